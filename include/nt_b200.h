@@ -141,6 +141,10 @@ int nt_host_unregister(void *ptr);
 int nt_zeros(int64_t n, int dtype, int device, nt_storage **out);
 int nt_ones(int64_t n, int dtype, int device, nt_storage **out);
 int nt_full(int64_t n, const nt_scalar *value, int dtype, int device, nt_storage **out);
+/* One Cuda element that holds `value`, for operands the host knows (a Python scalar beside a tensor, the seed of a
+ * backward pass; the reference copies a one-element tensor to the device for each).  No memory and no fill
+ * launch until something needs the address: the Float32 elementwise kernels take the value as an argument. */
+int nt_constant(const nt_scalar *value, int dtype, nt_storage **out);
 /* eye / arange are written by a kernel when device is Cuda (host loop + copy in the reference). */
 int nt_eye(int64_t n, int dtype, int device, nt_storage **out);
 int nt_arange(int64_t n, int64_t start, int64_t step, int dtype, int device, nt_storage **out);

@@ -502,6 +502,12 @@ def full(n: int, value, dtype: Dtype, device: Device) -> Storage:
     return _factory(_lib.nt_full, C.c_int64(n), C.byref(s), int(_dtype(dtype)), _device(device).value)
 
 
+def constant(value, dtype: Dtype) -> Storage:
+    """One Cuda element known to hold `value`: no fill launch until something needs its address."""
+    s = _scalar(value)
+    return _factory(_lib.nt_constant, C.byref(s), int(_dtype(dtype)))
+
+
 def eye(n: int, dtype: Dtype, device: Device) -> Storage:
     return _factory(_lib.nt_eye, C.c_int64(n), int(_dtype(dtype)), _device(device).value)
 

@@ -249,10 +249,21 @@ static void binary_checks(const nt_view *x1, const nt_view *x2, const char *fnam
   require_cuda(x1, fname);
 }
 
+// Both operands one-element constants: the host's own IEEE operation is the kernel's, and the result is a constant too
+// (the seed of a backward pass divided by a mean's count never becomes a launch).
+template <template <class> class F> static float fold(float a, float b) {
+  if constexpr (std::is_same_v<F<float>, AddF<float>>) return a + b;
+  else if constexpr (std::is_same_v<F<float>, SubF<float>>) return a - b;
+  else if constexpr (std::is_same_v<F<float>, MulF<float>>) return a * b;
+  else return a / b;
+}
+
 template <template <class> class F, bool ARITH_ONLY>
 static nt_storage *binary_same_dtype(const nt_view *x1, const nt_view *x2) {
   binary_checks(x1, x2, "_dispatch_binary");
   const int dt = x1->storage->dtype;
+  if (dt == NT_FLOAT32 && x1->storage->constant && x2->storage->constant && view_numel(*x1) == 1)
+    return storage_new_constant(fold<F>(x1->storage->value, x2->storage->value));
   StorageRef out(storage_new(view_numel(*x1), dt, NT_CUDA));
   nt_view ov = fresh_view(out.s, *x1);
   auto run = [&]<class T>() {
@@ -342,18 +353,18 @@ template <class F, int NIN> static nt_storage *produce_with_planes(F f, const nt
   if (!g_producer_planes.load() || nt_get_matmul_mode() != 1 || !dense_2d(a)) return nullptr;
   const int64_t R = a->shape[0], C = a->shape[1];
   if (C % 32 != 0 || R * C < (int64_t(1) << 20)) return nullptr;
-  const float *pa = static_cast<const float *>(a->storage->data) + a->offset, *pb = nullptr;
+  const float *pa = static_cast<const float *>(a->storage->ptr()) + a->offset, *pb = nullptr;
   if (!aligned16(pa)) return nullptr;
   if constexpr (NIN == 2) {
     if (!dense_2d(b) || b->shape[0] != R || b->shape[1] != C) return nullptr;
-    pb = static_cast<const float *>(b->storage->data) + b->offset;
+    pb = static_cast<const float *>(b->storage->ptr()) + b->offset;
     if (!aligned16(pb)) return nullptr;
   }
   StorageRef out(storage_new(R * C, NT_FLOAT32, NT_CUDA));
   float *hi = gemm_tc_adopt_planes(out.s, R, C);
   if (!hi) return nullptr;
   const int64_t n = R * C;
-  ew_contig_planes<F, NIN><<<unsigned(ceil_div(n >> 2, 256 * 4)), 256, 0, stream()>>>(f, static_cast<float *>(out->data), pa, pb, n,
+  ew_contig_planes<F, NIN><<<unsigned(ceil_div(n >> 2, 256 * 4)), 256, 0, stream()>>>(f, static_cast<float *>(out->ptr()), pa, pb, n,
                                                                                       hi, hi + n);
   check_launch("ew_contig_planes");
   return out.release();
@@ -385,13 +396,13 @@ template <class F> static void binary_backward_both(F f, const nt_view *g, const
       if (chk[i]->shape[d] != 1 && chk[i]->strides[d] != acc) return;
       acc *= chk[i]->shape[d];
     }
-    p[i] = static_cast<const float *>(chk[i]->storage->data) + chk[i]->offset;
+    p[i] = static_cast<const float *>(chk[i]->storage->ptr()) + chk[i]->offset;
     if (!aligned16(p[i])) return;
   }
   if (n < 4) return;
   StorageRef o1(storage_new(n, NT_FLOAT32, NT_CUDA)), o2(storage_new(n, NT_FLOAT32, NT_CUDA));
-  ew_contig_two<F><<<unsigned(ceil_div(n >> 2, 256 * 2)), 256, 0, stream()>>>(f, static_cast<float *>(o1->data),
-                                                                            static_cast<float *>(o2->data), p[0], p[1], p[2], n);
+  ew_contig_two<F><<<unsigned(ceil_div(n >> 2, 256 * 2)), 256, 0, stream()>>>(f, static_cast<float *>(o1->ptr()),
+                                                                            static_cast<float *>(o2->ptr()), p[0], p[1], p[2], n);
   check_launch("ew_contig_two");
   *out1 = o1.release();
   *out2 = o2.release();
@@ -450,15 +461,15 @@ int nt_equals(const nt_view *x1, const nt_view *x2, int *result) {
   // one int of device scratch from the arena; the compare kernel writes its first input back
   // into a throw-away buffer only to reuse the launcher (n is small wherever this is used).
   StorageRef flag(storage_new(1, NT_INT32, NT_CUDA));
-  NT_CUDA_CHECK(cudaMemsetAsync(flag->data, 0, sizeof(int), stream()));
+  NT_CUDA_CHECK(cudaMemsetAsync(flag->ptr(), 0, sizeof(int), stream()));
   StorageRef sink(storage_new(view_numel(*x1), x1->storage->dtype, NT_CUDA));
   nt_view sv = fresh_view(sink.s, *x1);
   dispatch_all(x1->storage->dtype, [&]<class T>() {
     const nt_view *views[3] = {&sv, x1, x2};
-    ew_launch<NeqFlagF<T>, 2>(NeqFlagF<T>{static_cast<int *>(flag->data)}, views);
+    ew_launch<NeqFlagF<T>, 2>(NeqFlagF<T>{static_cast<int *>(flag->ptr())}, views);
   });
   int host = 0;
-  NT_CUDA_CHECK(cudaMemcpyAsync(&host, flag->data, sizeof(int), cudaMemcpyDeviceToHost, stream()));
+  NT_CUDA_CHECK(cudaMemcpyAsync(&host, flag->ptr(), sizeof(int), cudaMemcpyDeviceToHost, stream()));
   NT_CUDA_CHECK(cudaStreamSynchronize(stream()));
   *result = (host == 0) ? 1 : 0;
   NT_API_END
@@ -682,8 +693,8 @@ int nt_sgd_update(const nt_view *param, const nt_view *grad, float lr, float gra
   if (g_producer_planes.load() && nt_get_matmul_mode() == 1 && dense_2d(param) && dense_2d(grad) && param->offset == 0 &&
       param->shape[0] * param->shape[1] == param->storage->n) {
     const int64_t R = param->shape[0], C = param->shape[1], n = R * C;
-    float *pp = static_cast<float *>(param->storage->data);
-    const float *pg = static_cast<const float *>(grad->storage->data) + grad->offset;
+    float *pp = static_cast<float *>(param->storage->ptr());
+    const float *pg = static_cast<const float *>(grad->storage->ptr()) + grad->offset;
     float *hi = (n >= 4 && aligned16(pp) && aligned16(pg)) ? gemm_tc_refresh_target(param->storage, R, C) : nullptr;
     if (hi) {
       ew_contig_planes<SgdF, 2><<<unsigned(ceil_div(n >> 2, 256 * 4)), 256, 0, stream()>>>(f, pp, pp, pg, n, hi, hi + n);

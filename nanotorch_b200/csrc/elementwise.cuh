@@ -555,17 +555,49 @@ bool ew_launch_tile_pipeline(F f, const IterSpace<NIN + 1> &it, float *out, cons
   return true;
 }
 
+// A functor with its first or second argument bound to a value the host knows: the op then runs as one of one
+// operand fewer, with the same arithmetic per element and without a scalar in memory (one launch and one broadcast
+// operand less: x * 2 on [4096, 4096] moves as a unary op).
+template <class F> struct BindFirst {
+  using in_t = typename F::in_t;
+  using out_t = typename F::out_t;
+  F f;
+  in_t v;
+  __device__ __forceinline__ out_t operator()(in_t b) const { return f(v, b); }
+};
+template <class F> struct BindSecond {
+  using in_t = typename F::in_t;
+  using out_t = typename F::out_t;
+  F f;
+  in_t v;
+  __device__ __forceinline__ out_t operator()(in_t a) const { return f(a, v); }
+};
+template <class F> struct is_bound : std::false_type {};
+template <class F> struct is_bound<BindFirst<F>> : std::true_type {};
+template <class F> struct is_bound<BindSecond<F>> : std::true_type {};
+
 // views[0] is the output view (for fresh outputs: contiguous, offset 0).
 template <class F, int NIN> void ew_launch(F f, const nt_view *const (&views)[NIN + 1]) {
   using TI = typename F::in_t;
   using TO = typename F::out_t;
+  if constexpr (NIN == 2 && std::is_same_v<TI, float> && std::is_same_v<TO, float>) {
+    const bool c1 = views[1]->storage->constant, c2 = views[2]->storage->constant;
+    if (c2 && !c1) {
+      const nt_view *rest[2] = {views[0], views[1]};
+      return ew_launch<BindSecond<F>, 1>(BindSecond<F>{f, views[2]->storage->value}, rest);
+    }
+    if (c1) {
+      const nt_view *rest[2] = {views[0], views[2]};
+      return ew_launch<BindFirst<F>, 1>(BindFirst<F>{f, views[1]->storage->value}, rest);
+    }
+  }
   IterSpace<NIN + 1> it = collapse<NIN + 1>(views);
   if (it.numel == 0) return;
   cudaStream_t st = stream();
 
-  TO *out = static_cast<TO *>(views[0]->storage->data) + it.offset[0];
+  TO *out = static_cast<TO *>(views[0]->storage->ptr()) + it.offset[0];
   const TI *in[EW_MAX_IN] = {nullptr, nullptr, nullptr};
-  for (int o = 0; o < NIN; ++o) in[o] = static_cast<const TI *>(views[o + 1]->storage->data) + it.offset[o + 1];
+  for (int o = 0; o < NIN; ++o) in[o] = static_cast<const TI *>(views[o + 1]->storage->ptr()) + it.offset[o + 1];
 
   constexpr bool VECTOR_TYPES = (sizeof(TI) == 4 && sizeof(TO) == 4);
 
@@ -608,7 +640,7 @@ template <class F, int NIN> void ew_launch(F f, const nt_view *const (&views)[NI
     }
   }
 
-  if constexpr (NIN == 1 && std::is_same<TI, float>::value && std::is_same<TO, float>::value) {
+  if constexpr (NIN == 1 && !is_bound<F>::value && std::is_same<TI, float>::value && std::is_same<TO, float>::value) {
     if (it.ndim == 2 && (it.shape[1] & 3) == 0 && (it.numel >> 2) < (int64_t(1) << 31) && it.strides[0][0] == it.shape[1] &&
         it.strides[0][1] == 1 && it.strides[1][0] == 0 && it.strides[1][1] == 1 && aligned16(out) && aligned16(in[0])) {
       uint32_t mul, shift;

@@ -923,7 +923,7 @@ static std::atomic<uint64_t> g_split_launches{0}, g_split_hits{0};
 
 static void run_split(const nt_storage *s, const PlaneEntry &e) {
   NatSplitArgs a{};
-  a.src = static_cast<const float *>(s->data) + e.offset;
+  a.src = static_cast<const float *>(s->ptr()) + e.offset;
   a.hi = e.planes;
   a.lo = e.planes + e.batch * e.R * e.Cp;
   a.R = e.R;

@@ -203,7 +203,7 @@ Plan make_plan(const char *fname, const int64_t *it_shape, int it_ndim, const in
     const int64_t dim = fancy_dims[q];
     if (dim < 0 || dim >= ix->ndim || fancy_of_dim[dim] != -1) fail_invalid(f + ": bad indexed dimension.");
     fancy_of_dim[dim] = q;
-    p.ind[q] = static_cast<const int64_t *>(iv.storage->data) + iv.offset;
+    p.ind[q] = static_cast<const int64_t *>(iv.storage->ptr()) + iv.offset;
     p.ind_extent[q] = ix->shape[dim];
     p.ix_fancy_stride[q] = ix->strides[dim];
   }
@@ -230,8 +230,8 @@ Plan make_plan(const char *fname, const int64_t *it_shape, int it_ndim, const in
   // zero-initialised counters; it must then have extent >= 1
   p.items = items;
   pl.itemsize = int(dtype_itemsize(ix->storage->dtype));
-  pl.lin_base = static_cast<const char *>(lin_storage->data) + lin_offset * pl.itemsize;
-  pl.ix_base = static_cast<const char *>(ix->storage->data) + ix->offset * pl.itemsize;
+  pl.lin_base = static_cast<const char *>(lin_storage->ptr()) + lin_offset * pl.itemsize;
+  pl.ix_base = static_cast<const char *>(ix->storage->ptr()) + ix->offset * pl.itemsize;
   {
     int64_t acc = 1;
     for (int d = it_ndim - 1; d >= 0; --d) {
@@ -295,7 +295,7 @@ void validate_indices(const nt_view *ix, const int64_t *fancy_dims, int n_fancy,
       vp.shape[d] = iv.shape[d];
       vp.strides[d] = iv.strides[d];
     }
-    vp.data = static_cast<const int64_t *>(iv.storage->data) + iv.offset;
+    vp.data = static_cast<const int64_t *>(iv.storage->ptr()) + iv.offset;
     vp.extent = ix->shape[fancy_dims[q]];
     if (vp.numel == 0) continue;
     index_validate<<<unsigned(ceil_div(vp.numel, 256)), 256, 0, stream()>>>(vp, err);

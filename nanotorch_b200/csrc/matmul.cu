@@ -384,9 +384,9 @@ static nt_storage *matmul_impl(const nt_view *x1, const nt_view *x2, const nt_vi
 
   if (dt == NT_FLOAT32) {
     GemmArgs g{};
-    g.A = static_cast<const float *>(x1->storage->data) + x1->offset;
-    g.B = static_cast<const float *>(x2->storage->data) + x2->offset;
-    g.C = static_cast<float *>(o->data);
+    g.A = static_cast<const float *>(x1->storage->ptr()) + x1->offset;
+    g.B = static_cast<const float *>(x2->storage->ptr()) + x2->offset;
+    g.C = static_cast<float *>(o->ptr());
     g.M = M; g.N = N; g.K = K;
     g.a_sm = a_sm; g.a_sk = a_sk; g.b_sk = b_sk; g.b_sn = b_sn;
     g.batch = bi;
@@ -411,7 +411,7 @@ static nt_storage *matmul_impl(const nt_view *x1, const nt_view *x2, const nt_vi
         a_sb = bi.a_strides[bi.ndim - 1];
         b_sb = bi.b_strides[bi.ndim - 1];
       }
-      const float *bp = bias ? static_cast<const float *>(bias->storage->data) + bias->offset : nullptr;
+      const float *bp = bias ? static_cast<const float *>(bias->storage->ptr()) + bias->offset : nullptr;
       if (single && mode == 1 && g_natural_planes.load())
         done = gemm_3xtf32_natural(x1->storage, x1->offset, x2->storage, x2->offset, g.C, nbatch, M, N, K, a_sb, a_sm,
                                    a_sk, b_sb, b_sk, b_sn, bp, bias ? bias->strides[0] : 0, &bias_done);
@@ -427,11 +427,11 @@ static nt_storage *matmul_impl(const nt_view *x1, const nt_view *x2, const nt_vi
   } else {
     dispatch_arith(dt, [&]<class T>() {
       if constexpr (!std::is_same_v<T, float>) {
-        const T *A = static_cast<const T *>(x1->storage->data) + x1->offset;
-        const T *B = static_cast<const T *>(x2->storage->data) + x2->offset;
+        const T *A = static_cast<const T *>(x1->storage->ptr()) + x1->offset;
+        const T *B = static_cast<const T *>(x2->storage->ptr()) + x2->offset;
         int64_t blocks = ceil_div(total, 256);
         if (blocks > 0x7fffffffLL) fail_runtime("matmul: output too large for one launch.");
-        matmul_naive<T><<<unsigned(blocks), 256, 0, stream()>>>(A, B, static_cast<T *>(o->data), M, N, K, a_sm, a_sk,
+        matmul_naive<T><<<unsigned(blocks), 256, 0, stream()>>>(A, B, static_cast<T *>(o->ptr()), M, N, K, a_sm, a_sk,
                                                                 b_sk, b_sn, bi, total);
         check_launch("matmul_naive");
       }

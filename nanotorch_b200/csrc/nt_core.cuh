@@ -144,7 +144,7 @@ void host_free(void *p, bool pinned, size_t nbytes);
 // The storage object behind the opaque handle.
 struct nt_storage {
   std::atomic<int64_t> refs{1};
-  void *data = nullptr;
+  void *block = nullptr; // read through ptr(): a constant has no memory until something needs it
   size_t rounded = 0; // arena block size (device) or byte size (host)
   int64_t n = 0;
   int dtype = NT_FLOAT32;
@@ -153,6 +153,19 @@ struct nt_storage {
   uint64_t version = 0;  // the reference's counter: bumped by the in-place ops only
   uint64_t mutation = 0; // bumped by EVERY entry point that writes into an existing storage (in-place ops,
                          // uploads, copy_view, scatter, all-reduce): what cached derived data is checked against
+  // One element whose value the host knows (a Python scalar beside a tensor, the seed of a backward pass).
+  // The Float32 kernels take the value as an argument instead of a pointer; memory is allocated and filled
+  // only when something asks for the address.  Writing to the storage ends it being a constant.
+  bool constant = false;
+  float value = 0.0f; // of a Float32 constant
+  nt_scalar scalar{};
+  nt_storage *prev = nullptr, *next = nullptr; // constants without memory, see constants_materialize_all
+
+  void *ptr() const {
+    if (constant && !block) materialize();
+    return block;
+  }
+  void materialize() const;
 };
 
 namespace ntb {
@@ -160,7 +173,15 @@ namespace ntb {
 nt_storage *storage_new(int64_t n, int dtype, int device);
 inline void storage_retain(nt_storage *s) { s->refs.fetch_add(1, std::memory_order_relaxed); }
 void storage_release(nt_storage *s);
-inline void storage_touch(nt_storage *s) { s->mutation += 1; }
+inline void storage_touch(nt_storage *s) {
+  s->constant = false;
+  s->mutation += 1;
+}
+nt_storage *storage_new_constant(const nt_scalar &value, int dtype);
+nt_storage *storage_new_constant(float value);
+// Gives every constant its memory: called before a graph capture starts, because a fill recorded inside the capture
+// would not have run yet for eager work, and would run again on every replay.
+void constants_materialize_all();
 // Cached operand planes of the tensor-core GEMM (gemm_tc.cu) die with the storage they were split from.
 void gemm_tc_forget(nt_storage *s);
 // Re-split, on the current stream(), every cached plane set of `s` (called right after a parameter

@@ -507,7 +507,7 @@ static Plan make_plan(const nt_view *x, const int64_t *axes, int32_t n_axes) {
 }
 
 template <class Op> static bool try_fast_f32(const nt_view *x, const Plan &pl, float *out, float divisor = 0.0f) {
-  const float *in = static_cast<const float *>(x->storage->data) + x->offset;
+  const float *in = static_cast<const float *>(x->storage->ptr()) + x->offset;
   cudaStream_t st = stream();
   const int sms = sm_count();
   const int64_t target_ctas = int64_t(sms) * 8;
@@ -609,7 +609,7 @@ template <class Op> static bool try_fast_f32(const nt_view *x, const Plan &pl, f
 }
 
 template <class T, class O, class Op> static void launch_generic(const nt_view *x, const Plan &pl, void *out) {
-  const T *in = static_cast<const T *>(x->storage->data) + x->offset;
+  const T *in = static_cast<const T *>(x->storage->ptr()) + x->offset;
   cudaStream_t st = stream();
   if (pl.n_drop > 256) {
     if (pl.n_keep > 0x7fffffffLL) fail_runtime("reduction: too many kept elements.");
@@ -637,11 +637,11 @@ static nt_storage *reduce_impl(const nt_view *x, const int64_t *axes, int32_t n_
 
   if constexpr (!std::is_same_v<FastOp, void>) {
     if (in_dtype == NT_FLOAT32 && out_dtype == NT_FLOAT32 && pl.n_drop > 0) {
-      if (try_fast_f32<FastOp>(x, pl, static_cast<float *>(out->data))) return out.release();
+      if (try_fast_f32<FastOp>(x, pl, static_cast<float *>(out->ptr()))) return out.release();
     }
   }
   dispatch_all(in_dtype, [&]<class T>() {
-    dispatch_arith(out_dtype, [&]<class O>() { launch_generic<T, O, GOp>(x, pl, out->data); });
+    dispatch_arith(out_dtype, [&]<class O>() { launch_generic<T, O, GOp>(x, pl, out->ptr()); });
   });
   return out.release();
 }
@@ -995,9 +995,9 @@ static bool extremum_backward_fused(const nt_view *g, const nt_view *x, const nt
     sc.m_keep.strides[k] = m->strides[d];
     sc.x_keep.ndim = sc.g_keep.ndim = sc.m_keep.ndim = k + 1;
   }
-  const float *xp = static_cast<const float *>(x->storage->data) + x->offset;
-  const float *gp = static_cast<const float *>(g->storage->data) + g->offset;
-  const float *mp = static_cast<const float *>(m->storage->data) + m->offset;
+  const float *xp = static_cast<const float *>(x->storage->ptr()) + x->offset;
+  const float *gp = static_cast<const float *>(g->storage->ptr()) + g->offset;
+  const float *mp = static_cast<const float *>(m->storage->ptr()) + m->offset;
   cudaStream_t st = stream();
   const bool rows = trailing && pl.drop.ndim == 1 && pl.drop.strides[0] == 1;
   const bool cols = !rows && leading && pl.drop.ndim == 1 && pl.keep.ndim == 1 && pl.keep.strides[0] == 1;
@@ -1167,7 +1167,7 @@ int nt_mean_f32(const nt_view *x, const int64_t *axes, int32_t n_axes, float cou
   Plan pl = make_plan(x, axes, n_axes);
   if (pl.n_keep == 0 || pl.n_drop == 0) return NT_OK;
   StorageRef o(storage_new(pl.n_keep, NT_FLOAT32, NT_CUDA));
-  if (try_fast_f32<RSum>(x, pl, static_cast<float *>(o->data), count)) *out = o.release();
+  if (try_fast_f32<RSum>(x, pl, static_cast<float *>(o->ptr()), count)) *out = o.release();
   NT_API_END
 }
 int nt_max(const nt_view *x, const int64_t *axes, int32_t n_axes, nt_storage **out) {
@@ -1209,7 +1209,7 @@ int nt_extremum_backward(const nt_view *g_expanded, const nt_view *x, const nt_v
   const int64_t n = view_numel(*x);
   if (n > 0) {
     StorageRef fused(storage_new(n, NT_FLOAT32, NT_CUDA));
-    if (extremum_backward_fused(g_expanded, x, m_expanded, axes, n_axes, static_cast<float *>(fused->data))) {
+    if (extremum_backward_fused(g_expanded, x, m_expanded, axes, n_axes, static_cast<float *>(fused->ptr()))) {
       *out = fused.release();
       return NT_OK;
     }

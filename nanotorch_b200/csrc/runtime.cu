@@ -364,9 +364,9 @@ nt_storage *storage_new(int64_t n, int dtype, int device) {
   s->device = device;
   try {
     if (device == NT_CUDA) {
-      s->data = device_alloc(nbytes, &s->rounded);
+      s->block = device_alloc(nbytes, &s->rounded);
     } else {
-      s->data = host_alloc(nbytes, &s->pinned);
+      s->block = host_alloc(nbytes, &s->pinned);
       s->rounded = nbytes;
     }
   } catch (...) {
@@ -375,14 +375,48 @@ nt_storage *storage_new(int64_t n, int dtype, int device) {
   }
   return s;
 }
+// Constants that have no memory yet, as a list through the storages themselves.
+static std::mutex g_constants_mu;
+static nt_storage *g_constants = nullptr;
+static void constants_unlink(nt_storage *s) {
+  std::lock_guard<std::mutex> lk(g_constants_mu);
+  if (s->prev) s->prev->next = s->next;
+  if (s->next) s->next->prev = s->prev;
+  if (g_constants == s) g_constants = s->next;
+  s->prev = s->next = nullptr;
+}
+template <class T> static T scalar_as(const nt_scalar *v);
+nt_storage *storage_new_constant(const nt_scalar &value, int dtype) {
+  dtype_itemsize(dtype);
+  stream(); // the same error as an allocation where there is no device
+  const float f32 = dtype == NT_FLOAT32 ? scalar_as<float>(&value) : 0.0f;
+  nt_storage *s = new nt_storage();
+  s->n = 1;
+  s->dtype = dtype;
+  s->device = NT_CUDA;
+  s->constant = true;
+  s->scalar = value;
+  s->value = f32;
+  std::lock_guard<std::mutex> lk(g_constants_mu);
+  s->next = g_constants;
+  if (g_constants) g_constants->prev = s;
+  g_constants = s;
+  return s;
+}
+nt_storage *storage_new_constant(float value) { return storage_new_constant(nt_scalar{2, 0, value}, NT_FLOAT32); }
 void storage_release(nt_storage *s) {
   if (!s) return;
   if (s->refs.fetch_sub(1, std::memory_order_acq_rel) == 1) {
+    if (s->constant && !s->block) {
+      constants_unlink(s);
+      delete s;
+      return;
+    }
     if (s->device == NT_CUDA) gemm_tc_forget(s);
     if (s->device == NT_CUDA)
-      device_free(s->data, s->rounded);
+      device_free(s->block, s->rounded);
     else
-      host_free(s->data, s->pinned, s->rounded);
+      host_free(s->block, s->pinned, s->rounded);
     delete s;
   }
 }
@@ -523,7 +557,7 @@ static int grid_for(int64_t n, int block) {
 
 template <class T> static void fill_device(nt_storage *s, T value) {
   if (s->n == 0) return;
-  fill_kernel<T><<<grid_for(s->n, 256), 256, 0, stream()>>>(static_cast<T *>(s->data), s->n, value);
+  fill_kernel<T><<<grid_for(s->n, 256), 256, 0, stream()>>>(static_cast<T *>(s->ptr()), s->n, value);
   check_launch("fill");
 }
 
@@ -536,6 +570,10 @@ template <class T> static T scalar_as(const nt_scalar *v) {
   }
 }
 
+static void fill_constant(nt_storage *s) {
+  s->block = device_alloc(size_t(dtype_itemsize(s->dtype)), &s->rounded);
+  dispatch_all(s->dtype, [&]<class T>() { fill_device<T>(s, scalar_as<T>(&s->scalar)); });
+}
 static nt_storage *full_impl(int64_t n, const nt_scalar *value, int dtype, int device) {
   StorageRef out(storage_new(n, dtype, device));
   dispatch_all(dtype, [&]<class T>() {
@@ -543,7 +581,7 @@ static nt_storage *full_impl(int64_t n, const nt_scalar *value, int dtype, int d
     if (device == NT_CUDA) {
       fill_device<T>(out.s, v);
     } else {
-      T *p = static_cast<T *>(out->data);
+      T *p = static_cast<T *>(out->ptr());
       for (int64_t i = 0; i < n; ++i) p[i] = v;
     }
   });
@@ -560,7 +598,7 @@ static nt_storage *to_device_impl(nt_storage *s, int device) {
   if (nbytes) {
     cudaStream_t st = stream();
     cudaMemcpyKind kind = (s->device == NT_CPU) ? cudaMemcpyHostToDevice : cudaMemcpyDeviceToHost;
-    NT_CUDA_CHECK(cudaMemcpyAsync(out->data, s->data, nbytes, kind, st));
+    NT_CUDA_CHECK(cudaMemcpyAsync(out->ptr(), s->ptr(), nbytes, kind, st));
     // The host side of either direction may be reused or read right after the call returns.
     NT_CUDA_CHECK(cudaStreamSynchronize(st));
     if (kind == cudaMemcpyDeviceToHost && !is_capturing()) check_device_errors(); // values are about to be read
@@ -568,7 +606,25 @@ static nt_storage *to_device_impl(nt_storage *s, int device) {
   return out.release();
 }
 
+void constants_materialize_all() {
+  for (;;) {
+    nt_storage *s;
+    {
+      std::lock_guard<std::mutex> lk(g_constants_mu);
+      s = g_constants;
+    }
+    if (!s) return;
+    s->materialize();
+  }
+}
+
 } // namespace ntb
+
+void nt_storage::materialize() const {
+  nt_storage *s = const_cast<nt_storage *>(this);
+  ntb::constants_unlink(s);
+  ntb::fill_constant(s);
+}
 
 using namespace ntb;
 
@@ -732,6 +788,7 @@ int nt_graph_begin_capture(int *graph_id) {
   // would find it uninitialised
   reduce_prepare();
   gemm_tc_prepare();
+  constants_materialize_all();
   Runtime &r = rt();
   std::lock_guard<std::mutex> lk(r.mu);
   if (r.capturing) fail_runtime("nt_graph_begin_capture: a capture is already in progress.");
@@ -793,7 +850,7 @@ int nt_storage_upload_async(nt_storage *dst, const void *host_src, int64_t nbyte
   Runtime &r = rt();
   NT_CUDA_CHECK(cudaEventRecord(r.copy_gate, st));
   NT_CUDA_CHECK(cudaStreamWaitEvent(r.copy, r.copy_gate, 0));
-  if (nbytes) NT_CUDA_CHECK(cudaMemcpyAsync(dst->data, host_src, size_t(nbytes), cudaMemcpyHostToDevice, r.copy));
+  if (nbytes) NT_CUDA_CHECK(cudaMemcpyAsync(dst->ptr(), host_src, size_t(nbytes), cudaMemcpyHostToDevice, r.copy));
   storage_touch(dst);
   NT_API_END
 }
@@ -845,7 +902,15 @@ int64_t nt_storage_itemsize(const nt_storage *s) {
 int nt_storage_dtype(const nt_storage *s) { return s->dtype; }
 int nt_storage_device(const nt_storage *s) { return s->device; }
 uint64_t nt_storage_version(const nt_storage *s) { return s->version; }
-void *nt_storage_data(nt_storage *s) { return s->data; }
+void *nt_storage_data(nt_storage *s) {
+  try {
+    void *p = s->ptr();
+    s->constant = false; // the caller may write through the pointer
+    return p;
+  } catch (...) {
+    return nullptr;
+  }
+}
 
 int nt_storage_clone(const nt_storage *s, nt_storage **out) {
   NT_API_BEGIN
@@ -853,9 +918,9 @@ int nt_storage_clone(const nt_storage *s, nt_storage **out) {
   size_t nbytes = size_t(s->n) * dtype_itemsize(s->dtype);
   if (nbytes) {
     if (s->device == NT_CPU)
-      std::memcpy(o->data, s->data, nbytes);
+      std::memcpy(o->ptr(), s->ptr(), nbytes);
     else
-      NT_CUDA_CHECK(cudaMemcpyAsync(o->data, s->data, nbytes, cudaMemcpyDeviceToDevice, stream()));
+      NT_CUDA_CHECK(cudaMemcpyAsync(o->ptr(), s->ptr(), nbytes, cudaMemcpyDeviceToDevice, stream()));
   }
   *out = o.release();
   NT_API_END
@@ -880,8 +945,8 @@ int nt_storage_cast(nt_storage *s, int dtype, nt_storage **out) {
   if (s->n) {
     dispatch_all(s->dtype, [&]<class S>() {
       dispatch_all(dtype, [&]<class D>() {
-        const S *in = static_cast<const S *>(s->data);
-        D *dst = static_cast<D *>(o->data);
+        const S *in = static_cast<const S *>(s->ptr());
+        D *dst = static_cast<D *>(o->ptr());
         if (s->device == NT_CUDA) {
           cast_kernel<S, D><<<grid_for(s->n, 256), 256, 0, stream()>>>(in, dst, s->n);
           check_launch("cast");
@@ -908,10 +973,10 @@ int nt_storage_upload(nt_storage *dst, const void *host_src, int64_t nbytes) {
     fail_runtime("nt_storage_upload: byte count exceeds the storage.");
   if (nbytes == 0) return NT_OK;
   if (dst->device == NT_CPU) {
-    std::memcpy(dst->data, host_src, size_t(nbytes));
+    std::memcpy(dst->ptr(), host_src, size_t(nbytes));
   } else {
     cudaStream_t st = stream();
-    NT_CUDA_CHECK(cudaMemcpyAsync(dst->data, host_src, size_t(nbytes), cudaMemcpyHostToDevice, st));
+    NT_CUDA_CHECK(cudaMemcpyAsync(dst->ptr(), host_src, size_t(nbytes), cudaMemcpyHostToDevice, st));
     NT_CUDA_CHECK(cudaStreamSynchronize(st));
   }
   storage_touch(dst);
@@ -924,10 +989,10 @@ int nt_storage_download(const nt_storage *src, void *host_dst, int64_t nbytes) {
     fail_runtime("nt_storage_download: byte count exceeds the storage.");
   if (nbytes == 0) return NT_OK;
   if (src->device == NT_CPU) {
-    std::memcpy(host_dst, src->data, size_t(nbytes));
+    std::memcpy(host_dst, src->ptr(), size_t(nbytes));
   } else {
     cudaStream_t st = stream();
-    NT_CUDA_CHECK(cudaMemcpyAsync(host_dst, src->data, size_t(nbytes), cudaMemcpyDeviceToHost, st));
+    NT_CUDA_CHECK(cudaMemcpyAsync(host_dst, src->ptr(), size_t(nbytes), cudaMemcpyDeviceToHost, st));
     NT_CUDA_CHECK(cudaStreamSynchronize(st));
     check_device_errors(); // the caller is about to read these values
   }
@@ -953,12 +1018,18 @@ int nt_full(int64_t n, const nt_scalar *value, int dtype, int device, nt_storage
   NT_API_END
 }
 
+int nt_constant(const nt_scalar *value, int dtype, nt_storage **out) {
+  NT_API_BEGIN
+  *out = storage_new_constant(*value, dtype);
+  NT_API_END
+}
+
 int nt_eye(int64_t n, int dtype, int device, nt_storage **out) {
   NT_API_BEGIN
   if (n < 0) fail_invalid("eye: negative size.");
   StorageRef o(storage_new(n * n, dtype, device));
   dispatch_all(dtype, [&]<class T>() {
-    T *p = static_cast<T *>(o->data);
+    T *p = static_cast<T *>(o->ptr());
     if (device == NT_CUDA) {
       if (n > 0) {
         eye_kernel<T><<<grid_for(n * n, 256), 256, 0, stream()>>>(p, n);
@@ -978,7 +1049,7 @@ int nt_arange(int64_t n, int64_t start, int64_t step, int dtype, int device, nt_
   if (n < 0) fail_invalid("arange: negative size.");
   StorageRef o(storage_new(n, dtype, device));
   dispatch_all(dtype, [&]<class T>() {
-    T *p = static_cast<T *>(o->data);
+    T *p = static_cast<T *>(o->ptr());
     if (device == NT_CUDA) {
       if (n > 0) {
         arange_kernel<T><<<grid_for(n, 256), 256, 0, stream()>>>(p, n, start, step);
@@ -1020,7 +1091,7 @@ int nt_uniform(int64_t n, int dtype, int device, nt_storage **out) {
       constexpr int per = std::is_same_v<T, float> ? 4 : 2;
       const int64_t blocks = ceil_div(n, per);
       if (n > 0) {
-        philox_uniform_kernel<T><<<grid_for(blocks, 256), 256, 0, stream()>>>(static_cast<T *>(o->data), n,
+        philox_uniform_kernel<T><<<grid_for(blocks, 256), 256, 0, stream()>>>(static_cast<T *>(o->ptr()), n,
                                                                               rt().philox_seed, rt().philox_offset);
         check_launch("philox_uniform");
       }
@@ -1031,7 +1102,7 @@ int nt_uniform(int64_t n, int dtype, int device, nt_storage **out) {
   }
   StorageRef host(storage_new(n, dtype, NT_CPU));
   dispatch_float(dtype, [&]<class T>() {
-    T *p = static_cast<T *>(host->data);
+    T *p = static_cast<T *>(host->ptr());
     std::uniform_real_distribution<T> dist(0.0, 1.0);
     auto &rng = rt().rng;
     for (int64_t i = 0; i < n; ++i) p[i] = static_cast<T>(dist(rng));

@@ -164,9 +164,9 @@ class Tensor:
 
     @classmethod
     def _scalar(cls, value, dtype: Dtype, device: Device) -> "Tensor":
-        """0-d tensor written by a device fill: no host->device copy, no synchronisation."""
-        t = cls._new_contiguous(_C.full(1, value, dtype, device), ())
-        return t
+        """0-d tensor: on Cuda a constant the kernels take as an argument, no copy and no launch."""
+        storage = _C.constant(value, dtype) if device == Device.Cuda else _C.full(1, value, dtype, device)
+        return cls._new_contiguous(storage, ())
 
     @classmethod
     def from_numpy(cls, array, device: Device | str = Device.Cuda, requires_grad: bool = False) -> "Tensor":
@@ -462,7 +462,7 @@ class Tensor:
                 "Cannot call .backward() on a tensor that does not require grad and does not have a grad_fn.")
         if self.numel != 1:
             raise RuntimeError(f"Cannot call .backward() on a non-scalar tensor of shape {self.shape}")
-        seed = Tensor._new_contiguous(_C.full(1, 1.0, self.dtype, self.device), ())
+        seed = Tensor._scalar(1.0, self.dtype, self.device)
         if self.shape != ():
             seed = seed.reshape(*self.shape)
         self._grad = seed
