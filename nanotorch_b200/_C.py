@@ -4,7 +4,8 @@ Same names, argument meaning and exception classes as the reference's pybind11 m
 (src/cpp/_C.cpp:12-24, typed in src/nanotorch/_C.pyi:1-136): ``Dtype``, ``Device``, ``Storage``,
 ``TensorView`` and the free functions that take views and return a fresh ``Storage``.  The extra
 entry points of include/nt_b200.h (fused backward kernels, SGD update, data-parallel exchange,
-matmul mode) are exposed under the same module.
+matmul mode) are exposed under the same module.  Storages, views and the ops themselves are bound natively
+(csrc/engine); what is called once in a while goes through ctypes.
 
 There is no fallback: if the shared library is missing the import fails, and every compute call
 on a machine without a GPU raises RuntimeError.
@@ -24,6 +25,8 @@ if not _LIB_PATH.exists():
         "(there is no CPU or PyTorch fallback for the op kernels)."
     )
 _lib = C.CDLL(str(_LIB_PATH))
+
+from . import _engine  # noqa: E402  (links against the library loaded above)
 
 NT_MAX_DIMS = 8
 
@@ -124,37 +127,10 @@ def _scalar(v) -> _Scalar:
     raise TypeError("Unknown scalar type.")
 
 
-class Storage:
+class Storage(_engine.StorageBase):
     """Pointer to a 1D contiguous, typed memory segment (src/cpp/storage.h:34-66)."""
 
-    __slots__ = ("_h", "_dtype", "_device", "_size", "__weakref__")
-
-    def __init__(self, *_a, **_k):
-        raise TypeError("Storage: use Storage.allocate or Storage.from_iterable")
-
-    @classmethod
-    def _wrap(cls, handle: int) -> "Storage":
-        self = object.__new__(cls)
-        self._h = handle
-        self._dtype = Dtype(_lib.nt_storage_dtype(handle))
-        self._device = Device(_lib.nt_storage_device(handle))
-        self._size = _lib.nt_storage_size(handle)
-        return self
-
-    def __del__(self):
-        h = getattr(self, "_h", None)
-        if h and _lib is not None:
-            try:
-                _lib.nt_storage_release(h)
-            except Exception:  # interpreter shutdown
-                pass
-            self._h = None
-
-    @staticmethod
-    def allocate(n: int, dtype: Dtype, device: Device) -> "Storage":
-        out = C.c_void_p()
-        _check(_lib.nt_storage_allocate(C.c_int64(n), int(_dtype(dtype)), _device(device).value, C.byref(out)))
-        return Storage._wrap(out.value)
+    __slots__ = ("__weakref__",)
 
     @staticmethod
     def from_iterable(values: Sequence, dtype: Dtype, device: Device) -> "Storage":
@@ -164,7 +140,7 @@ class Storage:
         host = Storage.allocate(n, dtype, Device.Cpu)
         if n:
             ctype = _CTYPE[dtype]
-            arr = (ctype * n).from_address(_lib.nt_storage_data(host._h))
+            arr = (ctype * n).from_address(host.data_ptr)
             if dtype in (Dtype.Int32, Dtype.Int64):
                 for i, v in enumerate(values):
                     if isinstance(v, float):
@@ -178,118 +154,47 @@ class Storage:
                     arr[i] = v
         return host if device == Device.Cpu else host.to(device)
 
-    @property
-    def size(self) -> int:
-        return self._size
-
-    @property
-    def itemsize(self) -> int:
-        return _ITEMSIZE[self._dtype]
-
-    @property
-    def dtype(self) -> Dtype:
-        return self._dtype
-
-    @property
-    def device(self) -> Device:
-        return self._device
-
-    @property
-    def version(self) -> int:
-        return _lib.nt_storage_version(self._h)
-
-    @property
-    def data_ptr(self) -> int:
-        return _lib.nt_storage_data(self._h) or 0
-
-    def clone(self) -> "Storage":
-        out = C.c_void_p()
-        _check(_lib.nt_storage_clone(C.c_void_p(self._h), C.byref(out)))
-        return Storage._wrap(out.value)
-
-    def to(self, device: Device) -> "Storage":
-        device = _device(device)
-        if device == self._device:
-            return self
-        out = C.c_void_p()
-        _check(_lib.nt_storage_to(C.c_void_p(self._h), device.value, C.byref(out)))
-        return Storage._wrap(out.value)
-
-    def cast(self, dtype: Dtype) -> "Storage":
-        dtype = _dtype(dtype)
-        if dtype == self._dtype:
-            return self
-        out = C.c_void_p()
-        _check(_lib.nt_storage_cast(C.c_void_p(self._h), int(dtype), C.byref(out)))
-        return Storage._wrap(out.value)
-
     # Buffer protocol, 1-D, writable (src/cpp/storage.cpp:67-70, 82-95).  As in the reference the
     # exported pointer of a Cuda storage is a device pointer: its length is meaningful, its
     # contents are not readable from the host.
     def __buffer__(self, flags: int) -> memoryview:
-        n = self._size
-        ctype = _CTYPE[self._dtype]
-        fmt = _FORMAT[self._dtype]
+        n = self.size
+        ctype = _CTYPE[self.dtype]
+        fmt = _FORMAT[self.dtype]
         if n == 0:
             return memoryview((ctype * 0)()).cast("B").cast(fmt)
-        arr = (ctype * n).from_address(_lib.nt_storage_data(self._h))
+        arr = (ctype * n).from_address(self.data_ptr)
         arr._owner = self  # keep the storage alive while the view is
         return memoryview(arr).cast("B").cast(fmt)
 
-    # fast paths used by the tensor layer and the tests (numpy arrays, bytes)
-    def upload(self, host_ptr: int, nbytes: int) -> None:
-        _check(_lib.nt_storage_upload(C.c_void_p(self._h), C.c_void_p(host_ptr), C.c_int64(nbytes)))
 
-    def download(self, host_ptr: int, nbytes: int) -> None:
-        _check(_lib.nt_storage_download(C.c_void_p(self._h), C.c_void_p(host_ptr), C.c_int64(nbytes)))
+_engine.register_storage(Storage, tuple(Dtype), tuple(Device))
+TensorView = _engine.TensorView
 
 
-class TensorView:
-    """Strided tensor view handed to the kernels (src/cpp/tensor_view.cuh:10-15, 93-102)."""
-
-    __slots__ = ("_storage", "_shape", "_strides", "_offset", "_c")
-
-    def __init__(self, storage: Storage = None, shape=(), strides=(), offset: int = 0) -> None:
-        self._storage = storage
-        self._shape = tuple(shape)
-        self._strides = tuple(strides)
-        self._offset = int(offset)
-        self._c = None
-
-    def _struct(self) -> _View:
-        c = self._c
-        if c is None:
-            nd = len(self._shape)
-            if len(self._strides) != nd:
-                raise RuntimeError("TensorView: shape and strides differ in length.")
-            if nd > NT_MAX_DIMS:
-                raise RuntimeError("TensorView: more than 8 dimensions are not supported on device.")
-            if not isinstance(self._storage, Storage):
-                raise TypeError("TensorView: storage must be a Storage.")
-            c = _View()
-            c.storage = self._storage._h
-            c.ndim = nd
-            for i in range(nd):
-                c.shape[i] = self._shape[i]
-                c.strides[i] = self._strides[i]
-            c.offset = self._offset
-            self._c = c
-        return c
-
-    def _set(self, name, value):
-        object.__setattr__(self, name, value)
-        object.__setattr__(self, "_c", None)
-
-    storage = property(lambda s: s._storage, lambda s, v: s._set("_storage", v))
-    shape = property(lambda s: list(s._shape), lambda s, v: s._set("_shape", tuple(v)))
-    strides = property(lambda s: list(s._strides), lambda s, v: s._set("_strides", tuple(v)))
-    offset = property(lambda s: s._offset, lambda s, v: s._set("_offset", int(v)))
+def _view_struct(v: TensorView) -> _View:
+    if not isinstance(v, TensorView):
+        raise TypeError(f"expected a TensorView, got {type(v).__name__}")
+    shape, strides = v.shape, v.strides
+    nd = len(shape)
+    if len(strides) != nd:
+        raise RuntimeError("TensorView: shape and strides differ in length.")
+    if nd > NT_MAX_DIMS:
+        raise RuntimeError("TensorView: more than 8 dimensions are not supported on device.")
+    if not isinstance(v.storage, Storage):
+        raise TypeError("TensorView: storage must be a Storage.")
+    c = _View()
+    c.storage = v.storage._h
+    c.ndim = nd
+    for i in range(nd):
+        c.shape[i] = shape[i]
+        c.strides[i] = strides[i]
+    c.offset = v.offset
+    return c
 
 
 def _vref(v: TensorView):
-    if not isinstance(v, TensorView):
-        raise TypeError(f"expected a TensorView, got {type(v).__name__}")
-    return C.byref(v._struct())
+    return C.byref(_view_struct(v))
 
 
 def _ret_storage(fn, *args) -> Storage:
@@ -298,52 +203,22 @@ def _ret_storage(fn, *args) -> Storage:
     return Storage._wrap(out.value)
 
 
-def _binary(name):
-    fn = getattr(_lib, "nt_" + name)
-
-    def op(x1: TensorView, x2: TensorView) -> Storage:
-        return _ret_storage(fn, _vref(x1), _vref(x2))
-
-    op.__name__ = name
-    return op
-
-
-def _unary(name):
-    fn = getattr(_lib, "nt_" + name)
-
-    def op(x: TensorView) -> Storage:
-        return _ret_storage(fn, _vref(x))
-
-    op.__name__ = name
-    return op
-
-
-def _inplace(name):
-    fn = getattr(_lib, "nt_" + name)
-
-    def op(x1: TensorView, x2: TensorView) -> None:
-        _check(fn(_vref(x1), _vref(x2)))
-
-    op.__name__ = name
-    return op
-
-
 # ---- pointwise (src/cpp/ops/binary_ops.cu:178-196, unary_ops.cu:109-128)
-add = _binary("add")
-subtract = _binary("subtract")
-multiply = _binary("multiply")
-divide = _binary("divide")
-pw_equal = _binary("pw_equal")
-pw_greater = _binary("pw_greater")
-pw_greater_eq = _binary("pw_greater_eq")
-matmul = _binary("matmul")
-exp = _unary("exp")
-log = _unary("log")
-sqrt = _unary("sqrt")
-tanh = _unary("tanh")
-sigmoid = _unary("sigmoid")
-neg = _unary("neg")
-relu = _unary("relu")
+add = _engine.add
+subtract = _engine.subtract
+multiply = _engine.multiply
+divide = _engine.divide
+pw_equal = _engine.pw_equal
+pw_greater = _engine.pw_greater
+pw_greater_eq = _engine.pw_greater_eq
+matmul = _engine.matmul
+exp = _engine.exp
+log = _engine.log
+sqrt = _engine.sqrt
+tanh = _engine.tanh
+sigmoid = _engine.sigmoid
+neg = _engine.neg
+relu = _engine.relu
 
 
 def equals(x1: TensorView, x2: TensorView) -> bool:
@@ -363,9 +238,7 @@ def _axes(axis: Sequence[int]):
     return (C.c_int64 * len(ax))(*ax), len(ax)
 
 
-def sum(x: TensorView, axis: Sequence[int], dtype: Dtype) -> Storage:  # noqa: A001
-    arr, n = _axes(axis)
-    return _ret_storage(_lib.nt_sum, _vref(x), arr, C.c_int32(n), int(_dtype(dtype)))
+sum = _engine.sum  # noqa: A001  (view, axes, dtype)
 
 
 def mean_f32(x: TensorView, axis: Sequence[int], count: int) -> "Storage | None":
@@ -377,28 +250,12 @@ def mean_f32(x: TensorView, axis: Sequence[int], count: int) -> "Storage | None"
     return Storage._wrap(out.value) if out.value else None
 
 
-def _reduction(name):
-    fn = getattr(_lib, "nt_" + name)
-
-    def op(x: TensorView, axis: Sequence[int]) -> Storage:
-        arr, n = _axes(axis)
-        return _ret_storage(fn, _vref(x), arr, C.c_int32(n))
-
-    op.__name__ = name
-    return op
-
-
-max = _reduction("max")  # noqa: A001
-min = _reduction("min")  # noqa: A001
-argmax = _reduction("argmax")
-argmin = _reduction("argmin")
-
-def matmul_pair(a1: TensorView, b1: TensorView, a2: TensorView, b2: TensorView) -> tuple[Storage, Storage]:
-    """(a1 @ b1, a2 @ b2): two independent products, the second overlapping the first's last wave of tiles
-    (addition to the reference's surface; the bits of two `matmul` calls)."""
-    o1, o2 = C.c_void_p(), C.c_void_p()
-    _check(_lib.nt_matmul_pair(_vref(a1), _vref(b1), _vref(a2), _vref(b2), C.byref(o1), C.byref(o2)))
-    return Storage._wrap(o1.value), Storage._wrap(o2.value)
+max = _engine.max  # noqa: A001  (view, axes)
+min = _engine.min  # noqa: A001
+argmax = _engine.argmax
+argmin = _engine.argmin
+matmul_pair = _engine.matmul_pair
+linear = _engine.linear
 
 
 def set_matmul_pair_overlap(on: bool = True) -> None:
@@ -406,17 +263,12 @@ def set_matmul_pair_overlap(on: bool = True) -> None:
     _check(_lib.nt_set_matmul_pair_overlap(int(bool(on))))
 
 
-def linear(x: TensorView, w: TensorView, bias: TensorView) -> Storage:
-    """x @ w + bias with the bias add fused into the GEMM epilogue (addition to the reference's surface)."""
-    return _ret_storage(_lib.nt_linear, _vref(x), _vref(w), _vref(bias))
-
-
 # ---- in-place (src/cpp/ops/inplace_ops.cu:81-92)
-add_inplace = _inplace("add_inplace")
-sub_inplace = _inplace("sub_inplace")
-mul_inplace = _inplace("mul_inplace")
-div_inplace = _inplace("div_inplace")
-copy_inplace = _inplace("copy_inplace")
+add_inplace = _engine.add_inplace
+sub_inplace = _engine.sub_inplace
+mul_inplace = _engine.mul_inplace
+div_inplace = _engine.div_inplace
+copy_inplace = _engine.copy_inplace
 
 
 # ---- core ops (src/cpp/storage.cpp:96-102, ops/copy_ops.cu:219-233)
@@ -433,8 +285,7 @@ def copy_view(*, src: TensorView, out: TensorView) -> Storage:
     return out.storage
 
 
-def clone_contiguous_view_from(src: TensorView) -> Storage:
-    return _ret_storage(_lib.nt_clone_contiguous_view_from, _vref(src))
+clone_contiguous_view_from = _engine.clone_contiguous_view_from
 
 
 # Index-array gather/scatter.  Keyword names are the reference's (src/cpp/ops/copy_ops.cu:219-233);
@@ -454,7 +305,7 @@ def _index_plan(fancy_dims_in_src, fancy_dims_data, out_axis_is_fancy, out_axis_
     dims = (C.c_int64 * (nf or 1))(*fancy_dims_in_src)
     views = (_View * (nf or 1))()
     for i, v in enumerate(fancy_dims_data):
-        views[i] = v._struct()
+        views[i] = _view_struct(v)
     is_fancy = (C.c_uint8 * (na or 1))(*[1 if f else 0 for f in out_axis_is_fancy])
     target = (C.c_int64 * (na or 1))(*out_axis_target)
     return dims, nf, views, is_fancy, target
@@ -669,20 +520,19 @@ def get_matmul_mode() -> int:
     return _lib.nt_get_matmul_mode()
 
 
-relu_backward = _binary("relu_backward")
-tanh_backward = _binary("tanh_backward")
-sigmoid_backward = _binary("sigmoid_backward")
-exp_backward = _binary("exp_backward")
-log_backward = _binary("log_backward")
-sqrt_backward = _binary("sqrt_backward")
+relu_backward = _engine.relu_backward
+tanh_backward = _engine.tanh_backward
+sigmoid_backward = _engine.sigmoid_backward
+exp_backward = _engine.exp_backward
+log_backward = _engine.log_backward
+sqrt_backward = _engine.sqrt_backward
 
 
 def pow_backward(g: TensorView, x: TensorView, exponent: float) -> Storage:
     return _ret_storage(_lib.nt_pow_backward, _vref(g), _vref(x), C.c_float(exponent))
 
 
-def div_backward_x2(g: TensorView, x1: TensorView, x2: TensorView) -> Storage:
-    return _ret_storage(_lib.nt_div_backward_x2, _vref(g), _vref(x1), _vref(x2))
+div_backward_x2 = _engine.div_backward_x2
 
 
 def extremum_backward(g_expanded: TensorView, x: TensorView, m_expanded: TensorView, axis: Sequence[int]) -> Storage:
@@ -690,16 +540,8 @@ def extremum_backward(g_expanded: TensorView, x: TensorView, m_expanded: TensorV
     return _ret_storage(_lib.nt_extremum_backward, _vref(g_expanded), _vref(x), _vref(m_expanded), arr, C.c_int32(n))
 
 
-def _backward_both(fn):
-    def op(g: TensorView, x1: TensorView, x2: TensorView):
-        a, b = C.c_void_p(), C.c_void_p()
-        _check(fn(_vref(g), _vref(x1), _vref(x2), C.byref(a), C.byref(b)))
-        return (Storage._wrap(a.value), Storage._wrap(b.value)) if a.value else None
-    return op
-
-
-mul_backward = _backward_both(_lib.nt_mul_backward)   # (x2*g, x1*g) in one pass, or None
-div_backward = _backward_both(_lib.nt_div_backward)   # (g/x2, ((-x1)/x2**2)*g) in one pass, or None
+mul_backward = _engine.mul_backward   # (x2*g, x1*g) in one pass, or None
+div_backward = _engine.div_backward   # (g/x2, ((-x1)/x2**2)*g) in one pass, or None
 
 
 def sgd_update(param: TensorView, grad: TensorView, lr: float, grad_scale: float = 1.0) -> None:

@@ -1,8 +1,9 @@
 """nanotorch op-kernel hot path on B200: Tensor/autograd API over hand-written sm_100a kernels.
 
 Mirrors the public surface of the reference package for this path (src/nanotorch/__init__.py):
-``Tensor``, dtypes, ``no_grad``, functional ops, factories, ``manual_seed``; operators are bound
-onto ``Tensor`` here exactly as the reference binds them at import (src/nanotorch/__init__.py:124-177).
+``Tensor``, dtypes, ``no_grad``, functional ops, factories, ``manual_seed``.  The arithmetic operators and op
+methods are slots of the native tensor type; the comparisons are bound onto ``Tensor`` here, as the reference
+binds all of them at import (src/nanotorch/__init__.py:124-177).
 """
 
 from . import _C
@@ -40,23 +41,6 @@ def _t(other, self):
     return totensor(other, anchor=self)
 
 
-Tensor.__add__ = lambda self, other: AddOp.apply(self, _t(other, self))
-Tensor.__radd__ = lambda self, other: AddOp.apply(self, _t(other, self))
-Tensor.__iadd__ = lambda self, other: AddOp.apply(self, _t(other, self), out=self)
-Tensor.__mul__ = lambda self, other: MulOp.apply(self, _t(other, self))
-Tensor.__rmul__ = lambda self, other: MulOp.apply(self, _t(other, self))
-Tensor.__imul__ = lambda self, other: MulOp.apply(self, _t(other, self), out=self)
-Tensor.__sub__ = lambda self, other: SubOp.apply(self, _t(other, self))
-Tensor.__rsub__ = lambda self, other: SubOp.apply(_t(other, self), self)
-Tensor.__isub__ = lambda self, other: SubOp.apply(self, _t(other, self), out=self)
-Tensor.__truediv__ = lambda self, other: TrueDivOp.apply(self, _t(other, self))
-Tensor.__rtruediv__ = lambda self, other: TrueDivOp.apply(_t(other, self), self)
-Tensor.__itruediv__ = lambda self, other: TrueDivOp.apply(self, _t(other, self), out=self)
-Tensor.__neg__ = lambda self: NegOp.apply(self)
-Tensor.__matmul__ = lambda self, other: MatmulOp.apply(self, _t(other, self))
-Tensor.__pow__ = lambda self, exponent: PowOp.apply(self, _t(exponent, self))
-Tensor.__rpow__ = lambda self, base: PowOp.apply(_t(base, self), self)
-
 
 def _compare(kernel):
     def op(x1: Tensor, x2: Tensor) -> Tensor:
@@ -77,20 +61,6 @@ Tensor.__gt__ = lambda self, other: greater_op_(self, _t(other, self))
 Tensor.__ge__ = lambda self, other: greater_eq_op_(self, _t(other, self))
 Tensor.__lt__ = lambda self, other: _t(other, self) > self
 Tensor.__le__ = lambda self, other: _t(other, self) >= self
-Tensor.exp = lambda self: ExpOp.apply(self)
-Tensor.log = lambda self: LogOp.apply(self)
-Tensor.sqrt = lambda self: SqrtOp.apply(self)
-Tensor.tanh = lambda self: TanhOp.apply(self)
-Tensor.sigmoid = lambda self: SigmoidOp.apply(self)
-Tensor.relu = lambda self: ReluOp.apply(self)
-Tensor.pow = lambda self, exponent: PowOp.apply(self, exponent)
-Tensor.sum = lambda self, axis=None, keepdim=False, dtype=None: SumOp.apply(self, axis, keepdim, dtype)
-Tensor.mean = lambda self, axis=None, keepdim=False, dtype=None: MeanOp.apply(self, axis, keepdim, dtype)
-Tensor.max = lambda self, axis=None, keepdim=False: MaxOp.apply(self, axis, keepdim)
-Tensor.min = lambda self, axis=None, keepdim=False: MinOp.apply(self, axis, keepdim)
-Tensor.reshape = lambda self, *dims: ReshapeOp.apply(self, *dims)
-Tensor.expand = lambda self, *dims: ExpandOp.apply(self, *dims)
-Tensor.transpose = lambda self, dim0, dim1: TransposeOp.apply(self, dim0, dim1)
 
 
 # ---- functional forms (src/nanotorch/ops.py)

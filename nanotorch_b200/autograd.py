@@ -8,8 +8,12 @@ Differences, none of which changes a value:
   - for Float32 tensors on Cuda each backward is ONE fused kernel that performs the reference's
     chain of primitive kernels with the same per-step rounding (include/nt_b200.h); any other
     dtype takes the reference's composition of primitives;
-  - Python scalars become device scalars by a fill kernel instead of a host->device copy, and
+  - Python scalars become constants the kernels take as arguments instead of a host->device copy, and
     PowOp never reads its exponent back from the device.
+
+For ordinary Float32 Cuda tensors ``apply`` and the backward sweep run natively (csrc/engine), with the
+same calls in the same order as the classes below; these classes are the specification and serve every
+other case (dtypes, devices, ``out=``, broadcast batches, subclasses).
 """
 
 from __future__ import annotations
@@ -17,28 +21,21 @@ from __future__ import annotations
 import math
 from typing import Any
 
-from . import _C
+from . import _C, _engine
 from ._C import Device, Dtype
 from .tensor import Shape, Tensor, broadcast_shapes, promote_dtypes, sizeof
 
-_grad_enabled = True
-
-
-def is_grad_enabled() -> bool:
-    return _grad_enabled
+is_grad_enabled = _engine.is_grad_enabled
 
 
 class no_grad:
     """Context manager disabling graph recording (src/nanotorch/autograd/grad_mode.py:11-21)."""
 
     def __enter__(self):
-        global _grad_enabled
-        self._prev = _grad_enabled
-        _grad_enabled = False
+        self._prev = _engine.set_grad_enabled(False)
 
     def __exit__(self, exc_type, exc, tb):
-        global _grad_enabled
-        _grad_enabled = self._prev
+        _engine.set_grad_enabled(self._prev)
 
 
 def totensor(x, *, anchor: Tensor) -> Tensor:
@@ -93,50 +90,12 @@ def normalize_axes(axis, x: Tensor) -> Shape:
     return axis
 
 
-class Function:
-    """Base class of the differentiable ops (src/nanotorch/autograd/function.py:11-93)."""
-
-    def __init__(self):
-        self._inputs: Any = None
-        self._inputs_kw: Any = None
-        self._saved: tuple[tuple[Tensor, int], ...] | None = None
-        self.needs_input_grad: tuple[bool, ...] = ()
+class Function(_engine.FunctionBase):
+    """Base class of the differentiable ops (src/nanotorch/autograd/function.py:11-93); ``apply``,
+    ``save_for_backward``, ``saved_tensors`` and ``inputs`` are the native base's."""
 
     def __repr__(self) -> str:
         return f"[{type(self).__name__}]"
-
-    @property
-    def inputs(self):
-        if self._inputs is None:
-            raise RuntimeError("No inputs saved during apply().")
-        return self._inputs
-
-    @property
-    def saved_tensors(self) -> tuple[Tensor, ...]:
-        if self._saved is None:
-            raise RuntimeError("No tensor was saved during forward.")
-        for t, v in self._saved:
-            if t.version != v:
-                raise RuntimeError("One of the tensors needed for grad computation was modified inplace.")
-        return tuple(t for t, _ in self._saved)
-
-    def save_for_backward(self, *tensors: Tensor) -> None:
-        if is_grad_enabled():
-            self._saved = tuple((t, t.version) for t in tensors)
-
-    @classmethod
-    def apply(cls, *args, **kwargs) -> Tensor:
-        self = cls()
-        self._inputs = args
-        self._inputs_kw = kwargs
-        out = self.forward(*args, **kwargs)
-        if is_grad_enabled():
-            if any(out is a for a in list(args) + list(kwargs.values())):
-                out = out._alias()
-            self.needs_input_grad = tuple(isinstance(a, Tensor) and a.requires_grad for a in args)
-            if any(self.needs_input_grad):
-                out.attach_grad_fn(self)
-        return out
 
     def forward(self, *inputs):
         raise NotImplementedError
@@ -181,6 +140,11 @@ def _binary(x1: Tensor, x2: Tensor, op, op_inplace, out: Tensor | None) -> Tenso
     return result
 
 
+def _input_shapes(fn: Function) -> tuple[Shape, Shape]:
+    x1, x2 = fn.inputs[:2]
+    return x1.shape, x2.shape
+
+
 class _BinaryOp(Function):
     @classmethod
     def flops(cls, x1, x2, _=None) -> int:
@@ -200,20 +164,18 @@ def _negated(g: Tensor) -> Tensor:
 
 class AddOp(_BinaryOp):
     def forward(self, x1, x2, out=None):
-        self._shapes = (x1.shape, x2.shape)
         return _binary(x1, x2, _C.add, _C.add_inplace, out)
 
     def backward(self, g):
-        return tuple(unbroadcast(g, s) if _need(self, i) else None for i, s in enumerate(self._shapes))
+        return tuple(unbroadcast(g, s) if _need(self, i) else None for i, s in enumerate(_input_shapes(self)))
 
 
 class SubOp(_BinaryOp):
     def forward(self, x1, x2, out=None):
-        self._shapes = (x1.shape, x2.shape)
         return _binary(x1, x2, _C.subtract, _C.sub_inplace, out)
 
     def backward(self, g):
-        s1, s2 = self._shapes
+        s1, s2 = _input_shapes(self)
         return (unbroadcast(g, s1) if _need(self, 0) else None,
                 unbroadcast(_negated(g), s2) if _need(self, 1) else None)
 
@@ -279,24 +241,25 @@ def _matmul_shapes(s1: Shape, s2: Shape) -> tuple[Shape, Shape, Shape]:
 class MatmulOp(Function):
     def forward(self, x1, x2):
         self.save_for_backward(x1, x2)
-        self._shape1, self._shape2, shape_out = _matmul_shapes(x1.shape, x2.shape)
+        shape1, shape2, shape_out = _matmul_shapes(x1.shape, x2.shape)
         dtype = promote_dtypes(x1.dtype, x2.dtype)
-        a = x1.to(dtype).expand(*self._shape1)
+        a = x1.to(dtype).expand(*shape1)
         b = x2
-        if b.ndim == 1 and self._shape2[-2:] == (b.shape[0], 1):
+        if b.ndim == 1 and shape2[-2:] == (b.shape[0], 1):
             b = b.reshape(b.shape[0], 1)
-        b = b.to(dtype).expand(*self._shape2)
+        b = b.to(dtype).expand(*shape2)
         return Tensor._new_contiguous(_C.matmul(a._C_view, b._C_view), shape_out)
 
     def backward(self, g):
         x1, x2 = self.saved_tensors
-        a = x1.expand(*self._shape1)
+        shape1, shape2, _ = _matmul_shapes(x1.shape, x2.shape)
+        a = x1.expand(*shape1)
         b = x2
-        if b.ndim == 1 and self._shape2[-2:] == (b.shape[0], 1):
+        if b.ndim == 1 and shape2[-2:] == (b.shape[0], 1):
             b = b.reshape(b.shape[0], 1)
         b_orig = b
-        b = b.expand(*self._shape2)
-        g = g.reshape(*broadcast_shapes(self._shape1[:-2], self._shape2[:-2]), self._shape1[-2], self._shape2[-1])
+        b = b.expand(*shape2)
+        g = g.reshape(*broadcast_shapes(shape1[:-2], shape2[:-2]), shape1[-2], shape2[-1])
         g1 = g2 = None
         if (_need(self, 0) and _need(self, 1) and x1.ndim == 2 and x2.ndim == 2 and g.ndim == 2
                 and x1.dtype == x2.dtype == g.dtype == Dtype.Float32 and x1.device == x2.device == Device.Cuda):
@@ -339,7 +302,6 @@ class LinearOp(Function):
 
     def forward(self, x, W, b):
         self.save_for_backward(x, W)
-        self._bias_shape = b.shape
         return Tensor._new_contiguous(_C.linear(x._C_view, W._C_view, b._C_view), (x.shape[0], W.shape[1]))
 
     def backward(self, g):
@@ -351,7 +313,7 @@ class LinearOp(Function):
         else:
             gx = g @ W.transpose(-2, -1) if _need(self, 0) else None
             gW = x.transpose(-2, -1) @ g if _need(self, 1) else None
-        gb = unbroadcast(g, self._bias_shape) if _need(self, 2) else None
+        gb = unbroadcast(g, self.inputs[2].shape) if _need(self, 2) else None
         return gx, gW, gb
 
     @classmethod
@@ -390,11 +352,10 @@ def _bwd2(kernel, g: Tensor, saved: Tensor) -> Tensor:
 
 class NegOp(_UnaryOp):
     def forward(self, x):
-        self._shape = x.shape
         return Tensor._new_contiguous(_C.neg(x._C_view), x.shape)
 
     def backward(self, g):
-        return (unbroadcast(_negated(g), self._shape),)
+        return (unbroadcast(_negated(g), self.inputs[0].shape),)
 
 
 class ExpOp(_UnaryOp):
@@ -524,15 +485,14 @@ class SumOp(_ReductionOp):
         if dtype is None:
             dtype = max(x.dtype, Dtype.Int64)
         new_shape = _reduced_shapes(x, self._axis, keepdim)
-        self._orig_shape = x.shape
         if x.is_empty:
             return Tensor._new_contiguous(_C.zeros(math.prod(new_shape), dtype, x.device), new_shape)
         return Tensor._new_contiguous(_C.sum(x._C_view, self._axis, dtype), new_shape)
 
     def backward(self, g):
-        if not self._orig_shape:
+        if not self.inputs[0].shape:
             return (g,)
-        return (_expand_back(g, self._orig_shape, self._axis),)
+        return (_expand_back(g, self.inputs[0].shape, self._axis),)
 
 
 class MeanOp(_ReductionOp):
@@ -542,7 +502,6 @@ class MeanOp(_ReductionOp):
         if dtype < Dtype.Float32:
             raise TypeError("Cannot take mean of integer tensor, cast to fp.")
         self._axis = normalize_axes(axis, x)
-        self._orig_shape = x.shape
         if _fused(x) and dtype == Dtype.Float32 and not x.is_empty:
             # sum and the true division by the count in one launch (same bits as the two steps below);
             # the count is exact in fp32 up to 2^24 elements per slice, beyond that the composed form runs
@@ -558,12 +517,12 @@ class MeanOp(_ReductionOp):
         return total / self._denom  # true division by the count, not a multiply by its reciprocal
 
     def backward(self, g):
-        if not self._orig_shape:
+        if not self.inputs[0].shape:
             return (g,)
         # The reference divides the expanded gradient element by element (autograd/ops_reduction.py:129-137);
         # dividing the kept elements once and expanding the quotient (a stride-0 view, like Sum's
         # gradient) yields the same bits without a division and a write per input element.
-        return (_expand_back(g / self._denom, self._orig_shape, self._axis),)
+        return (_expand_back(g / self._denom, self.inputs[0].shape, self._axis),)
 
 
 class _ExtremumOp(_ReductionOp):
@@ -572,7 +531,6 @@ class _ExtremumOp(_ReductionOp):
     def forward(self, x, axis=None, keepdim=False):
         self._axis = normalize_axes(axis, x)
         new_shape = _reduced_shapes(x, self._axis, keepdim)
-        self._orig_shape = x.shape
         if x.is_empty:
             if math.prod(new_shape) != 0:
                 raise IndexError("argmin() expects reduction dim to be specified for numel=0.")
@@ -582,14 +540,14 @@ class _ExtremumOp(_ReductionOp):
         return m
 
     def backward(self, g):
-        if not self._orig_shape:
+        if not self.inputs[0].shape:
             return (g,)
         x, m = self.saved_tensors
-        m_full = _expand_back(m, self._orig_shape, self._axis)
-        g_full = _expand_back(g, self._orig_shape, self._axis)
+        m_full = _expand_back(m, self.inputs[0].shape, self._axis)
+        g_full = _expand_back(g, self.inputs[0].shape, self._axis)
         if _fused(g, x, m):
             out = _C.extremum_backward(g_full._C_view, x._C_view, m_full._C_view, self._axis)
-            return (Tensor._new_contiguous(out, self._orig_shape),)
+            return (Tensor._new_contiguous(out, self.inputs[0].shape),)
         # The reference's mask arithmetic: Bool mask times the INTEGER quotient 1 // count, which is
         # 1 where the extremum is unique and 0 on every tied slice (autograd/ops_reduction.py:209-212).
         mask = x == m_full
@@ -611,21 +569,19 @@ class ReshapeOp(Function):
     def forward(self, x, *dims):
         if math.prod(dims) != x.numel:
             raise ValueError(f"Can't reshape {x.shape} into {dims}.")
-        self._shape = x.shape
         if dims == x.shape:
             return x
         x = x._to_contiguous()
         return Tensor._new_view(x.storage, tuple(dims), None, x._offset)
 
     def backward(self, g):
-        return (g.reshape(*self._shape),)
+        return (g.reshape(*self.inputs[0].shape),)
 
 
 class ExpandOp(Function):
     def forward(self, x, *dims):
         if len(dims) < x.ndim:
             raise ValueError(f"Cannot broadcast {x.shape} to {dims}.")
-        self._orig_shape = x.shape
         if dims == x.shape:
             return x
         pad = len(dims) - x.ndim
@@ -640,7 +596,7 @@ class ExpandOp(Function):
         return Tensor._new_view(x.storage, tuple(dims), tuple(strides), x._offset)
 
     def backward(self, g):
-        return (unbroadcast(g, self._orig_shape),)
+        return (unbroadcast(g, self.inputs[0].shape),)
 
 
 class TOp(Function):
@@ -655,7 +611,6 @@ class TOp(Function):
 
 class TransposeOp(Function):
     def forward(self, x, dim0, dim1):
-        self._dims = (dim0, dim1)
         if x.ndim < 2 or dim0 == dim1:
             return x
         shape, strides = list(x.shape), list(x._strides)
@@ -664,7 +619,7 @@ class TransposeOp(Function):
         return Tensor._new_view(x.storage, tuple(shape), tuple(strides), x._offset)
 
     def backward(self, g):
-        return (g.transpose(*self._dims),)
+        return (g.transpose(*self.inputs[1:]),)
 
 
 ALL_OPS_ = [AddOp, ExpOp, ExpandOp, LogOp, MatmulOp, MeanOp, MulOp, NegOp, PowOp, ReluOp, ReshapeOp, SigmoidOp,
@@ -679,51 +634,7 @@ ALL_OPS_ = [AddOp, ExpOp, ExpandOp, LogOp, MatmulOp, MeanOp, MulOp, NegOp, PowOp
 # rest of backward continues.
 leaf_grad_hooks: dict[int, Any] = {}
 
+# Reverse-topological sweep from a tensor whose ``_grad`` holds the seed (csrc/engine/autograd.cpp).
+run_backward = _engine.run_backward
 
-def run_backward(root: Tensor) -> None:
-    """Reverse-topological sweep from `root`, whose ``_grad`` holds the seed.
-
-    Same contract as the reference's ``_backpropagate_grad`` (src/nanotorch/core.py:836-872): a node
-    runs once every consumer has reported, leaf gradients accumulate, intermediate gradients are
-    dropped as soon as they have been consumed.
-    """
-    order: list[Tensor] = []
-    seen: set[int] = set()
-    stack: list[tuple[Tensor, bool]] = [(root, False)]
-    while stack:
-        node, expanded = stack.pop()
-        if expanded:
-            order.append(node)
-            continue
-        if id(node) in seen or node.grad_fn is None:
-            continue
-        seen.add(id(node))
-        stack.append((node, True))
-        for inp in node.grad_fn.inputs:
-            if isinstance(inp, Tensor) and inp.requires_grad and inp.grad_fn is not None and id(inp) not in seen:
-                stack.append((inp, False))
-    # contributions each hooked leaf is still to receive in this pass
-    pending: dict[int, int] = {}
-    if leaf_grad_hooks:
-        for node in order:
-            for a in node.grad_fn.inputs:
-                if isinstance(a, Tensor) and a.requires_grad and a.grad_fn is None and id(a) in leaf_grad_hooks:
-                    pending[id(a)] = pending.get(id(a), 0) + 1
-    with no_grad():  # gradients are values, not graph nodes
-        for node in reversed(order):
-            fn = node.grad_fn
-            if node._grad is None:
-                raise RuntimeError("f_x.grad is None.")
-            tensor_inputs = [a for a in fn.inputs if isinstance(a, Tensor)]
-            grads = fn.backward(node._grad)
-            for x, gx in zip(tensor_inputs, grads):
-                if not x.requires_grad:
-                    continue
-                if gx is not None:
-                    x._grad = gx if x._grad is None else x._grad + gx
-                left = pending.get(id(x))
-                if left is not None and x.grad_fn is None:
-                    pending[id(x)] = left - 1
-                    if left == 1 and x._grad is not None:
-                        leaf_grad_hooks[id(x)](x)
-            node._grad = None
+_engine.register_ops({op.__name__: op for op in [*ALL_OPS_, LinearOp]}, totensor, leaf_grad_hooks)

@@ -1,4 +1,5 @@
-"""Build step of the package: compiles csrc/*.cu for sm_100a and links lib/libnt_b200.so.
+"""Build step of the package: compiles csrc/*.cu for sm_100a and links lib/libnt_b200.so, then the host
+engine (csrc/engine/*.cpp, a CPython extension over that library) as _engine*.so beside the package's modules.
 
 Run as ``python nanotorch_b200/build.py`` (add ``--force`` to rebuild everything); it is run by
 path because importing the package needs the library this script produces.  Objects are
@@ -10,6 +11,7 @@ from __future__ import annotations
 import os
 import subprocess
 import sys
+import sysconfig
 from concurrent.futures import ThreadPoolExecutor
 from pathlib import Path
 
@@ -79,7 +81,33 @@ def build(force: bool = False, verbose: bool = False) -> Path:
         proc = subprocess.run(cmd, capture_output=True, text=True)
         if proc.returncode != 0:
             raise RuntimeError("link failed:\n" + proc.stdout + proc.stderr)
+    build_engine(force)
     return LIB
+
+
+def build_engine(force: bool = False) -> Path:
+    """Compile and link the CPython extension; returns its path."""
+    objs = []
+    ext = PKG / ("_engine" + sysconfig.get_config_var("EXT_SUFFIX"))
+    flags = ["-O2", "-std=c++20", "-fPIC", "-fvisibility=hidden", "-Wall", "-Wno-missing-field-initializers",
+             f"-I{sysconfig.get_paths()['include']}", f"-I{CUDA_HOME / 'include'}"]
+    jobs = []
+    for src in sorted((CSRC / "engine").glob("*.cpp")):
+        obj = OBJ / f"engine_{src.stem}.o"
+        objs.append(obj)
+        if force or _stale(obj, [src, *(CSRC / "engine").glob("*.h"), *_headers()]):
+            jobs.append(["g++", *flags, "-c", str(src), "-o", str(obj)])
+    with ThreadPoolExecutor(max_workers=4) as pool:
+        for proc in pool.map(lambda cmd: subprocess.run(cmd, capture_output=True, text=True), jobs):
+            if proc.returncode != 0:
+                raise RuntimeError("g++ failed:\n" + proc.stdout + proc.stderr)
+    if force or _stale(ext, objs):
+        cmd = ["g++", "-shared", "-o", str(ext), *map(str, objs), f"-L{LIB.parent}", f"-l:{LIB.name}",
+               "-Wl,-rpath,$ORIGIN/lib"]
+        proc = subprocess.run(cmd, capture_output=True, text=True)
+        if proc.returncode != 0:
+            raise RuntimeError("link failed:\n" + proc.stdout + proc.stderr)
+    return ext
 
 
 if __name__ == "__main__":

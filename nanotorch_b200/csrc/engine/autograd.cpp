@@ -1,0 +1,437 @@
+// Function (the base of the op classes), its apply(), and the backward sweep: see engine.h.
+#include "engine.h"
+
+#include <structmember.h>
+
+#include <cstddef>
+#include <unordered_map>
+#include <unordered_set>
+
+namespace eng {
+
+static TensorObj *T_(PyObject *o) { return reinterpret_cast<TensorObj *>(o); }
+static FunctionObj *F_(PyObject *o) { return reinterpret_cast<FunctionObj *>(o); }
+
+// =============================================================================================
+// Function
+static int function_traverse(PyObject *self, visitproc visit, void *arg) {
+  FunctionObj *f = F_(self);
+  Py_VISIT(f->inputs);
+  Py_VISIT(f->inputs_kw);
+  Py_VISIT(f->saved);
+  return 0;
+}
+static int function_clear(PyObject *self) {
+  FunctionObj *f = F_(self);
+  Py_CLEAR(f->inputs);
+  Py_CLEAR(f->inputs_kw);
+  Py_CLEAR(f->saved);
+  return 0;
+}
+static void function_dealloc(PyObject *self) {
+  PyObject_GC_UnTrack(self);
+  FunctionObj *f = F_(self);
+  function_clear(self);
+  Py_CLEAR(f->needs);
+  PyMem_Free(f->versions);
+  Py_TYPE(self)->tp_free(self);
+}
+
+static bool version_of(PyObject *tensor, uint64_t *out) {
+  TensorObj *t = T_(tensor);
+  if (is_tensor(tensor) && t->storage && is_storage(t->storage)) {
+    *out = storage_of(t)->version;
+    return true;
+  }
+  Ref v(PyObject_GetAttrString(tensor, "version"));
+  if (!v) return false;
+  *out = PyLong_AsUnsignedLongLong(v.p);
+  return !(*out == uint64_t(-1) && PyErr_Occurred());
+}
+static PyObject *function_save(PyObject *self, PyObject *const *args, Py_ssize_t n) {
+  if (!G.grad_enabled) Py_RETURN_NONE;
+  FunctionObj *f = F_(self);
+  PyObject *t = PyTuple_New(n);
+  uint64_t *v = static_cast<uint64_t *>(PyMem_Malloc(sizeof(uint64_t) * size_t(n ? n : 1)));
+  if (!t || !v) {
+    Py_XDECREF(t);
+    PyMem_Free(v);
+    return PyErr_NoMemory();
+  }
+  for (Py_ssize_t i = 0; i < n; ++i) {
+    PyTuple_SET_ITEM(t, i, own(args[i]));
+    if (!version_of(args[i], v + i)) {
+      Py_DECREF(t);
+      PyMem_Free(v);
+      return nullptr;
+    }
+  }
+  Py_XSETREF(f->saved, t);
+  PyMem_Free(f->versions);
+  f->versions = v;
+  Py_RETURN_NONE;
+}
+static PyObject *function_get_saved_tensors(PyObject *self, void *) {
+  FunctionObj *f = F_(self);
+  if (!f->saved) {
+    PyErr_SetString(PyExc_RuntimeError, "No tensor was saved during forward.");
+    return nullptr;
+  }
+  for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(f->saved); ++i) {
+    uint64_t v;
+    if (!version_of(PyTuple_GET_ITEM(f->saved, i), &v)) return nullptr;
+    if (v != f->versions[i]) {
+      PyErr_SetString(PyExc_RuntimeError, "One of the tensors needed for grad computation was modified inplace.");
+      return nullptr;
+    }
+  }
+  return own(f->saved);
+}
+static PyObject *function_get_inputs(PyObject *self, void *) {
+  if (!F_(self)->inputs) {
+    PyErr_SetString(PyExc_RuntimeError, "No inputs saved during apply().");
+    return nullptr;
+  }
+  return own(F_(self)->inputs);
+}
+static PyObject *function_get_needs(PyObject *self, void *) {
+  return F_(self)->needs ? own(F_(self)->needs) : PyTuple_New(0);
+}
+static int function_set_needs(PyObject *self, PyObject *value, void *) {
+  PyObject *t = value ? PySequence_Tuple(value) : nullptr;
+  if (!t) return -1;
+  Py_XSETREF(F_(self)->needs, t);
+  return 0;
+}
+static PyObject *function_get_axis(PyObject *self, void *) { return dims_tuple(F_(self)->n_axes, F_(self)->axes); }
+static int function_set_axis(PyObject *self, PyObject *value, void *) {
+  int n = 0;
+  if (!value || !parse_dims(value, F_(self)->axes, &n)) {
+    PyErr_SetString(PyExc_RuntimeError, "_axis: at most 8 axes.");
+    return -1;
+  }
+  F_(self)->n_axes = n;
+  return 0;
+}
+static PyObject *function_get_raw(PyObject *self, void *where) {
+  PyObject *o = *reinterpret_cast<PyObject **>(reinterpret_cast<char *>(self) + reinterpret_cast<intptr_t>(where));
+  return own(o ? o : Py_None);
+}
+
+// ---- apply
+Op op_of(PyTypeObject *cls) {
+  for (int i = 1; i < OP_COUNT; ++i)
+    if (G.op_class[i] == cls) return Op(i);
+  return OP_NONE;
+}
+
+PyObject *apply(PyTypeObject *cls, PyObject *const *args, Py_ssize_t n, PyObject *kwnames) {
+  const Py_ssize_t nkw = kwnames ? PyTuple_GET_SIZE(kwnames) : 0;
+  if (!nkw) {
+    const Op op = op_of(cls);
+    if (op != OP_NONE) {
+      PyObject *out = forward(op, cls, args, n);
+      if (out || PyErr_Occurred()) return out;
+    }
+  }
+  // the general form: cls().forward(*args, **kwargs)
+  Ref fn(PyObject_CallNoArgs(reinterpret_cast<PyObject *>(cls)));
+  if (!fn) return nullptr;
+  FunctionObj *f = F_(fn.p);
+  PyObject *in = PyTuple_New(n), *kw = PyDict_New();
+  Py_XSETREF(f->inputs, in);
+  Py_XSETREF(f->inputs_kw, kw);
+  if (!in || !kw) return nullptr;
+  for (Py_ssize_t i = 0; i < n; ++i) PyTuple_SET_ITEM(in, i, own(args[i]));
+  for (Py_ssize_t k = 0; k < nkw; ++k)
+    if (PyDict_SetItem(kw, PyTuple_GET_ITEM(kwnames, k), args[n + k]) < 0) return nullptr;
+  Ref method(PyObject_GetAttrString(fn.p, "forward"));
+  if (!method) return nullptr;
+  Ref out(PyObject_Vectorcall(method.p, args, size_t(n), kwnames));
+  if (!out) return nullptr;
+  if (!G.grad_enabled) return out.release();
+  bool same = false;
+  for (Py_ssize_t i = 0; i < n + nkw; ++i) same = same || args[i] == out.p;
+  if (same) {
+    out = Ref(PyObject_CallMethod(out.p, "_alias", nullptr));
+    if (!out) return nullptr;
+  }
+  Ref needs(PyTuple_New(n));
+  if (!needs) return nullptr;
+  bool any = false;
+  for (Py_ssize_t i = 0; i < n; ++i) {
+    const bool r = is_tensor(args[i]) && requires_grad(T_(args[i]));
+    any = any || r;
+    PyTuple_SET_ITEM(needs.p, i, own(r ? Py_True : Py_False));
+  }
+  Py_XSETREF(f->needs, needs.release());
+  if (!any) return out.release();
+  if (f->saved) { // a saved result would be a reference cycle: keep an alias over its storage instead
+    for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(f->saved); ++i)
+      if (PyTuple_GET_ITEM(f->saved, i) == out.p && is_tensor(out.p)) {
+        Ref alias(PyObject_CallMethod(out.p, "_alias", nullptr));
+        if (!alias) return nullptr;
+        PyTuple_SET_ITEM(f->saved, i, alias.release());
+        Py_DECREF(out.p);
+      }
+  }
+  if (is_tensor(out.p)) {
+    Py_XSETREF(T_(out.p)->grad_fn, fn.release());
+  } else {
+    Ref r(PyObject_CallMethod(out.p, "attach_grad_fn", "O", fn.p));
+    if (!r) return nullptr;
+  }
+  return out.release();
+}
+static PyObject *function_apply(PyObject *cls, PyObject *const *args, Py_ssize_t n, PyObject *kwnames) {
+  return apply(reinterpret_cast<PyTypeObject *>(cls), args, n, kwnames);
+}
+
+static PyMethodDef function_methods[] = {
+    {"apply", reinterpret_cast<PyCFunction>(reinterpret_cast<void *>(function_apply)), METH_CLASS | METH_FASTCALL | METH_KEYWORDS,
+     "Runs forward and, while gradients are enabled, records the node behind the result."},
+    {"save_for_backward", reinterpret_cast<PyCFunction>(function_save), METH_FASTCALL,
+     "Remembers tensors, and the versions of their storages, for backward."},
+    {}};
+static PyGetSetDef function_getset[] = {
+    {"inputs", function_get_inputs},
+    {"saved_tensors", function_get_saved_tensors},
+    {"needs_input_grad", function_get_needs, function_set_needs},
+    {"_inputs", function_get_raw, nullptr, nullptr, reinterpret_cast<void *>(offsetof(FunctionObj, inputs))},
+    {"_inputs_kw", function_get_raw, nullptr, nullptr, reinterpret_cast<void *>(offsetof(FunctionObj, inputs_kw))},
+    {"_saved", function_get_raw, nullptr, nullptr, reinterpret_cast<void *>(offsetof(FunctionObj, saved))},
+    {"_axis", function_get_axis, function_set_axis},
+    {}};
+static PyMemberDef function_members[] = {{"_e", T_DOUBLE, offsetof(FunctionObj, e), 0, nullptr},
+                                         {"_denom", T_LONGLONG, offsetof(FunctionObj, denom), 0, nullptr},
+                                         {}};
+PyTypeObject FunctionBase_Type = {.ob_base = PyVarObject_HEAD_INIT(nullptr, 0)};
+
+// =============================================================================================
+// Backward sweep.  Same contract as the reference's `_backpropagate_grad` (src/nanotorch/core.py:836-872): a node runs
+// once every consumer has reported, leaf gradients accumulate, intermediate gradients are dropped as soon as they have
+// been consumed.  The order of nodes, and so of the additions into shared gradients, is that of a depth-first sweep.
+static Ref inputs_of(PyObject *fn) {
+  if (PyObject_TypeCheck(fn, &FunctionBase_Type)) return Ref(function_get_inputs(fn, nullptr));
+  return Ref(PyObject_GetAttrString(fn, "inputs"));
+}
+
+struct NoGrad {
+  bool prev = G.grad_enabled;
+  NoGrad() { G.grad_enabled = false; }
+  ~NoGrad() { G.grad_enabled = prev; }
+};
+
+static bool accumulate(TensorObj *x, PyObject *gx) {
+  if (!x->grad) {
+    x->grad = own(gx);
+    return true;
+  }
+  PyObject *sum = reinterpret_cast<PyObject *>(add_tensors(x->grad, gx));
+  if (!sum && !PyErr_Occurred()) sum = PyNumber_Add(x->grad, gx);
+  if (!sum) return false;
+  Py_SETREF(x->grad, sum);
+  return true;
+}
+
+PyObject *run_backward(TensorObj *root) {
+  std::vector<Ref> order; // a node is followed by those it depends on... reversed below
+  std::unordered_set<PyObject *> seen;
+  std::vector<std::pair<PyObject *, bool>> stack;
+  stack.emplace_back(reinterpret_cast<PyObject *>(root), false);
+  while (!stack.empty()) {
+    const auto [node, expanded] = stack.back();
+    stack.pop_back();
+    if (expanded) {
+      order.emplace_back(own(node));
+      continue;
+    }
+    if (!T_(node)->grad_fn || !seen.insert(node).second) continue;
+    stack.emplace_back(node, true);
+    Ref in(inputs_of(T_(node)->grad_fn));
+    if (!in) return nullptr;
+    Ref fast(PySequence_Fast(in.p, "inputs must be a sequence"));
+    if (!fast) return nullptr;
+    for (Py_ssize_t i = 0; i < PySequence_Fast_GET_SIZE(fast.p); ++i) {
+      PyObject *x = PySequence_Fast_GET_ITEM(fast.p, i);
+      if (is_tensor(x) && T_(x)->grad_fn && !seen.count(x)) stack.emplace_back(x, false);
+    }
+  }
+  // contributions each hooked leaf is still to receive in this pass
+  std::unordered_map<PyObject *, int> pending;
+  if (G.hooks && PyDict_GET_SIZE(G.hooks)) {
+    for (Ref &node : order) {
+      Ref in(inputs_of(T_(node.p)->grad_fn));
+      Ref fast(in ? PySequence_Fast(in.p, "inputs must be a sequence") : nullptr);
+      if (!fast) return nullptr;
+      for (Py_ssize_t i = 0; i < PySequence_Fast_GET_SIZE(fast.p); ++i) {
+        PyObject *x = PySequence_Fast_GET_ITEM(fast.p, i);
+        if (!is_tensor(x) || T_(x)->grad_fn || !T_(x)->requires_grad) continue;
+        Ref key(PyLong_FromVoidPtr(x));
+        const int has = key ? PyDict_Contains(G.hooks, key.p) : -1;
+        if (has < 0) return nullptr;
+        if (has) pending[x] += 1;
+      }
+    }
+  }
+  NoGrad no_grad; // gradients are values, not graph nodes
+  for (auto it = order.rbegin(); it != order.rend(); ++it) {
+    TensorObj *node = T_(it->p);
+    if (!node->grad) {
+      PyErr_SetString(PyExc_RuntimeError, "f_x.grad is None.");
+      return nullptr;
+    }
+    Ref fn(own(node->grad_fn)), g(own(node->grad));
+    PyObject *out[3] = {};
+    int n_out = 0;
+    Ref grads; // of the Python backward
+    const bool native = PyObject_TypeCheck(fn.p, &FunctionBase_Type) && backward_fast(F_(fn.p), T_(g.p), out, &n_out);
+    Ref held[3] = {Ref(out[0]), Ref(out[1]), Ref(out[2])};
+    if (!native) {
+      if (PyErr_Occurred()) return nullptr;
+      Ref r(PyObject_CallMethod(fn.p, "backward", "O", g.p));
+      if (!r) return nullptr;
+      grads = Ref(PySequence_Fast(r.p, "backward must return one gradient per tensor input"));
+      if (!grads) return nullptr;
+      n_out = int(PySequence_Fast_GET_SIZE(grads.p));
+    }
+    Ref in(inputs_of(fn.p));
+    Ref fast(in ? PySequence_Fast(in.p, "inputs must be a sequence") : nullptr);
+    if (!fast) return nullptr;
+    int at = 0; // gradients come one per tensor input
+    for (Py_ssize_t i = 0; i < PySequence_Fast_GET_SIZE(fast.p) && at < n_out; ++i) {
+      PyObject *x = PySequence_Fast_GET_ITEM(fast.p, i);
+      if (!is_tensor(x)) continue;
+      PyObject *gx = native ? held[at].p : PySequence_Fast_GET_ITEM(grads.p, at);
+      ++at;
+      if (!requires_grad(T_(x))) continue;
+      if (gx && gx != Py_None && !accumulate(T_(x), gx)) return nullptr;
+      if (T_(x)->grad_fn || pending.empty()) continue;
+      auto p = pending.find(x);
+      if (p == pending.end()) continue;
+      if (p->second-- == 1 && T_(x)->grad) {
+        Ref key(PyLong_FromVoidPtr(x));
+        PyObject *hook = key ? PyDict_GetItemWithError(G.hooks, key.p) : nullptr;
+        if (!hook) {
+          if (!PyErr_Occurred()) PyErr_SetObject(PyExc_KeyError, key.p);
+          return nullptr;
+        }
+        Ref hold(own(hook)), r(PyObject_CallOneArg(hook, x));
+        if (!r) return nullptr;
+      }
+    }
+    Py_CLEAR(node->grad);
+    g = Ref();
+  }
+  Py_RETURN_NONE;
+}
+
+// =============================================================================================
+// Module functions
+static PyObject *m_run_backward(PyObject *, PyObject *root) {
+  if (!is_tensor(root)) {
+    PyErr_SetString(PyExc_TypeError, "run_backward: expected a Tensor");
+    return nullptr;
+  }
+  return run_backward(T_(root));
+}
+static PyObject *m_is_grad_enabled(PyObject *, PyObject *) { return PyBool_FromLong(G.grad_enabled); }
+static PyObject *m_set_grad_enabled(PyObject *, PyObject *on) { // returns the previous setting
+  const int v = PyObject_IsTrue(on);
+  if (v < 0) return nullptr;
+  const bool prev = G.grad_enabled;
+  G.grad_enabled = v != 0;
+  return PyBool_FromLong(prev);
+}
+// sgd_update(param, lr, scale): the fused update of one ordinary parameter; False when it is not one
+static PyObject *m_sgd_update(PyObject *, PyObject *const *args, Py_ssize_t n) {
+  if (n != 3) {
+    PyErr_SetString(PyExc_TypeError, "sgd_update(param, lr, grad_scale)");
+    return nullptr;
+  }
+  const double lr = PyFloat_AsDouble(args[1]), scale = PyFloat_AsDouble(args[2]);
+  if (PyErr_Occurred()) return nullptr;
+  if (!is_fast(args[0]) || !T_(args[0])->grad || !is_fast(T_(args[0])->grad)) Py_RETURN_FALSE;
+  TensorObj *p = T_(args[0]), *g = T_(p->grad);
+  if (!same_shape(p, g)) Py_RETURN_FALSE;
+  const nt_view vp = view_of(p), vg = view_of(g);
+  const int rc = nt_sgd_update(&vp, &vg, float(lr), float(scale));
+  if (rc) return raise_status(rc);
+  Py_RETURN_TRUE;
+}
+static PyObject *m_register_storage(PyObject *, PyObject *const *args, Py_ssize_t n) { // (Storage, dtypes, devices)
+  if (n != 3 || !PyType_Check(args[0]) || !PyTuple_Check(args[1]) || PyTuple_GET_SIZE(args[1]) != 5 ||
+      !PyTuple_Check(args[2]) || PyTuple_GET_SIZE(args[2]) != 2) {
+    PyErr_SetString(PyExc_TypeError, "register_storage(Storage, five dtypes, two devices)");
+    return nullptr;
+  }
+  G.storage_type = reinterpret_cast<PyTypeObject *>(own(args[0]));
+  for (int i = 0; i < 5; ++i) G.dtypes[i] = own(PyTuple_GET_ITEM(args[1], i));
+  for (int i = 0; i < 2; ++i) G.devices[i] = own(PyTuple_GET_ITEM(args[2], i));
+  Py_RETURN_NONE;
+}
+static PyObject *m_register_tensor(PyObject *, PyObject *type) {
+  if (!PyType_Check(type) || !PyType_IsSubtype(reinterpret_cast<PyTypeObject *>(type), &TensorBase_Type)) {
+    PyErr_SetString(PyExc_TypeError, "register_tensor: a class derived from TensorBase");
+    return nullptr;
+  }
+  G.tensor_type = reinterpret_cast<PyTypeObject *>(own(type));
+  Py_RETURN_NONE;
+}
+static PyObject *m_register_ops(PyObject *, PyObject *const *args, Py_ssize_t n) { // (name -> class, totensor, leaf_grad_hooks)
+  static const char *const names[OP_COUNT] = {"", "AddOp", "SubOp", "MulOp", "TrueDivOp", "MatmulOp", "LinearOp", "NegOp", "ExpOp",
+                                              "LogOp", "SqrtOp", "TanhOp", "SigmoidOp", "ReluOp", "PowOp", "SumOp", "MeanOp",
+                                              "MaxOp", "MinOp", "ReshapeOp", "ExpandOp", "TOp", "TransposeOp"};
+  if (n != 3 || !PyDict_Check(args[0]) || !PyDict_Check(args[2])) {
+    PyErr_SetString(PyExc_TypeError, "register_ops(classes by name, totensor, hooks)");
+    return nullptr;
+  }
+  for (int i = 1; i < OP_COUNT; ++i) {
+    PyObject *c = PyDict_GetItemString(args[0], names[i]);
+    if (!c || !PyType_Check(c) || !PyType_IsSubtype(reinterpret_cast<PyTypeObject *>(c), &FunctionBase_Type)) {
+      PyErr_Format(PyExc_TypeError, "register_ops: no Function class %s", names[i]);
+      return nullptr;
+    }
+    G.op_class[i] = reinterpret_cast<PyTypeObject *>(own(c));
+  }
+  G.totensor = own(args[1]);
+  G.hooks = own(args[2]);
+  Py_RETURN_NONE;
+}
+static PyMethodDef m_functions[] = {
+    {"run_backward", m_run_backward, METH_O, "Reverse-topological sweep from a tensor whose gradient holds the seed."},
+    {"is_grad_enabled", m_is_grad_enabled, METH_NOARGS, nullptr},
+    {"set_grad_enabled", m_set_grad_enabled, METH_O, nullptr},
+    {"sgd_update", reinterpret_cast<PyCFunction>(m_sgd_update), METH_FASTCALL, nullptr},
+    {"register_storage", reinterpret_cast<PyCFunction>(m_register_storage), METH_FASTCALL, nullptr},
+    {"register_tensor", m_register_tensor, METH_O, nullptr},
+    {"register_ops", reinterpret_cast<PyCFunction>(m_register_ops), METH_FASTCALL, nullptr},
+    {}};
+
+bool init_autograd(PyObject *m) {
+  FunctionBase_Type.tp_name = "nanotorch_b200._engine.FunctionBase";
+  FunctionBase_Type.tp_basicsize = sizeof(FunctionObj);
+  FunctionBase_Type.tp_flags = Py_TPFLAGS_DEFAULT | Py_TPFLAGS_BASETYPE | Py_TPFLAGS_HAVE_GC;
+  FunctionBase_Type.tp_traverse = function_traverse;
+  FunctionBase_Type.tp_clear = function_clear;
+  FunctionBase_Type.tp_dealloc = function_dealloc;
+  FunctionBase_Type.tp_new = PyType_GenericNew;
+  FunctionBase_Type.tp_methods = function_methods;
+  FunctionBase_Type.tp_getset = function_getset;
+  FunctionBase_Type.tp_members = function_members;
+  if (PyType_Ready(&FunctionBase_Type) < 0) return false;
+  if (PyModule_AddObjectRef(m, "FunctionBase", reinterpret_cast<PyObject *>(&FunctionBase_Type)) < 0) return false;
+  return PyModule_AddFunctions(m, m_functions) == 0;
+}
+
+} // namespace eng
+
+static PyModuleDef engine_module = {PyModuleDef_HEAD_INIT, "nanotorch_b200._engine",
+                                    "Native storages, tensors and autograd over libnt_b200.so.", -1};
+
+PyMODINIT_FUNC PyInit__engine(void) {
+  PyObject *m = PyModule_Create(&engine_module);
+  if (m && eng::init_objects(m) && eng::init_ops(m) && eng::init_autograd(m)) return m;
+  Py_XDECREF(m);
+  return nullptr;
+}

@@ -1,0 +1,181 @@
+// The host side of an eager op, native: storages, views, tensors and the autograd engine as CPython types over the
+// C ABI of libnt_b200.so.  What these types do is what nanotorch_b200/tensor.py and autograd.py describe; the Python
+// classes there derive from the ones here and keep every case that is not an ordinary Float32 Cuda one.
+//
+// Why: an op of a small model is bounded by the host, not by the device.  Through ctypes and Python-level view
+// arithmetic one op cost 15-25 us of interpreter time (argument marshalling, enum and tuple construction, three
+// function frames per broadcast operand) against 2-3 us for its launch.
+#pragma once
+
+#define PY_SSIZE_T_CLEAN
+#include <Python.h>
+
+#include "../nt_core.cuh"
+
+namespace eng {
+
+constexpr int MAXD = NT_MAX_DIMS;
+
+struct StorageObj {
+  PyObject_HEAD
+  nt_storage *h;
+};
+
+struct ViewObj { // TensorView
+  PyObject_HEAD
+  PyObject *storage, *shape, *strides; // storage: any object; shape, strides: tuples
+  int64_t offset;
+};
+
+// nd <= MAXD: sh / st are authoritative and the tuples are made when Python asks for them; larger tensors (host-side
+// bookkeeping only, no kernel takes them) keep tuples and have nd == -1.
+struct TensorObj {
+  PyObject_HEAD
+  PyObject *storage;
+  PyObject *shape, *strides; // cached tuples, may be null
+  PyObject *grad, *grad_fn, *pyvalue;
+  int64_t offset;
+  int64_t sh[MAXD], st[MAXD];
+  int nd, nst; // nst: strides set so far (the Python constructor assigns shape and strides one after the other)
+  char requires_grad;
+};
+
+enum Op : int {
+  OP_NONE = 0, OP_ADD, OP_SUB, OP_MUL, OP_DIV, OP_MATMUL, OP_LINEAR, OP_NEG, OP_EXP, OP_LOG, OP_SQRT, OP_TANH,
+  OP_SIGMOID, OP_RELU, OP_POW, OP_SUM, OP_MEAN, OP_MAX, OP_MIN, OP_RESHAPE, OP_EXPAND, OP_T, OP_TRANSPOSE, OP_COUNT
+};
+
+struct FunctionObj {
+  PyObject_HEAD
+  PyObject *inputs, *inputs_kw;        // null: None
+  PyObject *saved;                     // tuple of tensors, null: nothing saved
+  uint64_t *versions;                  // of the saved tensors' storages, one each
+  PyObject *needs;                     // needs_input_grad tuple, null: ()
+  // set by the native forward only; the native backward runs when `op` is set
+  int op;
+  int n_axes;
+  int64_t axes[MAXD];
+  double e;                            // pow
+  int64_t denom;                       // mean
+};
+
+struct Globals {
+  PyTypeObject *storage_type = nullptr; // the Python classes derived from the ones here
+  PyTypeObject *tensor_type = nullptr;
+  PyObject *dtypes[5] = {};             // Dtype and Device members by value
+  PyObject *devices[2] = {};
+  PyTypeObject *op_class[OP_COUNT] = {};
+  PyObject *totensor = nullptr;         // autograd.totensor(x, anchor=...)
+  PyObject *hooks = nullptr;            // autograd.leaf_grad_hooks
+  bool grad_enabled = true;
+};
+extern Globals G;
+
+extern PyTypeObject StorageBase_Type, View_Type, TensorBase_Type, FunctionBase_Type;
+
+// ---- errors
+PyObject *raise_status(int status);     // the Python exception of a non-zero nt status; returns null
+struct PyErr {};                        // thrown after a Python exception has been set
+
+// ---- references
+struct Ref {
+  PyObject *p = nullptr;
+  Ref() = default;
+  explicit Ref(PyObject *o) : p(o) {}
+  Ref(const Ref &) = delete;
+  Ref &operator=(const Ref &) = delete;
+  Ref(Ref &&o) noexcept : p(o.p) { o.p = nullptr; }
+  Ref &operator=(Ref &&o) noexcept {
+    if (this != &o) {
+      Py_XDECREF(p);
+      p = o.p;
+      o.p = nullptr;
+    }
+    return *this;
+  }
+  ~Ref() { Py_XDECREF(p); }
+  PyObject *release() {
+    PyObject *o = p;
+    p = nullptr;
+    return o;
+  }
+  explicit operator bool() const { return p != nullptr; }
+};
+inline PyObject *own(PyObject *o) {
+  Py_INCREF(o);
+  return o;
+}
+
+// ---- storages and tensors
+PyObject *wrap_storage(nt_storage *s);  // takes the reference; null with an exception set on failure
+inline bool is_storage(PyObject *o) { return PyObject_TypeCheck(o, &StorageBase_Type); }
+inline bool is_tensor(PyObject *o) { return PyObject_TypeCheck(o, &TensorBase_Type); }
+inline nt_storage *storage_of(const TensorObj *t) { return reinterpret_cast<StorageObj *>(t->storage)->h; }
+
+TensorObj *alloc_tensor();              // an empty tensor of the registered class
+// fresh contiguous tensor over `s` (takes the reference)
+TensorObj *new_tensor(nt_storage *s, int nd, const int64_t *shape);
+// view of the storage object of `like` (shares it)
+TensorObj *new_view(PyObject *storage, int nd, const int64_t *shape, const int64_t *strides, int64_t offset);
+inline TensorObj *alias_of(const TensorObj *t) { return new_view(t->storage, t->nd, t->sh, t->st, t->offset); }
+
+inline bool requires_grad(const TensorObj *t) { return t->requires_grad || t->grad_fn; }
+inline bool same_shape(const TensorObj *a, const TensorObj *b) {
+  return a->nd == b->nd && std::memcmp(a->sh, b->sh, sizeof(int64_t) * size_t(a->nd < 0 ? 0 : a->nd)) == 0;
+}
+inline int64_t numel(int nd, const int64_t *sh) {
+  int64_t n = 1;
+  for (int d = 0; d < nd; ++d) n *= sh[d];
+  return n;
+}
+inline bool dense(const TensorObj *t) { // row-major strides, exactly (the rule of Tensor._is_contiguous)
+  int64_t acc = 1;
+  for (int d = t->nd - 1; d >= 0; --d) {
+    if (t->st[d] != acc) return false;
+    acc *= t->sh[d];
+  }
+  return true;
+}
+// An ordinary tensor of the fast paths: exactly the registered class, Float32 on Cuda, at most MAXD dims, not empty.
+inline bool is_fast(PyObject *o) {
+  if (Py_TYPE(o) != G.tensor_type) return false;
+  const TensorObj *t = reinterpret_cast<const TensorObj *>(o);
+  if (t->nd < 0 || !t->storage || Py_TYPE(t->storage) != G.storage_type) return false;
+  const nt_storage *s = storage_of(t);
+  if (s->dtype != NT_FLOAT32 || s->device != NT_CUDA) return false;
+  for (int d = 0; d < t->nd; ++d)
+    if (t->sh[d] == 0) return false;
+  return true;
+}
+inline nt_view view_of(const TensorObj *t) {
+  nt_view v;
+  v.storage = storage_of(t);
+  v.ndim = t->nd;
+  for (int d = 0; d < t->nd; ++d) {
+    v.shape[d] = t->sh[d];
+    v.strides[d] = t->st[d];
+  }
+  v.offset = t->offset;
+  return v;
+}
+// `t` broadcast to a shape of nd >= t->nd dims; false when it does not broadcast
+bool expand_view(const TensorObj *t, int nd, const int64_t *shape, nt_view *out);
+
+bool parse_dims(PyObject *seq, int64_t *out, int *n); // sequence of at most MAXD integers; false (no exception) otherwise
+PyObject *dims_tuple(int n, const int64_t *v);
+
+// ---- ops (ops.cpp): a new tensor, or null with an exception set, or null without one: "not a fast case"
+PyObject *forward(Op op, PyTypeObject *cls, PyObject *const *args, Py_ssize_t n);
+// the gradients of a node whose native forward ran; false: take the Python backward (no exception) or an exception
+bool backward_fast(FunctionObj *fn, TensorObj *g, PyObject **out, int *n_out);
+TensorObj *add_tensors(PyObject *a, PyObject *b); // a + b of two fast tensors of one shape, no graph; null otherwise
+PyObject *apply(PyTypeObject *cls, PyObject *const *args, Py_ssize_t n, PyObject *kwnames);
+PyObject *to_operand(PyObject *x, TensorObj *anchor); // totensor(x, anchor=anchor)
+PyObject *run_backward(TensorObj *root);
+Op op_of(PyTypeObject *cls);
+
+bool init_objects(PyObject *m);
+bool init_ops(PyObject *m);
+bool init_autograd(PyObject *m);
+
+} // namespace eng

@@ -1,0 +1,837 @@
+// The ops of engine.h: the `_C` functions over TensorViews, and the forward and backward of the op classes for
+// ordinary Float32 Cuda tensors.  Each follows its class in nanotorch_b200/autograd.py call for call, so results are
+// bit for bit those of the Python path; whatever is out of the ordinary returns "not a fast case" and takes it.
+#include "engine.h"
+
+#include <algorithm>
+
+namespace eng {
+
+bool view_arg(PyObject *o, nt_view *out);
+int parse_dtype(PyObject *o);
+
+// =============================================================================================
+// `_C` functions
+using Fn1 = int (*)(const nt_view *, nt_storage **);
+using Fn2 = int (*)(const nt_view *, const nt_view *, nt_storage **);
+using Fn3 = int (*)(const nt_view *, const nt_view *, const nt_view *, nt_storage **);
+using FnIn = int (*)(const nt_view *, const nt_view *);
+using FnBoth = int (*)(const nt_view *, const nt_view *, const nt_view *, nt_storage **, nt_storage **);
+using FnAxes = int (*)(const nt_view *, const int64_t *, int32_t, nt_storage **);
+
+static bool count_is(Py_ssize_t n, Py_ssize_t want) {
+  if (n == want) return true;
+  PyErr_Format(PyExc_TypeError, "expected %zd arguments, got %zd", want, n);
+  return false;
+}
+template <Fn1 FN> static PyObject *c_unary(PyObject *, PyObject *const *a, Py_ssize_t n) {
+  nt_view x;
+  if (!count_is(n, 1) || !view_arg(a[0], &x)) return nullptr;
+  nt_storage *out = nullptr;
+  const int rc = FN(&x, &out);
+  return rc ? raise_status(rc) : wrap_storage(out);
+}
+template <Fn2 FN> static PyObject *c_binary(PyObject *, PyObject *const *a, Py_ssize_t n) {
+  nt_view x, y;
+  if (!count_is(n, 2) || !view_arg(a[0], &x) || !view_arg(a[1], &y)) return nullptr;
+  nt_storage *out = nullptr;
+  const int rc = FN(&x, &y, &out);
+  return rc ? raise_status(rc) : wrap_storage(out);
+}
+template <Fn3 FN> static PyObject *c_ternary(PyObject *, PyObject *const *a, Py_ssize_t n) {
+  nt_view x, y, z;
+  if (!count_is(n, 3) || !view_arg(a[0], &x) || !view_arg(a[1], &y) || !view_arg(a[2], &z)) return nullptr;
+  nt_storage *out = nullptr;
+  const int rc = FN(&x, &y, &z, &out);
+  return rc ? raise_status(rc) : wrap_storage(out);
+}
+template <FnIn FN> static PyObject *c_inplace(PyObject *, PyObject *const *a, Py_ssize_t n) {
+  nt_view x, y;
+  if (!count_is(n, 2) || !view_arg(a[0], &x) || !view_arg(a[1], &y)) return nullptr;
+  const int rc = FN(&x, &y);
+  if (rc) return raise_status(rc);
+  Py_RETURN_NONE;
+}
+static PyObject *pair_of(nt_storage *s1, nt_storage *s2) {
+  Ref a(wrap_storage(s1)), b(wrap_storage(s2));
+  return a && b ? PyTuple_Pack(2, a.p, b.p) : nullptr;
+}
+template <FnBoth FN> static PyObject *c_both(PyObject *, PyObject *const *a, Py_ssize_t n) {
+  nt_view g, x, y;
+  if (!count_is(n, 3) || !view_arg(a[0], &g) || !view_arg(a[1], &x) || !view_arg(a[2], &y)) return nullptr;
+  nt_storage *s1 = nullptr, *s2 = nullptr;
+  const int rc = FN(&g, &x, &y, &s1, &s2);
+  if (rc) return raise_status(rc);
+  if (!s1) Py_RETURN_NONE;
+  return pair_of(s1, s2);
+}
+static PyObject *c_matmul_pair(PyObject *, PyObject *const *a, Py_ssize_t n) {
+  nt_view v[4];
+  if (!count_is(n, 4)) return nullptr;
+  for (int i = 0; i < 4; ++i)
+    if (!view_arg(a[i], &v[i])) return nullptr;
+  nt_storage *s1 = nullptr, *s2 = nullptr;
+  const int rc = nt_matmul_pair(&v[0], &v[1], &v[2], &v[3], &s1, &s2);
+  return rc ? raise_status(rc) : pair_of(s1, s2);
+}
+static bool axes_arg(PyObject *o, std::vector<int64_t> *out) {
+  Ref t(PySequence_Tuple(o));
+  if (!t) return false;
+  for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(t.p); ++i) {
+    Ref x(PyNumber_Long(PyTuple_GET_ITEM(t.p, i)));
+    if (!x) return false;
+    const long long v = PyLong_AsLongLong(x.p);
+    if (v == -1 && PyErr_Occurred()) return false;
+    out->push_back(v);
+  }
+  return true;
+}
+template <FnAxes FN> static PyObject *c_reduce(PyObject *, PyObject *const *a, Py_ssize_t n) {
+  nt_view x;
+  std::vector<int64_t> ax;
+  if (!count_is(n, 2) || !view_arg(a[0], &x) || !axes_arg(a[1], &ax)) return nullptr;
+  nt_storage *out = nullptr;
+  const int rc = FN(&x, ax.data(), int32_t(ax.size()), &out);
+  return rc ? raise_status(rc) : wrap_storage(out);
+}
+static PyObject *c_sum(PyObject *, PyObject *const *a, Py_ssize_t n) {
+  nt_view x;
+  std::vector<int64_t> ax;
+  if (!count_is(n, 3) || !view_arg(a[0], &x) || !axes_arg(a[1], &ax)) return nullptr;
+  const int dt = parse_dtype(a[2]);
+  if (dt < 0) return nullptr;
+  nt_storage *out = nullptr;
+  const int rc = nt_sum(&x, ax.data(), int32_t(ax.size()), dt, &out);
+  return rc ? raise_status(rc) : wrap_storage(out);
+}
+
+#define BINARY(name) {#name, reinterpret_cast<PyCFunction>(c_binary<nt_##name>), METH_FASTCALL, nullptr}
+#define UNARY(name) {#name, reinterpret_cast<PyCFunction>(c_unary<nt_##name>), METH_FASTCALL, nullptr}
+#define INPLACE(name) {#name, reinterpret_cast<PyCFunction>(c_inplace<nt_##name>), METH_FASTCALL, nullptr}
+#define REDUCE(name) {#name, reinterpret_cast<PyCFunction>(c_reduce<nt_##name>), METH_FASTCALL, nullptr}
+#define BOTH(name) {#name, reinterpret_cast<PyCFunction>(c_both<nt_##name>), METH_FASTCALL, nullptr}
+static PyMethodDef c_functions[] = {
+    BINARY(add), BINARY(subtract), BINARY(multiply), BINARY(divide), BINARY(pw_equal), BINARY(pw_greater),
+    BINARY(pw_greater_eq), BINARY(matmul), BINARY(relu_backward), BINARY(tanh_backward), BINARY(sigmoid_backward),
+    BINARY(exp_backward), BINARY(log_backward), BINARY(sqrt_backward),
+    UNARY(exp), UNARY(log), UNARY(sqrt), UNARY(tanh), UNARY(sigmoid), UNARY(neg), UNARY(relu),
+    UNARY(clone_contiguous_view_from),
+    INPLACE(add_inplace), INPLACE(sub_inplace), INPLACE(mul_inplace), INPLACE(div_inplace), INPLACE(copy_inplace),
+    REDUCE(max), REDUCE(min), REDUCE(argmax), REDUCE(argmin),
+    BOTH(mul_backward), BOTH(div_backward),
+    {"linear", reinterpret_cast<PyCFunction>(c_ternary<nt_linear>), METH_FASTCALL,
+     "x @ w + bias with the bias add fused into the GEMM epilogue (addition to the reference's surface)."},
+    {"div_backward_x2", reinterpret_cast<PyCFunction>(c_ternary<nt_div_backward_x2>), METH_FASTCALL, nullptr},
+    {"matmul_pair", reinterpret_cast<PyCFunction>(c_matmul_pair), METH_FASTCALL,
+     "(a1 @ b1, a2 @ b2): two independent products in one call (addition to the reference's surface; the bits of two `matmul` calls)."},
+    {"sum", reinterpret_cast<PyCFunction>(c_sum), METH_FASTCALL, "sum(x, axes, dtype)"},
+    {}};
+
+bool init_ops(PyObject *m) { return PyModule_AddFunctions(m, c_functions) == 0; }
+
+// =============================================================================================
+// Helpers of the fast paths
+static nt_storage *checked(int rc, nt_storage *const &s) { // by reference: rc is what fills it
+  if (rc) {
+    raise_status(rc);
+    throw PyErr{};
+  }
+  return s;
+}
+static PyObject *fresh(nt_storage *s, int nd, const int64_t *shape) {
+  PyObject *t = reinterpret_cast<PyObject *>(new_tensor(s, nd, shape));
+  if (!t) throw PyErr{};
+  return t;
+}
+static TensorObj *T_(PyObject *o) { return reinterpret_cast<TensorObj *>(o); }
+
+// A storage reference of this file's own.
+struct Held {
+  nt_storage *s = nullptr;
+  Held() = default;
+  explicit Held(nt_storage *p) : s(p) {}
+  Held(const Held &) = delete;
+  Held &operator=(const Held &) = delete;
+  ~Held() {
+    if (s) nt_storage_release(s);
+  }
+};
+static nt_storage *constant(const nt_scalar &v) {
+  nt_storage *s = nullptr;
+  return checked(nt_constant(&v, NT_FLOAT32, &s), s);
+}
+
+static bool scalar_of(PyObject *x, nt_scalar *out) { // bool before int: bool is an int subclass
+  if (PyBool_Check(x)) {
+    *out = nt_scalar{0, x == Py_True, double(x == Py_True)};
+    return true;
+  }
+  if (PyLong_Check(x)) {
+    int overflow = 0;
+    const long long v = PyLong_AsLongLongAndOverflow(x, &overflow);
+    if (overflow) return false;
+    *out = nt_scalar{1, v, double(v)};
+    return true;
+  }
+  if (PyFloat_Check(x)) {
+    *out = nt_scalar{2, 0, PyFloat_AS_DOUBLE(x)};
+    return true;
+  }
+  return false;
+}
+
+PyObject *to_operand(PyObject *x, TensorObj *anchor) {
+  if (is_tensor(x)) return own(x);
+  nt_scalar v;
+  if (is_storage(anchor->storage) && storage_of(anchor)->device == NT_CUDA && scalar_of(x, &v)) {
+    nt_storage *s = nullptr;
+    const int rc = nt_constant(&v, v.kind == 0 ? NT_BOOL : v.kind == 1 ? NT_INT64 : NT_FLOAT32, &s);
+    if (rc) return raise_status(rc);
+    TensorObj *t = new_tensor(s, 0, nullptr);
+    if (t) t->pyvalue = own(x);
+    return reinterpret_cast<PyObject *>(t);
+  }
+  static PyObject *names = Py_BuildValue("(s)", "anchor");
+  PyObject *args[2] = {x, reinterpret_cast<PyObject *>(anchor)};
+  return PyObject_Vectorcall(G.totensor, args, 1, names);
+}
+
+// An operand of an elementwise op of Float32 result: a fast tensor, or a 0-d tensor that still knows its Python value
+// (then its value at Float32, whatever its own dtype).
+struct Operand {
+  TensorObj *t = nullptr;
+  Held scalar;
+  bool take(PyObject *o) {
+    if (is_fast(o)) {
+      t = T_(o);
+      return true;
+    }
+    if (Py_TYPE(o) != G.tensor_type) return false;
+    TensorObj *x = T_(o);
+    nt_scalar v;
+    if (!x->pyvalue || x->nd != 0 || !is_storage(x->storage) || storage_of(x)->device != NT_CUDA ||
+        storage_of(x)->dtype > NT_FLOAT32 || !scalar_of(x->pyvalue, &v))
+      return false;
+    t = x;
+    scalar.s = constant(v);
+    return true;
+  }
+  bool view(int nd, const int64_t *shape, nt_view *out) const {
+    if (!expand_view(t, nd, shape, out)) return false;
+    if (scalar.s) {
+      out->storage = scalar.s;
+      out->offset = 0;
+    }
+    return true;
+  }
+};
+
+static bool broadcast(const TensorObj *a, const TensorObj *b, int *nd, int64_t *shape) {
+  *nd = a->nd > b->nd ? a->nd : b->nd;
+  for (int d = 0; d < *nd; ++d) {
+    const int da = d - (*nd - a->nd), db = d - (*nd - b->nd);
+    const int64_t ea = da < 0 ? 1 : a->sh[da], eb = db < 0 ? 1 : b->sh[db];
+    if (ea != eb && ea != 1 && eb != 1) return false;
+    shape[d] = ea == 1 ? eb : ea;
+  }
+  return true;
+}
+
+// ---- the node of a result
+struct Node {
+  FunctionObj *fn = nullptr; // null when no graph is recorded
+  Ref holder;
+};
+static bool recording(PyObject *const *in, int n) {
+  if (!G.grad_enabled) return false;
+  for (int i = 0; i < n; ++i)
+    if (is_tensor(in[i]) && requires_grad(T_(in[i]))) return true;
+  return false;
+}
+// A function object of class `cls` over the given arguments, attached to `out`.
+static FunctionObj *attach(Op op, PyTypeObject *cls, PyObject *out, PyObject *const *in, Py_ssize_t n) {
+  PyObject *f = cls->tp_alloc(cls, 0);
+  if (!f) throw PyErr{};
+  FunctionObj *fn = reinterpret_cast<FunctionObj *>(f);
+  Ref holder(f);
+  fn->op = op;
+  fn->inputs = PyTuple_New(n);
+  fn->needs = PyTuple_New(n);
+  if (!fn->inputs || !fn->needs) throw PyErr{};
+  for (Py_ssize_t i = 0; i < n; ++i) {
+    PyTuple_SET_ITEM(fn->inputs, i, own(in[i]));
+    PyTuple_SET_ITEM(fn->needs, i, own(is_tensor(in[i]) && requires_grad(T_(in[i])) ? Py_True : Py_False));
+  }
+  T_(out)->grad_fn = holder.release();
+  return fn;
+}
+// Saves tensors for backward.  A result that is its own node's saved tensor would be a reference cycle (and keep its
+// memory until the cycle collector runs): an alias over the same storage is saved in its place.
+static void save(FunctionObj *fn, PyObject *result, std::initializer_list<PyObject *> tensors) {
+  fn->saved = PyTuple_New(Py_ssize_t(tensors.size()));
+  fn->versions = static_cast<uint64_t *>(PyMem_Malloc(sizeof(uint64_t) * tensors.size()));
+  if (!fn->saved || !fn->versions) throw PyErr{};
+  Py_ssize_t i = 0;
+  for (PyObject *t : tensors) {
+    PyObject *keep = t == result ? reinterpret_cast<PyObject *>(alias_of(T_(t))) : own(t);
+    if (!keep) throw PyErr{};
+    fn->versions[i] = storage_of(T_(t))->version;
+    PyTuple_SET_ITEM(fn->saved, i++, keep);
+  }
+}
+
+// =============================================================================================
+// Forward
+static PyObject *binary_forward(Op op, PyTypeObject *cls, PyObject *const *in) {
+  static const Fn2 fns[] = {nt_add, nt_subtract, nt_multiply, nt_divide};
+  Operand a, b;
+  if (!a.take(in[0]) || !b.take(in[1]) || (a.scalar.s && b.scalar.s)) return nullptr;
+  int nd;
+  int64_t shape[MAXD];
+  nt_view va, vb;
+  if (!broadcast(a.t, b.t, &nd, shape) || !a.view(nd, shape, &va) || !b.view(nd, shape, &vb)) return nullptr;
+  nt_storage *s = nullptr;
+  Ref out(fresh(checked(fns[op - OP_ADD](&va, &vb, &s), s), nd, shape));
+  if (recording(in, 2)) {
+    FunctionObj *fn = attach(op, cls, out.p, in, 2);
+    if (op == OP_MUL || op == OP_DIV) save(fn, out.p, {in[0], in[1]});
+  }
+  return out.release();
+}
+
+static PyObject *unary_forward(Op op, PyTypeObject *cls, PyObject *const *in) {
+  static const Fn1 fns[] = {nt_neg, nt_exp, nt_log, nt_sqrt, nt_tanh, nt_sigmoid, nt_relu};
+  if (!is_fast(in[0])) return nullptr;
+  TensorObj *x = T_(in[0]);
+  const nt_view v = view_of(x);
+  nt_storage *s = nullptr;
+  Ref out(fresh(checked(fns[op - OP_NEG](&v, &s), s), x->nd, x->sh));
+  if (recording(in, 1)) {
+    FunctionObj *fn = attach(op, cls, out.p, in, 1);
+    if (op == OP_LOG) save(fn, out.p, {in[0]});
+    else if (op != OP_NEG) save(fn, out.p, {out.p});
+  }
+  return out.release();
+}
+
+static PyObject *pow_forward(PyTypeObject *cls, PyObject *const *in) {
+  if (!is_fast(in[0])) return nullptr;
+  TensorObj *x = T_(in[0]);
+  Ref exponent;
+  nt_scalar e;
+  if (is_tensor(in[1])) {
+    TensorObj *t = T_(in[1]);
+    if (Py_TYPE(in[1]) != G.tensor_type || !t->pyvalue || t->nd != 0 || !is_storage(t->storage) ||
+        storage_of(t)->dtype > NT_FLOAT32 || !scalar_of(t->pyvalue, &e))
+      return nullptr;
+    exponent = Ref(own(in[1]));
+  } else {
+    if (!scalar_of(in[1], &e)) return nullptr;
+    exponent = Ref(to_operand(in[1], x));
+    if (!exponent) throw PyErr{};
+  }
+  e = nt_scalar{2, 0, e.d};
+  const nt_view v = view_of(x);
+  nt_storage *s = nullptr;
+  Ref out(fresh(checked(nt_pow(&v, &e, &s), s), x->nd, x->sh));
+  if (recording(in, 1) || (is_tensor(in[1]) && recording(in + 1, 1))) {
+    FunctionObj *fn = attach(OP_POW, cls, out.p, in, 2);
+    save(fn, out.p, {in[0], exponent.p});
+    fn->e = e.d;
+  }
+  return out.release();
+}
+
+static PyObject *matmul_forward(PyTypeObject *cls, PyObject *const *in) {
+  if (!is_fast(in[0]) || !is_fast(in[1])) return nullptr;
+  TensorObj *a = T_(in[0]), *b = T_(in[1]);
+  const int nd = a->nd;
+  if (nd < 2 || b->nd != nd || a->sh[nd - 1] != b->sh[nd - 2]) return nullptr;
+  int64_t shape[MAXD];
+  for (int d = 0; d < nd - 2; ++d) {
+    if (a->sh[d] != b->sh[d]) return nullptr; // broadcast batch dims: the Python path expands them
+    shape[d] = a->sh[d];
+  }
+  shape[nd - 2] = a->sh[nd - 2];
+  shape[nd - 1] = b->sh[nd - 1];
+  const nt_view va = view_of(a), vb = view_of(b);
+  nt_storage *s = nullptr;
+  Ref out(fresh(checked(nt_matmul(&va, &vb, &s), s), nd, shape));
+  if (recording(in, 2)) save(attach(OP_MATMUL, cls, out.p, in, 2), out.p, {in[0], in[1]});
+  return out.release();
+}
+
+static PyObject *linear_forward(PyTypeObject *cls, PyObject *const *in) {
+  for (int i = 0; i < 3; ++i)
+    if (!is_fast(in[i])) return nullptr;
+  TensorObj *x = T_(in[0]), *w = T_(in[1]), *b = T_(in[2]);
+  if (x->nd != 2 || w->nd != 2 || b->nd != 1 || x->sh[1] != w->sh[0] || b->sh[0] != w->sh[1]) return nullptr;
+  const nt_view vx = view_of(x), vw = view_of(w), vb = view_of(b);
+  const int64_t shape[2] = {x->sh[0], w->sh[1]};
+  nt_storage *s = nullptr;
+  Ref out(fresh(checked(nt_linear(&vx, &vw, &vb, &s), s), 2, shape));
+  if (recording(in, 3)) save(attach(OP_LINEAR, cls, out.p, in, 3), out.p, {in[0], in[1]});
+  return out.release();
+}
+
+// None | int | tuple of ints -> distinct non-negative axes; false: let the Python path decide (and raise)
+static bool axes_of(PyObject *axis, int nd, int64_t *axes, int *n) {
+  *n = 0;
+  if (axis != Py_None) {
+    if (PyLong_CheckExact(axis)) {
+      axes[(*n)++] = PyLong_AsLongLong(axis);
+    } else if (PyTuple_CheckExact(axis)) {
+      if (!parse_dims(axis, axes, n)) return false;
+    } else {
+      return false;
+    }
+  }
+  if (*n == 0) {
+    for (int d = 0; d < nd; ++d) axes[(*n)++] = d;
+    return true;
+  }
+  unsigned seen = 0;
+  for (int i = 0; i < *n; ++i) {
+    if (axes[i] < 0) axes[i] += nd;
+    if (axes[i] < 0 || axes[i] >= nd || (seen >> axes[i] & 1)) return false;
+    seen |= 1u << axes[i];
+  }
+  return true;
+}
+static int kept_shape(const TensorObj *x, const int64_t *axes, int n, bool keepdim, int64_t *shape) {
+  unsigned drop = 0;
+  for (int i = 0; i < n; ++i) drop |= 1u << axes[i];
+  int nd = 0;
+  for (int d = 0; d < x->nd; ++d) {
+    if (!(drop >> d & 1)) shape[nd++] = x->sh[d];
+    else if (keepdim) shape[nd++] = 1;
+  }
+  return nd;
+}
+static PyObject *reduce_forward(Op op, PyTypeObject *cls, PyObject *const *in, Py_ssize_t n) {
+  if (!is_fast(in[0])) return nullptr;
+  TensorObj *x = T_(in[0]);
+  PyObject *axis = n > 1 ? in[1] : Py_None, *keep = n > 2 ? in[2] : Py_False, *dtype = n > 3 ? in[3] : Py_None;
+  if (dtype != Py_None && dtype != G.dtypes[NT_FLOAT32]) return nullptr;
+  const int keepdim = keep == Py_False ? 0 : PyObject_IsTrue(keep);
+  if (keepdim < 0) throw PyErr{};
+  int64_t axes[MAXD], shape[MAXD];
+  int n_axes;
+  if (!axes_of(axis, x->nd, axes, &n_axes)) return nullptr;
+  const int nd = kept_shape(x, axes, n_axes, keepdim != 0, shape);
+  const nt_view v = view_of(x);
+  nt_storage *s = nullptr;
+  int64_t denom = 0;
+  switch (op) {
+  case OP_SUM: checked(nt_sum(&v, axes, n_axes, NT_FLOAT32, &s), s); break;
+  case OP_MEAN:
+    denom = numel(x->nd, x->sh) / numel(nd, shape);
+    if (denom > (int64_t(1) << 24)) return nullptr; // the count is no longer exact in fp32
+    checked(nt_mean_f32(&v, axes, n_axes, float(denom), &s), s);
+    if (!s) return nullptr;
+    break;
+  case OP_MAX: checked(nt_max(&v, axes, n_axes, &s), s); break;
+  default: checked(nt_min(&v, axes, n_axes, &s), s); break;
+  }
+  Ref out(fresh(s, nd, shape));
+  if (recording(in, 1)) {
+    FunctionObj *fn = attach(op, cls, out.p, in, n);
+    fn->n_axes = n_axes;
+    std::copy(axes, axes + n_axes, fn->axes);
+    fn->denom = denom;
+    if (op == OP_MAX || op == OP_MIN) save(fn, out.p, {in[0], out.p});
+  }
+  return out.release();
+}
+
+// The view ops take any tensor of up to MAXD dims: no kernel is involved unless a strided one is reshaped.
+static bool plain(PyObject *o) { return Py_TYPE(o) == G.tensor_type && T_(o)->nd >= 0 && T_(o)->storage; }
+static PyObject *view_result(Op op, PyTypeObject *cls, PyObject *out, PyObject *const *in, Py_ssize_t n) {
+  if (!out) throw PyErr{};
+  Ref holder(out);
+  if (recording(in, 1)) attach(op, cls, out, in, n);
+  return holder.release();
+}
+static PyObject *unchanged(Op op, PyTypeObject *cls, PyObject *const *in, Py_ssize_t n) { // the input itself, as a node of its own
+  return G.grad_enabled ? view_result(op, cls, reinterpret_cast<PyObject *>(alias_of(T_(in[0]))), in, n) : own(in[0]);
+}
+static bool dims_of(PyObject *const *in, Py_ssize_t n, int64_t *dims) {
+  if (n > MAXD) return false;
+  for (Py_ssize_t i = 0; i < n; ++i) {
+    int overflow = 0;
+    if (!PyLong_Check(in[i])) return false;
+    dims[i] = PyLong_AsLongLongAndOverflow(in[i], &overflow);
+    if (overflow) return false;
+  }
+  return true;
+}
+static PyObject *reshape_forward(PyTypeObject *cls, PyObject *const *in, Py_ssize_t n) {
+  int64_t dims[MAXD], st[MAXD];
+  if (!plain(in[0]) || !dims_of(in + 1, n - 1, dims)) return nullptr;
+  TensorObj *x = T_(in[0]);
+  const int nd = int(n - 1);
+  if (numel(nd, dims) != numel(x->nd, x->sh)) return nullptr;
+  for (int d = 0; d < nd; ++d)
+    if (dims[d] < 0) return nullptr;
+  if (nd == x->nd && std::equal(dims, dims + nd, x->sh)) return unchanged(OP_RESHAPE, cls, in, n);
+  if (!dense(x)) return nullptr; // has to be copied
+  int64_t acc = 1;
+  for (int d = nd - 1; d >= 0; --d) {
+    st[d] = acc;
+    acc *= dims[d];
+  }
+  return view_result(OP_RESHAPE, cls, reinterpret_cast<PyObject *>(new_view(x->storage, nd, dims, st, x->offset)), in, n);
+}
+static PyObject *expand_forward(PyTypeObject *cls, PyObject *const *in, Py_ssize_t n) {
+  int64_t dims[MAXD];
+  if (!plain(in[0]) || !is_storage(T_(in[0])->storage) || !dims_of(in + 1, n - 1, dims)) return nullptr;
+  TensorObj *x = T_(in[0]);
+  const int nd = int(n - 1);
+  if (nd == x->nd && std::equal(dims, dims + nd, x->sh)) return unchanged(OP_EXPAND, cls, in, n);
+  nt_view v;
+  if (numel(x->nd, x->sh) == 0 || !expand_view(x, nd, dims, &v)) return nullptr;
+  for (int d = 0; d < nd; ++d)
+    if (dims[d] < 0) return nullptr;
+  return view_result(OP_EXPAND, cls, reinterpret_cast<PyObject *>(new_view(x->storage, nd, v.shape, v.strides, v.offset)), in, n);
+}
+static PyObject *transposed_forward(Op op, PyTypeObject *cls, PyObject *const *in, Py_ssize_t n) {
+  if (!plain(in[0])) return nullptr;
+  TensorObj *x = T_(in[0]);
+  int64_t sh[MAXD], st[MAXD];
+  const int nd = x->nd;
+  if (op == OP_T) {
+    if (n != 1) return nullptr;
+    if (nd < 2) return unchanged(op, cls, in, n);
+    for (int d = 0; d < nd; ++d) {
+      sh[d] = x->sh[nd - 1 - d];
+      st[d] = x->st[nd - 1 - d];
+    }
+  } else {
+    int64_t d01[2];
+    if (n != 3 || !dims_of(in + 1, 2, d01)) return nullptr;
+    if (nd < 2 || d01[0] == d01[1]) return unchanged(op, cls, in, n);
+    for (int i = 0; i < 2; ++i) {
+      if (d01[i] < 0) d01[i] += nd;
+      if (d01[i] < 0 || d01[i] >= nd) return nullptr;
+    }
+    std::copy(x->sh, x->sh + nd, sh);
+    std::copy(x->st, x->st + nd, st);
+    std::swap(sh[d01[0]], sh[d01[1]]);
+    std::swap(st[d01[0]], st[d01[1]]);
+  }
+  return view_result(op, cls, reinterpret_cast<PyObject *>(new_view(x->storage, nd, sh, st, x->offset)), in, n);
+}
+
+PyObject *forward(Op op, PyTypeObject *cls, PyObject *const *in, Py_ssize_t n) {
+  try {
+    switch (op) {
+    case OP_ADD: case OP_SUB: case OP_MUL: case OP_DIV: return n == 2 ? binary_forward(op, cls, in) : nullptr;
+    case OP_MATMUL: return n == 2 ? matmul_forward(cls, in) : nullptr;
+    case OP_LINEAR: return n == 3 ? linear_forward(cls, in) : nullptr;
+    case OP_POW: return n == 2 ? pow_forward(cls, in) : nullptr;
+    case OP_NEG: case OP_EXP: case OP_LOG: case OP_SQRT: case OP_TANH: case OP_SIGMOID: case OP_RELU:
+      return n == 1 ? unary_forward(op, cls, in) : nullptr;
+    case OP_SUM: case OP_MEAN: return n >= 1 && n <= 4 ? reduce_forward(op, cls, in, n) : nullptr;
+    case OP_MAX: case OP_MIN: return n >= 1 && n <= 3 ? reduce_forward(op, cls, in, n) : nullptr;
+    case OP_RESHAPE: return n >= 1 ? reshape_forward(cls, in, n) : nullptr;
+    case OP_EXPAND: return n >= 1 ? expand_forward(cls, in, n) : nullptr;
+    case OP_T: case OP_TRANSPOSE: return n >= 1 ? transposed_forward(op, cls, in, n) : nullptr;
+    default: return nullptr;
+    }
+  } catch (const PyErr &) {
+    return nullptr;
+  }
+}
+
+// =============================================================================================
+// Backward
+static bool need(const FunctionObj *fn, int i) {
+  return i >= PyTuple_GET_SIZE(fn->needs) || PyTuple_GET_ITEM(fn->needs, i) == Py_True;
+}
+// The saved tensors, after the check that none was modified in place; false with an exception set.
+static bool saved_ok(FunctionObj *fn) {
+  for (Py_ssize_t i = 0; i < PyTuple_GET_SIZE(fn->saved); ++i)
+    if (storage_of(T_(PyTuple_GET_ITEM(fn->saved, i)))->version != fn->versions[i]) {
+      PyErr_SetString(PyExc_RuntimeError, "One of the tensors needed for grad computation was modified inplace.");
+      throw PyErr{};
+    }
+  return true;
+}
+static TensorObj *saved(FunctionObj *fn, int i) { return T_(PyTuple_GET_ITEM(fn->saved, i)); }
+static TensorObj *input(FunctionObj *fn, int i) { return T_(PyTuple_GET_ITEM(fn->inputs, i)); }
+
+// x summed over its broadcast axes down to `shape`: the leading ones first, then the kept ones of extent 1
+static Ref unbroadcast(TensorObj *x, int nd, const int64_t *shape) {
+  Ref cur(own(reinterpret_cast<PyObject *>(x)));
+  const int lead = x->nd - nd;
+  int64_t axes[MAXD];
+  if (lead > 0) {
+    for (int d = 0; d < lead; ++d) axes[d] = d;
+    const nt_view v = view_of(x);
+    nt_storage *s = nullptr;
+    cur = Ref(fresh(checked(nt_sum(&v, axes, lead, NT_FLOAT32, &s), s), nd, x->sh + lead));
+  }
+  TensorObj *t = T_(cur.p);
+  int n = 0;
+  int64_t kept[MAXD];
+  for (int d = 0; d < nd; ++d) {
+    kept[d] = t->sh[d];
+    if (t->sh[d] != 1 && shape[d] == 1) {
+      axes[n++] = d;
+      kept[d] = 1;
+    }
+  }
+  if (n) {
+    const nt_view v = view_of(t);
+    nt_storage *s = nullptr;
+    cur = Ref(fresh(checked(nt_sum(&v, axes, n, NT_FLOAT32, &s), s), nd, kept));
+  }
+  return cur;
+}
+static Ref unbroadcast(TensorObj *x, const TensorObj *like) { return unbroadcast(x, like->nd, like->sh); }
+static Ref unbroadcast(Ref x, const TensorObj *like) { return unbroadcast(T_(x.p), like->nd, like->sh); }
+
+// the gradient of a reduction as a stride-0 view of the input's shape: no kernel, no bytes
+static PyObject *expand_back(const TensorObj *g, const TensorObj *x, const FunctionObj *fn) {
+  unsigned drop = 0;
+  for (int i = 0; i < fn->n_axes; ++i) drop |= 1u << fn->axes[i];
+  const bool keepdim = g->nd == x->nd;
+  int64_t st[MAXD];
+  int k = 0;
+  for (int d = 0; d < x->nd; ++d) {
+    if (drop >> d & 1) {
+      st[d] = 0;
+      k += keepdim;
+    } else {
+      st[d] = g->st[k++];
+    }
+  }
+  PyObject *t = reinterpret_cast<PyObject *>(new_view(g->storage, x->nd, x->sh, st, g->offset));
+  if (!t) throw PyErr{};
+  return t;
+}
+static nt_view expanded(const TensorObj *t, int nd, const int64_t *shape) {
+  nt_view v;
+  if (!expand_view(t, nd, shape, &v)) {
+    PyErr_SetString(PyExc_RuntimeError, "backward: a saved tensor does not broadcast to the gradient's shape.");
+    throw PyErr{};
+  }
+  return v;
+}
+static Ref elementwise(Fn2 f, const nt_view &a, const nt_view &b, const TensorObj *like) {
+  nt_storage *s = nullptr;
+  return Ref(fresh(checked(f(&a, &b, &s), s), like->nd, like->sh));
+}
+static nt_view transposed(const TensorObj *t) { // the last two dims swapped
+  nt_view v = view_of(t);
+  std::swap(v.shape[t->nd - 1], v.shape[t->nd - 2]);
+  std::swap(v.strides[t->nd - 1], v.strides[t->nd - 2]);
+  return v;
+}
+
+// A product's operand as it took part: a scalar tensor keeps its own dtype in the graph, so only fast ones qualify.
+static bool fast_pair(FunctionObj *fn) {
+  return is_fast(reinterpret_cast<PyObject *>(saved(fn, 0))) && is_fast(reinterpret_cast<PyObject *>(saved(fn, 1)));
+}
+
+static bool backward_op(FunctionObj *fn, TensorObj *g, PyObject **out, int *n_out) {
+  switch (fn->op) {
+  case OP_ADD:
+  case OP_SUB: {
+    *n_out = 2;
+    if (need(fn, 0)) out[0] = unbroadcast(g, input(fn, 0)).release();
+    if (need(fn, 1)) {
+      if (fn->op == OP_ADD) {
+        out[1] = unbroadcast(g, input(fn, 1)).release();
+      } else {
+        const nt_view v = view_of(g);
+        nt_storage *s = nullptr;
+        Ref neg(fresh(checked(nt_neg(&v, &s), s), g->nd, g->sh));
+        out[1] = unbroadcast(std::move(neg), input(fn, 1)).release();
+      }
+    }
+    return true;
+  }
+  case OP_MUL:
+  case OP_DIV: {
+    const bool mul = fn->op == OP_MUL;
+    *n_out = 2;
+    saved_ok(fn);
+    TensorObj *x1 = saved(fn, 0), *x2 = saved(fn, 1);
+    const nt_view vg = view_of(g);
+    const bool both = need(fn, 0) && need(fn, 1);
+    if (both && !fast_pair(fn)) return false;
+    if (both && same_shape(g, x1) && same_shape(g, x2)) { // one pass when all three are dense
+      const nt_view v1 = view_of(x1), v2 = view_of(x2);
+      nt_storage *s1 = nullptr, *s2 = nullptr;
+      checked((mul ? nt_mul_backward : nt_div_backward)(&vg, &v1, &v2, &s1, &s2), s1);
+      if (s1) {
+        PyObject *first = reinterpret_cast<PyObject *>(new_tensor(s1, g->nd, g->sh));
+        PyObject *second = reinterpret_cast<PyObject *>(new_tensor(s2, g->nd, g->sh));
+        out[0] = first;
+        out[1] = second;
+        if (!first || !second) throw PyErr{};
+        return true;
+      }
+    }
+    Operand o1, o2;
+    nt_view v1, v2;
+    if (!o1.take(reinterpret_cast<PyObject *>(x1)) || !o2.take(reinterpret_cast<PyObject *>(x2)) ||
+        !o1.view(g->nd, g->sh, &v1) || !o2.view(g->nd, g->sh, &v2))
+      return false;
+    if (need(fn, 0)) out[0] = unbroadcast(mul ? elementwise(nt_multiply, v2, vg, g) : elementwise(nt_divide, vg, v2, g), x1).release();
+    if (need(fn, 1)) {
+      if (mul) {
+        out[1] = unbroadcast(elementwise(nt_multiply, v1, vg, g), x2).release();
+      } else {
+        if (!fast_pair(fn)) return false;
+        nt_storage *s = nullptr;
+        out[1] = unbroadcast(Ref(fresh(checked(nt_div_backward_x2(&vg, &v1, &v2, &s), s), g->nd, g->sh)), x2).release();
+      }
+    }
+    return true;
+  }
+  case OP_MATMUL:
+  case OP_LINEAR: {
+    saved_ok(fn);
+    TensorObj *a = saved(fn, 0), *b = saved(fn, 1);
+    if (g->nd != a->nd) return false;
+    *n_out = fn->op == OP_LINEAR ? 3 : 2;
+    const nt_view vg = view_of(g), vat = transposed(a), vbt = transposed(b);
+    if (need(fn, 0) && need(fn, 1) && g->nd == 2) {
+      // both gradients in one call: the second product may start on the SMs the first one's last wave leaves idle
+      nt_storage *s1 = nullptr, *s2 = nullptr;
+      checked(nt_matmul_pair(&vg, &vbt, &vat, &vg, &s1, &s2), s1);
+      out[0] = reinterpret_cast<PyObject *>(new_tensor(s1, a->nd, a->sh));
+      out[1] = reinterpret_cast<PyObject *>(new_tensor(s2, b->nd, b->sh));
+      if (!out[0] || !out[1]) throw PyErr{};
+    } else {
+      if (need(fn, 0)) out[0] = elementwise(nt_matmul, vg, vbt, a).release();
+      if (need(fn, 1)) out[1] = elementwise(nt_matmul, vat, vg, b).release();
+    }
+    if (fn->op == OP_LINEAR && need(fn, 2)) out[2] = unbroadcast(g, input(fn, 2)).release();
+    return true;
+  }
+  case OP_NEG: {
+    *n_out = 1;
+    const nt_view v = view_of(g);
+    nt_storage *s = nullptr;
+    out[0] = fresh(checked(nt_neg(&v, &s), s), g->nd, g->sh);
+    return true;
+  }
+  case OP_EXP: case OP_LOG: case OP_SQRT: case OP_TANH: case OP_SIGMOID: case OP_RELU: {
+    static const Fn2 fns[] = {nt_exp_backward, nt_log_backward, nt_sqrt_backward, nt_tanh_backward, nt_sigmoid_backward, nt_relu_backward};
+    saved_ok(fn);
+    TensorObj *x = saved(fn, 0);
+    if (!same_shape(g, x)) return false;
+    *n_out = 1;
+    out[0] = elementwise(fns[fn->op - OP_EXP], view_of(g), view_of(x), g).release();
+    return true;
+  }
+  case OP_POW: {
+    saved_ok(fn);
+    TensorObj *x = saved(fn, 0);
+    if (!same_shape(g, x)) return false;
+    *n_out = 1;
+    const nt_view vg = view_of(g), vx = view_of(x);
+    nt_storage *s = nullptr;
+    out[0] = fresh(checked(nt_pow_backward(&vg, &vx, float(fn->e), &s), s), g->nd, g->sh);
+    return true;
+  }
+  case OP_SUM:
+  case OP_MEAN:
+  case OP_MAX:
+  case OP_MIN: {
+    TensorObj *x = input(fn, 0);
+    *n_out = 1;
+    if (x->nd == 0) {
+      out[0] = own(reinterpret_cast<PyObject *>(g));
+      return true;
+    }
+    if (fn->op == OP_SUM) {
+      out[0] = expand_back(g, x, fn);
+    } else if (fn->op == OP_MEAN) {
+      // the kept elements are divided by the count once, then expanded
+      Held count(constant(nt_scalar{1, fn->denom, double(fn->denom)}));
+      nt_view c{};
+      c.storage = count.s;
+      c.ndim = g->nd;
+      std::copy(g->sh, g->sh + g->nd, c.shape);
+      Ref q(elementwise(nt_divide, view_of(g), c, g));
+      out[0] = expand_back(T_(q.p), x, fn);
+    } else {
+      saved_ok(fn);
+      Ref ge(expand_back(g, x, fn)), me(expand_back(saved(fn, 1), x, fn));
+      const nt_view vg = view_of(T_(ge.p)), vx = view_of(saved(fn, 0)), vm = view_of(T_(me.p));
+      nt_storage *s = nullptr;
+      out[0] = fresh(checked(nt_extremum_backward(&vg, &vx, &vm, fn->axes, fn->n_axes, &s), s), x->nd, x->sh);
+    }
+    return true;
+  }
+  case OP_RESHAPE: {
+    TensorObj *x = input(fn, 0);
+    if (!dense(g)) return false;
+    int64_t st[MAXD], acc = 1;
+    for (int d = x->nd - 1; d >= 0; --d) {
+      st[d] = acc;
+      acc *= x->sh[d];
+    }
+    *n_out = 1;
+    out[0] = reinterpret_cast<PyObject *>(new_view(g->storage, x->nd, x->sh, st, g->offset));
+    if (!out[0]) throw PyErr{};
+    return true;
+  }
+  case OP_EXPAND:
+    *n_out = 1;
+    out[0] = unbroadcast(g, input(fn, 0)).release();
+    return true;
+  case OP_T:
+  case OP_TRANSPOSE: {
+    const int nd = g->nd;
+    int64_t sh[MAXD], st[MAXD], d01[2] = {0, 0};
+    if (fn->op == OP_TRANSPOSE && !dims_of(&PyTuple_GET_ITEM(fn->inputs, 1), 2, d01)) return false;
+    for (int d = 0; d < nd; ++d) {
+      const int from = fn->op == OP_T && nd >= 2 ? nd - 1 - d : d;
+      sh[d] = g->sh[from];
+      st[d] = g->st[from];
+    }
+    if (fn->op == OP_TRANSPOSE && nd >= 2) {
+      for (int64_t &d : d01) d += d < 0 ? nd : 0;
+      std::swap(sh[d01[0]], sh[d01[1]]);
+      std::swap(st[d01[0]], st[d01[1]]);
+    }
+    *n_out = 1;
+    out[0] = reinterpret_cast<PyObject *>(new_view(g->storage, nd, sh, st, g->offset));
+    if (!out[0]) throw PyErr{};
+    return true;
+  }
+  default: return false;
+  }
+}
+
+bool backward_fast(FunctionObj *fn, TensorObj *g, PyObject **out, int *n_out) {
+  if (fn->op == OP_NONE || !is_fast(reinterpret_cast<PyObject *>(g))) return false;
+  out[0] = out[1] = out[2] = nullptr;
+  bool ok = false;
+  try {
+    ok = backward_op(fn, g, out, n_out);
+  } catch (const PyErr &) {
+  }
+  if (!ok)
+    for (int i = 0; i < 3; ++i) Py_CLEAR(out[i]);
+  return ok;
+}
+
+TensorObj *add_tensors(PyObject *a, PyObject *b) {
+  if (!is_fast(a) || !is_fast(b) || !same_shape(T_(a), T_(b))) return nullptr;
+  const nt_view va = view_of(T_(a)), vb = view_of(T_(b));
+  nt_storage *s = nullptr;
+  const int rc = nt_add(&va, &vb, &s);
+  if (rc) {
+    raise_status(rc);
+    return nullptr;
+  }
+  return new_tensor(s, T_(a)->nd, T_(a)->sh);
+}
+
+} // namespace eng

@@ -11,10 +11,10 @@ from __future__ import annotations
 import math
 from typing import Any, Sequence
 
-from . import _C, compute_on_device, rand, zeros
+from . import _engine, compute_on_device, rand, zeros
 from .autograd import LinearOp, ReluOp, TanhOp, no_grad
 from .tensor import Tensor
-from ._C import Device, Dtype
+from ._C import Device
 
 
 class Module:
@@ -137,12 +137,9 @@ class GradientDescent(Optimizer):
                 continue
             if p.grad is None:
                 raise RuntimeError("Gradients not set, did you call backward?")
-            g = p.grad
-            if (p.dtype == Dtype.Float32 and g.dtype == Dtype.Float32 and p.device == Device.Cuda
-                    and g.shape == p.shape):
-                _C.sgd_update(p._C_view, g._C_view, self._lr, self._grad_scale)
-            else:
+            if not _engine.sgd_update(p, self._lr, self._grad_scale):
                 with no_grad():
+                    g = p.grad
                     if self._grad_scale != 1.0:
                         g = g * self._grad_scale
                     p -= g * self._lr

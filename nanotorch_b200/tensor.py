@@ -3,7 +3,8 @@
 Host-side mirror of the reference's ``nanotorch.Tensor`` for the op-kernel hot path
 (src/nanotorch/core.py:47-139, 255-334, 489-563): same view model (strides and offset in elements,
 stride 0 = broadcast, views never copy), same attribute and method names, same error classes.
-Everything numeric happens in ``_C`` (libnt_b200.so); this file only does bookkeeping.
+Everything numeric happens in ``_C`` (libnt_b200.so); this file only does bookkeeping.  The fields, view
+construction, operators and ``backward`` live in the native base class (csrc/engine/objects.cpp).
 
 Index-array and mask indexing (src/nanotorch/core.py:172-254, 666-772) follows the reference's plan
 (the numpy rule for where the index dimensions land) and runs as device gather/scatter kernels; the
@@ -15,7 +16,7 @@ from __future__ import annotations
 import math
 from typing import Any, Sequence
 
-from . import _C
+from . import _C, _engine
 from ._C import Device, Dtype
 
 Shape = tuple[int, ...]
@@ -109,10 +110,10 @@ def _flatten_nested(data, max_depth: int = 32):
     return tuple(shape), flat, (auto if auto is not None else Dtype.Float32)
 
 
-class Tensor:
+class Tensor(_engine.TensorBase):
     """Typed n-dimensional array with autograd; see the module docstring."""
 
-    __slots__ = ("_storage", "_shape", "_strides", "_offset", "_requires_grad", "_grad", "_grad_fn", "_pyvalue")
+    __slots__ = ()
 
     def __init__(self, data, *, dtype: Dtype | None = None, requires_grad: bool = False,
                  device: Device | str = Device.Cpu):
@@ -137,31 +138,6 @@ class Tensor:
         self._pyvalue = data if (shape == () and dtype is None) else None
 
     # ------------------------------------------------------------------ constructors
-    @classmethod
-    def _new_view(cls, storage: _C.Storage, shape: Shape, strides: Shape | None, offset: int | None) -> "Tensor":
-        shape = tuple(shape)
-        strides = contiguous_strides(shape) if strides is None else tuple(strides)
-        offset = 0 if offset is None else offset
-        if math.prod(shape) > 0:
-            lo = offset + sum((s - 1) * st for s, st in zip(shape, strides) if st < 0)
-            hi = offset + sum((s - 1) * st for s, st in zip(shape, strides) if st > 0)
-            if lo < 0 or hi >= storage.size:
-                raise IndexError(f"View max index {hi} exceeds storage capacity {storage.size}.")
-        t = object.__new__(cls)
-        t._storage = storage
-        t._shape = shape
-        t._strides = strides
-        t._offset = offset
-        t._requires_grad = False
-        t._grad = None
-        t._grad_fn = None
-        t._pyvalue = None
-        return t
-
-    @classmethod
-    def _new_contiguous(cls, storage: _C.Storage, shape: Shape) -> "Tensor":
-        return cls._new_view(storage, shape, None, None)
-
     @classmethod
     def _scalar(cls, value, dtype: Dtype, device: Device) -> "Tensor":
         """0-d tensor: on Cuda a constant the kernels take as an argument, no copy and no launch."""
@@ -209,20 +185,6 @@ class Tensor:
             src._storage.download(out.ctypes.data, out.nbytes)
         return out
 
-    # ------------------------------------------------------------------ metadata
-    dtype = property(lambda self: self._storage.dtype)
-    shape = property(lambda self: self._shape)
-    ndim = property(lambda self: len(self._shape))
-    numel = property(lambda self: math.prod(self._shape))
-    is_empty = property(lambda self: math.prod(self._shape) == 0)
-    storage = property(lambda self: self._storage)
-    strides = property(lambda self: (self._strides, self._offset))
-    device = property(lambda self: self._storage.device)
-    version = property(lambda self: self._storage.version)
-
-    def __len__(self) -> int:
-        return self._shape[0] if self._shape else 0
-
     def __repr__(self) -> str:
         """The reference's format (src/nanotorch/core.py:141-164): values for 0-d, 1-D (first and last three
         beyond 7 elements) and 2-D tensors (first and last two rows beyond 5), a summary line otherwise.
@@ -243,16 +205,6 @@ class Tensor:
             lines = ["..." if i is None else compact(self[i]) for i in rows]
             return "nt.Tensor(" + ("\n" + " " * 10).join(lines) + ")"
         return f"nt.Tensor(shape={self.shape}, {self.numel} x <{self.dtype.name}>, d: {self.device.name})"
-
-    @property
-    def T(self) -> "Tensor":
-        from .autograd import TOp
-
-        return TOp.apply(self)
-
-    @property
-    def _C_view(self) -> _C.TensorView:
-        return _C.TensorView(self._storage, self._shape, self._strides, self._offset)
 
     # ------------------------------------------------------------------ moves and copies
     def to(self, target: Dtype | Device | str) -> "Tensor":
@@ -325,19 +277,10 @@ class Tensor:
             raise RuntimeError("Tensor on device, call .cpu() first.")
         return memoryview(self._storage)[self._offset]
 
-    def _is_contiguous(self, full_span: bool = False) -> bool:
-        dense = self._strides == contiguous_strides(self._shape)
-        if not full_span:
-            return dense
-        return dense and self._offset == 0 and self.numel == self._storage.size
-
     def _to_contiguous(self, force: bool = False) -> "Tensor":
         if not force and self._is_contiguous():
             return self
         return Tensor._new_contiguous(_C.clone_contiguous_view_from(self._C_view), self._shape)
-
-    def _alias(self) -> "Tensor":
-        return Tensor._new_view(self._storage, self._shape, self._strides, self._offset)
 
     # ------------------------------------------------------------------ indexing
     def _basic_index(self, index) -> "tuple[Tensor, tuple | None]":
@@ -426,53 +369,10 @@ class Tensor:
             fancy_dims_data=[t._C_view for t in plan.fancy_dims_data], out_axis_is_fancy=plan.out_axis_is_fancy,
             out_axis_target=plan.out_axis_target, checked=plan.checked, unique=plan.unique)
 
-    # ------------------------------------------------------------------ autograd
-    @property
-    def requires_grad(self) -> bool:
-        return self._requires_grad or self._grad_fn is not None
-
-    @property
-    def is_leaf(self) -> bool:
-        return self._grad_fn is None
-
-    @property
-    def grad(self) -> "Tensor | None":
-        return self._grad
-
-    @property
-    def grad_fn(self):
-        return self._grad_fn
-
-    def attach_grad_fn(self, grad_fn) -> None:
-        self._grad_fn = grad_fn
-
-    def zero_grad(self) -> None:
-        self._grad = None
-
-    def enable_grad(self) -> None:
-        """Enables gradient tracking after construction.  Unlike the constructor this does not look at
-        the dtype, as in the reference (src/nanotorch/core.py:536-538; its tests call
-        ``arange(60, requires_grad=True)`` on an Int64 range)."""
-        self._requires_grad = True
-
-    def backward(self) -> None:
-        """Backpropagate from a one-element tensor through the recorded graph."""
-        if not self.requires_grad:
-            raise RuntimeError(
-                "Cannot call .backward() on a tensor that does not require grad and does not have a grad_fn.")
-        if self.numel != 1:
-            raise RuntimeError(f"Cannot call .backward() on a non-scalar tensor of shape {self.shape}")
-        seed = Tensor._scalar(1.0, self.dtype, self.device)
-        if self.shape != ():
-            seed = seed.reshape(*self.shape)
-        self._grad = seed
-        if not self.is_leaf:
-            from .autograd import run_backward
-
-            run_backward(self)
-
     __hash__ = None  # elementwise __eq__
 
+
+_engine.register_tensor(Tensor)
 
 # what the operators accept on either side (src/nanotorch/core.py: TensorLike)
 TensorLike = Tensor | float | int | bool | list

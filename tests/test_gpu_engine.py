@@ -1,0 +1,68 @@
+"""The native apply / backward sweep against the Python op classes they restate: same bits, forward and gradients.
+A subclass of an op class is not the registered class, so it takes the Python forward and backward."""
+
+import gc
+
+import numpy as np
+import pytest
+
+from tests.util import bits
+
+pytestmark = pytest.mark.gpu
+
+CASES = [
+    ("AddOp", ((5, 7), (5, 7))), ("AddOp", ((5, 7), (7,))), ("SubOp", ((5, 1), (1, 7))), ("MulOp", ((4, 8), (4, 8))),
+    ("MulOp", ((3, 5, 7), (5, 1))), ("TrueDivOp", ((4, 8), (4, 8))), ("TrueDivOp", ((5, 7), (7,))),
+    ("MatmulOp", ((9, 17), (17, 5))), ("MatmulOp", ((3, 9, 17), (3, 17, 5))), ("LinearOp", ((9, 17), (17, 5), (5,))),
+    *[(name, ((6, 11),)) for name in ("NegOp", "ExpOp", "LogOp", "SqrtOp", "TanhOp", "SigmoidOp", "ReluOp", "SumOp",
+                                      "MeanOp", "MaxOp", "MinOp", "TOp")],
+    ("PowOp", ((6, 11),), 3), ("PowOp", ((6, 11),), -1.5), ("SumOp", ((6, 11),), (0,), True), ("MeanOp", ((6, 11),), -1),
+    ("MaxOp", ((2, 3, 4),), 1, True), ("MinOp", ((6, 11),), 0), ("ReshapeOp", ((6, 4),), 3, 8),
+    ("ExpandOp", ((6, 1),), 2, 6, 5), ("TransposeOp", ((2, 3, 4),), 0, -1),
+]
+
+
+@pytest.mark.parametrize("case", CASES, ids=lambda c: f"{c[0]}-{'x'.join(map(str, c[1]))}-{c[2:]}")
+def test_native_path_has_the_bits_of_the_op_classes(nt, case):
+    name, shapes, extra = case[0], case[1], case[2:]
+    native = getattr(__import__("nanotorch_b200.autograd", fromlist=[name]), name)
+    python = type(name + "Python", (native,), {})
+    rng = np.random.default_rng(3)
+    data = [rng.uniform(0.5, 2, s).astype(np.float32) for s in shapes]
+    got = []
+    for cls in (native, python):
+        leaves = [nt.Tensor.from_numpy(d, "cuda", requires_grad=True) for d in data]
+        y = cls.apply(*leaves, *extra)
+        w = nt.Tensor.from_numpy(np.random.default_rng(4).standard_normal(y.shape).astype(np.float32), "cuda")
+        assert type(y.grad_fn) is cls and y.grad_fn.needs_input_grad[:len(leaves)] == (True,) * len(leaves)
+        (y * w).sum().backward()
+        got.append([y.numpy()] + [t.grad.numpy() for t in leaves])
+    for a, b in zip(*got):
+        assert a.shape == b.shape and np.array_equal(bits(a), bits(b))
+
+
+def test_results_are_freed_without_the_cycle_collector(nt):
+    """A node that saves its own result must not keep it alive: memory comes back by reference count alone."""
+    x = nt.Tensor.from_numpy(np.ones((64, 64), np.float32), "cuda", requires_grad=True)
+    nt.tanh(x).max(axis=0).exp().sum().backward()
+    x.zero_grad()
+    gc.collect()
+    gc.disable()
+    try:
+        before = nt.cuda.memory_stats()["bytes_in_use"]
+        for _ in range(3):
+            nt.tanh(x).max(axis=0).exp().sum().backward()
+            x.zero_grad()
+        assert nt.cuda.memory_stats()["bytes_in_use"] == before
+    finally:
+        gc.enable()
+
+
+def test_saved_tensor_modified_in_place_is_refused(nt):
+    x = nt.Tensor.from_numpy(np.ones((4, 4), np.float32), "cuda", requires_grad=True)
+    y = x * 2
+    z = y * y
+    with nt.no_grad():
+        y += 1
+    with pytest.raises(RuntimeError, match="modified inplace"):
+        z.sum().backward()
