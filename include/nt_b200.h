@@ -234,9 +234,10 @@ int nt_linear(const nt_view *x, const nt_view *w, const nt_view *bias, nt_storag
 int nt_set_matmul_mode(int mode);
 int nt_get_matmul_mode(void);
 /* In modes 1 and 3 a product of at most this many multiply-adds (batch*M*N*K, default 2^21) takes the
- * exact FP32 kernel of mode 0 instead: that small, the tensor-core path's operand-split launches cost more
- * than they save, and tiny products keep the accuracy of the reference's CUDA kernels.  0 sends every fp32
- * product to the tensor cores. */
+ * exact FP32 kernels instead: tiny products keep the accuracy of the reference's CUDA kernels.  (There a
+ * product may be split along k, its parts added in a fixed order; modes 0 and 2 are never split.)  Above it,
+ * mode 1 picks between the plane-fed kernel and one that splits the operands itself, by expected time; the
+ * bits are the same.  0 sends every fp32 product through the planes. */
 /* Mode 1 splits each fp32 operand into two TF32 planes (hi, lo) before the product.  natural != 0 (default):
  * the planes keep the operand's own row-major order whichever of its two matrix dims has unit stride -- the
  * kernel reads them K-major or MN-major -- so no operand is transposed on the way.  cached != 0 (default): the
@@ -281,6 +282,12 @@ int nt_matmul_pair(const nt_view *a1, const nt_view *b1, const nt_view *a2, cons
                    nt_storage **out2);
 int nt_set_matmul_pair_overlap(int on);
 int nt_set_matmul_tc_min_macs(int64_t macs);
+/* on != 0: mode-1 products of this thread may also run on the CUDA cores in exact FP32, where that is expected to be
+ * faster; returns the previous setting (default 0).  A product's sum is then rounded in another order than on the
+ * tensor cores -- at no lower accuracy -- so the host layer allows it where no later decision hangs on the last bit:
+ * for gradients and for products outside a recorded graph, not for a recorded forward product, whose values decide
+ * the side of a ReLU's kink or which element is an extremum. */
+int nt_matmul_allow_reorder(int on);
 int64_t nt_get_matmul_tc_min_macs(void);
 
 /* ------------------------------------------------------------------ in-place (src/cpp/ops/inplace_ops.cu:75-79); bump the version */

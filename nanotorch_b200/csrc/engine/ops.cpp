@@ -342,6 +342,13 @@ static PyObject *pow_forward(PyTypeObject *cls, PyObject *const *in) {
   return out.release();
 }
 
+// Products whose last bit decides nothing may be summed in any order (nt_matmul_allow_reorder).
+struct Reorder {
+  int was;
+  explicit Reorder(bool on) : was(nt_matmul_allow_reorder(on)) {}
+  ~Reorder() { nt_matmul_allow_reorder(was); }
+};
+
 static PyObject *matmul_forward(PyTypeObject *cls, PyObject *const *in) {
   if (!is_fast(in[0]) || !is_fast(in[1])) return nullptr;
   TensorObj *a = T_(in[0]), *b = T_(in[1]);
@@ -355,6 +362,7 @@ static PyObject *matmul_forward(PyTypeObject *cls, PyObject *const *in) {
   shape[nd - 2] = a->sh[nd - 2];
   shape[nd - 1] = b->sh[nd - 1];
   const nt_view va = view_of(a), vb = view_of(b);
+  const Reorder reorder(!recording(in, 2));
   nt_storage *s = nullptr;
   Ref out(fresh(checked(nt_matmul(&va, &vb, &s), s), nd, shape));
   if (recording(in, 2)) save(attach(OP_MATMUL, cls, out.p, in, 2), out.p, {in[0], in[1]});
@@ -368,6 +376,7 @@ static PyObject *linear_forward(PyTypeObject *cls, PyObject *const *in) {
   if (x->nd != 2 || w->nd != 2 || b->nd != 1 || x->sh[1] != w->sh[0] || b->sh[0] != w->sh[1]) return nullptr;
   const nt_view vx = view_of(x), vw = view_of(w), vb = view_of(b);
   const int64_t shape[2] = {x->sh[0], w->sh[1]};
+  const Reorder reorder(!recording(in, 3));
   nt_storage *s = nullptr;
   Ref out(fresh(checked(nt_linear(&vx, &vw, &vb, &s), s), 2, shape));
   if (recording(in, 3)) save(attach(OP_LINEAR, cls, out.p, in, 3), out.p, {in[0], in[1]});
@@ -696,6 +705,7 @@ static bool backward_op(FunctionObj *fn, TensorObj *g, PyObject **out, int *n_ou
     saved_ok(fn);
     TensorObj *a = saved(fn, 0), *b = saved(fn, 1);
     if (g->nd != a->nd) return false;
+    const Reorder reorder(true);
     *n_out = fn->op == OP_LINEAR ? 3 : 2;
     const nt_view vg = view_of(g), vat = transposed(a), vbt = transposed(b);
     if (need(fn, 0) && need(fn, 1) && g->nd == 2) {

@@ -33,6 +33,7 @@
 #include <mutex>
 #include <unordered_map>
 
+#include "gemm_common.cuh"
 #include "nt_core.cuh"
 #include "tf32_split.cuh"
 #include "tma.cuh"
@@ -134,10 +135,6 @@ __global__ void __launch_bounds__(256) split_pack(SplitArgs a) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// PTX wrappers (the mbarrier and TMA ones are in tma.cuh)
-__device__ __forceinline__ void tcgen05_fence_before() { asm volatile("tcgen05.fence::before_thread_sync;" ::: "memory"); }
-__device__ __forceinline__ void tcgen05_fence_after() { asm volatile("tcgen05.fence::after_thread_sync;" ::: "memory"); }
-
 // K-major operand tile in the 64-byte swizzle layout that TMA wrote: rows of 64 bytes, groups of 8
 // rows (512 bytes) back to back.  Fields: start address >> 4 in bits [0,14); leading byte offset >> 4
 // in [16,30) (unused for this layout, set to 1); stride byte offset >> 4 in [32,46) = 512 bytes between
@@ -170,20 +167,9 @@ __device__ __forceinline__ uint64_t umma_desc_mn_sw128(uint32_t smem_addr, uint3
 // [10,13); A and B K-major (0) in bits 15, 16; N >> 3 in [17,23); M >> 4 in [24,29).
 constexpr uint32_t TC_IDESC = (1u << 4) | (2u << 7) | (2u << 10) | (uint32_t(TC_BN >> 3) << 17) | (uint32_t(TC_BM >> 4) << 24);
 
-__device__ __forceinline__ void umma_tf32_idesc(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t idesc, uint32_t accumulate) {
-  asm volatile("{\n\t.reg .pred p;\n\t"
-               "setp.ne.b32 p, %4, 0;\n\t"
-               "tcgen05.mma.cta_group::1.kind::tf32 [%0], %1, %2, %3, p;\n\t}"
-               ::"r"(tmem_d), "l"(adesc), "l"(bdesc), "r"(idesc), "r"(accumulate)
-               : "memory");
-}
 __device__ __forceinline__ void umma_tf32(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t accumulate) {
   umma_tf32_idesc(tmem_d, adesc, bdesc, TC_IDESC, accumulate);
 }
-__device__ __forceinline__ void umma_commit(uint32_t bar) {
-  asm volatile("tcgen05.commit.cta_group::1.mbarrier::arrive::one.shared::cluster.b64 [%0];" ::"r"(bar) : "memory");
-}
-
 struct TcArgs {
   float *C;
   int64_t M, N;
@@ -403,20 +389,7 @@ gemm_3xtf32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
 // tcgen05.ld and add it -- round-to-nearest -- into running sums they keep in registers (128 per
 // thread).  The result has the error of an ordinary fp32 summation (2e-6 of max|C| at K = 4096 and 16384;
 // chains of 128 measured 1e-6 at 3 % more time, one chain per output 1e-5 .. 4e-5).
-constexpr int TC_PERIOD_KB = 16; // k-blocks (of TC_BK = 16) per accumulation chain
-
-__device__ __forceinline__ void tmem_ld32(uint32_t taddr, uint32_t (&v)[32]) {
-  asm volatile(
-      "tcgen05.ld.sync.aligned.32x32b.x32.b32 "
-      "{%0, %1, %2, %3, %4, %5, %6, %7, %8, %9, %10, %11, %12, %13, %14, %15, "
-      "%16, %17, %18, %19, %20, %21, %22, %23, %24, %25, %26, %27, %28, %29, %30, %31}, [%32];"
-      : "=r"(v[0]), "=r"(v[1]), "=r"(v[2]), "=r"(v[3]), "=r"(v[4]), "=r"(v[5]), "=r"(v[6]), "=r"(v[7]),
-        "=r"(v[8]), "=r"(v[9]), "=r"(v[10]), "=r"(v[11]), "=r"(v[12]), "=r"(v[13]), "=r"(v[14]), "=r"(v[15]),
-        "=r"(v[16]), "=r"(v[17]), "=r"(v[18]), "=r"(v[19]), "=r"(v[20]), "=r"(v[21]), "=r"(v[22]), "=r"(v[23]),
-        "=r"(v[24]), "=r"(v[25]), "=r"(v[26]), "=r"(v[27]), "=r"(v[28]), "=r"(v[29]), "=r"(v[30]), "=r"(v[31])
-      : "r"(taddr)
-      : "memory");
-}
+constexpr int TC_PERIOD_KB = TC_PERIOD / TC_BK; // k-blocks per accumulation chain
 
 // A_MN / B_MN: the operand's planes keep the source tensor's own row-major order and the contraction
 // index k runs down the rows (A seen as its transpose, B as stored): the tile arrives through a 4-D
@@ -1143,6 +1116,32 @@ static int unit_dim(int64_t P, int64_t Q, int64_t s_p, int64_t s_q) {
   return -1;
 }
 
+// CTAs that share an output tile along k, see gemm_3xtf32_natural.
+KSplit gemm_tc_k_split(int64_t batch, int64_t M, int64_t N, int64_t K) {
+  KSplit best;
+  const int64_t tiles = ceil_div(M, TC_BM) * ceil_div(N, TC_BN) * batch, num_kb = ceil_div(K, TC_BK);
+  const int sms = sm_count();
+  const int max_splits = g_tc_max_splits.load(std::memory_order_relaxed);
+  for (int sp = 2; sp <= max_splits && tiles <= TC_MAX_TICKETS; ++sp) {
+    const int per = int(ceil_div(ceil_div(num_kb, int64_t(sp)), int64_t(TC_PERIOD_KB))) * TC_PERIOD_KB;
+    if (per < 2 * TC_PERIOD_KB || int64_t(sp - 1) * per >= num_kb) continue; // at least 512 of k each, none empty
+    if (tiles * sp > sms) break;
+    best.splits = sp;
+    best.kb_per_split = per;
+  }
+  return best;
+}
+
+// Expected time of a product through planes: half a microsecond per 16-deep k-block of a tile, one tile per SM at a time;
+// 11 us around it (pipeline fill, epilogue, one operand split); 4.5 us per part for the finish of a k-split.  Measured, with
+// one split: 256 x 64 x 256 14 us, 784 x 256 x 256 20, 1024 x 512 x 512 26, 1024^3 40, 100 x 2000 x 60 (4 parts) 44.
+double gemm_tc_expected_us(int64_t batch, int64_t M, int64_t N, int64_t K) {
+  const int64_t tiles = ceil_div(M, TC_BM) * ceil_div(N, TC_BN) * batch, num_kb = ceil_div(K, TC_BK);
+  const KSplit ks = gemm_tc_k_split(batch, M, N, K);
+  const double waves = double(ceil_div(tiles * ks.splits, sm_count()));
+  return 11.0 + waves * double(ks.splits > 1 ? ks.kb_per_split : num_kb) * 0.5 + (ks.splits > 1 ? 4.5 * ks.splits : 0.0);
+}
+
 // The promoted-accumulation kernel over natural-layout planes.  Returns false when an operand has no
 // unit-stride matrix dim (the caller then takes the transposing split below).
 bool gemm_3xtf32_natural(nt_storage *sa, int64_t a_off, nt_storage *sb, int64_t b_off, float *C, int64_t batch, int64_t M,
@@ -1192,18 +1191,11 @@ bool gemm_3xtf32_natural(nt_storage *sa, int64_t a_off, nt_storage *sb, int64_t 
     // SMs, 2 waves against 1.75 with four k-quarters) the split costs more than it saves, 10.4 ms per step
     // against 8.3 -- four short pipelines with four epilogues and 134 MB of partial sums per launch.
     size_t part_owned = 0;
-    g.splits = 1;
     {
       const int64_t tiles = tiles_m * tiles_n * batch;
-      const int sms = sm_count();
-      const int max_splits = g_tc_max_splits.load(std::memory_order_relaxed);
-      for (int sp = 2; sp <= max_splits && tiles <= TC_MAX_TICKETS; ++sp) {
-        const int per = int(ceil_div(ceil_div(int64_t(g.num_kb), int64_t(sp)), int64_t(TC_PERIOD_KB))) * TC_PERIOD_KB;
-        if (per < 2 * TC_PERIOD_KB || int64_t(sp - 1) * per >= g.num_kb) continue; // at least 512 of k each, none empty
-        if (tiles * sp > sms) break;
-        g.splits = sp;
-        g.kb_per_split = per;
-      }
+      const KSplit ks = gemm_tc_k_split(batch, M, N, K);
+      g.splits = ks.splits;
+      g.kb_per_split = ks.kb_per_split;
       if (g.splits > 1) {
         g.partials = static_cast<float *>(device_alloc(size_t(tiles) * g.splits * TC_BM * TC_BN * 4, &part_owned));
         g.tickets = g_tickets;

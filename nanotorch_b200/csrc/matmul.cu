@@ -3,18 +3,22 @@
 // fp32 has three modes (nt_set_matmul_mode):
 //   1 (default) 3xTF32 on the tcgen05 tensor cores with promoted accumulation, see gemm_tc.cu;
 //   3           3xTF32 with one accumulation chain per output (1 % faster, 5-20x the rounding bias);
-//   0           exact FP32 on the CUDA cores: 128x128x16 shared-memory tiles, 8x8 register
-//               micro-tiles, register-prefetch double buffering, one FMA per multiply-add,
-//               accumulated in ascending k -- the rounding of the reference's CUDA kernels
-//               (src/cpp/ops/matmul.cu:60-205);
-//   2           same kernel with separate multiply and add roundings: bit for bit the reference's
+//   0           exact FP32 on the CUDA cores (sgemm.cuh), one FMA per multiply-add, accumulated in
+//               ascending k -- the rounding of the reference's CUDA kernels (src/cpp/ops/matmul.cu:60-205);
+//   2           same kernels with separate multiply and add roundings: bit for bit the reference's
 //               CPU triple loop (src/cpp/ops/matmul.cu:21-57).
+// Tiny products of modes 1 and 3 take the exact kernels too, where they may also be split along k; small and middle
+// ones of mode 1 take the tensor-core kernel of gemm_fused.cu.
 // Operand tiles are read straight from the strided views -- vectorised along whichever of the two
 // matrix dims has unit stride -- so the transposed views of MatmulOp.backward
 // (autograd/ops_binary.py:265-266) and N % 4 != 0 never drop to a one-thread-per-output kernel as
 // they do in the reference (src/cpp/ops/matmul.cu:218-233).
 // Other dtypes (Int32/Int64/Float64) use a plain one-output-per-thread kernel.
 #include "nt_core.cuh"
+#include "sgemm.cuh"
+
+#include <algorithm>
+#include <cmath>
 
 namespace ntb {
 
@@ -23,6 +27,11 @@ bool gemm_3xtf32(const float *A, const float *B, float *C, int64_t batch, int64_
                  int64_t a_sb, int64_t a_sm, int64_t a_sk, int64_t b_sb, int64_t b_sk, int64_t b_sn,
                  const float *bias, int64_t bias_stride, bool *bias_done);
 void gemm_tc_set_promoted(bool on);
+double gemm_tc_expected_us(int64_t batch, int64_t M, int64_t N, int64_t K);
+// gemm_fused.cu: mode 1 without planes
+double gemm_fused_expected_us(int64_t batch, int64_t M, int64_t N, int64_t K);
+bool gemm_fused(const float *A, const float *B, float *C, int64_t batch, int64_t M, int64_t N, int64_t K, int64_t a_sb, int64_t a_sm,
+                int64_t a_sk, int64_t b_sb, int64_t b_sk, int64_t b_sn, const float *bias, int64_t bias_stride);
 // mode 1 over natural-layout, cached operand planes; false when an operand has no unit-stride matrix dim
 bool gemm_3xtf32_natural(nt_storage *sa, int64_t a_off, nt_storage *sb, int64_t b_off, float *C, int64_t batch, int64_t M,
                          int64_t N, int64_t K, int64_t a_sb, int64_t a_sm, int64_t a_sk, int64_t b_sb, int64_t b_sk,
@@ -33,207 +42,10 @@ void gemm_tc_pair_role(int role);
 void gemm_tc_set_pair_overlap(bool on);
 void gemm_tc_split_stats(uint64_t *launches, uint64_t *hits);
 static std::atomic<int> g_natural_planes{1};
+static thread_local bool t_reorder = false; // nt_matmul_allow_reorder
 
 static std::atomic<int> g_matmul_mode{1};
 static std::atomic<int64_t> g_tc_min_macs{int64_t(1) << 21}; // batch*M*N*K at or below this: exact FP32 kernel
-
-constexpr int BM = 128, BN = 128, BK = 16;
-
-struct BatchIndex {
-  int ndim;
-  int64_t shape[NT_MAX_DIMS];
-  int64_t a_strides[NT_MAX_DIMS];
-  int64_t b_strides[NT_MAX_DIMS];
-};
-
-enum LoadMode { LOAD_SCALAR = 0, LOAD_VEC_K = 1, LOAD_VEC_MN = 2 };
-
-struct GemmArgs {
-  const float *A, *B;
-  float *C;
-  int64_t M, N, K;
-  int64_t a_sm, a_sk, b_sk, b_sn;
-  BatchIndex batch;
-  int c_vec; // C rows may be written 128 bits at a time
-};
-
-template <int AMODE, int BMODE, bool FUSED_MAD>
-__global__ void __launch_bounds__(256) sgemm_tiled(GemmArgs g) {
-  __shared__ __align__(16) float As[2][BK][BM];
-  __shared__ __align__(16) float Bs[2][BK][BN];
-
-  const int tid = threadIdx.x;
-  const int64_t m0 = int64_t(blockIdx.y) * BM, n0 = int64_t(blockIdx.x) * BN;
-
-  const float *A = g.A, *B = g.B;
-  {
-    int64_t lin = blockIdx.z;
-    for (int d = g.batch.ndim - 1; d >= 0; --d) {
-      int64_t q = lin / g.batch.shape[d];
-      int64_t r = lin - q * g.batch.shape[d];
-      lin = q;
-      A += r * g.batch.a_strides[d];
-      B += r * g.batch.b_strides[d];
-    }
-  }
-  float *C = g.C + int64_t(blockIdx.z) * g.M * g.N;
-
-  float ra[8], rb[8]; // staged global loads of the next k-tile
-
-  auto load_a = [&](int64_t k0) {
-    if constexpr (AMODE == LOAD_VEC_K) {
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int64_t m = m0 + (tid >> 2) + 64 * i, k = k0 + (tid & 3) * 4;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (m < g.M && k < g.K) v = *reinterpret_cast<const float4 *>(A + m * g.a_sm + k);
-        ra[4 * i + 0] = v.x; ra[4 * i + 1] = v.y; ra[4 * i + 2] = v.z; ra[4 * i + 3] = v.w;
-      }
-    } else if constexpr (AMODE == LOAD_VEC_MN) {
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int64_t k = k0 + (tid >> 5) + 8 * i, m = m0 + (tid & 31) * 4;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (m < g.M && k < g.K) v = *reinterpret_cast<const float4 *>(A + k * g.a_sk + m);
-        ra[4 * i + 0] = v.x; ra[4 * i + 1] = v.y; ra[4 * i + 2] = v.z; ra[4 * i + 3] = v.w;
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int idx = tid + 256 * i;
-        const int64_t m = m0 + (idx & (BM - 1)), k = k0 + (idx >> 7);
-        ra[i] = (m < g.M && k < g.K) ? A[m * g.a_sm + k * g.a_sk] : 0.f;
-      }
-    }
-  };
-  auto load_b = [&](int64_t k0) {
-    if constexpr (BMODE == LOAD_VEC_K) {
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int64_t n = n0 + (tid >> 2) + 64 * i, k = k0 + (tid & 3) * 4;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (n < g.N && k < g.K) v = *reinterpret_cast<const float4 *>(B + n * g.b_sn + k);
-        rb[4 * i + 0] = v.x; rb[4 * i + 1] = v.y; rb[4 * i + 2] = v.z; rb[4 * i + 3] = v.w;
-      }
-    } else if constexpr (BMODE == LOAD_VEC_MN) {
-#pragma unroll
-      for (int i = 0; i < 2; ++i) {
-        const int64_t k = k0 + (tid >> 5) + 8 * i, n = n0 + (tid & 31) * 4;
-        float4 v = make_float4(0.f, 0.f, 0.f, 0.f);
-        if (n < g.N && k < g.K) v = *reinterpret_cast<const float4 *>(B + k * g.b_sk + n);
-        rb[4 * i + 0] = v.x; rb[4 * i + 1] = v.y; rb[4 * i + 2] = v.z; rb[4 * i + 3] = v.w;
-      }
-    } else {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int idx = tid + 256 * i;
-        const int64_t n = n0 + (idx & (BN - 1)), k = k0 + (idx >> 7);
-        rb[i] = (n < g.N && k < g.K) ? B[k * g.b_sk + n * g.b_sn] : 0.f;
-      }
-    }
-  };
-  auto store_a = [&](int buf) {
-    if constexpr (AMODE == LOAD_VEC_K) {
-#pragma unroll
-      for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) As[buf][(tid & 3) * 4 + e][(tid >> 2) + 64 * i] = ra[4 * i + e];
-    } else if constexpr (AMODE == LOAD_VEC_MN) {
-#pragma unroll
-      for (int i = 0; i < 2; ++i)
-        *reinterpret_cast<float4 *>(&As[buf][(tid >> 5) + 8 * i][(tid & 31) * 4]) =
-            make_float4(ra[4 * i], ra[4 * i + 1], ra[4 * i + 2], ra[4 * i + 3]);
-    } else {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int idx = tid + 256 * i;
-        As[buf][idx >> 7][idx & (BM - 1)] = ra[i];
-      }
-    }
-  };
-  auto store_b = [&](int buf) {
-    if constexpr (BMODE == LOAD_VEC_K) {
-#pragma unroll
-      for (int i = 0; i < 2; ++i)
-#pragma unroll
-        for (int e = 0; e < 4; ++e) Bs[buf][(tid & 3) * 4 + e][(tid >> 2) + 64 * i] = rb[4 * i + e];
-    } else if constexpr (BMODE == LOAD_VEC_MN) {
-#pragma unroll
-      for (int i = 0; i < 2; ++i)
-        *reinterpret_cast<float4 *>(&Bs[buf][(tid >> 5) + 8 * i][(tid & 31) * 4]) =
-            make_float4(rb[4 * i], rb[4 * i + 1], rb[4 * i + 2], rb[4 * i + 3]);
-    } else {
-#pragma unroll
-      for (int i = 0; i < 8; ++i) {
-        const int idx = tid + 256 * i;
-        Bs[buf][idx >> 7][idx & (BN - 1)] = rb[i];
-      }
-    }
-  };
-
-  // thread (ty, tx) owns rows {4ty..4ty+3, 64+4ty..} and columns {4tx..4tx+3, 64+4tx..}
-  const int ty = tid >> 4, tx = tid & 15;
-  float acc[8][8];
-#pragma unroll
-  for (int i = 0; i < 8; ++i)
-#pragma unroll
-    for (int j = 0; j < 8; ++j) acc[i][j] = 0.f;
-
-  load_a(0);
-  load_b(0);
-  store_a(0);
-  store_b(0);
-  __syncthreads();
-
-  int buf = 0;
-  for (int64_t k0 = 0; k0 < g.K; k0 += BK) {
-    const bool more = (k0 + BK < g.K);
-    if (more) {
-      load_a(k0 + BK);
-      load_b(k0 + BK);
-    }
-#pragma unroll
-    for (int k = 0; k < BK; ++k) {
-      float4 a_lo = *reinterpret_cast<const float4 *>(&As[buf][k][4 * ty]);
-      float4 a_hi = *reinterpret_cast<const float4 *>(&As[buf][k][64 + 4 * ty]);
-      float4 b_lo = *reinterpret_cast<const float4 *>(&Bs[buf][k][4 * tx]);
-      float4 b_hi = *reinterpret_cast<const float4 *>(&Bs[buf][k][64 + 4 * tx]);
-      const float av[8] = {a_lo.x, a_lo.y, a_lo.z, a_lo.w, a_hi.x, a_hi.y, a_hi.z, a_hi.w};
-      const float bv[8] = {b_lo.x, b_lo.y, b_lo.z, b_lo.w, b_hi.x, b_hi.y, b_hi.z, b_hi.w};
-#pragma unroll
-      for (int i = 0; i < 8; ++i)
-#pragma unroll
-        for (int j = 0; j < 8; ++j) {
-          if constexpr (FUSED_MAD) acc[i][j] = fmaf(av[i], bv[j], acc[i][j]);
-          else acc[i][j] = __fadd_rn(acc[i][j], __fmul_rn(av[i], bv[j]));
-        }
-    }
-    if (more) {
-      store_a(buf ^ 1);
-      store_b(buf ^ 1);
-      __syncthreads();
-      buf ^= 1;
-    }
-  }
-
-#pragma unroll
-  for (int i = 0; i < 8; ++i) {
-    const int64_t m = m0 + ((i < 4) ? (4 * ty + i) : (64 + 4 * ty + i - 4));
-    if (m >= g.M) continue;
-#pragma unroll
-    for (int h = 0; h < 2; ++h) {
-      const int64_t n = n0 + 64 * h + 4 * tx;
-      float *dst = C + m * g.N + n;
-      if (g.c_vec && n + 3 < g.N) {
-        *reinterpret_cast<float4 *>(dst) = make_float4(acc[i][4 * h], acc[i][4 * h + 1], acc[i][4 * h + 2], acc[i][4 * h + 3]);
-      } else {
-#pragma unroll
-        for (int e = 0; e < 4; ++e)
-          if (n + e < g.N) dst[e] = acc[i][4 * h + e];
-      }
-    }
-  }
-}
 
 // One output element per thread, any arithmetic dtype (the shape of the reference's fallback).
 template <class T>
@@ -258,46 +70,102 @@ __global__ void matmul_naive(const T *A, const T *B, T *C, int64_t M, int64_t N,
 
 static bool al16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-template <int AMODE, int BMODE> static void launch_simt(const GemmArgs &g, dim3 grid, bool fused) {
-  if (fused)
-    sgemm_tiled<AMODE, BMODE, true><<<grid, 256, 0, stream()>>>(g);
-  else
-    sgemm_tiled<AMODE, BMODE, false><<<grid, 256, 0, stream()>>>(g);
+// How a product runs on the CUDA cores: tile edge, CTAs along k (a cluster), and the time that is expected of it.
+// Clocks per k of one CTA, measured: alone on its SM (a chain of shared-memory loads and multiply-adds: 50 for the
+// 32-wide tile, 75 for 64, 345 for 128 x 256) and with the SM full (20, 70, 350).  So a product with few tiles takes
+// the small tile and many k-splits (256 x 784 x 256: 8.4 us with 64 tiles x 8, against 21 us unsplit and 145 us in two
+// 128 x 256 tiles), one with many tiles the large tile (52 TFLOP/s; 35 with the 64-wide tile).
+struct SimtPlan {
+  int tile = 32, splits = 1;
+  int64_t k_per_split = 0;
+  double us = 1e30;
+};
+static SimtPlan plan_simt(int64_t batch, int64_t M, int64_t N, int64_t K, bool may_split) {
+  SimtPlan best;
+  for (int tile : {128, 64, 32}) {
+    const double tiles = double(ceil_div(M, tile)) * double(ceil_div(N, tile == 128 ? LG_N : tile)) * double(batch);
+    if (ceil_div(M, tile) > 65535) continue;
+    const double full = tile == 128 ? 350 : tile == 64 ? 70 : 20, alone = tile == 128 ? 345 : tile == 64 ? 75 : 50;
+    for (int s = 1; s <= (may_split && tile < 128 ? 8 : 1); ++s) {
+      const int64_t per = s == 1 ? K : ceil_div(ceil_div(K, s), SG_BK) * SG_BK;
+      if (s > 1 && (s - 1) * per >= K) continue;
+      const double rounds = std::ceil(tiles * s / sm_count());
+      const double clocks = std::max(rounds * full, alone) * double(per) + (s > 1 ? 1500 : 0) + 3000;
+      if (clocks / 1900 < best.us) best = SimtPlan{tile, s, per, clocks / 1900};
+    }
+  }
+  return best;
 }
 
-static void sgemm_simt(GemmArgs g, int64_t nbatch, bool fused) {
-  bool batch_al = true;
-  for (int d = 0; d < g.batch.ndim; ++d) batch_al = batch_al && (g.batch.a_strides[d] % 4 == 0);
-  int amode = LOAD_SCALAR;
-  if (al16(g.A) && batch_al) {
-    if (g.a_sk == 1 && g.K % 4 == 0 && g.a_sm % 4 == 0) amode = LOAD_VEC_K;
-    else if (g.a_sm == 1 && g.M % 4 == 0 && g.a_sk % 4 == 0) amode = LOAD_VEC_MN;
+template <int T, bool A_K, bool B_K, bool FUSED> static void launch_small(const GemmArgs &g, dim3 grid) {
+  constexpr int smem = sg_smem_bytes<T, A_K, B_K>;
+  auto *kernel = sgemm_small<T, A_K, B_K, FUSED>;
+  static bool configured = false;
+  if (!configured) {
+    NT_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
+    configured = true;
   }
-  batch_al = true;
-  for (int d = 0; d < g.batch.ndim; ++d) batch_al = batch_al && (g.batch.b_strides[d] % 4 == 0);
-  int bmode = LOAD_SCALAR;
-  if (al16(g.B) && batch_al) {
-    if (g.b_sn == 1 && g.N % 4 == 0 && g.b_sk % 4 == 0) bmode = LOAD_VEC_MN;
-    else if (g.b_sk == 1 && g.K % 4 == 0 && g.b_sn % 4 == 0) bmode = LOAD_VEC_K;
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = dim3((T / 4) * (T / 4), 1, 1);
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream();
+  cudaLaunchAttribute attr[1];
+  attr[0].id = cudaLaunchAttributeClusterDimension;
+  attr[0].val.clusterDim.x = unsigned(g.splits);
+  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
+  cfg.attrs = attr;
+  cfg.numAttrs = g.splits > 1 ? 1 : 0;
+  NT_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, g));
+}
+template <int T, bool FUSED> static void launch_small(const GemmArgs &g, dim3 grid, bool a_k, bool b_k) {
+  if (a_k && b_k) launch_small<T, true, true, FUSED>(g, grid);
+  else if (a_k) launch_small<T, true, false, FUSED>(g, grid);
+  else if (b_k) launch_small<T, false, true, FUSED>(g, grid);
+  else launch_small<T, false, false, FUSED>(g, grid);
+}
+
+template <bool A_K, bool B_K, bool FUSED> static void launch_large(const GemmArgs &g, dim3 grid) {
+  auto *kernel = sgemm_large<A_K, B_K, FUSED>;
+  static bool configured = false;
+  if (!configured) {
+    NT_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LG_SMEM));
+    configured = true;
   }
-  g.c_vec = (g.N % 4 == 0) ? 1 : 0;
-  if (nbatch > 65535 || ceil_div(g.M, BM) > 65535) fail_runtime("matmul: too many tiles for one launch.");
-  dim3 grid{unsigned(ceil_div(g.N, BN)), unsigned(ceil_div(g.M, BM)), unsigned(nbatch)};
-#define NT_CASE(a, b)                                                                              \
-  if (amode == a && bmode == b) {                                                                  \
-    launch_simt<a, b>(g, grid, fused);                                                             \
-  } else
-  NT_CASE(LOAD_SCALAR, LOAD_SCALAR)
-  NT_CASE(LOAD_SCALAR, LOAD_VEC_K)
-  NT_CASE(LOAD_SCALAR, LOAD_VEC_MN)
-  NT_CASE(LOAD_VEC_K, LOAD_SCALAR)
-  NT_CASE(LOAD_VEC_K, LOAD_VEC_K)
-  NT_CASE(LOAD_VEC_K, LOAD_VEC_MN)
-  NT_CASE(LOAD_VEC_MN, LOAD_SCALAR)
-  NT_CASE(LOAD_VEC_MN, LOAD_VEC_K)
-  NT_CASE(LOAD_VEC_MN, LOAD_VEC_MN) {}
-#undef NT_CASE
-  check_launch("sgemm_tiled");
+  kernel<<<grid, LG_NT, LG_SMEM, stream()>>>(g);
+}
+template <bool FUSED> static void launch_large(const GemmArgs &g, dim3 grid, bool a_k, bool b_k) {
+  if (a_k && b_k) launch_large<true, true, FUSED>(g, grid);
+  else if (a_k) launch_large<true, false, FUSED>(g, grid);
+  else if (b_k) launch_large<false, true, FUSED>(g, grid);
+  else launch_large<false, false, FUSED>(g, grid);
+}
+
+static void sgemm_simt(GemmArgs g, int64_t nbatch, bool fused, const SimtPlan &plan) {
+  bool a_al = al16(g.A), b_al = al16(g.B);
+  for (int d = 0; d < g.batch.ndim; ++d) {
+    a_al = a_al && g.batch.a_strides[d] % 4 == 0;
+    b_al = b_al && g.batch.b_strides[d] % 4 == 0;
+  }
+  const bool a_k = g.a_sk == 1 && g.a_sm != 1, b_k = g.b_sk == 1 && g.b_sn != 1;
+  g.a_vec = a_k ? (a_al && g.K % 4 == 0 && g.a_sm % 4 == 0) : (a_al && g.a_sm == 1 && g.M % 4 == 0 && g.a_sk % 4 == 0);
+  g.b_vec = b_k ? (b_al && g.K % 4 == 0 && g.b_sn % 4 == 0) : (b_al && g.b_sn == 1 && g.N % 4 == 0 && g.b_sk % 4 == 0);
+  g.c_vec = g.N % 4 == 0 && al16(g.C);
+  g.splits = plan.splits;
+  g.k_per_split = plan.k_per_split;
+  if (nbatch > 65535 || ceil_div(g.M, plan.tile) > 65535) fail_runtime("matmul: too many tiles for one launch.");
+  dim3 grid{unsigned(ceil_div(g.N, plan.tile == 128 ? LG_N : plan.tile) * plan.splits), unsigned(ceil_div(g.M, plan.tile)), unsigned(nbatch)};
+  if (plan.tile == 128) {
+    if (fused) launch_large<true>(g, grid, a_k, b_k);
+    else launch_large<false>(g, grid, a_k, b_k);
+  } else if (plan.tile == 64) {
+    if (fused) launch_small<64, true>(g, grid, a_k, b_k);
+    else launch_small<64, false>(g, grid, a_k, b_k);
+  } else {
+    if (fused) launch_small<32, true>(g, grid, a_k, b_k);
+    else launch_small<32, false>(g, grid, a_k, b_k);
+  }
+  check_launch("sgemm");
 }
 
 } // namespace ntb
@@ -313,6 +181,11 @@ int nt_set_matmul_mode(int mode) {
   g_matmul_mode.store(mode);
   gemm_tc_set_promoted(mode == 1);
   NT_API_END
+}
+int nt_matmul_allow_reorder(int on) {
+  const int was = t_reorder;
+  t_reorder = on != 0;
+  return was;
 }
 int nt_get_matmul_mode(void) { return g_matmul_mode.load(); }
 int nt_set_matmul_schedule(int max_splits, int panel) {
@@ -394,8 +267,16 @@ static nt_storage *matmul_impl(const nt_view *x1, const nt_view *x2, const nt_vi
     bool done = false;
     // Tiny products (a single tile of the exact kernel) take the exact FP32 kernel: one launch instead of
     // up to three, and the full fp32 accuracy of the reference's own CUDA kernels on the small cases.
-    const bool big_enough = double(nbatch) * double(M) * double(N) * double(K) > double(g_tc_min_macs.load());
-    if ((mode == 1 || mode == 3) && K > 0 && big_enough) {
+    const int64_t min_macs = g_tc_min_macs.load();
+    const bool big_enough = double(nbatch) * double(M) * double(N) * double(K) > double(min_macs);
+    // Above that threshold mode 1 goes by expected time (a threshold of 0 sends everything through planes): planes, the
+    // tensor-core kernel that does without them -- same bits -- and, where the caller does not need those very bits,
+    // the CUDA cores, which finish first below some 5e8 multiply-adds (784 x 256 x 256: 7 us against 11.5 and 20).
+    const SimtPlan simt = plan_simt(nbatch, M, N, K, /*may_split=*/mode == 1 || mode == 3);
+    const bool by_time = mode == 1 && big_enough && min_macs > 0;
+    const double tc_us = by_time ? gemm_tc_expected_us(nbatch, M, N, K) : 0, fused_us = by_time ? gemm_fused_expected_us(nbatch, M, N, K) : 0;
+    const bool on_cuda_cores = by_time && t_reorder && simt.us < std::min(tc_us, fused_us);
+    if ((mode == 1 || mode == 3) && K > 0 && big_enough && !on_cuda_cores) {
       // the tensor-core path takes a single (collapsed) batch stride per operand
       int64_t a_sb = 0, b_sb = 0;
       bool single = true;
@@ -412,7 +293,9 @@ static nt_storage *matmul_impl(const nt_view *x1, const nt_view *x2, const nt_vi
         b_sb = bi.b_strides[bi.ndim - 1];
       }
       const float *bp = bias ? static_cast<const float *>(bias->storage->ptr()) + bias->offset : nullptr;
-      if (single && mode == 1 && g_natural_planes.load())
+      if (single && by_time && fused_us < tc_us)
+        bias_done = done = gemm_fused(g.A, g.B, g.C, nbatch, M, N, K, a_sb, a_sm, a_sk, b_sb, b_sk, b_sn, bp, bias ? bias->strides[0] : 0);
+      if (single && !done && mode == 1 && g_natural_planes.load())
         done = gemm_3xtf32_natural(x1->storage, x1->offset, x2->storage, x2->offset, g.C, nbatch, M, N, K, a_sb, a_sm,
                                    a_sk, b_sb, b_sk, b_sn, bp, bias ? bias->strides[0] : 0, &bias_done);
       if (single && !done)
@@ -420,8 +303,11 @@ static nt_storage *matmul_impl(const nt_view *x1, const nt_view *x2, const nt_vi
                            bias ? bias->strides[0] : 0, &bias_done);
     }
     if (!done) {
+      g.bias = bias ? static_cast<const float *>(bias->storage->ptr()) + bias->offset : nullptr;
+      g.bias_stride = bias ? bias->strides[0] : 0;
+      bias_done = true;
       matmul_profile_begin();
-      sgemm_simt(g, nbatch, /*fused=*/mode != 2);
+      sgemm_simt(g, nbatch, /*fused=*/mode != 2, simt);
       matmul_profile_end();
     }
   } else {

@@ -1,0 +1,345 @@
+// Exact FP32 products on the CUDA cores: two kernels over strided operands, each output accumulated in ascending k
+// with one rounding per multiply-add (FUSED) or a rounded product and a rounded sum (the reference's CPU loop).
+//
+//   sgemm_small<T>  T x T output tiles (T = 64 or 32), cp.async into a 3-stage ring of 32-deep k-slices, 4 x 4 outputs
+//                   per thread.  What bounds a small product is not arithmetic but how many SMs take part and the
+//                   chain of loads each CTA waits for: 256 x 256 x 10 through one 128-wide tile per CTA used 2 SMs
+//                   and took 42 us.  With `splits` > 1 a cluster of CTAs shares a tile, each over its own k-range; the
+//                   partial tiles meet in distributed shared memory and are added in rank order, so the result
+//                   does not depend on timing (one launch, no workspace).
+//   sgemm_large     128 x 256 tiles, 8 x 16 outputs per thread as packed pairs: fma.rn.f32x2 does two IEEE fused
+//                   multiply-adds per instruction, which leaves issue slots for loads and moves (a scalar FFMA takes
+//                   every slot of its scheduler).  8 x 16 because shared memory feeds registers at 128 bytes a clock:
+//                   8 x 8 outputs need 64 bytes per 64 multiply-adds and tie with the arithmetic, 8 x 16 need 96 per 128.
+#pragma once
+
+#include <cooperative_groups.h>
+
+#include "cp_async.cuh"
+#include "nt_core.cuh"
+
+namespace ntb {
+
+struct BatchIndex {
+  int ndim;
+  int64_t shape[NT_MAX_DIMS];
+  int64_t a_strides[NT_MAX_DIMS];
+  int64_t b_strides[NT_MAX_DIMS];
+};
+
+struct GemmArgs {
+  const float *A, *B;
+  float *C;
+  const float *bias;   // C[m][n] = fl(fl(sum) + bias[n * bias_stride]) when non-null
+  int64_t bias_stride;
+  int64_t M, N, K;
+  int64_t a_sm, a_sk, b_sk, b_sn;
+  BatchIndex batch;
+  int a_vec, b_vec;    // 16-byte loads along the unit-stride dim are aligned and whole
+  int c_vec;           // C rows may be written 128 bits at a time
+  int splits;          // small kernel: CTAs of a cluster along k
+  int64_t k_per_split;
+};
+
+__device__ __forceinline__ void gemm_batch_base(const GemmArgs &g, int64_t lin, const float *&A, const float *&B) {
+  for (int d = g.batch.ndim - 1; d >= 0; --d) {
+    const int64_t q = lin / g.batch.shape[d];
+    const int64_t r = lin - q * g.batch.shape[d];
+    lin = q;
+    A += r * g.batch.a_strides[d];
+    B += r * g.batch.b_strides[d];
+  }
+}
+
+template <bool FUSED> __device__ __forceinline__ float mad(float a, float b, float c) {
+  if constexpr (FUSED) return fmaf(a, b, c);
+  else return __fadd_rn(c, __fmul_rn(a, b));
+}
+
+// ---------------------------------------------------------------------------------------------
+// Small products.  A_K / B_K: the operand's unit-stride dim is k (shared tile [row][k]); otherwise rows run along the
+// unit stride (shared tile [k][row]).  Thread (ty, tx) of the (T/4)^2 owns rows r(ty, i) and columns r(tx, j): 4 t + i
+// where the tile is [k][row], so that a 128-bit load covers them, and t + (T/4) i where it is [row][k], so that the
+// 128-bit loads along k of neighbouring threads fall into different banks.
+constexpr int SG_BK = 32;
+template <int T> constexpr int sg_stages = 3;
+template <int T, bool K_MAJOR> constexpr int sg_tile_floats = K_MAJOR ? T * (SG_BK + 4) : SG_BK * (T + 4);
+template <int T, bool A_K, bool B_K> // the ring; a partial tile of T x T is smaller
+constexpr int sg_smem_bytes = sg_stages<T> * (sg_tile_floats<T, A_K> + sg_tile_floats<T, B_K>) * 4;
+
+template <int T, bool A_K, bool B_K, bool FUSED>
+__global__ void __launch_bounds__((T / 4) * (T / 4)) sgemm_small(GemmArgs g) {
+  constexpr int G = T / 4, NT = G * G;
+  constexpr int SG_STAGES = sg_stages<T>;
+  constexpr int AF = sg_tile_floats<T, A_K>, BF = sg_tile_floats<T, B_K>;
+  extern __shared__ __align__(16) float sg_smem[];
+  const int tid = threadIdx.x, tx = tid % G, ty = tid / G;
+  const int split = blockIdx.x % g.splits;
+  const int64_t n0 = int64_t(blockIdx.x / g.splits) * T, m0 = int64_t(blockIdx.y) * T;
+  const float *A = g.A, *B = g.B;
+  gemm_batch_base(g, blockIdx.z, A, B);
+  const int64_t k_lo = split * g.k_per_split, k_hi = min(g.K, k_lo + g.k_per_split);
+  const int steps = k_hi > k_lo ? int((k_hi - k_lo + SG_BK - 1) / SG_BK) : 0;
+
+  // one operand's slice [T rows][SG_BK of k] into shared memory; what lies outside is zero
+  auto load = [&](auto k_major, const float *src, int64_t r0, int64_t R, int64_t s_r, int64_t s_k, int vec, float *dst, int64_t k0) {
+    constexpr bool KM = decltype(k_major)::value;
+    if (vec) { // the unit-stride extent is a multiple of 4: a group is inside or outside as a whole
+#pragma unroll
+      for (int i = 0; i < T * SG_BK / 4 / NT; ++i) {
+        const int v = tid + i * NT;
+        const int r = KM ? v / (SG_BK / 4) : (v % (T / 4)) * 4, k = KM ? (v % (SG_BK / 4)) * 4 : v / (T / 4);
+        const bool live = r0 + r < R && k0 + k < k_hi;
+        const float *p = live ? src + (r0 + r) * s_r + (k0 + k) * s_k : src;
+        cp_async16(dst + (KM ? r * (SG_BK + 4) + k : k * (T + 4) + r), p, live);
+      }
+    } else {
+#pragma unroll 4
+      for (int i = 0; i < T * SG_BK / NT; ++i) {
+        const int v = tid + i * NT;
+        const int r = KM ? v / SG_BK : v % T, k = KM ? v % SG_BK : v / T;
+        const bool live = r0 + r < R && k0 + k < k_hi;
+        const float *p = live ? src + (r0 + r) * s_r + (k0 + k) * s_k : src;
+        cp_async4(dst + (KM ? r * (SG_BK + 4) + k : k * (T + 4) + r), p, live);
+      }
+    }
+  };
+  auto fetch = [&](int step) {
+    float *st = sg_smem + (step % SG_STAGES) * (AF + BF);
+    const int64_t k0 = k_lo + int64_t(step) * SG_BK;
+    load(std::bool_constant<A_K>{}, A, m0, g.M, g.a_sm, g.a_sk, g.a_vec, st, k0);
+    load(std::bool_constant<B_K>{}, B, n0, g.N, g.b_sn, g.b_sk, g.b_vec, st + AF, k0);
+  };
+
+  float acc[4][4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
+
+#pragma unroll
+  for (int s = 0; s < SG_STAGES - 1; ++s) {
+    if (s < steps) fetch(s);
+    cp_async_commit();
+  }
+  for (int s = 0; s < steps; ++s) {
+    cp_async_wait<SG_STAGES - 2>();
+    __syncthreads(); // slice s has landed for everyone, and slice s - 1 has been read by everyone
+    if (s + SG_STAGES - 1 < steps) fetch(s + SG_STAGES - 1);
+    cp_async_commit();
+    const float *as = sg_smem + (s % SG_STAGES) * (AF + BF), *bs = as + AF;
+#pragma unroll
+    for (int k = 0; k < SG_BK; k += 4) {
+      float a[4][4], b[4][4]; // [row][k]
+#pragma unroll
+      for (int i = 0; i < 4; ++i) {
+        const float4 va = A_K ? *reinterpret_cast<const float4 *>(as + (ty + G * i) * (SG_BK + 4) + k)
+                              : *reinterpret_cast<const float4 *>(as + (k + i) * (T + 4) + 4 * ty);
+        const float4 vb = B_K ? *reinterpret_cast<const float4 *>(bs + (tx + G * i) * (SG_BK + 4) + k)
+                              : *reinterpret_cast<const float4 *>(bs + (k + i) * (T + 4) + 4 * tx);
+        const float fa[4] = {va.x, va.y, va.z, va.w}, fb[4] = {vb.x, vb.y, vb.z, vb.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          if (A_K) a[i][e] = fa[e];
+          else a[e][i] = fa[e];
+          if (B_K) b[i][e] = fb[e];
+          else b[e][i] = fb[e];
+        }
+      }
+#pragma unroll
+      for (int kk = 0; kk < 4; ++kk)
+#pragma unroll
+        for (int i = 0; i < 4; ++i)
+#pragma unroll
+          for (int j = 0; j < 4; ++j) acc[i][j] = mad<FUSED>(a[i][kk], b[j][kk], acc[i][j]);
+    }
+  }
+
+  float *C = g.C + int64_t(blockIdx.z) * g.M * g.N;
+  auto row = [&](int i) { return A_K ? ty + G * i : 4 * ty + i; };
+  auto col = [&](int j) { return B_K ? tx + G * j : 4 * tx + j; };
+  if (g.splits == 1) {
+#pragma unroll
+    for (int i = 0; i < 4; ++i) {
+      const int64_t m = m0 + row(i);
+      if (m >= g.M) continue;
+      if (!B_K && g.c_vec && !g.bias && n0 + 4 * tx < g.N) {
+        *reinterpret_cast<float4 *>(C + m * g.N + n0 + 4 * tx) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+        continue;
+      }
+#pragma unroll
+      for (int j = 0; j < 4; ++j) {
+        const int64_t n = n0 + col(j);
+        if (n < g.N) C[m * g.N + n] = g.bias ? acc[i][j] + __ldg(g.bias + n * g.bias_stride) : acc[i][j];
+      }
+    }
+    return;
+  }
+  // the cluster's partial tiles, added in rank order; each CTA finishes its share of the tile
+  namespace cg = cooperative_groups;
+  cg::cluster_group cluster = cg::this_cluster();
+  __syncthreads(); // the ring is free
+#pragma unroll
+  for (int i = 0; i < 4; ++i)
+#pragma unroll
+    for (int j = 0; j < 4; ++j) sg_smem[row(i) * T + col(j)] = acc[i][j];
+  cluster.sync();
+  const float *part[8];
+#pragma unroll
+  for (int r = 0; r < 8; ++r) part[r] = cluster.map_shared_rank(sg_smem, r < g.splits ? r : 0);
+  for (int e = split * NT + tid; e < T * T; e += NT * g.splits) {
+    const int64_t m = m0 + e / T, n = n0 + e % T;
+    if (m >= g.M || n >= g.N) continue;
+    float v[8];
+#pragma unroll
+    for (int r = 0; r < 8; ++r) v[r] = r < g.splits ? part[r][e] : 0.0f;
+    float sum = v[0];
+#pragma unroll
+    for (int r = 1; r < 8; ++r)
+      if (r < g.splits) sum += v[r];
+    C[m * g.N + n] = g.bias ? sum + __ldg(g.bias + n * g.bias_stride) : sum;
+  }
+  cluster.sync(); // nobody leaves while its tile is being read
+}
+
+// ---------------------------------------------------------------------------------------------
+// Large products: 128 x 256 tiles, 256 threads of 8 x 16 outputs.
+constexpr int LG_M = 128, LG_N = 256, LG_BK = 8, LG_NT = 256, LG_STAGES = 4;
+constexpr int LG_AP = LG_M + 4, LG_BP = LG_N + 4; // pitches of the shared rows [k][m|n], in floats
+constexpr int LG_SMEM = LG_STAGES * LG_BK * (LG_AP + LG_BP) * 4;
+
+using f32x2 = unsigned long long;
+template <bool FUSED> __device__ __forceinline__ void mad2(f32x2 &c, f32x2 a, f32x2 b) {
+  if constexpr (FUSED) {
+    asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
+  } else { // as scalars: the packed multiply and add came out of the assembler as one fused operation
+    float x, y, a0, a1, b0, b1;
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(c));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(a0), "=f"(a1) : "l"(a));
+    asm("mov.b64 {%0, %1}, %2;" : "=f"(b0), "=f"(b1) : "l"(b));
+    x = __fadd_rn(x, __fmul_rn(a0, b0));
+    y = __fadd_rn(y, __fmul_rn(a1, b1));
+    asm("mov.b64 %0, {%1, %2};" : "=l"(c) : "f"(x), "f"(y));
+  }
+}
+__device__ __forceinline__ f32x2 twice(float x) {
+  f32x2 r;
+  asm("mov.b64 %0, {%1, %1};" : "=l"(r) : "f"(x));
+  return r;
+}
+
+// A [R rows][8 k] slice into shared rows [k][row]: 16 bytes at a time along aligned rows, else value by value (along k,
+// a lane per k, where that is the unit stride).  What lies outside the operand is zero.
+template <int R, bool K_MAJOR>
+__device__ __forceinline__ void lg_load(float *st, const float *base, int64_t s_r, int64_t s_k, int64_t rows, bool vec, int64_t k0, int64_t K) {
+  constexpr int P = R + 4;
+  const int tid = threadIdx.x;
+  if (!K_MAJOR && vec) {
+#pragma unroll
+    for (int i = 0; i < R / 128; ++i) {
+      const int v = tid + 256 * i, r = (v * 4) % R, k = (v * 4) / R;
+      const bool live = r < rows && k0 + k < K;
+      cp_async16(st + k * P + r, live ? base + r + (k0 + k) * s_k : base, live);
+    }
+  } else {
+#pragma unroll
+    for (int i = 0; i < R / 32; ++i) {
+      const int v = tid + 256 * i;
+      const int r = K_MAJOR ? v / LG_BK : v % R, k = K_MAJOR ? v % LG_BK : v / R;
+      const bool live = r < rows && k0 + k < K;
+      cp_async4(st + k * P + r, live ? base + r * s_r + (k0 + k) * s_k : base, live);
+    }
+  }
+}
+
+// Two warps per scheduler is all that 8 x 16 outputs leave registers for, so latencies are covered inside a warp: the
+// operands of step k + 1 are loaded while step k multiplies, and slices arrive by cp.async three steps ahead.
+template <bool A_K, bool B_K, bool FUSED> __global__ void __launch_bounds__(LG_NT, 1) sgemm_large(GemmArgs g) {
+  extern __shared__ __align__(16) float lg_smem[];
+  constexpr int AF = LG_BK * LG_AP, SF = LG_BK * (LG_AP + LG_BP); // floats of A's part and of a stage
+  const int tid = threadIdx.x, tx = tid & 15, ty = tid >> 4;
+  const int64_t m0 = int64_t(blockIdx.y) * LG_M, n0 = int64_t(blockIdx.x) * LG_N;
+  const float *A = g.A, *B = g.B;
+  gemm_batch_base(g, blockIdx.z, A, B);
+  A += m0 * g.a_sm;
+  B += n0 * g.b_sn;
+  const int steps = int((g.K + LG_BK - 1) / LG_BK);
+  auto fetch = [&](int s) {
+    if (s < steps) {
+      float *st = lg_smem + (s % LG_STAGES) * SF;
+      lg_load<LG_M, A_K>(st, A, g.a_sm, g.a_sk, g.M - m0, g.a_vec, int64_t(s) * LG_BK, g.K);
+      lg_load<LG_N, B_K>(st + AF, B, g.b_sn, g.b_sk, g.N - n0, g.b_vec, int64_t(s) * LG_BK, g.K);
+    }
+    cp_async_commit();
+  };
+  // rows {4 ty .. + 3, 64 + 4 ty .. + 3}; columns 64 h + 4 tx .. + 3 for h = 0 .. 3, as pairs
+  f32x2 acc[8][8];
+#pragma unroll
+  for (int i = 0; i < 8; ++i)
+#pragma unroll
+    for (int j = 0; j < 8; ++j) acc[i][j] = 0ull;
+  float4 a[2][2];
+  ulonglong2 b[2][4];
+  auto operands = [&](int to, int s, int k) {
+    const float *st = lg_smem + (s % LG_STAGES) * SF;
+#pragma unroll
+    for (int h = 0; h < 2; ++h) a[to][h] = *reinterpret_cast<const float4 *>(st + k * LG_AP + 64 * h + 4 * ty);
+#pragma unroll
+    for (int h = 0; h < 4; ++h) b[to][h] = *reinterpret_cast<const ulonglong2 *>(st + AF + k * LG_BP + 64 * h + 4 * tx);
+  };
+
+#pragma unroll
+  for (int s = 0; s < LG_STAGES - 1; ++s) fetch(s);
+  cp_async_wait<LG_STAGES - 2>();
+  __syncthreads();
+  operands(0, 0, 0);
+  for (int s = 0; s < steps; ++s) {
+#pragma unroll
+    for (int k = 0; k < LG_BK; ++k) {
+      const int cur = k & 1;
+      if (k == 0) fetch(s + LG_STAGES - 1); // into the slot that every warp left before the last barrier
+      if (k < LG_BK - 1) {
+        operands(cur ^ 1, s, k + 1);
+      } else { // the first operands of the next slice (of a stale slot after the last one, unused)
+        cp_async_wait<LG_STAGES - 2>();
+        __syncthreads();
+        operands(cur ^ 1, s + 1, 0);
+      }
+      const f32x2 bb[8] = {b[cur][0].x, b[cur][0].y, b[cur][1].x, b[cur][1].y, b[cur][2].x, b[cur][2].y, b[cur][3].x, b[cur][3].y};
+#pragma unroll
+      for (int h = 0; h < 2; ++h) {
+        const float aa[4] = {a[cur][h].x, a[cur][h].y, a[cur][h].z, a[cur][h].w};
+#pragma unroll
+        for (int i = 0; i < 4; ++i) {
+          const f32x2 pair = twice(aa[i]);
+#pragma unroll
+          for (int j = 0; j < 8; ++j) mad2<FUSED>(acc[4 * h + i][j], pair, bb[j]);
+        }
+      }
+    }
+  }
+
+  float *C = g.C + int64_t(blockIdx.z) * g.M * g.N;
+#pragma unroll
+  for (int i = 0; i < 8; ++i) {
+    const int64_t m = m0 + (i < 4 ? 4 * ty + i : 64 + 4 * ty + i - 4);
+    if (m >= g.M) continue;
+#pragma unroll
+    for (int h = 0; h < 4; ++h) {
+      const int64_t n = n0 + 64 * h + 4 * tx;
+      float v[4];
+      *reinterpret_cast<f32x2 *>(v) = acc[i][2 * h];
+      *reinterpret_cast<f32x2 *>(v + 2) = acc[i][2 * h + 1];
+      float *dst = C + m * g.N + n;
+      if (g.c_vec && !g.bias && n < g.N) {
+        *reinterpret_cast<float4 *>(dst) = make_float4(v[0], v[1], v[2], v[3]);
+      } else {
+#pragma unroll
+        for (int e = 0; e < 4; ++e)
+          if (n + e < g.N) dst[e] = g.bias ? v[e] + __ldg(g.bias + (n + e) * g.bias_stride) : v[e];
+      }
+    }
+  }
+}
+
+} // namespace ntb
