@@ -234,8 +234,7 @@ int nt_linear(const nt_view *x, const nt_view *w, const nt_view *bias, nt_storag
 int nt_set_matmul_mode(int mode);
 int nt_get_matmul_mode(void);
 /* In modes 1 and 3 a product of at most this many multiply-adds (batch*M*N*K, default 2^21) takes the
- * exact FP32 kernels instead: tiny products keep the accuracy of the reference's CUDA kernels.  (There a
- * product may be split along k, its parts added in a fixed order; modes 0 and 2 are never split.)  Above it,
+ * exact FP32 kernels instead: tiny products keep the bits of the reference's CUDA kernels.  Above it,
  * mode 1 picks between the plane-fed kernel and one that splits the operands itself, by expected time; the
  * bits are the same.  0 sends every fp32 product through the planes. */
 /* Mode 1 splits each fp32 operand into two TF32 planes (hi, lo) before the product.  natural != 0 (default):
@@ -282,12 +281,13 @@ int nt_matmul_pair(const nt_view *a1, const nt_view *b1, const nt_view *a2, cons
                    nt_storage **out2);
 int nt_set_matmul_pair_overlap(int on);
 int nt_set_matmul_tc_min_macs(int64_t macs);
-/* on != 0: mode-1 products of this thread may also run on the CUDA cores in exact FP32, where that is expected to be
- * faster; returns the previous setting (default 0).  A product's sum is then rounded in another order than on the
- * tensor cores -- at no lower accuracy -- so the host layer allows it where no later decision hangs on the last bit:
- * for gradients and for products outside a recorded graph, not for a recorded forward product, whose values decide
- * the side of a ReLU's kink or which element is an extremum. */
-int nt_matmul_allow_reorder(int on);
+/* How free the order of a sum is in this thread's products of modes 1 and 3; returns the previous level (default 0).
+ * 1: a product above the threshold may also run on the CUDA cores in exact FP32, split along k where that is expected
+ * to be faster (the parts are added in a fixed order); 2: one below it may be split as well.  The result is rounded
+ * in another order at no lower accuracy, so the host layer allows it where no later decision hangs on the last bit --
+ * level 2 for gradients, 1 for products outside a recorded graph -- and not for a recorded forward product, whose
+ * values decide the side of a ReLU's kink or which element is an extremum. */
+int nt_matmul_allow_reorder(int level);
 int64_t nt_get_matmul_tc_min_macs(void);
 
 /* ------------------------------------------------------------------ in-place (src/cpp/ops/inplace_ops.cu:75-79); bump the version */

@@ -364,7 +364,7 @@ template <class F, int NIN> static nt_storage *produce_with_planes(F f, const nt
   float *hi = gemm_tc_adopt_planes(out.s, R, C);
   if (!hi) return nullptr;
   const int64_t n = R * C;
-  ew_contig_planes<F, NIN><<<unsigned(ceil_div(n >> 2, 256 * 4)), 256, 0, stream()>>>(f, static_cast<float *>(out->ptr()), pa, pb, n,
+  launch(ew_contig_planes<F, NIN>, unsigned(ceil_div(n >> 2, 256 * 4)), 256, 0, f, static_cast<float *>(out->ptr()), pa, pb, n,
                                                                                       hi, hi + n);
   check_launch("ew_contig_planes");
   return out.release();
@@ -401,7 +401,7 @@ template <class F> static void binary_backward_both(F f, const nt_view *g, const
   }
   if (n < 4) return;
   StorageRef o1(storage_new(n, NT_FLOAT32, NT_CUDA)), o2(storage_new(n, NT_FLOAT32, NT_CUDA));
-  ew_contig_two<F><<<unsigned(ceil_div(n >> 2, 256 * 2)), 256, 0, stream()>>>(f, static_cast<float *>(o1->ptr()),
+  launch(ew_contig_two<F>, unsigned(ceil_div(n >> 2, 256 * 2)), 256, 0, f, static_cast<float *>(o1->ptr()),
                                                                             static_cast<float *>(o2->ptr()), p[0], p[1], p[2], n);
   check_launch("ew_contig_two");
   *out1 = o1.release();
@@ -697,7 +697,7 @@ int nt_sgd_update(const nt_view *param, const nt_view *grad, float lr, float gra
     const float *pg = static_cast<const float *>(grad->storage->ptr()) + grad->offset;
     float *hi = (n >= 4 && aligned16(pp) && aligned16(pg)) ? gemm_tc_refresh_target(param->storage, R, C) : nullptr;
     if (hi) {
-      ew_contig_planes<SgdF, 2><<<unsigned(ceil_div(n >> 2, 256 * 4)), 256, 0, stream()>>>(f, pp, pp, pg, n, hi, hi + n);
+      launch(ew_contig_planes<SgdF, 2>, unsigned(ceil_div(n >> 2, 256 * 4)), 256, 0, f, pp, pp, pg, n, hi, hi + n);
       check_launch("ew_contig_planes");
       param->storage->version += 1;
       storage_touch(param->storage);

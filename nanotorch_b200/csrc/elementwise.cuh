@@ -23,6 +23,7 @@
 #include <type_traits>
 
 #include "ew_tile_tma.cuh"
+#include "launch.cuh"
 #include "nt_core.cuh"
 #include "tf32_split.cuh"
 
@@ -56,6 +57,8 @@ __device__ __forceinline__ void st_stream(float4 *p, float4 v) { __stcs(p, v); }
 template <class F, int NIN>
 __global__ void __launch_bounds__(256) ew_contig(F f, typename F::out_t *out, const typename F::in_t *a,
                                                  const typename F::in_t *b, const typename F::in_t *c, int64_t n) {
+  pdl_trigger();
+  pdl_wait();
   // no __restrict__: in-place ops pass the same pointer as `out` and `a`
   using TI = typename F::in_t;
   using TO = typename F::out_t;
@@ -107,6 +110,8 @@ __global__ void __launch_bounds__(256) ew_contig(F f, typename F::out_t *out, co
 template <class F, int NIN>
 __global__ void __launch_bounds__(256) ew_contig_planes(F f, float *out, const float *a, const float *b, int64_t n,
                                                         float *hi, float *lo) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int UNROLL = 4;
   const int64_t nvec = n >> 2;
   const int64_t base = (int64_t(blockIdx.x) * UNROLL) * blockDim.x + threadIdx.x;
@@ -141,6 +146,8 @@ __global__ void __launch_bounds__(256) ew_contig_planes(F f, float *out, const f
 template <class F, bool ROW_FIRST>
 __global__ void __launch_bounds__(256) ew_contig_rowbcast(F f, float *out, const float *a, const float *row, int64_t nvec,
                                                           uint32_t cvec, uint32_t div_mul, uint32_t div_shift) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int UNROLL = 4;
   const int64_t base = (int64_t(blockIdx.x) * UNROLL) * blockDim.x + threadIdx.x;
   float4 va[UNROLL], vr[UNROLL];
@@ -171,6 +178,8 @@ __global__ void __launch_bounds__(256) ew_contig_rowbcast(F f, float *out, const
 template <class F>
 __global__ void __launch_bounds__(256) ew_contig_rowbcast1(F f, float *out, const float *row, int64_t nvec, uint32_t cvec,
                                                            uint32_t div_mul, uint32_t div_shift) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int UNROLL = 4;
   const int64_t base = (int64_t(blockIdx.x) * UNROLL) * blockDim.x + threadIdx.x;
 #pragma unroll
@@ -190,6 +199,8 @@ __global__ void __launch_bounds__(256) ew_contig_rowbcast1(F f, float *out, cons
 template <class F>
 __global__ void __launch_bounds__(256) ew_contig_two(F f, float *out1, float *out2, const float *g, const float *x1,
                                                      const float *x2, int64_t n) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int UNROLL = 2;
   const int64_t nvec = n >> 2;
   const int64_t base = (int64_t(blockIdx.x) * UNROLL) * blockDim.x + threadIdx.x;
@@ -268,6 +279,8 @@ inline void ew_fast_divisor(int64_t d, uint32_t *mul, uint32_t *shift) {
 
 template <class F, int NIN, int VEC, class IDX, int ND = 0>
 __global__ void __launch_bounds__(256) ew_strided(F f, EwParams p) {
+  pdl_trigger();
+  pdl_wait();
   using TI = typename F::in_t;
   using TO = typename F::out_t;
   if constexpr (VEC == 1) {
@@ -550,7 +563,7 @@ bool ew_launch_tile_pipeline(F f, const IterSpace<NIN + 1> &it, float *out, cons
   }
   const int64_t tiles = int64_t(a.tiles_i) * a.tiles_j * lead;
   const unsigned grid = unsigned(std::min<int64_t>(tiles, sm_count()));
-  tile_tma::ew_tile_tma<F, NIN><<<grid, tile_tma::THREADS, smem, stream()>>>(f, m_out, m0, m1, pf0, pf1, a);
+  launch_ordered(tile_tma::ew_tile_tma<F, NIN>, grid, tile_tma::THREADS, smem, f, m_out, m0, m1, pf0, pf1, a);
   check_launch("ew_tile_tma");
   return true;
 }
@@ -611,7 +624,7 @@ template <class F, int NIN> void ew_launch(F f, const nt_view *const (&views)[NI
     if (all_contig && al && it.numel >= 4) {
       int64_t nvec = it.numel >> 2;
       int64_t blocks = ceil_div(nvec, 256 * 4);
-      ew_contig<F, NIN><<<unsigned(blocks), 256, 0, st>>>(f, out, in[0], in[1], in[2], it.numel);
+      launch(ew_contig<F, NIN>, unsigned(blocks), 256, 0, f, out, in[0], in[1], in[2], it.numel);
       check_launch("ew_contig");
       return;
     }
@@ -631,9 +644,9 @@ template <class F, int NIN> void ew_launch(F f, const nt_view *const (&views)[NI
         const int64_t nvec = it.numel >> 2;
         const unsigned blocks = unsigned(ceil_div(nvec, 256 * 4));
         if (which == 1)
-          ew_contig_rowbcast<F, true><<<blocks, 256, 0, st>>>(f, out, in[1], in[0], nvec, uint32_t(C >> 2), mul, shift);
+          launch(ew_contig_rowbcast<F, true>, blocks, 256, 0, f, out, in[1], in[0], nvec, uint32_t(C >> 2), mul, shift);
         else
-          ew_contig_rowbcast<F, false><<<blocks, 256, 0, st>>>(f, out, in[0], in[1], nvec, uint32_t(C >> 2), mul, shift);
+          launch(ew_contig_rowbcast<F, false>, blocks, 256, 0, f, out, in[0], in[1], nvec, uint32_t(C >> 2), mul, shift);
         check_launch("ew_contig_rowbcast");
         return;
       }
@@ -646,7 +659,7 @@ template <class F, int NIN> void ew_launch(F f, const nt_view *const (&views)[NI
       uint32_t mul, shift;
       ew_fast_divisor(it.shape[1] >> 2, &mul, &shift);
       const int64_t nvec = it.numel >> 2;
-      ew_contig_rowbcast1<F><<<unsigned(ceil_div(nvec, 256 * 4)), 256, 0, st>>>(f, out, in[0], nvec, uint32_t(it.shape[1] >> 2), mul, shift);
+      launch(ew_contig_rowbcast1<F>, unsigned(ceil_div(nvec, 256 * 4)), 256, 0, f, out, in[0], nvec, uint32_t(it.shape[1] >> 2), mul, shift);
       check_launch("ew_contig_rowbcast1");
       return;
     }
@@ -703,7 +716,7 @@ template <class F, int NIN> void ew_launch(F f, const nt_view *const (&views)[NI
         }
         dim3 grid(unsigned(ceil_div(it.shape[dJ], TILE)), unsigned(ceil_div(it.shape[dI], TILE)), unsigned(lead));
         const size_t smem = size_t(n_col) * TILE * TILE_PITCH * sizeof(TI); // at most 2 slots = 33 KB: below the 48 KB default limit
-        ew_tile2d<F, NIN><<<grid, 256, smem, st>>>(f, p);
+        launch_ordered(ew_tile2d<F, NIN>, grid, 256, smem, f, p);
         check_launch("ew_tile2d");
         return;
       }
@@ -737,11 +750,11 @@ template <class F, int NIN> void ew_launch(F f, const nt_view *const (&views)[NI
     if (vec4) {
       int64_t blocks = ceil_div(it.numel / 4, 256 * 4);
       if (idx32 && p.ndim == 2) // the common case ([R, C] with a broadcast or sliced operand): unrolled index math
-        ew_strided<F, NIN, 4, uint32_t, 2><<<unsigned(blocks), 256, 0, st>>>(f, p);
+        launch(ew_strided<F, NIN, 4, uint32_t, 2>, unsigned(blocks), 256, 0, f, p);
       else if (idx32)
-        ew_strided<F, NIN, 4, uint32_t><<<unsigned(blocks), 256, 0, st>>>(f, p);
+        launch(ew_strided<F, NIN, 4, uint32_t>, unsigned(blocks), 256, 0, f, p);
       else
-        ew_strided<F, NIN, 4, uint64_t><<<unsigned(blocks), 256, 0, st>>>(f, p);
+        launch(ew_strided<F, NIN, 4, uint64_t>, unsigned(blocks), 256, 0, f, p);
       check_launch("ew_strided");
       return;
     }
@@ -749,9 +762,9 @@ template <class F, int NIN> void ew_launch(F f, const nt_view *const (&views)[NI
   int64_t blocks = ceil_div(it.numel, 256);
   if (blocks > 0x7fffffffLL) fail_runtime("elementwise: tensor too large for one launch.");
   if (idx32)
-    ew_strided<F, NIN, 1, uint32_t><<<unsigned(blocks), 256, 0, st>>>(f, p);
+    launch(ew_strided<F, NIN, 1, uint32_t>, unsigned(blocks), 256, 0, f, p);
   else
-    ew_strided<F, NIN, 1, uint64_t><<<unsigned(blocks), 256, 0, st>>>(f, p);
+    launch(ew_strided<F, NIN, 1, uint64_t>, unsigned(blocks), 256, 0, f, p);
   check_launch("ew_strided");
 }
 

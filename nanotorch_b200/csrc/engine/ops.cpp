@@ -345,7 +345,7 @@ static PyObject *pow_forward(PyTypeObject *cls, PyObject *const *in) {
 // Products whose last bit decides nothing may be summed in any order (nt_matmul_allow_reorder).
 struct Reorder {
   int was;
-  explicit Reorder(bool on) : was(nt_matmul_allow_reorder(on)) {}
+  explicit Reorder(int level) : was(nt_matmul_allow_reorder(level)) {}
   ~Reorder() { nt_matmul_allow_reorder(was); }
 };
 
@@ -705,7 +705,7 @@ static bool backward_op(FunctionObj *fn, TensorObj *g, PyObject **out, int *n_ou
     saved_ok(fn);
     TensorObj *a = saved(fn, 0), *b = saved(fn, 1);
     if (g->nd != a->nd) return false;
-    const Reorder reorder(true);
+    const Reorder reorder(2);
     *n_out = fn->op == OP_LINEAR ? 3 : 2;
     const nt_view vg = view_of(g), vat = transposed(a), vbt = transposed(b);
     if (need(fn, 0) && need(fn, 1) && g->nd == 2) {

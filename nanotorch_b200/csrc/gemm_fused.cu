@@ -23,6 +23,7 @@
 #include <cmath>
 
 #include "gemm_common.cuh"
+#include "launch.cuh"
 #include "nt_core.cuh"
 #include "tf32_split.cuh"
 #include "tma.cuh"
@@ -468,18 +469,7 @@ template <int BN, bool CLUSTER> static void fg_launch(const FgArgs &g, dim3 grid
     NT_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     configured = smem;
   }
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(fg_threads<BN>, 1, 1);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream();
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = unsigned(g.csize);
-  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = CLUSTER ? 1 : 0;
-  NT_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, g));
+  launch_with(false, CLUSTER ? unsigned(g.csize) : 1u, kernel, grid, fg_threads<BN>, smem, g);
 }
 
 // C = A @ B (+ bias), one collapsed batch stride per operand; false when the shape is outside one launch's limits.

@@ -34,6 +34,7 @@
 #include <unordered_map>
 
 #include "gemm_common.cuh"
+#include "launch.cuh"
 #include "nt_core.cuh"
 #include "tf32_split.cuh"
 #include "tma.cuh"
@@ -71,6 +72,8 @@ __device__ __forceinline__ void split_store4(const SplitArgs &a, int64_t idx, fl
 // One CTA converts a 64 (r) x 64 (k) tile.  Kp is a multiple of 32, so every 4-group of k inside Kp is
 // either fully stored or fully outside.
 __global__ void __launch_bounds__(256) split_pack(SplitArgs a) {
+  pdl_trigger();
+  pdl_wait();
   __shared__ float tile[64][65];
   const int64_t r0 = int64_t(blockIdx.y) * 64, k0 = int64_t(blockIdx.x) * 64;
   const int64_t b = blockIdx.z;
@@ -776,7 +779,7 @@ static void launch_split(const float *src, float *planes, int64_t batch, int64_t
   if (s_k == 1 && base_al && s_r % 4 == 0) a.mode = 1;
   else if (s_r == 1 && s_k != 1 && base_al && s_k % 4 == 0) a.mode = 2;
   dim3 grid{unsigned(ceil_div(Kp, 64)), unsigned(ceil_div(R, 64)), unsigned(batch)};
-  split_pack<<<grid, 256, 0, stream()>>>(a);
+  launch(split_pack, grid, 256, 0, a);
   check_launch("split_pack");
 }
 
@@ -841,6 +844,8 @@ struct NatSplitArgs {
 };
 
 __global__ void __launch_bounds__(256) split_planes(NatSplitArgs a) {
+  pdl_trigger();
+  pdl_wait();
   const int64_t c = (int64_t(blockIdx.x) * 64 + (threadIdx.x & 63)) * 4;
   if (c >= a.Cp) return;
   const int64_t r0 = int64_t(blockIdx.y) * 16 + (threadIdx.x >> 6);
@@ -906,7 +911,7 @@ static void run_split(const nt_storage *s, const PlaneEntry &e) {
   a.s_b = e.s_b;
   a.vec = ((reinterpret_cast<uintptr_t>(a.src) & 15) == 0 && e.s_r % 4 == 0 && e.s_b % 4 == 0) ? 1 : 0;
   dim3 grid{unsigned(ceil_div(e.Cp, 256)), unsigned(ceil_div(e.R, 16)), unsigned(e.batch)};
-  split_planes<<<grid, 256, 0, stream()>>>(a);
+  launch(split_planes, grid, 256, 0, a);
   check_launch("split_planes");
   g_split_launches.fetch_add(1, std::memory_order_relaxed);
 }

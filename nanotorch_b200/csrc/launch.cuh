@@ -1,0 +1,58 @@
+// Kernel launches that overlap with the end of the kernel before them (programmatic dependent launch).
+//
+// A step of a small model is a chain of kernels of 2-5 us each, and between two of them the device spends about as long
+// again draining one grid and setting up the next.  Launched by launch() a grid is set up, and its CTAs take the slots
+// that free up, while the last CTAs of the kernel before it still run; such a kernel starts with pdl_wait(), which waits
+// until that kernel has completed and its writes are visible.  A kernel completes only after its own wait, so by
+// induction everything earlier in the stream has completed too.
+//   - pdl_trigger() lets the next kernel's CTAs in once every CTA of this one is running.  Only the elementwise kernels,
+//     whose CTAs come and go, call it: behind a kernel that holds its SMs to the end, the next one's CTAs piled up on the
+//     SMs that happened to have room (a 384 x 3584 x 1856 product with both gradients 549 -> 604 us).
+//   - launch_ordered() starts a kernel the ordinary way: those whose CTAs must be spread evenly over the SMs.
+//   - Not inside a graph capture: replays went through such edges slower than through plain ones (64 -> 74 us for a
+//     17-launch step).  Not on other streams than the compute stream: kernels there follow events, not kernels.
+// Small training step issued eagerly 97 -> 77 us, softmax loss over 4096 x 1000 205 -> 160 us.
+#pragma once
+
+#include <utility>
+
+#include "nt_core.cuh"
+
+namespace ntb {
+
+// First statement of every kernel that launch() starts, executed by every thread.
+__device__ __forceinline__ void pdl_wait() { asm volatile("griddepcontrol.wait;" ::: "memory"); }
+__device__ __forceinline__ void pdl_trigger() { asm volatile("griddepcontrol.launch_dependents;" ::: "memory"); }
+
+// `overlap`: as the dependent of the kernel before it; `cluster`: CTAs of a cluster along x
+template <class... P, class... A>
+void launch_with(bool overlap, unsigned cluster, void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A &&...args) {
+  cudaLaunchConfig_t cfg{};
+  cfg.gridDim = grid;
+  cfg.blockDim = block;
+  cfg.dynamicSmemBytes = smem;
+  cfg.stream = stream();
+  cudaLaunchAttribute attr[2];
+  unsigned n = 0;
+  if (overlap && !stream_redirected() && !is_capturing()) {
+    attr[n].id = cudaLaunchAttributeProgrammaticStreamSerialization;
+    attr[n++].val.programmaticStreamSerializationAllowed = 1;
+  }
+  if (cluster > 1) {
+    attr[n].id = cudaLaunchAttributeClusterDimension;
+    attr[n].val.clusterDim.x = cluster;
+    attr[n].val.clusterDim.y = attr[n].val.clusterDim.z = 1;
+    ++n;
+  }
+  cfg.attrs = attr;
+  cfg.numAttrs = n;
+  NT_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, std::forward<A>(args)...));
+}
+template <class... P, class... A> void launch(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A &&...args) {
+  launch_with(true, 1, kernel, grid, block, smem, std::forward<A>(args)...);
+}
+template <class... P, class... A> void launch_ordered(void (*kernel)(P...), dim3 grid, dim3 block, size_t smem, A &&...args) {
+  launch_with(false, 1, kernel, grid, block, smem, std::forward<A>(args)...);
+}
+
+} // namespace ntb

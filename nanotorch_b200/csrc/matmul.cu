@@ -7,13 +7,14 @@
 //               ascending k -- the rounding of the reference's CUDA kernels (src/cpp/ops/matmul.cu:60-205);
 //   2           same kernels with separate multiply and add roundings: bit for bit the reference's
 //               CPU triple loop (src/cpp/ops/matmul.cu:21-57).
-// Tiny products of modes 1 and 3 take the exact kernels too, where they may also be split along k; small and middle
-// ones of mode 1 take the tensor-core kernel of gemm_fused.cu.
+// Tiny products of modes 1 and 3 take the exact kernels too; small and middle ones of mode 1 take the tensor-core
+// kernel of gemm_fused.cu or, where the order of the sum is free, the exact kernels with k-splits.
 // Operand tiles are read straight from the strided views -- vectorised along whichever of the two
 // matrix dims has unit stride -- so the transposed views of MatmulOp.backward
 // (autograd/ops_binary.py:265-266) and N % 4 != 0 never drop to a one-thread-per-output kernel as
 // they do in the reference (src/cpp/ops/matmul.cu:218-233).
 // Other dtypes (Int32/Int64/Float64) use a plain one-output-per-thread kernel.
+#include "launch.cuh"
 #include "nt_core.cuh"
 #include "sgemm.cuh"
 
@@ -42,7 +43,7 @@ void gemm_tc_pair_role(int role);
 void gemm_tc_set_pair_overlap(bool on);
 void gemm_tc_split_stats(uint64_t *launches, uint64_t *hits);
 static std::atomic<int> g_natural_planes{1};
-static thread_local bool t_reorder = false; // nt_matmul_allow_reorder
+static thread_local int t_reorder = 0; // nt_matmul_allow_reorder
 
 static std::atomic<int> g_matmul_mode{1};
 static std::atomic<int64_t> g_tc_min_macs{int64_t(1) << 21}; // batch*M*N*K at or below this: exact FP32 kernel
@@ -71,7 +72,7 @@ __global__ void matmul_naive(const T *A, const T *B, T *C, int64_t M, int64_t N,
 static bool al16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
 // How a product runs on the CUDA cores: tile edge, CTAs along k (a cluster), and the time that is expected of it.
-// Clocks per k of one CTA, measured: alone on its SM (a chain of shared-memory loads and multiply-adds: 50 for the
+// Tile 8 stands for the kernel for a few rows.  Clocks per k of one CTA, measured: alone on its SM (a chain of shared-memory loads and multiply-adds: 50 for the
 // 32-wide tile, 75 for 64, 345 for 128 x 256) and with the SM full (20, 70, 350).  So a product with few tiles takes
 // the small tile and many k-splits (256 x 784 x 256: 8.4 us with 64 tiles x 8, against 21 us unsplit and 145 us in two
 // 128 x 256 tiles), one with many tiles the large tile (52 TFLOP/s; 35 with the 64-wide tile).
@@ -80,8 +81,12 @@ struct SimtPlan {
   int64_t k_per_split = 0;
   double us = 1e30;
 };
-static SimtPlan plan_simt(int64_t batch, int64_t M, int64_t N, int64_t K, bool may_split) {
+static SimtPlan plan_simt(int64_t batch, int64_t M, int64_t N, int64_t K, bool thin, bool may_split) {
   SimtPlan best;
+  if (thin) {
+    const double rounds = std::ceil(double(ceil_div(N, TH_N)) * double(batch) / sm_count());
+    best = SimtPlan{8, 1, K, 3.0 + rounds * double(K) * 6.5 / 1900};
+  }
   for (int tile : {128, 64, 32}) {
     const double tiles = double(ceil_div(M, tile)) * double(ceil_div(N, tile == 128 ? LG_N : tile)) * double(batch);
     if (ceil_div(M, tile) > 65535) continue;
@@ -105,18 +110,7 @@ template <int T, bool A_K, bool B_K, bool FUSED> static void launch_small(const 
     NT_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     configured = true;
   }
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3((T / 4) * (T / 4), 1, 1);
-  cfg.dynamicSmemBytes = smem;
-  cfg.stream = stream();
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeClusterDimension;
-  attr[0].val.clusterDim.x = unsigned(g.splits);
-  attr[0].val.clusterDim.y = attr[0].val.clusterDim.z = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = g.splits > 1 ? 1 : 0;
-  NT_CUDA_CHECK(cudaLaunchKernelEx(&cfg, kernel, g));
+  launch_with(false, unsigned(g.splits), kernel, grid, (T / 4) * (T / 4), smem, g);
 }
 template <int T, bool FUSED> static void launch_small(const GemmArgs &g, dim3 grid, bool a_k, bool b_k) {
   if (a_k && b_k) launch_small<T, true, true, FUSED>(g, grid);
@@ -132,7 +126,7 @@ template <bool A_K, bool B_K, bool FUSED> static void launch_large(const GemmArg
     NT_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, LG_SMEM));
     configured = true;
   }
-  kernel<<<grid, LG_NT, LG_SMEM, stream()>>>(g);
+  launch_ordered(kernel, grid, LG_NT, LG_SMEM, g);
 }
 template <bool FUSED> static void launch_large(const GemmArgs &g, dim3 grid, bool a_k, bool b_k) {
   if (a_k && b_k) launch_large<true, true, FUSED>(g, grid);
@@ -153,6 +147,17 @@ static void sgemm_simt(GemmArgs g, int64_t nbatch, bool fused, const SimtPlan &p
   g.c_vec = g.N % 4 == 0 && al16(g.C);
   g.splits = plan.splits;
   g.k_per_split = plan.k_per_split;
+  if (plan.tile == 8) {
+    static bool configured = false;
+    if (!configured) {
+      NT_CUDA_CHECK(cudaFuncSetAttribute(sgemm_thin<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, TH_SMEM));
+      NT_CUDA_CHECK(cudaFuncSetAttribute(sgemm_thin<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, TH_SMEM));
+      configured = true;
+    }
+    launch_ordered(fused ? sgemm_thin<true> : sgemm_thin<false>, dim3(unsigned(ceil_div(g.N, TH_N)), 1, unsigned(nbatch)), TH_NT, TH_SMEM, g);
+    check_launch("sgemm");
+    return;
+  }
   if (nbatch > 65535 || ceil_div(g.M, plan.tile) > 65535) fail_runtime("matmul: too many tiles for one launch.");
   dim3 grid{unsigned(ceil_div(g.N, plan.tile == 128 ? LG_N : plan.tile) * plan.splits), unsigned(ceil_div(g.M, plan.tile)), unsigned(nbatch)};
   if (plan.tile == 128) {
@@ -182,9 +187,9 @@ int nt_set_matmul_mode(int mode) {
   gemm_tc_set_promoted(mode == 1);
   NT_API_END
 }
-int nt_matmul_allow_reorder(int on) {
+int nt_matmul_allow_reorder(int level) {
   const int was = t_reorder;
-  t_reorder = on != 0;
+  t_reorder = level < 0 ? 0 : level;
   return was;
 }
 int nt_get_matmul_mode(void) { return g_matmul_mode.load(); }
@@ -272,9 +277,11 @@ static nt_storage *matmul_impl(const nt_view *x1, const nt_view *x2, const nt_vi
     // Above that threshold mode 1 goes by expected time (a threshold of 0 sends everything through planes): planes, the
     // tensor-core kernel that does without them -- same bits -- and, where the caller does not need those very bits,
     // the CUDA cores, which finish first below some 5e8 multiply-adds (784 x 256 x 256: 7 us against 11.5 and 20).
-    const SimtPlan simt = plan_simt(nbatch, M, N, K, /*may_split=*/mode == 1 || mode == 3);
     const bool by_time = mode == 1 && big_enough && min_macs > 0;
     const double tc_us = by_time ? gemm_tc_expected_us(nbatch, M, N, K) : 0, fused_us = by_time ? gemm_fused_expected_us(nbatch, M, N, K) : 0;
+    const bool thin = M <= TH_M && b_sn == 1 && nbatch <= 65535;
+    const bool may_split = (mode == 1 || mode == 3) && t_reorder >= (big_enough ? 1 : 2);
+    const SimtPlan simt = plan_simt(nbatch, M, N, K, thin, may_split);
     const bool on_cuda_cores = by_time && t_reorder && simt.us < std::min(tc_us, fused_us);
     if ((mode == 1 || mode == 3) && K > 0 && big_enough && !on_cuda_cores) {
       // the tensor-core path takes a single (collapsed) batch stride per operand
@@ -317,7 +324,7 @@ static nt_storage *matmul_impl(const nt_view *x1, const nt_view *x2, const nt_vi
         const T *B = static_cast<const T *>(x2->storage->ptr()) + x2->offset;
         int64_t blocks = ceil_div(total, 256);
         if (blocks > 0x7fffffffLL) fail_runtime("matmul: output too large for one launch.");
-        matmul_naive<T><<<unsigned(blocks), 256, 0, stream()>>>(A, B, static_cast<T *>(o->ptr()), M, N, K, a_sm, a_sk,
+        launch_ordered(matmul_naive<T>, unsigned(blocks), 256, 0, A, B, static_cast<T *>(o->ptr()), M, N, K, a_sm, a_sk,
                                                                 b_sk, b_sn, bi, total);
         check_launch("matmul_naive");
       }

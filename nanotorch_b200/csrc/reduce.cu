@@ -71,6 +71,7 @@ template <class Op>
 __global__ void __launch_bounds__(256) reduce_rows(const float *__restrict__ in, float *__restrict__ out,
                                                    float *__restrict__ partials, unsigned *__restrict__ tickets,
                                                    KeepIndex keep, int64_t L, int S, int64_t chunk, float divisor) {
+  pdl_wait();
   // divisor != 0: the finished value is divided by it (one IEEE division of the rounded fp32 result:
   // the bits of a sum kernel followed by a divide kernel -- MeanOp's two steps in one launch)
   __shared__ float warp_part[8];
@@ -156,6 +157,7 @@ __global__ void __launch_bounds__(256) reduce_rows(const float *__restrict__ in,
 template <class Op>
 __global__ void __launch_bounds__(256) reduce_rows_warp(const float *__restrict__ in, float *__restrict__ out,
                                                         KeepIndex keep, int64_t n_rows, int64_t L, float divisor) {
+  pdl_wait();
   const int64_t row0 = (int64_t(blockIdx.x) * 8 + (threadIdx.x >> 5)) * 4;
   if (row0 >= n_rows) return;
   const int lane = threadIdx.x & 31;
@@ -203,6 +205,7 @@ __global__ void __launch_bounds__(256) reduce_cols(const float *__restrict__ in,
                                                    float *__restrict__ partials, unsigned *__restrict__ tickets,
                                                    KeepIndex keep_outer, int64_t R, int64_t C, int64_t sR,
                                                    int64_t rows_per_split, float divisor) {
+  pdl_wait();
   constexpr int TW = 32 * VEC; // tile width in columns
   __shared__ float part[8][TW];
   __shared__ bool is_last;
@@ -292,6 +295,7 @@ __global__ void __launch_bounds__(256) reduce_cols_wide(const float *__restrict_
                                                         float *__restrict__ partials, unsigned *__restrict__ tickets,
                                                         KeepIndex keep_outer, int64_t R, int64_t C, int64_t sR,
                                                         int64_t rows_per_split, float divisor) {
+  pdl_wait();
   __shared__ bool is_last;
   const int64_t c0 = int64_t(blockIdx.x) * 1024 + threadIdx.x * 4;
   const int S = gridDim.y, split = blockIdx.y;
@@ -415,6 +419,7 @@ template <class T, class O, class Op, int GROUP>
 __global__ void __launch_bounds__(256) reduce_generic(const T *__restrict__ in, void *__restrict__ out_raw,
                                                       KeepIndex keep, KeepIndex drop, int64_t n_keep,
                                                       int64_t n_drop) {
+  pdl_wait();
   constexpr int PER_CTA = 256 / GROUP;
   __shared__ Item<O> buf[256];
   const int sub = threadIdx.x / GROUP, t = threadIdx.x % GROUP;
@@ -518,7 +523,7 @@ template <class Op> static bool try_fast_f32(const nt_view *x, const Plan &pl, f
     if (L < 1024 && n_rows >= 64) {
       int64_t blocks = ceil_div(n_rows, 32);
       if (blocks > 0x7fffffffLL) return false;
-      reduce_rows_warp<Op><<<unsigned(blocks), 256, 0, st>>>(in, out, pl.keep, n_rows, L, divisor);
+      launch(reduce_rows_warp<Op>, unsigned(blocks), 256, 0, in, out, pl.keep, n_rows, L, divisor);
       check_launch("reduce_rows_warp");
       return true;
     }
@@ -537,7 +542,7 @@ template <class Op> static bool try_fast_f32(const nt_view *x, const Plan &pl, f
       partials = static_cast<float *>(device_alloc(size_t(n_rows * S) * sizeof(float), &rounded));
       tk = tickets(n_rows);
     }
-    reduce_rows<Op><<<unsigned(n_rows * S), 256, 0, st>>>(in, out, partials, tk, pl.keep, L, int(S), chunk, divisor);
+    launch(reduce_rows<Op>, unsigned(n_rows * S), 256, 0, in, out, partials, tk, pl.keep, L, int(S), chunk, divisor);
     if (partials) device_free(partials, rounded); // stream-ordered reuse: later work queues behind this launch
     check_launch("reduce_rows");
     return true;
@@ -574,7 +579,7 @@ template <class Op> static bool try_fast_f32(const nt_view *x, const Plan &pl, f
         tk = tickets(Z * tiles);
       }
       dim3 grid{unsigned(tiles), unsigned(S), unsigned(Z)};
-      reduce_cols_wide<Op><<<grid, 256, 0, st>>>(in, out, partials, tk, outer, R, C, sR, rows_per_split, divisor);
+      launch(reduce_cols_wide<Op>, grid, 256, 0, in, out, partials, tk, outer, R, C, sR, rows_per_split, divisor);
       if (partials) device_free(partials, rounded);
       check_launch("reduce_cols_wide");
       return true;
@@ -598,9 +603,9 @@ template <class Op> static bool try_fast_f32(const nt_view *x, const Plan &pl, f
     }
     dim3 grid{unsigned(tiles), unsigned(S), unsigned(Z)};
     if (vec)
-      reduce_cols<Op, 4><<<grid, 256, 0, st>>>(in, out, partials, tk, outer, R, C, sR, rows_per_split, divisor);
+      launch(reduce_cols<Op, 4>, grid, 256, 0, in, out, partials, tk, outer, R, C, sR, rows_per_split, divisor);
     else
-      reduce_cols<Op, 1><<<grid, 256, 0, st>>>(in, out, partials, tk, outer, R, C, sR, rows_per_split, divisor);
+      launch(reduce_cols<Op, 1>, grid, 256, 0, in, out, partials, tk, outer, R, C, sR, rows_per_split, divisor);
     if (partials) device_free(partials, rounded);
     check_launch("reduce_cols");
     return true;
@@ -613,11 +618,11 @@ template <class T, class O, class Op> static void launch_generic(const nt_view *
   cudaStream_t st = stream();
   if (pl.n_drop > 256) {
     if (pl.n_keep > 0x7fffffffLL) fail_runtime("reduction: too many kept elements.");
-    reduce_generic<T, O, Op, 256><<<unsigned(pl.n_keep), 256, 0, st>>>(in, out, pl.keep, pl.drop, pl.n_keep, pl.n_drop);
+    launch(reduce_generic<T, O, Op, 256>, unsigned(pl.n_keep), 256, 0, in, out, pl.keep, pl.drop, pl.n_keep, pl.n_drop);
   } else {
     int64_t blocks = ceil_div(pl.n_keep, 8);
     if (blocks > 0x7fffffffLL) fail_runtime("reduction: too many kept elements.");
-    reduce_generic<T, O, Op, 32><<<unsigned(blocks), 256, 0, st>>>(in, out, pl.keep, pl.drop, pl.n_keep, pl.n_drop);
+    launch(reduce_generic<T, O, Op, 32>, unsigned(blocks), 256, 0, in, out, pl.keep, pl.drop, pl.n_keep, pl.n_drop);
   }
   check_launch("reduce_generic");
 }
@@ -683,6 +688,7 @@ __device__ __forceinline__ int64_t slice_offset(const KeepIndex &k, int64_t lin)
 __global__ void __launch_bounds__(256) extremum_count_rows(const float *__restrict__ x, const float *__restrict__ m,
                                                            int *__restrict__ count, SliceScalars sc, int64_t L,
                                                            int chunks_per_row, int64_t chunk) {
+  pdl_wait();
   __shared__ int warp_cnt[8];
   const int64_t row = blockIdx.x / chunks_per_row;
   const int c = int(blockIdx.x - row * chunks_per_row);
@@ -719,6 +725,7 @@ __global__ void __launch_bounds__(256) extremum_count_rows(const float *__restri
 __global__ void __launch_bounds__(256) extremum_count_cols(const float *__restrict__ x, const float *__restrict__ m,
                                                            int *__restrict__ count, SliceScalars sc, int64_t R, int64_t C,
                                                            int64_t sR, int64_t rows_per_block, int vec) {
+  pdl_wait();
   __shared__ int part[8][128];
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
   const int64_t c0 = int64_t(blockIdx.x) * 128 + lane * 4;
@@ -760,6 +767,7 @@ __global__ void __launch_bounds__(256) extremum_apply(const float *__restrict__ 
                                                       const float *__restrict__ m, const int *__restrict__ count,
                                                       float *__restrict__ out, SliceScalars sc, int64_t n_outer, int64_t L,
                                                       int64_t sR, int vec) {
+  pdl_wait();
   // ROWS: n_outer slices of L elements; COLS: n_outer rows of L columns (slice = column).
   // total < 2^40 is guaranteed by the host; the common case fits 32-bit division.
   const int64_t total = n_outer * L;
@@ -815,6 +823,7 @@ __global__ void __launch_bounds__(256) extremum_apply_vec(const float *__restric
                                                           const float *__restrict__ m, const int *__restrict__ count,
                                                           float *__restrict__ out, SliceScalars sc, int64_t L, int64_t sR,
                                                           int chunks) {
+  pdl_wait();
   const int64_t outer = blockIdx.x / chunks;
   const int64_t inner = int64_t(blockIdx.x - outer * chunks) * 1024 + threadIdx.x * 4;
   if (inner >= L) return;
@@ -847,6 +856,7 @@ __global__ void __launch_bounds__(256) extremum_apply_count_vec(const float *__r
                                                                 const float *__restrict__ m, int *__restrict__ count,
                                                                 float *__restrict__ out, SliceScalars sc, int64_t L,
                                                                 int64_t sR, int chunks, int gm_vec) {
+  pdl_wait();
   // a CTA owns 4096 consecutive elements of ONE outer index (a slice for ROWS, a matrix row for COLS); a thread
   // owns four 128-bit vectors 1024 elements apart, all loaded before the first use
   const int64_t outer = blockIdx.x / chunks;
@@ -902,6 +912,7 @@ __global__ void __launch_bounds__(256) extremum_fix_ties(const float *__restrict
                                                          const float *__restrict__ m, const int *__restrict__ count,
                                                          float *__restrict__ out, SliceScalars sc, int64_t n_slices,
                                                          int64_t n_drop, int64_t sR) {
+  pdl_wait();
   if (ROWS) {
     const int64_t slice = blockIdx.x;
     if (count[slice] <= 1) return;
@@ -925,6 +936,7 @@ template <int VPT>
 __global__ void __launch_bounds__(256) extremum_rows_onepass(const float *__restrict__ x, const float *__restrict__ g,
                                                              const float *__restrict__ m, float *__restrict__ out,
                                                              SliceScalars sc, int64_t L) {
+  pdl_wait();
   __shared__ int warp_cnt[8];
   const int64_t row = blockIdx.x;
   const float4 *pv = reinterpret_cast<const float4 *>(x + slice_offset(sc.x_keep, row));
@@ -1010,11 +1022,11 @@ static bool extremum_backward_fused(const nt_view *g, const nt_view *x, const nt
     if (vec && L <= 16384 && pl.n_keep >= sm_count() && pl.n_keep <= 0x7fffffffLL) {
       const unsigned grid = unsigned(pl.n_keep);
       const int64_t per_thread = ceil_div(L / 4, 256);
-      if (per_thread <= 1) extremum_rows_onepass<1><<<grid, 256, 0, st>>>(xp, gp, mp, out, sc, L);
-      else if (per_thread <= 2) extremum_rows_onepass<2><<<grid, 256, 0, st>>>(xp, gp, mp, out, sc, L);
-      else if (per_thread <= 4) extremum_rows_onepass<4><<<grid, 256, 0, st>>>(xp, gp, mp, out, sc, L);
-      else if (per_thread <= 8) extremum_rows_onepass<8><<<grid, 256, 0, st>>>(xp, gp, mp, out, sc, L);
-      else extremum_rows_onepass<16><<<grid, 256, 0, st>>>(xp, gp, mp, out, sc, L);
+      if (per_thread <= 1) launch(extremum_rows_onepass<1>, grid, 256, 0, xp, gp, mp, out, sc, L);
+      else if (per_thread <= 2) launch(extremum_rows_onepass<2>, grid, 256, 0, xp, gp, mp, out, sc, L);
+      else if (per_thread <= 4) launch(extremum_rows_onepass<4>, grid, 256, 0, xp, gp, mp, out, sc, L);
+      else if (per_thread <= 8) launch(extremum_rows_onepass<8>, grid, 256, 0, xp, gp, mp, out, sc, L);
+      else launch(extremum_rows_onepass<16>, grid, 256, 0, xp, gp, mp, out, sc, L);
       check_launch("extremum_rows_onepass");
       return true;
     }
@@ -1036,14 +1048,14 @@ static bool extremum_backward_fused(const nt_view *g, const nt_view *x, const nt
     for (int k = 0; k < sc.x_keep.ndim; ++k) vec = vec && (sc.x_keep.strides[k] % 4 == 0);
     const int64_t vchunks = ceil_div(L, 4096);
     if (vec && pl.n_keep * vchunks <= 0x7fffffffLL) {
-      extremum_apply_count_vec<true><<<unsigned(pl.n_keep * vchunks), 256, 0, st>>>(xp, gp, mp, count, out, sc, L, 0, int(vchunks), 0);
+      launch(extremum_apply_count_vec<true>, unsigned(pl.n_keep * vchunks), 256, 0, xp, gp, mp, count, out, sc, L, 0, int(vchunks), 0);
       check_launch("extremum_apply_count_vec");
-      extremum_fix_ties<true><<<unsigned(pl.n_keep), 256, 0, st>>>(xp, gp, mp, count, out, sc, pl.n_keep, L, 0);
+      launch(extremum_fix_ties<true>, unsigned(pl.n_keep), 256, 0, xp, gp, mp, count, out, sc, pl.n_keep, L, 0);
       check_launch("extremum_fix_ties");
     } else {
-      extremum_count_rows<<<unsigned(pl.n_keep * chunks), 256, 0, st>>>(xp, mp, count, sc, L, int(chunks), chunk);
+      launch(extremum_count_rows, unsigned(pl.n_keep * chunks), 256, 0, xp, mp, count, sc, L, int(chunks), chunk);
       check_launch("extremum_count_rows");
-      extremum_apply<true><<<unsigned(apply_blocks), 256, 0, st>>>(xp, gp, mp, count, out, sc, pl.n_keep, L, 0, vec ? 1 : 0);
+      launch(extremum_apply<true>, unsigned(apply_blocks), 256, 0, xp, gp, mp, count, out, sc, pl.n_keep, L, 0, vec ? 1 : 0);
       check_launch("extremum_apply");
     }
   } else {
@@ -1065,14 +1077,14 @@ static bool extremum_backward_fused(const nt_view *g, const nt_view *x, const nt
     if (vec && R * vchunks <= 0x7fffffffLL) {
       const int gm_vec = (sc.g_keep.ndim == 1 && sc.g_keep.strides[0] == 1 && sc.m_keep.ndim == 1 && sc.m_keep.strides[0] == 1 &&
                           aligned16(gp) && aligned16(mp)) ? 1 : 0;
-      extremum_apply_count_vec<false><<<unsigned(R * vchunks), 256, 0, st>>>(xp, gp, mp, count, out, sc, C, sR, int(vchunks), gm_vec);
+      launch(extremum_apply_count_vec<false>, unsigned(R * vchunks), 256, 0, xp, gp, mp, count, out, sc, C, sR, int(vchunks), gm_vec);
       check_launch("extremum_apply_count_vec");
-      extremum_fix_ties<false><<<unsigned(ceil_div(C, 256)), 256, 0, st>>>(xp, gp, mp, count, out, sc, C, R, sR);
+      launch(extremum_fix_ties<false>, unsigned(ceil_div(C, 256)), 256, 0, xp, gp, mp, count, out, sc, C, R, sR);
       check_launch("extremum_fix_ties");
     } else {
-      extremum_count_cols<<<grid, 256, 0, st>>>(xp, mp, count, sc, R, C, sR, rows_per_block, vec ? 1 : 0);
+      launch(extremum_count_cols, grid, 256, 0, xp, mp, count, sc, R, C, sR, rows_per_block, vec ? 1 : 0);
       check_launch("extremum_count_cols");
-      extremum_apply<false><<<unsigned(apply_blocks), 256, 0, st>>>(xp, gp, mp, count, out, sc, R, C, sR, vec ? 1 : 0);
+      launch(extremum_apply<false>, unsigned(apply_blocks), 256, 0, xp, gp, mp, count, out, sc, R, C, sR, vec ? 1 : 0);
       check_launch("extremum_apply");
     }
   }
@@ -1128,7 +1140,7 @@ int nt_sum_rows_noalloc(const float *in, int64_t n_rows, int64_t row_len, float 
   if (row_len < 1024 && n_rows >= 64) {
     int64_t blocks = ceil_div(n_rows, 32);
     if (blocks > 0x7fffffffLL) fail_invalid("nt_sum_rows_noalloc: too many rows for one launch.");
-    reduce_rows_warp<RSum><<<unsigned(blocks), 256, 0, st>>>(in, out, keep, n_rows, row_len, 0.0f);
+    launch(reduce_rows_warp<RSum>, unsigned(blocks), 256, 0, in, out, keep, n_rows, row_len, 0.0f);
     check_launch("reduce_rows_warp");
     return NT_OK;
   }
@@ -1146,7 +1158,7 @@ int nt_sum_rows_noalloc(const float *in, int64_t n_rows, int64_t row_len, float 
                  " partials and " + std::to_string(NOALLOC_MAX_ROWS) + " row tickets. Use nt_sum for larger inputs.");
   if (S > 1) // tickets must start at zero whatever the previous call left behind
     NT_CUDA_CHECK(cudaMemsetAsync(scratch->tickets, 0, size_t(n_rows) * sizeof(unsigned), st));
-  reduce_rows<RSum><<<unsigned(n_rows * S), 256, 0, st>>>(in, out, scratch->partials, scratch->tickets, keep, row_len,
+  launch(reduce_rows<RSum>, unsigned(n_rows * S), 256, 0, in, out, scratch->partials, scratch->tickets, keep, row_len,
                                                         int(S), chunk, 0.0f);
   check_launch("reduce_rows");
   NT_API_END

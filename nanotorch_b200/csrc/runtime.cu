@@ -8,6 +8,7 @@
 #include <set>
 #include <unordered_map>
 
+#include "launch.cuh"
 #include "nt_core.cuh"
 
 namespace ntb {
@@ -120,6 +121,7 @@ cudaStream_t compute_stream() {
   ensure_streams_locked(r);
   return r.compute;
 }
+bool stream_redirected() { return rt().redirect != nullptr; }
 StreamRedirect::StreamRedirect(cudaStream_t to) {
   Runtime &r = rt();
   std::lock_guard<std::mutex> lk(r.mu);
@@ -460,6 +462,8 @@ void require_same_device(const nt_view *a, const nt_view *b, const char *fname) 
 // ------------------------------------------------------------------------------------------
 // kernels of this file
 template <class T> __global__ void fill_kernel(T *out, int64_t n, T value) {
+  pdl_trigger();
+  pdl_wait();
   int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   int64_t step = int64_t(gridDim.x) * blockDim.x;
   for (; i < n; i += step) out[i] = value;
@@ -483,6 +487,8 @@ template <class S, class D> __device__ __forceinline__ D cast_value(S x) {
   }
 }
 template <class S, class D> __global__ void cast_kernel(const S *in, D *out, int64_t n) {
+  pdl_trigger();
+  pdl_wait();
   int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   int64_t step = int64_t(gridDim.x) * blockDim.x;
   for (; i < n; i += step) out[i] = cast_value<S, D>(in[i]);
@@ -490,6 +496,8 @@ template <class S, class D> __global__ void cast_kernel(const S *in, D *out, int
 
 // eye(n): ones where row == column, i.e. at every (n + 1)-th element (src/cpp/factory.cu:51-59)
 template <class T> __global__ void eye_kernel(T *out, int64_t n) {
+  pdl_trigger();
+  pdl_wait();
   int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   int64_t step = int64_t(gridDim.x) * blockDim.x;
   for (; i < n * n; i += step) out[i] = static_cast<T>(i % (n + 1) == 0 ? 1 : 0);
@@ -497,6 +505,8 @@ template <class T> __global__ void eye_kernel(T *out, int64_t n) {
 
 // arange: static_cast<T>(start + i * step) in int64, as the reference's host loop (src/cpp/factory.cu:62-71)
 template <class T> __global__ void arange_kernel(T *out, int64_t n, int64_t start, int64_t inc) {
+  pdl_trigger();
+  pdl_wait();
   int64_t i = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
   int64_t step = int64_t(gridDim.x) * blockDim.x;
   for (; i < n; i += step) out[i] = static_cast<T>(start + i * inc);
@@ -522,6 +532,8 @@ __host__ __device__ inline void philox4x32_10(uint32_t (&c)[4], uint32_t k0, uin
 
 // U[0,1): float = top 24 bits * 2^-24 (4 per block); double = top 53 bits of two words * 2^-53 (2 per block)
 template <class T> __global__ void philox_uniform_kernel(T *out, int64_t n, uint64_t seed, uint64_t offset) {
+  pdl_trigger();
+  pdl_wait();
   constexpr int PER = std::is_same_v<T, float> ? 4 : 2;
   const int64_t blocks = (n + PER - 1) / PER;
   int64_t b = int64_t(blockIdx.x) * blockDim.x + threadIdx.x;
@@ -557,7 +569,7 @@ static int grid_for(int64_t n, int block) {
 
 template <class T> static void fill_device(nt_storage *s, T value) {
   if (s->n == 0) return;
-  fill_kernel<T><<<grid_for(s->n, 256), 256, 0, stream()>>>(static_cast<T *>(s->ptr()), s->n, value);
+  launch(fill_kernel<T>, grid_for(s->n, 256), 256, 0, static_cast<T *>(s->ptr()), s->n, value);
   check_launch("fill");
 }
 
@@ -948,7 +960,7 @@ int nt_storage_cast(nt_storage *s, int dtype, nt_storage **out) {
         const S *in = static_cast<const S *>(s->ptr());
         D *dst = static_cast<D *>(o->ptr());
         if (s->device == NT_CUDA) {
-          cast_kernel<S, D><<<grid_for(s->n, 256), 256, 0, stream()>>>(in, dst, s->n);
+          launch(cast_kernel<S, D>, grid_for(s->n, 256), 256, 0, in, dst, s->n);
           check_launch("cast");
         } else {
           // host staging buffers only: the cast of a CPU storage is bookkeeping for tensor
@@ -1032,7 +1044,7 @@ int nt_eye(int64_t n, int dtype, int device, nt_storage **out) {
     T *p = static_cast<T *>(o->ptr());
     if (device == NT_CUDA) {
       if (n > 0) {
-        eye_kernel<T><<<grid_for(n * n, 256), 256, 0, stream()>>>(p, n);
+        launch(eye_kernel<T>, grid_for(n * n, 256), 256, 0, p, n);
         check_launch("eye");
       }
     } else {
@@ -1052,7 +1064,7 @@ int nt_arange(int64_t n, int64_t start, int64_t step, int dtype, int device, nt_
     T *p = static_cast<T *>(o->ptr());
     if (device == NT_CUDA) {
       if (n > 0) {
-        arange_kernel<T><<<grid_for(n, 256), 256, 0, stream()>>>(p, n, start, step);
+        launch(arange_kernel<T>, grid_for(n, 256), 256, 0, p, n, start, step);
         check_launch("arange");
       }
     } else {
@@ -1091,7 +1103,7 @@ int nt_uniform(int64_t n, int dtype, int device, nt_storage **out) {
       constexpr int per = std::is_same_v<T, float> ? 4 : 2;
       const int64_t blocks = ceil_div(n, per);
       if (n > 0) {
-        philox_uniform_kernel<T><<<grid_for(blocks, 256), 256, 0, stream()>>>(static_cast<T *>(o->ptr()), n,
+        launch(philox_uniform_kernel<T>, grid_for(blocks, 256), 256, 0, static_cast<T *>(o->ptr()), n,
                                                                               rt().philox_seed, rt().philox_offset);
         check_launch("philox_uniform");
       }

@@ -1,4 +1,4 @@
-// Exact FP32 products on the CUDA cores: two kernels over strided operands, each output accumulated in ascending k
+// Exact FP32 products on the CUDA cores: three kernels over strided operands, each output accumulated in ascending k
 // with one rounding per multiply-add (FUSED) or a rounded product and a rounded sum (the reference's CPU loop).
 //
 //   sgemm_small<T>  T x T output tiles (T = 64 or 32), cp.async into a 3-stage ring of 32-deep k-slices, 4 x 4 outputs
@@ -7,6 +7,7 @@
 //                   and took 42 us.  With `splits` > 1 a cluster of CTAs shares a tile, each over its own k-range; the
 //                   partial tiles meet in distributed shared memory and are added in rank order, so the result
 //                   does not depend on timing (one launch, no workspace).
+//   sgemm_thin      at most 8 rows: a column per lane, see there.
 //   sgemm_large     128 x 256 tiles, 8 x 16 outputs per thread as packed pairs: fma.rn.f32x2 does two IEEE fused
 //                   multiply-adds per instruction, which leaves issue slots for loads and moves (a scalar FFMA takes
 //                   every slot of its scheduler).  8 x 16 because shared memory feeds registers at 128 bytes a clock:
@@ -16,6 +17,7 @@
 #include <cooperative_groups.h>
 
 #include "cp_async.cuh"
+#include "launch.cuh"
 #include "nt_core.cuh"
 
 namespace ntb {
@@ -128,9 +130,10 @@ __global__ void __launch_bounds__((T / 4) * (T / 4)) sgemm_small(GemmArgs g) {
     if (s + SG_STAGES - 1 < steps) fetch(s + SG_STAGES - 1);
     cp_async_commit();
     const float *as = sg_smem + (s % SG_STAGES) * (AF + BF), *bs = as + AF;
-#pragma unroll
-    for (int k = 0; k < SG_BK; k += 4) {
-      float a[4][4], b[4][4]; // [row][k]
+    // operands of four values of k at a time, the next four on their way while these multiply: few warps share an SM
+    // here, so a load's latency is covered inside the warp or not at all
+    float a[2][4][4], b[2][4][4]; // [buffer][row][k]
+    auto operands = [&](int to, int k) {
 #pragma unroll
       for (int i = 0; i < 4; ++i) {
         const float4 va = A_K ? *reinterpret_cast<const float4 *>(as + (ty + G * i) * (SG_BK + 4) + k)
@@ -140,18 +143,24 @@ __global__ void __launch_bounds__((T / 4) * (T / 4)) sgemm_small(GemmArgs g) {
         const float fa[4] = {va.x, va.y, va.z, va.w}, fb[4] = {vb.x, vb.y, vb.z, vb.w};
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          if (A_K) a[i][e] = fa[e];
-          else a[e][i] = fa[e];
-          if (B_K) b[i][e] = fb[e];
-          else b[e][i] = fb[e];
+          if (A_K) a[to][i][e] = fa[e];
+          else a[to][e][i] = fa[e];
+          if (B_K) b[to][i][e] = fb[e];
+          else b[to][e][i] = fb[e];
         }
       }
+    };
+    operands(0, 0);
+#pragma unroll
+    for (int k = 0; k < SG_BK; k += 4) {
+      const int cur = (k >> 2) & 1;
+      if (k + 4 < SG_BK) operands(cur ^ 1, k + 4);
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk)
 #pragma unroll
         for (int i = 0; i < 4; ++i)
 #pragma unroll
-          for (int j = 0; j < 4; ++j) acc[i][j] = mad<FUSED>(a[i][kk], b[j][kk], acc[i][j]);
+          for (int j = 0; j < 4; ++j) acc[i][j] = mad<FUSED>(a[cur][i][kk], b[cur][j][kk], acc[i][j]);
     }
   }
 
@@ -200,6 +209,81 @@ __global__ void __launch_bounds__((T / 4) * (T / 4)) sgemm_small(GemmArgs g) {
     C[m * g.N + n] = g.bias ? sum + __ldg(g.bias + n * g.bias_stride) : sum;
   }
   cluster.sync(); // nobody leaves while its tile is being read
+}
+
+// ---------------------------------------------------------------------------------------------
+// A few rows (M <= 8) times a row-major matrix: a prediction for one sample or a handful.  A CTA owns 32 columns and
+// keeps up to TH_STAGES slices of 64 k on their way; warp w multiplies rows w and w + 4, a column per lane: a chain of
+// one multiply-add per k and row, which is what bounds it.  (The 32 x 32 tiles spend 31 of 32 rows on nothing.)
+constexpr int TH_M = 8, TH_N = 32, TH_BK = 64, TH_STAGES = 10, TH_NT = 128;
+constexpr int TH_STAGE = TH_BK * (TH_N + TH_M); // floats: [k][32] of B, then [row][64] of A
+constexpr int TH_SMEM = TH_STAGES * TH_STAGE * 4;
+
+template <bool FUSED> __global__ void __launch_bounds__(TH_NT) sgemm_thin(GemmArgs g) {
+  extern __shared__ __align__(16) float th_smem[];
+  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const int64_t n0 = int64_t(blockIdx.x) * TH_N;
+  const float *A = g.A, *B = g.B;
+  gemm_batch_base(g, blockIdx.z, A, B);
+  const int steps = int((g.K + TH_BK - 1) / TH_BK);
+  auto fetch = [&](int s) {
+    if (s < steps) {
+      float *st = th_smem + (s % TH_STAGES) * TH_STAGE;
+      const int64_t k0 = int64_t(s) * TH_BK;
+      if (g.b_vec) {
+#pragma unroll
+        for (int i = 0; i < TH_BK * TH_N / 4 / TH_NT; ++i) {
+          const int v = tid + TH_NT * i, k = v / (TH_N / 4), n = (v % (TH_N / 4)) * 4;
+          const bool live = k0 + k < g.K && n0 + n < g.N;
+          cp_async16(st + k * TH_N + n, live ? B + (k0 + k) * g.b_sk + n0 + n : B, live);
+        }
+      } else {
+#pragma unroll 4
+        for (int i = 0; i < TH_BK * TH_N / TH_NT; ++i) {
+          const int v = tid + TH_NT * i, k = v / TH_N, n = v % TH_N;
+          const bool live = k0 + k < g.K && n0 + n < g.N;
+          cp_async4(st + k * TH_N + n, live ? B + (k0 + k) * g.b_sk + n0 + n : B, live);
+        }
+      }
+#pragma unroll
+      for (int i = 0; i < TH_BK * TH_M / TH_NT; ++i) {
+        const int v = tid + TH_NT * i, k = v % TH_BK, m = v / TH_BK;
+        const bool live = k0 + k < g.K && m < g.M;
+        cp_async4(st + TH_BK * TH_N + m * TH_BK + k, live ? A + m * g.a_sm + (k0 + k) * g.a_sk : A, live);
+      }
+    }
+    cp_async_commit();
+  };
+  float acc[2] = {0.0f, 0.0f};
+  const bool second = warp + 4 < g.M;
+  for (int s = 0; s < TH_STAGES - 1; ++s) fetch(s);
+  for (int s = 0; s < steps; ++s) {
+    cp_async_wait<TH_STAGES - 2>();
+    __syncthreads(); // slice s has landed for everyone, slice s - 1 has been read by everyone
+    fetch(s + TH_STAGES - 1);
+    const float *bs = th_smem + (s % TH_STAGES) * TH_STAGE + lane, *as = th_smem + (s % TH_STAGES) * TH_STAGE + TH_BK * TH_N + warp * TH_BK;
+    if (warp < g.M) {
+#pragma unroll
+      for (int k = 0; k < TH_BK; k += 4) {
+        const float4 a0 = *reinterpret_cast<const float4 *>(as + k);
+        const float4 a1 = second ? *reinterpret_cast<const float4 *>(as + 4 * TH_BK + k) : make_float4(0.f, 0.f, 0.f, 0.f);
+        const float b[4] = {bs[k * TH_N], bs[(k + 1) * TH_N], bs[(k + 2) * TH_N], bs[(k + 3) * TH_N]};
+        const float r0[4] = {a0.x, a0.y, a0.z, a0.w}, r1[4] = {a1.x, a1.y, a1.z, a1.w};
+#pragma unroll
+        for (int e = 0; e < 4; ++e) {
+          acc[0] = mad<FUSED>(r0[e], b[e], acc[0]);
+          acc[1] = mad<FUSED>(r1[e], b[e], acc[1]);
+        }
+      }
+    }
+  }
+  const int64_t n = n0 + lane;
+  float *C = g.C + int64_t(blockIdx.z) * g.M * g.N;
+#pragma unroll
+  for (int h = 0; h < 2; ++h) {
+    const int64_t m = warp + 4 * h;
+    if (m < g.M && n < g.N) C[m * g.N + n] = g.bias ? acc[h] + __ldg(g.bias + n * g.bias_stride) : acc[h];
+  }
 }
 
 // ---------------------------------------------------------------------------------------------
