@@ -71,11 +71,12 @@ __global__ void matmul_naive(const T *A, const T *B, T *C, int64_t M, int64_t N,
 
 static bool al16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 15) == 0; }
 
-// How a product runs on the CUDA cores: tile edge, CTAs along k (a cluster), and the time that is expected of it.
-// Tile 8 stands for the kernel for a few rows.  Clocks per k of one CTA, measured: alone on its SM (a chain of shared-memory loads and multiply-adds: 50 for the
-// 32-wide tile, 75 for 64, 345 for 128 x 256) and with the SM full (20, 70, 350).  So a product with few tiles takes
-// the small tile and many k-splits (256 x 784 x 256: 8.4 us with 64 tiles x 8, against 21 us unsplit and 145 us in two
-// 128 x 256 tiles), one with many tiles the large tile (52 TFLOP/s; 35 with the 64-wide tile).
+// How a product runs on the CUDA cores: tile edge (8: the kernel for a few rows), CTAs along k (a cluster), and the time
+// that is expected of it.  Clocks per k of one CTA, measured: alone on its SM (a chain of shared-memory loads and
+// multiply-adds: 26 for the 16-wide tile, 35 for 32, 70 for 64, 345 for 128 x 256) and with the SM full (9, 23, 70, 350);
+// 550 for a CTA's share of a cluster's sum, and 2.2 us for the launch.  So a product with few tiles takes a small tile and
+// many k-splits (256 x 784 x 256: 9 us with 64 tiles x 8, 15 us unsplit, 145 us in two 128 x 256 tiles), one with many
+// tiles the large tile (52 TFLOP/s; 35 with the 64-wide one).
 struct SimtPlan {
   int tile = 32, splits = 1;
   int64_t k_per_split = 0;
@@ -83,20 +84,26 @@ struct SimtPlan {
 };
 static SimtPlan plan_simt(int64_t batch, int64_t M, int64_t N, int64_t K, bool thin, bool may_split) {
   SimtPlan best;
+  const double sms = sm_count();
   if (thin) {
-    const double rounds = std::ceil(double(ceil_div(N, TH_N)) * double(batch) / sm_count());
-    best = SimtPlan{8, 1, K, 3.0 + rounds * double(K) * 6.5 / 1900};
+    const double rounds = std::ceil(double(ceil_div(N, TH_N)) * double(batch) / sms);
+    best = SimtPlan{8, 1, K, 2.2 + rounds * double(K) * (M <= 4 ? 13 : 21) / 1900};
   }
-  for (int tile : {128, 64, 32}) {
+  static const struct {
+    int tile;
+    double full, alone;
+  } kinds[] = {{128, 350, 345}, {64, 70, 70}, {32, 23, 35}, {16, 9, 26}};
+  for (const auto &kind : kinds) {
+    const int tile = kind.tile;
     const double tiles = double(ceil_div(M, tile)) * double(ceil_div(N, tile == 128 ? LG_N : tile)) * double(batch);
     if (ceil_div(M, tile) > 65535) continue;
-    const double full = tile == 128 ? 350 : tile == 64 ? 70 : 20, alone = tile == 128 ? 345 : tile == 64 ? 75 : 50;
     for (int s = 1; s <= (may_split && tile < 128 ? 8 : 1); ++s) {
       const int64_t per = s == 1 ? K : ceil_div(ceil_div(K, s), SG_BK) * SG_BK;
       if (s > 1 && (s - 1) * per >= K) continue;
-      const double rounds = std::ceil(tiles * s / sm_count());
-      const double clocks = std::max(rounds * full, alone) * double(per) + (s > 1 ? 1500 : 0) + 3000;
-      if (clocks / 1900 < best.us) best = SimtPlan{tile, s, per, clocks / 1900};
+      // the CTAs of a cluster like to share SMs: from half the SMs on, expect two on some
+      const double rounds = std::max(std::ceil(tiles * s / sms), s > 1 && 2 * tiles * s > sms ? 2.0 : 1.0), finish = s > 1 ? 550 : 0;
+      const double us = 2.2 + std::max(rounds * (kind.full * double(per) + finish), kind.alone * double(per) + 2 * finish) / 1900;
+      if (us < best.us) best = SimtPlan{tile, s, per, us};
     }
   }
   return best;
@@ -110,7 +117,7 @@ template <int T, bool A_K, bool B_K, bool FUSED> static void launch_small(const 
     NT_CUDA_CHECK(cudaFuncSetAttribute(kernel, cudaFuncAttributeMaxDynamicSharedMemorySize, smem));
     configured = true;
   }
-  launch_with(false, unsigned(g.splits), kernel, grid, (T / 4) * (T / 4), smem, g);
+  launch_with(false, unsigned(g.splits), kernel, grid, sg_threads<T>, smem, g);
 }
 template <int T, bool FUSED> static void launch_small(const GemmArgs &g, dim3 grid, bool a_k, bool b_k) {
   if (a_k && b_k) launch_small<T, true, true, FUSED>(g, grid);
@@ -148,13 +155,14 @@ static void sgemm_simt(GemmArgs g, int64_t nbatch, bool fused, const SimtPlan &p
   g.splits = plan.splits;
   g.k_per_split = plan.k_per_split;
   if (plan.tile == 8) {
+    using Kernel = void (*)(GemmArgs);
+    static const Kernel kernels[4] = {sgemm_thin<false, false>, sgemm_thin<false, true>, sgemm_thin<true, false>, sgemm_thin<true, true>};
     static bool configured = false;
     if (!configured) {
-      NT_CUDA_CHECK(cudaFuncSetAttribute(sgemm_thin<true>, cudaFuncAttributeMaxDynamicSharedMemorySize, TH_SMEM));
-      NT_CUDA_CHECK(cudaFuncSetAttribute(sgemm_thin<false>, cudaFuncAttributeMaxDynamicSharedMemorySize, TH_SMEM));
+      for (Kernel k : kernels) NT_CUDA_CHECK(cudaFuncSetAttribute(k, cudaFuncAttributeMaxDynamicSharedMemorySize, TH_SMEM));
       configured = true;
     }
-    launch_ordered(fused ? sgemm_thin<true> : sgemm_thin<false>, dim3(unsigned(ceil_div(g.N, TH_N)), 1, unsigned(nbatch)), TH_NT, TH_SMEM, g);
+    launch_ordered(kernels[(fused ? 2 : 0) + (g.M <= 4 ? 1 : 0)], dim3(unsigned(ceil_div(g.N, TH_N)), 1, unsigned(nbatch)), TH_NT, TH_SMEM, g);
     check_launch("sgemm");
     return;
   }
@@ -166,9 +174,12 @@ static void sgemm_simt(GemmArgs g, int64_t nbatch, bool fused, const SimtPlan &p
   } else if (plan.tile == 64) {
     if (fused) launch_small<64, true>(g, grid, a_k, b_k);
     else launch_small<64, false>(g, grid, a_k, b_k);
-  } else {
+  } else if (plan.tile == 32) {
     if (fused) launch_small<32, true>(g, grid, a_k, b_k);
     else launch_small<32, false>(g, grid, a_k, b_k);
+  } else {
+    if (fused) launch_small<16, true>(g, grid, a_k, b_k);
+    else launch_small<16, false>(g, grid, a_k, b_k);
   }
   check_launch("sgemm");
 }

@@ -60,124 +60,174 @@ template <bool FUSED> __device__ __forceinline__ float mad(float a, float b, flo
 
 // ---------------------------------------------------------------------------------------------
 // Small products.  A_K / B_K: the operand's unit-stride dim is k (shared tile [row][k]); otherwise rows run along the
-// unit stride (shared tile [k][row]).  Thread (ty, tx) of the (T/4)^2 owns rows r(ty, i) and columns r(tx, j): 4 t + i
-// where the tile is [k][row], so that a 128-bit load covers them, and t + (T/4) i where it is [row][k], so that the
-// 128-bit loads along k of neighbouring threads fall into different banks.
-constexpr int SG_BK = 32;
-template <int T> constexpr int sg_stages = 3;
+// unit stride (shared tile [k][row]).  A thread owns RM x RN outputs: rows RM ty + i where the tile is [k][row], so that
+// one load covers them, and ty + GM i where it is [row][k], so that the 128-bit loads along k of neighbouring threads fall
+// into different banks; columns likewise.  What bounds a CTA that has its SM for itself is the shared-memory pipe -- a
+// 128-bit load fills 512 bytes of registers, four clocks, also when lanes share the address -- against the latency that
+// few warps leave open: per 32-deep slice the 32-wide tile took 1600 clocks with 2 warps of 4 x 4 outputs, 1190 with 4 of
+// 4 x 2 and 1000 with 8 of 2 x 2, but the last is 15 % slower once the SMs are full.  So: 64 x 64 with 4 x 4, 32 x 32 with
+// 4 x 2, and 16 x 16 with 2 x 2 for products whose chain is all that counts.
+constexpr int SG_BK = 32, SG_STAGES = 4;
 template <int T, bool K_MAJOR> constexpr int sg_tile_floats = K_MAJOR ? T * (SG_BK + 4) : SG_BK * (T + 4);
 template <int T, bool A_K, bool B_K> // the ring; a partial tile of T x T is smaller
-constexpr int sg_smem_bytes = sg_stages<T> * (sg_tile_floats<T, A_K> + sg_tile_floats<T, B_K>) * 4;
+constexpr int sg_smem_bytes = SG_STAGES * (sg_tile_floats<T, A_K> + sg_tile_floats<T, B_K>) * 4;
+template <int T> constexpr int sg_rm = T == 16 ? 2 : 4; // outputs of a thread: sg_rm x sg_rn
+template <int T> constexpr int sg_rn = T == 64 ? 4 : 2;
+template <int T> constexpr int sg_threads = (T / sg_rm<T>) * (T / sg_rn<T>);
 
-template <int T, bool A_K, bool B_K, bool FUSED>
-__global__ void __launch_bounds__((T / 4) * (T / 4)) sgemm_small(GemmArgs g) {
-  constexpr int G = T / 4, NT = G * G;
-  constexpr int SG_STAGES = sg_stages<T>;
+// R values of an operand at each of 4 k, as v[row][k]
+template <int R, int G, int PITCH, bool KM> __device__ __forceinline__ void sg_operands(const float *st, int t, int k, float (&v)[R][4]) {
+  if constexpr (KM) {
+#pragma unroll
+    for (int i = 0; i < R; ++i) {
+      const float4 x = *reinterpret_cast<const float4 *>(st + (t + G * i) * PITCH + k);
+      v[i][0] = x.x, v[i][1] = x.y, v[i][2] = x.z, v[i][3] = x.w;
+    }
+  } else {
+#pragma unroll
+    for (int e = 0; e < 4; ++e) {
+      const float *q = st + (k + e) * PITCH + R * t;
+      if constexpr (R == 4) {
+        const float4 x = *reinterpret_cast<const float4 *>(q);
+        v[0][e] = x.x, v[1][e] = x.y, v[2][e] = x.z, v[3][e] = x.w;
+      } else {
+        const float2 x = *reinterpret_cast<const float2 *>(q);
+        v[0][e] = x.x, v[1][e] = x.y;
+      }
+    }
+  }
+}
+
+// One thread's copies of an operand's [T rows][SG_BK of k] slices: a first address, uniform steps between the copies of a
+// slice, and one between slices.  What lies outside the operand becomes zero.
+template <int T, int NT, bool KM> struct SgLoad {
+  static constexpr int NV = T * SG_BK / 4 / NT, NS = T * SG_BK / NT; // 16-byte and 4-byte copies per slice
+  const float *p, *safe;
+  int64_t step;      // between this thread's copies
+  int64_t next;      // to the next slice
+  int k, k_step;     // k of the first copy inside a slice, and of each further one (0 along rows)
+  unsigned rows;     // bit i: copy i's row exists
+  int dst, dst_step; // floats
+  bool vec;
+
+  __device__ __forceinline__ void init(const float *base, int64_t r0, int64_t R, int64_t s_r, int64_t s_k, bool v, int64_t k0) {
+    const int tid = threadIdx.x;
+    vec = v;
+    safe = base;
+    next = SG_BK * s_k;
+    const int W = v ? 4 : 1; // values per copy
+    int r, r_step;
+    if constexpr (KM) {
+      r = tid / (SG_BK / W);
+      k = (tid % (SG_BK / W)) * W;
+      r_step = NT / (SG_BK / W);
+      k_step = 0;
+      dst = r * (SG_BK + 4) + k;
+      dst_step = r_step * (SG_BK + 4);
+      step = r_step * s_r;
+    } else {
+      r = (tid % (T / W)) * W;
+      k = tid / (T / W);
+      r_step = 0;
+      k_step = NT / (T / W);
+      dst = k * (T + 4) + r;
+      dst_step = k_step * (T + 4);
+      step = k_step * s_k;
+    }
+    rows = 0;
+#pragma unroll
+    for (int i = 0; i < NS; ++i)
+      if (r0 + r + i * r_step < R) rows |= 1u << i;
+    p = base + (r0 + r) * s_r + (k0 + k) * s_k;
+  }
+  __device__ __forceinline__ void fetch(float *st, int left) { // left: values of k that remain, counted from this slice
+    const float *q = p;
+    float *d = st + dst;
+    if (vec) { // the unit-stride extent is a multiple of 4: a group is inside or outside as a whole
+#pragma unroll
+      for (int i = 0; i < NV; ++i, q += step, d += dst_step) {
+        const bool live = (rows >> i & 1) && k + i * k_step < left;
+        cp_async16(d, live ? q : safe, live);
+      }
+    } else {
+#pragma unroll 4
+      for (int i = 0; i < NS; ++i, q += step, d += dst_step) {
+        const bool live = (rows >> i & 1) && k + i * k_step < left;
+        cp_async4(d, live ? q : safe, live);
+      }
+    }
+    p += next;
+  }
+};
+
+template <int T, bool A_K, bool B_K, bool FUSED> __global__ void __launch_bounds__(sg_threads<T>) sgemm_small(GemmArgs g) {
+  constexpr int RM = sg_rm<T>, RN = sg_rn<T>, GM = T / RM, GN = T / RN, NT = GM * GN;
   constexpr int AF = sg_tile_floats<T, A_K>, BF = sg_tile_floats<T, B_K>;
   extern __shared__ __align__(16) float sg_smem[];
-  const int tid = threadIdx.x, tx = tid % G, ty = tid / G;
+  const int tid = threadIdx.x, tx = tid % GN, ty = tid / GN;
   const int split = blockIdx.x % g.splits;
   const int64_t n0 = int64_t(blockIdx.x / g.splits) * T, m0 = int64_t(blockIdx.y) * T;
   const float *A = g.A, *B = g.B;
   gemm_batch_base(g, blockIdx.z, A, B);
   const int64_t k_lo = split * g.k_per_split, k_hi = min(g.K, k_lo + g.k_per_split);
-  const int steps = k_hi > k_lo ? int((k_hi - k_lo + SG_BK - 1) / SG_BK) : 0;
+  const int depth = k_hi > k_lo ? int(k_hi - k_lo) : 0, steps = (depth + SG_BK - 1) / SG_BK;
 
-  // one operand's slice [T rows][SG_BK of k] into shared memory; what lies outside is zero
-  auto load = [&](auto k_major, const float *src, int64_t r0, int64_t R, int64_t s_r, int64_t s_k, int vec, float *dst, int64_t k0) {
-    constexpr bool KM = decltype(k_major)::value;
-    if (vec) { // the unit-stride extent is a multiple of 4: a group is inside or outside as a whole
-#pragma unroll
-      for (int i = 0; i < T * SG_BK / 4 / NT; ++i) {
-        const int v = tid + i * NT;
-        const int r = KM ? v / (SG_BK / 4) : (v % (T / 4)) * 4, k = KM ? (v % (SG_BK / 4)) * 4 : v / (T / 4);
-        const bool live = r0 + r < R && k0 + k < k_hi;
-        const float *p = live ? src + (r0 + r) * s_r + (k0 + k) * s_k : src;
-        cp_async16(dst + (KM ? r * (SG_BK + 4) + k : k * (T + 4) + r), p, live);
-      }
-    } else {
-#pragma unroll 4
-      for (int i = 0; i < T * SG_BK / NT; ++i) {
-        const int v = tid + i * NT;
-        const int r = KM ? v / SG_BK : v % T, k = KM ? v % SG_BK : v / T;
-        const bool live = r0 + r < R && k0 + k < k_hi;
-        const float *p = live ? src + (r0 + r) * s_r + (k0 + k) * s_k : src;
-        cp_async4(dst + (KM ? r * (SG_BK + 4) + k : k * (T + 4) + r), p, live);
-      }
-    }
-  };
+  SgLoad<T, NT, A_K> la;
+  SgLoad<T, NT, B_K> lb;
+  la.init(A, m0, g.M, g.a_sm, g.a_sk, g.a_vec, k_lo);
+  lb.init(B, n0, g.N, g.b_sn, g.b_sk, g.b_vec, k_lo);
   auto fetch = [&](int step) {
-    float *st = sg_smem + (step % SG_STAGES) * (AF + BF);
-    const int64_t k0 = k_lo + int64_t(step) * SG_BK;
-    load(std::bool_constant<A_K>{}, A, m0, g.M, g.a_sm, g.a_sk, g.a_vec, st, k0);
-    load(std::bool_constant<B_K>{}, B, n0, g.N, g.b_sn, g.b_sk, g.b_vec, st + AF, k0);
+    if (step < steps) {
+      float *st = sg_smem + (step % SG_STAGES) * (AF + BF);
+      la.fetch(st, depth - step * SG_BK);
+      lb.fetch(st + AF, depth - step * SG_BK);
+    }
+    cp_async_commit();
   };
 
-  float acc[4][4];
+  float acc[RM][RN];
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < RM; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) acc[i][j] = 0.0f;
+    for (int j = 0; j < RN; ++j) acc[i][j] = 0.0f;
 
 #pragma unroll
-  for (int s = 0; s < SG_STAGES - 1; ++s) {
-    if (s < steps) fetch(s);
-    cp_async_commit();
-  }
+  for (int s = 0; s < SG_STAGES - 1; ++s) fetch(s);
   for (int s = 0; s < steps; ++s) {
     cp_async_wait<SG_STAGES - 2>();
     __syncthreads(); // slice s has landed for everyone, and slice s - 1 has been read by everyone
-    if (s + SG_STAGES - 1 < steps) fetch(s + SG_STAGES - 1);
-    cp_async_commit();
+    fetch(s + SG_STAGES - 1);
     const float *as = sg_smem + (s % SG_STAGES) * (AF + BF), *bs = as + AF;
-    // operands of four values of k at a time, the next four on their way while these multiply: few warps share an SM
-    // here, so a load's latency is covered inside the warp or not at all
-    float a[2][4][4], b[2][4][4]; // [buffer][row][k]
-    auto operands = [&](int to, int k) {
-#pragma unroll
-      for (int i = 0; i < 4; ++i) {
-        const float4 va = A_K ? *reinterpret_cast<const float4 *>(as + (ty + G * i) * (SG_BK + 4) + k)
-                              : *reinterpret_cast<const float4 *>(as + (k + i) * (T + 4) + 4 * ty);
-        const float4 vb = B_K ? *reinterpret_cast<const float4 *>(bs + (tx + G * i) * (SG_BK + 4) + k)
-                              : *reinterpret_cast<const float4 *>(bs + (k + i) * (T + 4) + 4 * tx);
-        const float fa[4] = {va.x, va.y, va.z, va.w}, fb[4] = {vb.x, vb.y, vb.z, vb.w};
-#pragma unroll
-        for (int e = 0; e < 4; ++e) {
-          if (A_K) a[to][i][e] = fa[e];
-          else a[to][e][i] = fa[e];
-          if (B_K) b[to][i][e] = fb[e];
-          else b[to][e][i] = fb[e];
-        }
-      }
-    };
-    operands(0, 0);
 #pragma unroll
     for (int k = 0; k < SG_BK; k += 4) {
-      const int cur = (k >> 2) & 1;
-      if (k + 4 < SG_BK) operands(cur ^ 1, k + 4);
+      float a[RM][4], b[RN][4];
+      sg_operands<RM, GM, A_K ? SG_BK + 4 : T + 4, A_K>(as, ty, k, a);
+      sg_operands<RN, GN, B_K ? SG_BK + 4 : T + 4, B_K>(bs, tx, k, b);
 #pragma unroll
       for (int kk = 0; kk < 4; ++kk)
 #pragma unroll
-        for (int i = 0; i < 4; ++i)
+        for (int i = 0; i < RM; ++i)
 #pragma unroll
-          for (int j = 0; j < 4; ++j) acc[i][j] = mad<FUSED>(a[cur][i][kk], b[cur][j][kk], acc[i][j]);
+          for (int j = 0; j < RN; ++j) acc[i][j] = mad<FUSED>(a[i][kk], b[j][kk], acc[i][j]);
     }
   }
 
   float *C = g.C + int64_t(blockIdx.z) * g.M * g.N;
-  auto row = [&](int i) { return A_K ? ty + G * i : 4 * ty + i; };
-  auto col = [&](int j) { return B_K ? tx + G * j : 4 * tx + j; };
+  auto row = [&](int i) { return A_K ? ty + GM * i : RM * ty + i; };
+  auto col = [&](int j) { return B_K ? tx + GN * j : RN * tx + j; };
   if (g.splits == 1) {
 #pragma unroll
-    for (int i = 0; i < 4; ++i) {
+    for (int i = 0; i < RM; ++i) {
       const int64_t m = m0 + row(i);
       if (m >= g.M) continue;
-      if (!B_K && g.c_vec && !g.bias && n0 + 4 * tx < g.N) {
-        *reinterpret_cast<float4 *>(C + m * g.N + n0 + 4 * tx) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
-        continue;
+      if constexpr (!B_K && RN == 4) {
+        if (g.c_vec && !g.bias && n0 + 4 * tx < g.N) {
+          *reinterpret_cast<float4 *>(C + m * g.N + n0 + 4 * tx) = make_float4(acc[i][0], acc[i][1], acc[i][2], acc[i][3]);
+          continue;
+        }
       }
 #pragma unroll
-      for (int j = 0; j < 4; ++j) {
+      for (int j = 0; j < RN; ++j) {
         const int64_t n = n0 + col(j);
         if (n < g.N) C[m * g.N + n] = g.bias ? acc[i][j] + __ldg(g.bias + n * g.bias_stride) : acc[i][j];
       }
@@ -189,9 +239,9 @@ __global__ void __launch_bounds__((T / 4) * (T / 4)) sgemm_small(GemmArgs g) {
   cg::cluster_group cluster = cg::this_cluster();
   __syncthreads(); // the ring is free
 #pragma unroll
-  for (int i = 0; i < 4; ++i)
+  for (int i = 0; i < RM; ++i)
 #pragma unroll
-    for (int j = 0; j < 4; ++j) sg_smem[row(i) * T + col(j)] = acc[i][j];
+    for (int j = 0; j < RN; ++j) sg_smem[row(i) * T + col(j)] = acc[i][j];
   cluster.sync();
   const float *part[8];
 #pragma unroll
@@ -219,43 +269,50 @@ constexpr int TH_M = 8, TH_N = 32, TH_BK = 64, TH_STAGES = 10, TH_NT = 128;
 constexpr int TH_STAGE = TH_BK * (TH_N + TH_M); // floats: [k][32] of B, then [row][64] of A
 constexpr int TH_SMEM = TH_STAGES * TH_STAGE * 4;
 
-template <bool FUSED> __global__ void __launch_bounds__(TH_NT) sgemm_thin(GemmArgs g) {
+// FOUR: M <= 4
+template <bool FUSED, bool FOUR> __global__ void __launch_bounds__(TH_NT) sgemm_thin(GemmArgs g) {
   extern __shared__ __align__(16) float th_smem[];
   const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
   const int64_t n0 = int64_t(blockIdx.x) * TH_N;
   const float *A = g.A, *B = g.B;
   gemm_batch_base(g, blockIdx.z, A, B);
   const int steps = int((g.K + TH_BK - 1) / TH_BK);
+  // copies of B: rows kb, kb + kb_step, ... of a slice, 16 bytes (or single values) each; of A: k = tid % 64 of every
+  // second row
+  const int W = g.b_vec ? 4 : 1, kb = tid / (TH_N / W), nb = (tid % (TH_N / W)) * W, kb_step = TH_NT / (TH_N / W);
+  const bool nb_in = n0 + nb < g.N;
+  const float *pb = B + kb * g.b_sk + n0 + nb, *pa = A + (tid / TH_BK) * g.a_sm + (tid % TH_BK) * g.a_sk;
+  const int64_t b_step = kb_step * g.b_sk, b_next = TH_BK * g.b_sk, a_next = TH_BK * g.a_sk;
   auto fetch = [&](int s) {
     if (s < steps) {
       float *st = th_smem + (s % TH_STAGES) * TH_STAGE;
-      const int64_t k0 = int64_t(s) * TH_BK;
-      if (g.b_vec) {
+      const int left = int(min(g.K - int64_t(s) * TH_BK, int64_t(TH_BK)));
+      const float *q = pb;
+      float *d = st + kb * TH_N + nb;
+      if (W == 4) {
 #pragma unroll
-        for (int i = 0; i < TH_BK * TH_N / 4 / TH_NT; ++i) {
-          const int v = tid + TH_NT * i, k = v / (TH_N / 4), n = (v % (TH_N / 4)) * 4;
-          const bool live = k0 + k < g.K && n0 + n < g.N;
-          cp_async16(st + k * TH_N + n, live ? B + (k0 + k) * g.b_sk + n0 + n : B, live);
+        for (int i = 0; i < TH_BK * TH_N / 4 / TH_NT; ++i, q += b_step, d += kb_step * TH_N) {
+          const bool live = nb_in && kb + i * kb_step < left;
+          cp_async16(d, live ? q : B, live);
         }
       } else {
 #pragma unroll 4
-        for (int i = 0; i < TH_BK * TH_N / TH_NT; ++i) {
-          const int v = tid + TH_NT * i, k = v / TH_N, n = v % TH_N;
-          const bool live = k0 + k < g.K && n0 + n < g.N;
-          cp_async4(st + k * TH_N + n, live ? B + (k0 + k) * g.b_sk + n0 + n : B, live);
+        for (int i = 0; i < TH_BK * TH_N / TH_NT; ++i, q += b_step, d += kb_step * TH_N) {
+          const bool live = nb_in && kb + i * kb_step < left;
+          cp_async4(d, live ? q : B, live);
         }
       }
-#pragma unroll
-      for (int i = 0; i < TH_BK * TH_M / TH_NT; ++i) {
-        const int v = tid + TH_NT * i, k = v % TH_BK, m = v / TH_BK;
-        const bool live = k0 + k < g.K && m < g.M;
-        cp_async4(st + TH_BK * TH_N + m * TH_BK + k, live ? A + m * g.a_sm + (k0 + k) * g.a_sk : A, live);
+      const float *qa = pa;
+      for (int m = tid / TH_BK; m < g.M; m += TH_NT / TH_BK, qa += (TH_NT / TH_BK) * g.a_sm) {
+        const bool live = tid % TH_BK < left;
+        cp_async4(st + TH_BK * TH_N + m * TH_BK + tid % TH_BK, live ? qa : A, live);
       }
+      pb += b_next;
+      pa += a_next;
     }
     cp_async_commit();
   };
   float acc[2] = {0.0f, 0.0f};
-  const bool second = warp + 4 < g.M;
   for (int s = 0; s < TH_STAGES - 1; ++s) fetch(s);
   for (int s = 0; s < steps; ++s) {
     cp_async_wait<TH_STAGES - 2>();
@@ -263,16 +320,26 @@ template <bool FUSED> __global__ void __launch_bounds__(TH_NT) sgemm_thin(GemmAr
     fetch(s + TH_STAGES - 1);
     const float *bs = th_smem + (s % TH_STAGES) * TH_STAGE + lane, *as = th_smem + (s % TH_STAGES) * TH_STAGE + TH_BK * TH_N + warp * TH_BK;
     if (warp < g.M) {
+      // 16 values of k at a time, the next 16 on their way while these multiply
+      float b[2][16], r0[2][16], r1[2][16];
+      auto operands = [&](int to, int k) {
 #pragma unroll
-      for (int k = 0; k < TH_BK; k += 4) {
-        const float4 a0 = *reinterpret_cast<const float4 *>(as + k);
-        const float4 a1 = second ? *reinterpret_cast<const float4 *>(as + 4 * TH_BK + k) : make_float4(0.f, 0.f, 0.f, 0.f);
-        const float b[4] = {bs[k * TH_N], bs[(k + 1) * TH_N], bs[(k + 2) * TH_N], bs[(k + 3) * TH_N]};
-        const float r0[4] = {a0.x, a0.y, a0.z, a0.w}, r1[4] = {a1.x, a1.y, a1.z, a1.w};
+        for (int e = 0; e < 16; ++e) b[to][e] = bs[(k + e) * TH_N];
 #pragma unroll
         for (int e = 0; e < 4; ++e) {
-          acc[0] = mad<FUSED>(r0[e], b[e], acc[0]);
-          acc[1] = mad<FUSED>(r1[e], b[e], acc[1]);
+          *reinterpret_cast<float4 *>(&r0[to][4 * e]) = *reinterpret_cast<const float4 *>(as + k + 4 * e);
+          if constexpr (!FOUR) *reinterpret_cast<float4 *>(&r1[to][4 * e]) = *reinterpret_cast<const float4 *>(as + 4 * TH_BK + k + 4 * e);
+        }
+      };
+      operands(0, 0);
+#pragma unroll
+      for (int k = 0; k < TH_BK; k += 16) {
+        const int cur = (k >> 4) & 1;
+        if (k + 16 < TH_BK) operands(cur ^ 1, k + 16);
+#pragma unroll
+        for (int e = 0; e < 16; ++e) {
+          acc[0] = mad<FUSED>(r0[cur][e], b[cur][e], acc[0]);
+          if constexpr (!FOUR) acc[1] = mad<FUSED>(r1[cur][e], b[cur][e], acc[1]); // without a row: what lies in its slot, unused
         }
       }
     }
@@ -280,7 +347,7 @@ template <bool FUSED> __global__ void __launch_bounds__(TH_NT) sgemm_thin(GemmAr
   const int64_t n = n0 + lane;
   float *C = g.C + int64_t(blockIdx.z) * g.M * g.N;
 #pragma unroll
-  for (int h = 0; h < 2; ++h) {
+  for (int h = 0; h < (FOUR ? 1 : 2); ++h) {
     const int64_t m = warp + 4 * h;
     if (m < g.M && n < g.N) C[m * g.N + n] = g.bias ? acc[h] + __ldg(g.bias + n * g.bias_stride) : acc[h];
   }
