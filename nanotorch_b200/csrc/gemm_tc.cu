@@ -28,6 +28,7 @@
 // kernels, for fp32 operands.
 #include <cuda.h>
 
+#include <algorithm>
 #include <atomic>
 #include <cstdlib>
 #include <mutex>
@@ -50,7 +51,8 @@ constexpr int TC_TMEM_COLS = 512; // two fp32 accumulators of 256 columns: hi*hi
 constexpr uint32_t TC_A_PLANE_BYTES = TC_BM * TC_BK * 4;  // 8 KB
 constexpr uint32_t TC_B_PLANE_BYTES = TC_BN * TC_BK * 4;  // 16 KB
 constexpr uint32_t TC_STAGE_BYTES = 2 * TC_A_PLANE_BYTES + 2 * TC_B_PLANE_BYTES; // 48 KB
-constexpr uint32_t TC_SMEM_BYTES = TC_STAGES * TC_STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/;
+constexpr uint32_t TC_CORNER_BYTES = 32 * 32 * 4; // per epilogue warp of the promoted kernel
+constexpr uint32_t TC_SMEM_BYTES = TC_STAGES * TC_STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/ + 8 * TC_CORNER_BYTES;
 
 // ---------------------------------------------------------------------------------------------
 // split_pack
@@ -194,25 +196,29 @@ struct TcArgs {
   // promoted kernel: launched as the programmatic dependent of the product before it (nt_matmul_pair): it did not
   // wait for that grid on entry, so every CTA waits for it before leaving -- this grid never completes first
   int32_t wait_for_primary_at_end;
+  int32_t tiles_m, tiles_n; // promoted kernel: output tiles of one batch
+  int32_t work;             // tiles x splits x batches; a CTA takes items blockIdx.x, + gridDim.x, ...
 };
 
-// Output tile of this CTA.  CTAs are dispatched in the order of their linear index (x fastest); walking the
-// n-tiles of a whole row before the next m-tile makes every wave of CTAs touch all of B, which at these
+// Output tile of a work item.  CTAs take items in the order of their index, one wave after the other; taking the n-tiles
+// of a whole row before the next m-tile would make every wave touch all of B, which at these
 // sizes (two planes of B: 134 MB for 4096 x 4096) no longer fits the L2 and is fetched from DRAM once per
 // wave.  With panels of `panel` n-tiles a wave covers more m-tiles and fewer n-tiles, and a panel's slice of
 // B stays in the L2 while the CTAs walk down the m-tiles.
-__device__ __forceinline__ void tile_of_cta(const TcArgs &g, int &tm, int &tn, int &split) {
-  const int splits = g.splits > 1 ? g.splits : 1;
-  tm = blockIdx.y;
-  tn = blockIdx.x / splits; // the CTAs of one tile are neighbours in the dispatch order: their partial sums meet in the L2
-  split = blockIdx.x - tn * splits;
+__device__ __forceinline__ void tile_of_work(const TcArgs &g, int w, int &tm, int &tn, int &split, int &b) {
+  const int splits = g.splits > 1 ? g.splits : 1, per_batch = g.tiles_m * g.tiles_n * splits;
+  b = w / per_batch;
+  int lin = w - b * per_batch;
+  const int t = lin / splits; // the CTAs of one tile are neighbours in the order: their partial sums meet in the L2
+  split = lin - t * splits;
+  lin = t;
+  tm = lin / g.tiles_n;
+  tn = lin - tm * g.tiles_n;
   if (g.panel > 0) {
-    const int tiles_n = gridDim.x / splits, tiles_m = gridDim.y;
-    const int lin = tm * tiles_n + tn;
-    const int per_panel = g.panel * tiles_m;
+    const int per_panel = g.panel * g.tiles_m;
     const int p = lin / per_panel;
     const int within = lin - p * per_panel;
-    const int pw = min(g.panel, tiles_n - p * g.panel);
+    const int pw = min(g.panel, g.tiles_n - p * g.panel);
     tm = within / pw;
     tn = p * g.panel + within % pw;
   }
@@ -385,6 +391,11 @@ gemm_3xtf32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
 // ---------------------------------------------------------------------------------------------
 // Variant with promoted accumulation (matmul mode 1, the default; the kernel above is mode 3).
 //
+// One persistent CTA per SM walks over the output tiles: the producer runs ahead into the next tile's k-blocks, and the
+// epilogue warps store a tile while the MMA warp works on the next.  With a CTA per tile every tile paid for its own
+// start, pipeline fill and drain (32 x 512^3: two waves of 30 us for 13 us of products; 142 -> 161 TFLOP/s; 8192 x 1024 x
+// 4096 237 -> 266, 4096^3 250 -> 256).
+//
 // The tensor core adds into its fp32 accumulator with round-toward-zero, so a long accumulation chain
 // carries a bias that grows with its length.  Here a chain is only TC_PERIOD_KB k-blocks (256 values of
 // k, 96 MMAs) long: the two 256-column halves of tensor memory alternate as the accumulator of
@@ -416,13 +427,18 @@ gemm_3xtf32_promoted_kernel(const __grid_constant__ CUtensorMap map_a, const __g
   // A grid launched behind this one with the programmatic-serialization attribute may take the SMs this grid's
   // last wave leaves idle; it has nothing to wait for here.
   asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
-  int tile_m, tile_n, split;
-  tile_of_cta(g, tile_m, tile_n, split);
-  const int m0 = tile_m * TC_BM, n0 = tile_n * TC_BN, b = blockIdx.z;
-  // this CTA's share of the contraction: k-blocks [kb0, kb0 + nkb)
-  const int kb0 = g.splits > 1 ? split * g.kb_per_split : 0;
-  const int nkb = g.splits > 1 ? min(g.kb_per_split, g.num_kb - kb0) : g.num_kb;
-  const int num_periods = (nkb + TC_PERIOD_KB - 1) / TC_PERIOD_KB;
+  // a work item: an output tile and, with split-K, this CTA's share of the contraction, k-blocks [kb0, kb0 + nkb)
+  struct Item {
+    int tile_m, tile_n, split, b, kb0, nkb, periods;
+  };
+  auto item_of = [&](int w) {
+    Item it;
+    tile_of_work(g, w, it.tile_m, it.tile_n, it.split, it.b);
+    it.kb0 = g.splits > 1 ? it.split * g.kb_per_split : 0;
+    it.nkb = g.splits > 1 ? min(g.kb_per_split, g.num_kb - it.kb0) : g.num_kb;
+    it.periods = (it.nkb + TC_PERIOD_KB - 1) / TC_PERIOD_KB;
+    return it;
+  };
 
   if (threadIdx.x == 0) {
     for (int s = 0; s < TC_STAGES; ++s) {
@@ -451,85 +467,98 @@ gemm_3xtf32_promoted_kernel(const __grid_constant__ CUtensorMap map_a, const __g
     if (lane == 0 && !poisoned) {
       uint32_t phase = 0;
       int s = 0;
-      for (int kb = 0; kb < nkb; ++kb) {
-        if (!mbar_wait(empty0 + 8 * s, phase ^ 1, g.wait_limit)) {
-          atomicExch(g.error_flag, 1);
-          break;
-        }
-        const uint32_t st = smem_base + s * TC_STAGE_BYTES;
-        mbar_expect_tx(full0 + 8 * s, TC_STAGE_BYTES);
-        const int k = (kb0 + kb) * TC_BK;
-        if constexpr (A_MN) {
-          tma_load_4d(st, &map_a, full0 + 8 * s, 0, k, m0 >> 5, b);
-          tma_load_4d(st + TC_A_PLANE_BYTES, &map_a, full0 + 8 * s, 0, k, m0 >> 5, g.batch + b);
-        } else {
-          tma_load_3d(st, &map_a, full0 + 8 * s, k, m0, b);
-          tma_load_3d(st + TC_A_PLANE_BYTES, &map_a, full0 + 8 * s, k, m0, g.batch + b);
-        }
-        if constexpr (B_MN) {
-          tma_load_4d(st + 2 * TC_A_PLANE_BYTES, &map_b, full0 + 8 * s, 0, k, n0 >> 5, b);
-          tma_load_4d(st + 2 * TC_A_PLANE_BYTES + TC_B_PLANE_BYTES, &map_b, full0 + 8 * s, 0, k, n0 >> 5, g.batch + b);
-        } else {
-          tma_load_3d(st + 2 * TC_A_PLANE_BYTES, &map_b, full0 + 8 * s, k, n0, b);
-          tma_load_3d(st + 2 * TC_A_PLANE_BYTES + TC_B_PLANE_BYTES, &map_b, full0 + 8 * s, k, n0, g.batch + b);
-        }
-        if (++s == TC_STAGES) {
-          s = 0;
-          phase ^= 1;
+      bool ok = true;
+      for (int w = blockIdx.x; w < g.work && ok; w += gridDim.x) {
+        const Item it = item_of(w);
+        const int m0 = it.tile_m * TC_BM, n0 = it.tile_n * TC_BN, b = it.b;
+        for (int kb = 0; kb < it.nkb; ++kb) {
+          if (!mbar_wait(empty0 + 8 * s, phase ^ 1, g.wait_limit)) {
+            atomicExch(g.error_flag, 1);
+            ok = false;
+            break;
+          }
+          const uint32_t st = smem_base + s * TC_STAGE_BYTES;
+          mbar_expect_tx(full0 + 8 * s, TC_STAGE_BYTES);
+          const int k = (it.kb0 + kb) * TC_BK;
+          if constexpr (A_MN) {
+            tma_load_4d(st, &map_a, full0 + 8 * s, 0, k, m0 >> 5, b);
+            tma_load_4d(st + TC_A_PLANE_BYTES, &map_a, full0 + 8 * s, 0, k, m0 >> 5, g.batch + b);
+          } else {
+            tma_load_3d(st, &map_a, full0 + 8 * s, k, m0, b);
+            tma_load_3d(st + TC_A_PLANE_BYTES, &map_a, full0 + 8 * s, k, m0, g.batch + b);
+          }
+          if constexpr (B_MN) {
+            tma_load_4d(st + 2 * TC_A_PLANE_BYTES, &map_b, full0 + 8 * s, 0, k, n0 >> 5, b);
+            tma_load_4d(st + 2 * TC_A_PLANE_BYTES + TC_B_PLANE_BYTES, &map_b, full0 + 8 * s, 0, k, n0 >> 5, g.batch + b);
+          } else {
+            tma_load_3d(st + 2 * TC_A_PLANE_BYTES, &map_b, full0 + 8 * s, k, n0, b);
+            tma_load_3d(st + 2 * TC_A_PLANE_BYTES + TC_B_PLANE_BYTES, &map_b, full0 + 8 * s, k, n0, g.batch + b);
+          }
+          if (++s == TC_STAGES) {
+            s = 0;
+            phase ^= 1;
+          }
         }
       }
     }
   } else if (warp == 1) {
     if (lane == 0 && !poisoned) {
       uint32_t phase = 0;
-      int s = 0, kb = 0;
+      int s = 0;
+      uint32_t done = 0; // periods of the items before
       bool ok = true;
-      for (int p = 0; p < num_periods && ok; ++p) {
-        const int buf = p & 1;
-        // the epilogue must have drained this half (two periods ago) before it is overwritten
-        if (!mbar_wait(acc_empty0 + 8 * buf, ((p >> 1) & 1) ^ 1, g.wait_limit)) {
-          atomicExch(g.error_flag, 4);
-          ok = false;
-          break;
-        }
-        tcgen05_fence_after();
-        const uint32_t d = tmem_acc + uint32_t(buf * TC_BN);
-        const int kb_end = min(kb + TC_PERIOD_KB, nkb);
-        bool first = true;
-        for (; kb < kb_end; ++kb) {
-          if (!mbar_wait(full0 + 8 * s, phase, g.wait_limit)) {
-            atomicExch(g.error_flag, 2);
+      for (int w = blockIdx.x; w < g.work && ok; w += gridDim.x) {
+        const Item it = item_of(w);
+        int kb = 0;
+        for (int q = 0; q < it.periods && ok; ++q) {
+          const uint32_t p = done + q;
+          const int buf = p & 1;
+          // the epilogue must have drained this half (two periods ago) before it is overwritten
+          if (!mbar_wait(acc_empty0 + 8 * buf, ((p >> 1) & 1) ^ 1, g.wait_limit)) {
+            atomicExch(g.error_flag, 4);
             ok = false;
             break;
           }
           tcgen05_fence_after();
-          const uint32_t st = smem_base + s * TC_STAGE_BYTES;
+          const uint32_t d = tmem_acc + uint32_t(buf * TC_BN);
+          const int kb_end = min(kb + TC_PERIOD_KB, it.nkb);
+          bool first = true;
+          for (; kb < kb_end; ++kb) {
+            if (!mbar_wait(full0 + 8 * s, phase, g.wait_limit)) {
+              atomicExch(g.error_flag, 2);
+              ok = false;
+              break;
+            }
+            tcgen05_fence_after();
+            const uint32_t st = smem_base + s * TC_STAGE_BYTES;
 #pragma unroll
-          for (int ks = 0; ks < TC_BK / TC_UMMA_K; ++ks) {
-            // one instruction consumes 8 values of k: 32 bytes along a K-major row, 8 rows of 128 bytes
-            // of an MN-major tile
-            const uint32_t a_off = A_MN ? ks * 1024u : ks * TC_UMMA_K * 4u;
-            const uint32_t b_off = B_MN ? ks * 1024u : ks * TC_UMMA_K * 4u;
-            const uint32_t pa = st + a_off, pb = st + 2 * TC_A_PLANE_BYTES + b_off;
-            const uint64_t a_hi = A_MN ? umma_desc_mn_sw128(pa, g.mn_lbo, g.mn_sbo) : umma_desc_sw64(pa);
-            const uint64_t a_lo = A_MN ? umma_desc_mn_sw128(pa + TC_A_PLANE_BYTES, g.mn_lbo, g.mn_sbo)
-                                       : umma_desc_sw64(pa + TC_A_PLANE_BYTES);
-            const uint64_t b_hi = B_MN ? umma_desc_mn_sw128(pb, g.mn_lbo, g.mn_sbo) : umma_desc_sw64(pb);
-            const uint64_t b_lo = B_MN ? umma_desc_mn_sw128(pb + TC_B_PLANE_BYTES, g.mn_lbo, g.mn_sbo)
-                                       : umma_desc_sw64(pb + TC_B_PLANE_BYTES);
-            // small terms first, the large one last
-            umma_tf32_idesc(d, a_hi, b_lo, IDESC, first ? 0u : 1u);
-            umma_tf32_idesc(d, a_lo, b_hi, IDESC, 1);
-            umma_tf32_idesc(d, a_hi, b_hi, IDESC, 1);
-            first = false;
+            for (int ks = 0; ks < TC_BK / TC_UMMA_K; ++ks) {
+              // one instruction consumes 8 values of k: 32 bytes along a K-major row, 8 rows of 128 bytes
+              // of an MN-major tile
+              const uint32_t a_off = A_MN ? ks * 1024u : ks * TC_UMMA_K * 4u;
+              const uint32_t b_off = B_MN ? ks * 1024u : ks * TC_UMMA_K * 4u;
+              const uint32_t pa = st + a_off, pb = st + 2 * TC_A_PLANE_BYTES + b_off;
+              const uint64_t a_hi = A_MN ? umma_desc_mn_sw128(pa, g.mn_lbo, g.mn_sbo) : umma_desc_sw64(pa);
+              const uint64_t a_lo = A_MN ? umma_desc_mn_sw128(pa + TC_A_PLANE_BYTES, g.mn_lbo, g.mn_sbo)
+                                         : umma_desc_sw64(pa + TC_A_PLANE_BYTES);
+              const uint64_t b_hi = B_MN ? umma_desc_mn_sw128(pb, g.mn_lbo, g.mn_sbo) : umma_desc_sw64(pb);
+              const uint64_t b_lo = B_MN ? umma_desc_mn_sw128(pb + TC_B_PLANE_BYTES, g.mn_lbo, g.mn_sbo)
+                                         : umma_desc_sw64(pb + TC_B_PLANE_BYTES);
+              // small terms first, the large one last
+              umma_tf32_idesc(d, a_hi, b_lo, IDESC, first ? 0u : 1u);
+              umma_tf32_idesc(d, a_lo, b_hi, IDESC, 1);
+              umma_tf32_idesc(d, a_hi, b_hi, IDESC, 1);
+              first = false;
+            }
+            umma_commit(empty0 + 8 * s);
+            if (++s == TC_STAGES) {
+              s = 0;
+              phase ^= 1;
+            }
           }
-          umma_commit(empty0 + 8 * s);
-          if (++s == TC_STAGES) {
-            s = 0;
-            phase ^= 1;
-          }
+          if (ok) umma_commit(acc_full0 + 8 * buf);
         }
-        if (ok) umma_commit(acc_full0 + 8 * buf);
+        done += it.periods;
       }
       if (!ok) { // release the epilogue warps from whatever they wait on
         for (int i = 0; i < 2; ++i)
@@ -540,98 +569,126 @@ gemm_3xtf32_promoted_kernel(const __grid_constant__ CUtensorMap map_a, const __g
     // ------------------------------------------------------------------ epilogue, warps 2..9
     const int quad = warp & 3;          // 32-lane group of tensor memory this warp may read
     const int half = (warp - 2) >> 2;   // which 128 of the 256 columns
-    float sum[128];
-#pragma unroll
-    for (int i = 0; i < 128; ++i) sum[i] = 0.0f;
+    // a 32 x 32 corner of the tile on its way from a lane per row to whole 128-byte lines, 16-byte groups swizzled
+    char *corner = reinterpret_cast<char *>(smem_raw + (bar_base - smem_u32(smem_raw))) + 256 + (warp - 2) * TC_CORNER_BYTES;
     bool ok = !poisoned;
-    for (int p = 0; p < (poisoned ? 0 : num_periods); ++p) {
-      const int buf = p & 1;
-      if (ok && !mbar_wait(acc_full0 + 8 * buf, (p >> 1) & 1, g.wait_limit)) {
-        atomicExch(g.error_flag, 3);
-        ok = false;
-      }
-      if (!ok || *reinterpret_cast<volatile int *>(g.error_flag) != 0) {
-        ok = false;
-        break;
-      }
-      tcgen05_fence_after();
-      const uint32_t taddr = tmem_acc + (uint32_t(quad * 32) << 16) + uint32_t(buf * TC_BN + half * 128);
+    uint32_t done = 0; // periods of the items before
+    for (int w = blockIdx.x; w < g.work && ok; w += gridDim.x) {
+      const Item it = item_of(w);
+      const int m0 = it.tile_m * TC_BM, n0 = it.tile_n * TC_BN, b = it.b;
+      float sum[128];
 #pragma unroll
-      for (int c = 0; c < 4; ++c) {
-        uint32_t v[32];
-        tmem_ld32(taddr + uint32_t(c * 32), v);
-        asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-        for (int e = 0; e < 32; ++e) sum[c * 32 + e] = sum[c * 32 + e] + __uint_as_float(v[e]);
-      }
-      tcgen05_fence_before();
-      __syncwarp();
-      if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(acc_empty0 + 8 * buf) : "memory");
-    }
-    const int64_t m = int64_t(m0) + quad * 32 + lane;
-    if (g.splits > 1 && !poisoned) {
-      // Split-K: leave this CTA's sums in the workspace; whoever draws the tile's last ticket adds the
-      // partial sums up in split order (the order never depends on which CTA finishes last).  All eight
-      // epilogue warps pass the two barriers whatever happened to them; a warp whose wait ran out says so.
-      volatile int *fail_slot = poison_slot + 1;
-      volatile unsigned int *ticket_slot = reinterpret_cast<volatile unsigned int *>(poison_slot + 2);
-      const int et = int(threadIdx.x) - 64; // 0..255 among the epilogue threads
-      const int64_t tile_lin = (int64_t(b) * gridDim.y + tile_m) * (gridDim.x / g.splits) + tile_n;
-      float *mine = g.partials + ((tile_lin * g.splits + split) * 32 * 256 + et) * 4;
-      if (!ok) *fail_slot = 1;
-      if (ok && m < g.M) {
-#pragma unroll
-        for (int q = 0; q < 32; ++q)
-          __stcg(reinterpret_cast<float4 *>(mine + q * 1024), make_float4(sum[4 * q], sum[4 * q + 1], sum[4 * q + 2], sum[4 * q + 3]));
-      }
-      __threadfence();
-      asm volatile("bar.sync 1, 256;" ::: "memory");
-      if (et == 0) *ticket_slot = (*fail_slot != 0) ? 0xffffffffu : atomicAdd(g.tickets + tile_lin, 1u);
-      asm volatile("bar.sync 1, 256;" ::: "memory");
-      const unsigned int ticket = *ticket_slot;
-      ok = ok && ticket == unsigned(g.splits - 1);
-      if (ok) {
-        __threadfence();
-        if (m < g.M) {
-          const float *first = g.partials + (tile_lin * g.splits * 32 * 256 + et) * 4;
-#pragma unroll
-          for (int q = 0; q < 32; ++q) {
-            float4 acc = __ldcg(reinterpret_cast<const float4 *>(first + q * 1024));
-            for (int sp = 1; sp < g.splits; ++sp) {
-              const float4 v = __ldcg(reinterpret_cast<const float4 *>(first + int64_t(sp) * 32 * 256 * 4 + q * 1024));
-              acc.x += v.x;
-              acc.y += v.y;
-              acc.z += v.z;
-              acc.w += v.w;
-            }
-            sum[4 * q] = acc.x;
-            sum[4 * q + 1] = acc.y;
-            sum[4 * q + 2] = acc.z;
-            sum[4 * q + 3] = acc.w;
-          }
+      for (int i = 0; i < 128; ++i) sum[i] = 0.0f;
+      for (int q = 0; q < it.periods; ++q) {
+        const uint32_t p = done + q;
+        const int buf = p & 1;
+        if (ok && !mbar_wait(acc_full0 + 8 * buf, (p >> 1) & 1, g.wait_limit)) {
+          atomicExch(g.error_flag, 3);
+          ok = false;
         }
-        if (et == 0) g.tickets[tile_lin] = 0; // ready for the next launch
+        if (!ok || *reinterpret_cast<volatile int *>(g.error_flag) != 0) {
+          ok = false;
+          break;
+        }
+        tcgen05_fence_after();
+        const uint32_t taddr = tmem_acc + (uint32_t(quad * 32) << 16) + uint32_t(buf * TC_BN + half * 128);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          uint32_t v[32];
+          tmem_ld32(taddr + uint32_t(c * 32), v);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int e = 0; e < 32; ++e) sum[c * 32 + e] = sum[c * 32 + e] + __uint_as_float(v[e]);
+        }
+        tcgen05_fence_before();
+        __syncwarp();
+        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(acc_empty0 + 8 * buf) : "memory");
       }
-    }
-    if (ok && m < g.M) {
-      float *crow = g.C + (int64_t(b) * g.M + m) * g.N;
-      const int64_t n = int64_t(n0) + half * 128;
-      if (g.bias) {
-        // the second rounded step of x @ W + b: the fp32 product that a separate launch would have
-        // stored, plus the bias, rounded once more (every lane reads the same bias word: one broadcast)
+      done += it.periods;
+      const int64_t m = int64_t(m0) + quad * 32 + lane;
+      bool last = ok; // this CTA finishes the tile
+      if (g.splits > 1 && !poisoned) {
+        // Split-K: leave this CTA's sums in the workspace; whoever draws the tile's last ticket adds the
+        // partial sums up in split order (the order never depends on which CTA finishes last).  All eight
+        // epilogue warps pass the two barriers whatever happened to them; a warp whose wait ran out says so.
+        volatile int *fail_slot = poison_slot + 1;
+        volatile unsigned int *ticket_slot = reinterpret_cast<volatile unsigned int *>(poison_slot + 2);
+        const int et = int(threadIdx.x) - 64; // 0..255 among the epilogue threads
+        const int64_t tile_lin = (int64_t(b) * g.tiles_m + it.tile_m) * g.tiles_n + it.tile_n;
+        float *mine = g.partials + ((tile_lin * g.splits + it.split) * 32 * 256 + et) * 4;
+        if (!ok) *fail_slot = 1;
+        if (ok && m < g.M) {
 #pragma unroll
-        for (int i = 0; i < 128; ++i)
-          if (n + i < g.N) sum[i] = sum[i] + __ldg(g.bias + (n + i) * g.bias_stride);
+          for (int q = 0; q < 32; ++q)
+            __stcg(reinterpret_cast<float4 *>(mine + q * 1024), make_float4(sum[4 * q], sum[4 * q + 1], sum[4 * q + 2], sum[4 * q + 3]));
+        }
+        __threadfence();
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        if (et == 0) *ticket_slot = (*fail_slot != 0) ? 0xffffffffu : atomicAdd(g.tickets + tile_lin, 1u);
+        asm volatile("bar.sync 1, 256;" ::: "memory");
+        const unsigned int ticket = *ticket_slot;
+        last = ok && ticket == unsigned(g.splits - 1);
+        if (last) {
+          __threadfence();
+          if (m < g.M) {
+            const float *first = g.partials + (tile_lin * g.splits * 32 * 256 + et) * 4;
+#pragma unroll
+            for (int q = 0; q < 32; ++q) {
+              float4 acc = __ldcg(reinterpret_cast<const float4 *>(first + q * 1024));
+              for (int sp = 1; sp < g.splits; ++sp) {
+                const float4 v = __ldcg(reinterpret_cast<const float4 *>(first + int64_t(sp) * 32 * 256 * 4 + q * 1024));
+                acc.x += v.x;
+                acc.y += v.y;
+                acc.z += v.z;
+                acc.w += v.w;
+              }
+              sum[4 * q] = acc.x;
+              sum[4 * q + 1] = acc.y;
+              sum[4 * q + 2] = acc.z;
+              sum[4 * q + 3] = acc.w;
+            }
+          }
+          if (et == 0) g.tickets[tile_lin] = 0; // ready for the next launch
+        }
       }
+      if (__all_sync(0xffffffffu, last)) {
+        // A lane holds a row; stored like that, every instruction would touch 32 lines with 16 bytes each.  The next item's
+        // products run meanwhile: tensor memory takes two periods before it needs this warp again.
+        float *C = g.C + (int64_t(b) * g.M + m0 + quad * 32) * g.N;
+        const int64_t rows = g.M - m0 - quad * 32;
 #pragma unroll
-      for (int q = 0; q < 32; ++q) {
-        const int64_t nn = n + 4 * q;
-        if (g.c_vec && nn + 3 < g.N) {
-          *reinterpret_cast<float4 *>(crow + nn) = make_float4(sum[4 * q], sum[4 * q + 1], sum[4 * q + 2], sum[4 * q + 3]);
-        } else {
+        for (int c = 0; c < 4; ++c) {
+          const int64_t n = int64_t(n0) + half * 128 + c * 32;
 #pragma unroll
-          for (int e = 0; e < 4; ++e)
-            if (nn + e < g.N) crow[nn + e] = sum[4 * q + e];
+          for (int j = 0; j < 8; ++j)
+            *reinterpret_cast<float4 *>(corner + lane * 128 + ((j ^ (lane & 7)) << 4)) =
+                make_float4(sum[c * 32 + 4 * j], sum[c * 32 + 4 * j + 1], sum[c * 32 + 4 * j + 2], sum[c * 32 + 4 * j + 3]);
+          __syncwarp();
+          // the second rounded step of x @ W + b: the fp32 product that a separate launch would have stored, plus the bias,
+          // rounded once more
+          if (g.c_vec) {
+            const int j = lane & 7;
+            const int64_t nn = n + 4 * j;
+            float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
+            if (g.bias && nn < g.N)
+              bias = make_float4(__ldg(g.bias + nn * g.bias_stride), __ldg(g.bias + (nn + 1) * g.bias_stride),
+                                 __ldg(g.bias + (nn + 2) * g.bias_stride), __ldg(g.bias + (nn + 3) * g.bias_stride));
+#pragma unroll
+            for (int i = 0; i < 8; ++i) {
+              const int r = 4 * i + (lane >> 3);
+              float4 v = *reinterpret_cast<const float4 *>(corner + r * 128 + ((j ^ (r & 7)) << 4));
+              if (g.bias) v = make_float4(v.x + bias.x, v.y + bias.y, v.z + bias.z, v.w + bias.w);
+              if (r < rows && nn < g.N) *reinterpret_cast<float4 *>(C + r * g.N + nn) = v;
+            }
+          } else {
+            const int64_t nn = n + lane;
+            const float bias = g.bias && nn < g.N ? __ldg(g.bias + nn * g.bias_stride) : 0.0f;
+            for (int r = 0; r < 32 && r < rows; ++r) {
+              const float v = *reinterpret_cast<const float *>(corner + r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4);
+              if (nn < g.N) C[r * g.N + nn] = g.bias ? v + bias : v;
+            }
+          }
+          __syncwarp();
         }
       }
     }
@@ -1156,6 +1213,7 @@ bool gemm_3xtf32_natural(nt_storage *sa, int64_t a_off, nt_storage *sb, int64_t 
   if (!g_promoted.load()) return false;
   if (batch < 1 || batch > 32767 || M < 1 || N < 1 || K < 1) return false;
   if (ceil_div(M, TC_BM) > 65535 || ceil_div(N, TC_BN) > 0x7fffffff) return false;
+  if (ceil_div(M, TC_BM) * ceil_div(N, TC_BN) * batch >= (int64_t(1) << 27)) return false; // times up to 8 splits, plus a grid
   if (M >= (int64_t(1) << 31) || N >= (int64_t(1) << 31) || K >= (int64_t(1) << 31)) return false;
   const int ua = unit_dim(M, K, a_sm, a_sk), ub = unit_dim(K, N, b_sk, b_sn);
   if (ua < 0 || ub < 0) return false;
@@ -1209,7 +1267,10 @@ bool gemm_3xtf32_natural(nt_storage *sa, int64_t a_off, nt_storage *sb, int64_t 
     g.bias = bias;
     g.bias_stride = bias ? bias_stride : 0;
     if (bias && bias_done) *bias_done = true;
-    dim3 grid{unsigned(tiles_n * g.splits), unsigned(tiles_m), unsigned(batch)};
+    g.tiles_m = int32_t(tiles_m);
+    g.tiles_n = int32_t(tiles_n);
+    g.work = int32_t(tiles_m * tiles_n * g.splits * batch);
+    const dim3 grid{unsigned(std::min(g.work, sm_count())), 1, 1};
     const bool overlap = g_pair_overlap.load(std::memory_order_relaxed) != 0;
     g.wait_for_primary_at_end = (t_pair_second && overlap && launches_so_far() == g_promoted_seq) ? 1 : 0;
     // the matmul profile times an overlapped pair as one interval of two launches: no event between them
@@ -1252,6 +1313,7 @@ bool gemm_3xtf32(const float *A, const float *B, float *C, int64_t batch, int64_
   // limits of one launch / one tensor map
   if (batch < 1 || batch > 32767 || M < 1 || N < 1 || K < 1) return false;
   if (ceil_div(M, TC_BM) > 65535 || ceil_div(N, TC_BN) > 0x7fffffff) return false;
+  if (ceil_div(M, TC_BM) * ceil_div(N, TC_BN) * batch >= (int64_t(1) << 27)) return false; // times up to 8 splits, plus a grid
   if (M >= (int64_t(1) << 31) || N >= (int64_t(1) << 31) || K >= (int64_t(1) << 31)) return false;
   gemm_tc_prepare();
   const int64_t Kp = ceil_div(K, 32) * 32;
@@ -1281,9 +1343,12 @@ bool gemm_3xtf32(const float *A, const float *B, float *C, int64_t batch, int64_
     }
     dim3 grid{unsigned(ceil_div(N, TC_BN)), unsigned(ceil_div(M, TC_BM)), unsigned(batch)};
     matmul_profile_begin();
-    if (g_promoted.load())
-      gemm_3xtf32_promoted_kernel<false, false><<<grid, 320, TC_SMEM_BYTES, stream()>>>(map_a, map_b, g);
-    else
+    if (g_promoted.load()) {
+      g.tiles_m = int32_t(grid.y);
+      g.tiles_n = int32_t(grid.x);
+      g.work = int32_t(grid.x * grid.y * grid.z);
+      gemm_3xtf32_promoted_kernel<false, false><<<unsigned(std::min(g.work, sm_count())), 320, TC_SMEM_BYTES, stream()>>>(map_a, map_b, g);
+    } else
       gemm_3xtf32_kernel<<<grid, 192, TC_SMEM_BYTES, stream()>>>(map_a, map_b, g);
     matmul_profile_end();
     check_launch("gemm_3xtf32_kernel");
