@@ -351,6 +351,8 @@ int nt_extremum_backward(const nt_view *g_expanded, const nt_view *x, const nt_v
 /* SGD update p <- p - (g*lr), the two rounded steps of `p -= p.grad * lr` (nn/optimizers.py:45-51); bumps the version.
  * `grad_scale` multiplies g first when != 1 (data-parallel mean over ranks). */
 int nt_sgd_update(const nt_view *param, const nt_view *grad, float lr, float grad_scale);
+/* `count` such updates, the small ones among them in one launch. */
+int nt_sgd_update_many(const nt_view *params, const nt_view *grads, int32_t count, float lr, float grad_scale);
 
 /* ------------------------------------------------------------------ data-parallel exchange (NCCL; no counterpart in the reference) */
 #define NT_COMM_ID_BYTES 128

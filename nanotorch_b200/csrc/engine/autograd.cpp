@@ -343,19 +343,28 @@ static PyObject *m_set_grad_enabled(PyObject *, PyObject *on) { // returns the p
   G.grad_enabled = v != 0;
   return PyBool_FromLong(prev);
 }
-// sgd_update(param, lr, scale): the fused update of one ordinary parameter; False when it is not one
+// sgd_update(params, lr, scale): the fused updates of a list of ordinary parameters; False, and nothing done, when one of
+// those that take gradients is not ordinary or has no gradient
 static PyObject *m_sgd_update(PyObject *, PyObject *const *args, Py_ssize_t n) {
   if (n != 3) {
-    PyErr_SetString(PyExc_TypeError, "sgd_update(param, lr, grad_scale)");
+    PyErr_SetString(PyExc_TypeError, "sgd_update(params, lr, grad_scale)");
     return nullptr;
   }
   const double lr = PyFloat_AsDouble(args[1]), scale = PyFloat_AsDouble(args[2]);
   if (PyErr_Occurred()) return nullptr;
-  if (!is_fast(args[0]) || !T_(args[0])->grad || !is_fast(T_(args[0])->grad)) Py_RETURN_FALSE;
-  TensorObj *p = T_(args[0]), *g = T_(p->grad);
-  if (!same_shape(p, g)) Py_RETURN_FALSE;
-  const nt_view vp = view_of(p), vg = view_of(g);
-  const int rc = nt_sgd_update(&vp, &vg, float(lr), float(scale));
+  Ref seq(PySequence_Fast(args[0], "sgd_update: a sequence of tensors"));
+  if (!seq) return nullptr;
+  std::vector<nt_view> ps, gs;
+  for (Py_ssize_t i = 0; i < PySequence_Fast_GET_SIZE(seq.p); ++i) {
+    PyObject *o = PySequence_Fast_GET_ITEM(seq.p, i);
+    if (!is_tensor(o)) Py_RETURN_FALSE;
+    TensorObj *p = T_(o);
+    if (!requires_grad(p)) continue;
+    if (!is_fast(o) || !p->grad || !is_fast(p->grad) || !same_shape(p, T_(p->grad))) Py_RETURN_FALSE;
+    ps.push_back(view_of(p));
+    gs.push_back(view_of(T_(p->grad)));
+  }
+  const int rc = nt_sgd_update_many(ps.data(), gs.data(), int32_t(ps.size()), float(lr), float(scale));
   if (rc) return raise_status(rc);
   Py_RETURN_TRUE;
 }

@@ -132,12 +132,14 @@ class GradientDescent(Optimizer):
         self._grad_scale = grad_scale
 
     def step(self) -> None:
+        if _engine.sgd_update(self.parameters, self._lr, self._grad_scale):
+            return
         for p in self.parameters:
             if not p.requires_grad:
                 continue
             if p.grad is None:
                 raise RuntimeError("Gradients not set, did you call backward?")
-            if not _engine.sgd_update(p, self._lr, self._grad_scale):
+            if not _engine.sgd_update([p], self._lr, self._grad_scale):
                 with no_grad():
                     g = p.grad
                     if self._grad_scale != 1.0:
