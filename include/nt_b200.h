@@ -145,6 +145,12 @@ int nt_full(int64_t n, const nt_scalar *value, int dtype, int device, nt_storage
  * backward pass; the reference copies a one-element tensor to the device for each).  No memory and no fill
  * launch until something needs the address: the Float32 elementwise kernels take the value as an argument. */
 int nt_constant(const nt_scalar *value, int dtype, nt_storage **out);
+/* factor * x for a dense Float32 Cuda view, without a launch: kernels that take the result as an operand multiply as they
+ * read x, others find it written when they ask for its address (nt_storage_settle does that at once).  x must not be
+ * written in between, so this is for use inside one call -- a backward sweep, where the gradient of a squared error is
+ * the saved difference times a number.  *out stays NULL when x is not dense. */
+int nt_scaled(const nt_view *x, float factor, nt_storage **out);
+int nt_storage_settle(nt_storage *s);
 /* eye / arange are written by a kernel when device is Cuda (host loop + copy in the reference). */
 int nt_eye(int64_t n, int dtype, int device, nt_storage **out);
 int nt_arange(int64_t n, int64_t start, int64_t step, int dtype, int device, nt_storage **out);

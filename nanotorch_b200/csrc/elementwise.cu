@@ -322,6 +322,14 @@ template <template <class> class F, bool ARITH_ONLY> static void inplace_impl(co
   storage_touch(out->storage);
 }
 
+static bool row_major(const nt_view *v) {
+  int64_t acc = 1;
+  for (int d = v->ndim - 1; d >= 0; --d) {
+    if (v->shape[d] != 1 && v->strides[d] != acc) return false;
+    acc *= v->shape[d];
+  }
+  return true;
+}
 // fp32-only fused entry: every view must be Float32 on Cuda with the shape of `shape_of`.
 static void fused_checks(const nt_view *const *views, int n, const char *fname) {
   for (int i = 0; i < n; ++i) {
@@ -334,6 +342,12 @@ static void fused_checks(const nt_view *const *views, int n, const char *fname) 
 template <class F> static nt_storage *fused2(F f, const nt_view *a, const nt_view *b, const char *fname) {
   const nt_view *chk[2] = {a, b};
   fused_checks(chk, 2, fname);
+  if constexpr (!is_bound<F>::value) {
+    if (a->storage->scaled()) {
+      const nt_view u = unscaled_view(*a);
+      return fused2(ScaledFirst<F>{f, a->storage->value}, &u, b, fname);
+    }
+  }
   StorageRef out(storage_new(view_numel(*a), NT_FLOAT32, NT_CUDA));
   nt_view ov = fresh_view(out.s, *a);
   const nt_view *views[3] = {&ov, a, b};
@@ -351,6 +365,12 @@ static bool dense_2d(const nt_view *v) {
          v->storage->device == NT_CUDA;
 }
 template <class F, int NIN> static nt_storage *produce_with_planes(F f, const nt_view *a, const nt_view *b) {
+  if constexpr (NIN == 2 && !is_bound<F>::value) {
+    if (a->storage->scaled()) {
+      const nt_view u = unscaled_view(*a);
+      return produce_with_planes<ScaledFirst<F>, 2>(ScaledFirst<F>{f, a->storage->value}, &u, b);
+    }
+  }
   if (!g_producer_planes.load() || nt_get_matmul_mode() != 1 || !dense_2d(a)) return nullptr;
   const int64_t R = a->shape[0], C = a->shape[1];
   if (C % 32 != 0 || R * C < (int64_t(1) << 20)) return nullptr;
@@ -389,6 +409,12 @@ template <class F> static void binary_backward_both(F f, const nt_view *g, const
   *out1 = *out2 = nullptr;
   const nt_view *chk[3] = {g, x1, x2};
   fused_checks(chk, 3, fname);
+  if constexpr (!is_bound<F>::value) {
+    if (g->storage->scaled()) {
+      const nt_view u = unscaled_view(*g);
+      return binary_backward_both(ScaledFirst<F>{f, g->storage->value}, &u, x1, x2, out1, out2, fname);
+    }
+  }
   const int64_t n = view_numel(*g);
   const float *p[3];
   for (int i = 0; i < 3; ++i) {
@@ -412,14 +438,6 @@ template <class F> static void binary_backward_both(F f, const nt_view *g, const
 // ---- SGD.  A weight that has been a matmul operand: its TF32 planes follow the update.  When the parameter is the whole
 // of a dense 2-D storage the update writes them itself (20 bytes per element in one launch instead of 12 + 12 in two);
 // otherwise the cached views are split again behind the update.
-static bool row_major(const nt_view *v) {
-  int64_t acc = 1;
-  for (int d = v->ndim - 1; d >= 0; --d) {
-    if (v->shape[d] != 1 && v->strides[d] != acc) return false;
-    acc *= v->shape[d];
-  }
-  return true;
-}
 static float *sgd_planes(const nt_view *param) {
   if (!g_producer_planes.load() || nt_get_matmul_mode() != 1 || !dense_2d(param) || param->offset != 0 ||
       param->shape[0] * param->shape[1] != param->storage->n)
@@ -491,6 +509,20 @@ __global__ void __launch_bounds__(256) sgd_batch(SgdF f, const __grid_constant__
       }
     }
   }
+}
+
+void scale_into(float *out, const float *in, int64_t n, float factor) {
+  nt_storage dst, src; // views of the two runs
+  dst.block = out;
+  src.block = const_cast<float *>(in);
+  nt_view ov{}, iv{};
+  ov.storage = &dst;
+  iv.storage = &src;
+  ov.ndim = iv.ndim = 1;
+  ov.shape[0] = iv.shape[0] = n;
+  ov.strides[0] = iv.strides[0] = 1;
+  const nt_view *views[2] = {&ov, &iv};
+  ew_launch<BindFirst<MulF<float>>, 1>(BindFirst<MulF<float>>{{}, factor}, views);
 }
 
 } // namespace ntb
@@ -606,6 +638,11 @@ int nt_sigmoid(const nt_view *x, nt_storage **out) {
 }
 int nt_neg(const nt_view *x, nt_storage **out) {
   NT_API_BEGIN
+  check_view(x, "neg");
+  if (x->storage->scaled() && x->offset == 0 && x->storage->n == view_numel(*x) && row_major(x)) { // the other factor: exact
+    *out = storage_new_scaled(x->storage->src, x->storage->src_offset, x->storage->n, -x->storage->value);
+    return NT_OK;
+  }
   *out = unary_impl<NegF, 1>(x, "neg");
   NT_API_END
 }
@@ -631,7 +668,10 @@ int nt_pow(const nt_view *x, const nt_scalar *exponent, nt_storage **out) {
     if constexpr (std::is_same_v<T, float>) {
       f.special = pow_special(v);
       if (f.special == 3) {
-        ew_launch<SquareF, 1>(SquareF{}, views);
+        const float *in = static_cast<const float *>(x->storage->ptr()) + x->offset;
+        const int64_t n = view_numel(*x);
+        if (n > 0 && row_major(x) && aligned16(in)) square_with_sums(in, o.s, n);
+        else ew_launch<SquareF, 1>(SquareF{}, views);
         return;
       }
     }

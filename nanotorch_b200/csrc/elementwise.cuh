@@ -585,7 +585,26 @@ template <class F> struct BindSecond {
   in_t v;
   __device__ __forceinline__ out_t operator()(in_t a) const { return f(a, v); }
 };
+// A functor whose first argument -- the gradient -- is a value times a factor, rounded as the product of its own launch
+// would be (nt_scaled).
+template <class F> struct ScaledFirst {
+  using in_t = float;
+  using out_t = float;
+  F f;
+  float k;
+  __device__ __forceinline__ float operator()(float g, float x) const { return f(k * g, x); }
+  __device__ __forceinline__ void operator()(float g, float x1, float x2, float *d1, float *d2) const { f(k * g, x1, x2, d1, d2); }
+};
+// The view of what a scaled storage is a multiple of, for a view of that storage.
+inline nt_view unscaled_view(const nt_view &v) {
+  nt_view u = v;
+  u.storage = v.storage->src;
+  u.offset += v.storage->src_offset;
+  return u;
+}
+
 template <class F> struct is_bound : std::false_type {};
+template <class F> struct is_bound<ScaledFirst<F>> : std::true_type {};
 template <class F> struct is_bound<BindFirst<F>> : std::true_type {};
 template <class F> struct is_bound<BindSecond<F>> : std::true_type {};
 
@@ -593,7 +612,7 @@ template <class F> struct is_bound<BindSecond<F>> : std::true_type {};
 template <class F, int NIN> void ew_launch(F f, const nt_view *const (&views)[NIN + 1]) {
   using TI = typename F::in_t;
   using TO = typename F::out_t;
-  if constexpr (NIN == 2 && std::is_same_v<TI, float> && std::is_same_v<TO, float>) {
+  if constexpr (NIN == 2 && !is_bound<F>::value && std::is_same_v<TI, float> && std::is_same_v<TO, float>) {
     const bool c1 = views[1]->storage->constant, c2 = views[2]->storage->constant;
     if (c2 && !c1) {
       const nt_view *rest[2] = {views[0], views[1]};
@@ -631,7 +650,7 @@ template <class F, int NIN> void ew_launch(F f, const nt_view *const (&views)[NI
   }
 
   // (1b) a dense [R, C] operand against one broadcast row
-  if constexpr (NIN == 2 && std::is_same<TI, float>::value && std::is_same<TO, float>::value) {
+  if constexpr (NIN == 2 && !is_bound<F>::value && std::is_same<TI, float>::value && std::is_same<TO, float>::value) {
     if (it.ndim == 2 && (it.shape[1] & 3) == 0 && (it.numel >> 2) < (int64_t(1) << 31) && it.strides[0][0] == it.shape[1] &&
         it.strides[0][1] == 1 && aligned16(out) && aligned16(in[0]) && aligned16(in[1])) {
       const int64_t C = it.shape[1];

@@ -222,7 +222,15 @@ struct NoGrad {
   ~NoGrad() { G.grad_enabled = prev; }
 };
 
+// What leaves the sweep is in memory: see nt_scaled.
+static bool settle(PyObject *g) {
+  if (!is_tensor(g) || !T_(g)->storage || !is_storage(T_(g)->storage)) return true;
+  const int rc = nt_storage_settle(storage_of(T_(g)));
+  if (rc) raise_status(rc);
+  return rc == 0;
+}
 static bool accumulate(TensorObj *x, PyObject *gx) {
+  if (!x->grad_fn && !settle(gx)) return false;
   if (!x->grad) {
     x->grad = own(gx);
     return true;
@@ -288,7 +296,7 @@ PyObject *run_backward(TensorObj *root) {
     const bool native = PyObject_TypeCheck(fn.p, &FunctionBase_Type) && backward_fast(F_(fn.p), T_(g.p), out, &n_out);
     Ref held[3] = {Ref(out[0]), Ref(out[1]), Ref(out[2])};
     if (!native) {
-      if (PyErr_Occurred()) return nullptr;
+      if (PyErr_Occurred() || !settle(g.p)) return nullptr;
       Ref r(PyObject_CallMethod(fn.p, "backward", "O", g.p));
       if (!r) return nullptr;
       grads = Ref(PySequence_Fast(r.p, "backward must return one gradient per tensor input"));

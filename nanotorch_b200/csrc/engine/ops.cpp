@@ -745,6 +745,15 @@ static bool backward_op(FunctionObj *fn, TensorObj *g, PyObject **out, int *n_ou
     *n_out = 1;
     const nt_view vg = view_of(g), vx = view_of(x);
     nt_storage *s = nullptr;
+    // a squared error: the gradient is the saved difference times a number (unless that difference is a leaf, whose
+    // values a hook may change during the sweep)
+    if (fn->e == 2.0 && vg.storage->constant && x->grad_fn) {
+      checked(nt_scaled(&vx, vg.storage->value * 2.0f, &s), s);
+      if (s) {
+        out[0] = fresh(s, g->nd, g->sh);
+        return true;
+      }
+    }
     out[0] = fresh(checked(nt_pow_backward(&vg, &vx, float(fn->e), &s), s), g->nd, g->sh);
     return true;
   }

@@ -898,6 +898,7 @@ struct NatSplitArgs {
   float *hi, *lo;
   int64_t R, C, Cp, s_r, s_b;
   int vec; // rows of the source may be read 128 bits at a time
+  float factor;
 };
 
 __global__ void __launch_bounds__(256) split_planes(NatSplitArgs a) {
@@ -923,6 +924,7 @@ __global__ void __launch_bounds__(256) split_planes(NatSplitArgs a) {
         if (c + 2 < a.C) x[i].z = p[2];
         if (c + 3 < a.C) x[i].w = p[3];
       }
+      x[i] = make_float4(a.factor * x[i].x, a.factor * x[i].y, a.factor * x[i].z, a.factor * x[i].w);
     }
   }
 #pragma unroll
@@ -958,7 +960,13 @@ static std::atomic<uint64_t> g_split_launches{0}, g_split_hits{0};
 
 static void run_split(const nt_storage *s, const PlaneEntry &e) {
   NatSplitArgs a{};
-  a.src = static_cast<const float *>(s->ptr()) + e.offset;
+  a.factor = 1.0f;
+  if (s->scaled()) { // the product with the factor is rounded here, as it would be in memory
+    a.src = static_cast<const float *>(s->src->ptr()) + s->src_offset + e.offset;
+    a.factor = s->value;
+  } else {
+    a.src = static_cast<const float *>(s->ptr()) + e.offset;
+  }
   a.hi = e.planes;
   a.lo = e.planes + e.batch * e.R * e.Cp;
   a.R = e.R;

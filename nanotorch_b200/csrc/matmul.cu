@@ -273,8 +273,11 @@ static nt_storage *matmul_impl(const nt_view *x1, const nt_view *x2, const nt_vi
 
   if (dt == NT_FLOAT32) {
     GemmArgs g{};
-    g.A = static_cast<const float *>(x1->storage->ptr()) + x1->offset;
-    g.B = static_cast<const float *>(x2->storage->ptr()) + x2->offset;
+    // the operands in memory; the kernel that reads planes does without them
+    auto operands = [&] {
+      g.A = static_cast<const float *>(x1->storage->ptr()) + x1->offset;
+      g.B = static_cast<const float *>(x2->storage->ptr()) + x2->offset;
+    };
     g.C = static_cast<float *>(o->ptr());
     g.M = M; g.N = N; g.K = K;
     g.a_sm = a_sm; g.a_sk = a_sk; g.b_sk = b_sk; g.b_sn = b_sn;
@@ -311,16 +314,21 @@ static nt_storage *matmul_impl(const nt_view *x1, const nt_view *x2, const nt_vi
         b_sb = bi.b_strides[bi.ndim - 1];
       }
       const float *bp = bias ? static_cast<const float *>(bias->storage->ptr()) + bias->offset : nullptr;
-      if (single && by_time && fused_us < tc_us)
+      if (single && by_time && fused_us < tc_us) {
+        operands();
         bias_done = done = gemm_fused(g.A, g.B, g.C, nbatch, M, N, K, a_sb, a_sm, a_sk, b_sb, b_sk, b_sn, bp, bias ? bias->strides[0] : 0);
+      }
       if (single && !done && mode == 1 && g_natural_planes.load())
         done = gemm_3xtf32_natural(x1->storage, x1->offset, x2->storage, x2->offset, g.C, nbatch, M, N, K, a_sb, a_sm,
                                    a_sk, b_sb, b_sk, b_sn, bp, bias ? bias->strides[0] : 0, &bias_done);
-      if (single && !done)
+      if (single && !done) {
+        operands();
         done = gemm_3xtf32(g.A, g.B, g.C, nbatch, M, N, K, a_sb, a_sm, a_sk, b_sb, b_sk, b_sn, bp,
                            bias ? bias->strides[0] : 0, &bias_done);
+      }
     }
     if (!done) {
+      operands();
       g.bias = bias ? static_cast<const float *>(bias->storage->ptr()) + bias->offset : nullptr;
       g.bias_stride = bias ? bias->strides[0] : 0;
       bias_done = true;

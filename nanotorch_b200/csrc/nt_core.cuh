@@ -162,8 +162,16 @@ struct nt_storage {
   nt_scalar scalar{};
   nt_storage *prev = nullptr, *next = nullptr; // constants without memory, see constants_materialize_all
 
+  // value * (n elements of `src` from src_offset on), another storage's product with a known factor: the gradient of a
+  // squared error, inside a backward sweep (see nt_scaled).  Kernels that can take the factor read `src` itself.
+  nt_storage *src = nullptr;
+  int64_t src_offset = 0;
+  // The sum and the mean of all elements, when the kernel that wrote them left those too; handed out once.
+  nt_storage *side_sum = nullptr, *side_mean = nullptr;
+
+  bool scaled() const { return src && !block; }
   void *ptr() const {
-    if (constant && !block) materialize();
+    if (!block && (constant || src)) materialize();
     return block;
   }
   void materialize() const;
@@ -179,6 +187,11 @@ inline void storage_touch(nt_storage *s) {
   s->mutation += 1;
 }
 nt_storage *storage_new_constant(const nt_scalar &value, int dtype);
+nt_storage *storage_new_scaled(nt_storage *src, int64_t offset, int64_t n, float factor);
+void scale_into(float *out, const float *in, int64_t n, float factor); // elementwise.cu
+// x * x for n contiguous, 16-byte aligned values, leaving sum and mean of the result with `out` (reduce.cu)
+void square_with_sums(const float *in, nt_storage *out, int64_t n);
+void drop_side_sums(nt_storage *s);
 nt_storage *storage_new_constant(float value);
 // Gives every constant its memory: called before a graph capture starts, because a fill recorded inside the capture
 // would not have run yet for eager work, and would run again on every replay.

@@ -406,9 +406,34 @@ nt_storage *storage_new_constant(const nt_scalar &value, int dtype) {
   return s;
 }
 nt_storage *storage_new_constant(float value) { return storage_new_constant(nt_scalar{2, 0, value}, NT_FLOAT32); }
+nt_storage *storage_new_scaled(nt_storage *src, int64_t offset, int64_t n, float factor) {
+  nt_storage *s = new nt_storage();
+  s->n = n;
+  s->dtype = NT_FLOAT32;
+  s->device = NT_CUDA;
+  s->value = factor;
+  s->src = src;
+  s->src_offset = offset;
+  storage_retain(src);
+  return s;
+}
+void drop_side_sums(nt_storage *s) {
+  storage_release(s->side_sum);
+  storage_release(s->side_mean);
+  s->side_sum = s->side_mean = nullptr;
+}
 void storage_release(nt_storage *s) {
   if (!s) return;
   if (s->refs.fetch_sub(1, std::memory_order_acq_rel) == 1) {
+    drop_side_sums(s);
+    if (s->src) {
+      storage_release(s->src);
+      if (!s->block) {
+        gemm_tc_forget(s);
+        delete s;
+        return;
+      }
+    }
     if (s->constant && !s->block) {
       constants_unlink(s);
       delete s;
@@ -634,6 +659,12 @@ void constants_materialize_all() {
 
 void nt_storage::materialize() const {
   nt_storage *s = const_cast<nt_storage *>(this);
+  if (s->src) {
+    void *p = ntb::device_alloc(size_t(s->n) * sizeof(float), &s->rounded);
+    ntb::scale_into(static_cast<float *>(p), static_cast<const float *>(s->src->ptr()) + s->src_offset, s->n, s->value);
+    s->block = p;
+    return;
+  }
   ntb::constants_unlink(s);
   ntb::fill_constant(s);
 }
@@ -918,6 +949,7 @@ void *nt_storage_data(nt_storage *s) {
   try {
     void *p = s->ptr();
     s->constant = false; // the caller may write through the pointer
+    drop_side_sums(s);
     return p;
   } catch (...) {
     return nullptr;
@@ -1033,6 +1065,26 @@ int nt_full(int64_t n, const nt_scalar *value, int dtype, int device, nt_storage
 int nt_constant(const nt_scalar *value, int dtype, nt_storage **out) {
   NT_API_BEGIN
   *out = storage_new_constant(*value, dtype);
+  NT_API_END
+}
+
+int nt_scaled(const nt_view *x, float factor, nt_storage **out) {
+  NT_API_BEGIN
+  *out = nullptr;
+  check_view(x, "scaled");
+  require_cuda(x, "scaled");
+  int64_t acc = 1;
+  for (int d = x->ndim - 1; d >= 0; --d) {
+    if (x->shape[d] != 1 && x->strides[d] != acc) return NT_OK;
+    acc *= x->shape[d];
+  }
+  if (x->storage->dtype != NT_FLOAT32 || acc == 0 || x->storage->constant || x->storage->src) return NT_OK;
+  *out = storage_new_scaled(x->storage, x->offset, acc, factor);
+  NT_API_END
+}
+int nt_storage_settle(nt_storage *s) {
+  NT_API_BEGIN
+  s->ptr();
   NT_API_END
 }
 

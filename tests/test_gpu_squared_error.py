@@ -1,0 +1,56 @@
+"""A squared error's mean and gradient: the sums that the square leaves, and gradients kept as a factor of the saved
+difference, against NumPy in double precision and against the op-by-op path; sizes around a CTA's chunk."""
+
+import numpy as np
+import pytest
+
+from tests.util import bits
+
+pytestmark = pytest.mark.gpu
+
+
+@pytest.mark.parametrize("shape", [(), (1,), (5,), (3, 7), (1023, 4), (64, 64), (4097,), (129, 513), (1200, 1027)], ids=str)
+def test_mean_and_sum_of_squares(nt, shape):
+    x = np.asarray(np.random.default_rng(1).standard_normal(shape), np.float32)
+    t = nt.Tensor.from_numpy(x, "cuda") if shape else nt.Tensor(float(x)).to("cuda")
+    square = t ** 2
+    assert np.array_equal(bits(square.numpy()), bits(x * x))
+    want = np.square(x.astype(np.float64))
+    for _ in range(2):  # the second time the sums come from the square in memory
+        assert abs(float(nt.mean(square).numpy()) - want.mean()) <= 2e-6 * want.mean()
+        assert abs(float(nt.sum(square).numpy()) - want.sum()) <= 2e-6 * want.sum()
+    square = t ** 2
+    with nt.no_grad():
+        square += 1.0  # the sums that came with it are out of date
+    assert abs(float(nt.mean(square).numpy()) - (want + 1).mean()) <= 2e-6 * (want + 1).mean()
+
+
+OPS = {"add": lambda a, b: a + b, "mul": lambda a, b: a * b, "truediv": lambda a, b: a / b, "tanh": lambda a, b: a.tanh(),
+       "sigmoid": lambda a, b: a.sigmoid(), "relu": lambda a, b: a.relu(), "exp": lambda a, b: a.exp(), "log": lambda a, b: a.log(),
+       "sqrt": lambda a, b: a.sqrt(), "neg": lambda a, b: -a, "pow": lambda a, b: a ** 3.0, "matmul": lambda a, b: a @ b.T,
+       "transposed": lambda a, b: a.T * b.T, "sum": lambda a, b: a.sum(axis=0), "max": lambda a, b: a.max(axis=1),
+       "reshape": lambda a, b: a.reshape(a.numel), "twice": lambda a, b: a * a + b}
+
+
+@pytest.mark.parametrize("op", OPS)
+@pytest.mark.parametrize("shape", [(5, 7), (64, 132), (1024, 1056)], ids=str)
+def test_gradients_of_a_squared_error(nt, op, shape):
+    rng = np.random.default_rng(2)
+    a, b = (rng.uniform(0.5, 2, shape).astype(np.float32) for _ in range(2))
+    got = []
+    for k in (2, nt.Tensor(2.0).to("cuda")):  # a tensor exponent takes the classes' own path
+        ta, tb = (nt.Tensor.from_numpy(v, "cuda", requires_grad=True) for v in (a, b))
+        y = OPS[op](ta, tb)
+        target = nt.Tensor.from_numpy(np.random.default_rng(3).standard_normal(y.shape).astype(np.float32), "cuda")
+        nt.mean((y - target) ** k).backward()
+        got.append([t.grad.numpy() for t in (ta, tb) if t.grad is not None])
+    assert len(got[0]) == len(got[1])
+    for g, h in zip(*got):
+        assert np.array_equal(bits(g), bits(h)) if op != "matmul" else np.allclose(g, h, rtol=1e-5, atol=1e-9)
+
+
+def test_a_leaf_under_the_square(nt):
+    x = np.random.default_rng(4).standard_normal((33, 5)).astype(np.float32)
+    t = nt.Tensor.from_numpy(x, "cuda", requires_grad=True)
+    (t ** 2).mean().backward()
+    assert np.array_equal(bits(t.grad.numpy()), bits(np.float32(np.float32(1) / np.float32(x.size) * 2) * x))
