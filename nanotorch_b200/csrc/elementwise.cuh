@@ -51,6 +51,13 @@ struct EwParams {
 
 __device__ __forceinline__ float4 ld_stream(const float4 *p) { return __ldcs(p); }
 __device__ __forceinline__ void st_stream(float4 *p, float4 v) { __stcs(p, v); }
+// A result of up to 96 MB stays in the L2 for the op that reads it next ((a * b - t) ** 2 at 4096 x 4096 with its
+// gradients: 131 -> 122 us); a larger one would only push itself out.  Operands are read with the streaming hint either
+// way: keeping them too displaced the results (139 us).
+__device__ __forceinline__ void st_result(float4 *p, float4 v, int64_t nvec) {
+  if (nvec <= (int64_t(6) << 20)) *p = v;
+  else __stcs(p, v);
+}
 
 // ---------------------------------------------------------------------------------------------
 // Contiguous fp32-sized kernel.  TI/TO are 4-byte types.
@@ -91,7 +98,7 @@ __global__ void __launch_bounds__(256) ew_contig(F f, typename F::out_t *out, co
         if constexpr (NIN == 2) pr[e] = f(pa[e], pb[e]);
         if constexpr (NIN == 3) pr[e] = f(pa[e], pb[e], pc[e]);
       }
-      st_stream(reinterpret_cast<float4 *>(out) + i, r);
+      st_result(reinterpret_cast<float4 *>(out) + i, r, nvec);
     }
   }
   // ragged tail (n % 4 elements) by the first threads of block 0
@@ -169,7 +176,51 @@ __global__ void __launch_bounds__(256) ew_contig_rowbcast(F f, float *out, const
       float4 y;
       if constexpr (ROW_FIRST) y = make_float4(f(r.x, x.x), f(r.y, x.y), f(r.z, x.z), f(r.w, x.w));
       else y = make_float4(f(x.x, r.x), f(x.y, r.y), f(x.z, r.z), f(x.w, r.w));
-      st_stream(reinterpret_cast<float4 *>(out) + i, y);
+      st_result(reinterpret_cast<float4 *>(out) + i, y, nvec);
+    }
+  }
+}
+
+// [R, C] op [R, 1]: every operand is dense (mode 0) or one value per row (mode 1) -- a softmax's maximum and sum, and the
+// backward of either.  The contiguous kernel with the row number from one multiply-high per vector; the general strided
+// kernel spends a chain of them, and 500 bytes of parameters, on any number of dims.  C % 4 == 0, fewer than 2^31 vectors.
+template <class F, int NIN>
+__global__ void __launch_bounds__(256) ew_contig_colbcast(F f, float *out, const float *a, const float *b, const float *c, int modes,
+                                                          int64_t nvec, uint32_t div_mul, uint32_t div_shift) {
+  pdl_trigger();
+  pdl_wait();
+  constexpr int UNROLL = 4;
+  const int64_t base = (int64_t(blockIdx.x) * UNROLL) * blockDim.x + threadIdx.x;
+  float4 v[UNROLL][NIN];
+#pragma unroll
+  for (int u = 0; u < UNROLL; ++u) {
+    const int64_t i = base + int64_t(u) * blockDim.x;
+    if (i < nvec) {
+      const uint32_t lin = uint32_t(i), row = div_mul ? (__umulhi(lin, div_mul) >> div_shift) : lin;
+#pragma unroll
+      for (int o = 0; o < NIN; ++o) {
+        const float *p = o == 0 ? a : o == 1 ? b : c;
+        if (modes >> o & 1) {
+          const float x = __ldg(p + row);
+          v[u][o] = make_float4(x, x, x, x);
+        } else {
+          v[u][o] = ld_stream(reinterpret_cast<const float4 *>(p) + i);
+        }
+      }
+    }
+  }
+#pragma unroll
+  for (int u = 0; u < UNROLL; ++u) {
+    const int64_t i = base + int64_t(u) * blockDim.x;
+    if (i < nvec) {
+      float4 y;
+      if constexpr (NIN == 2) {
+        y = make_float4(f(v[u][0].x, v[u][1].x), f(v[u][0].y, v[u][1].y), f(v[u][0].z, v[u][1].z), f(v[u][0].w, v[u][1].w));
+      } else {
+        y = make_float4(f(v[u][0].x, v[u][1].x, v[u][2].x), f(v[u][0].y, v[u][1].y, v[u][2].y),
+                        f(v[u][0].z, v[u][1].z, v[u][2].z), f(v[u][0].w, v[u][1].w, v[u][2].w));
+      }
+      st_result(reinterpret_cast<float4 *>(out) + i, y, nvec);
     }
   }
 }
@@ -667,6 +718,27 @@ template <class F, int NIN> void ew_launch(F f, const nt_view *const (&views)[NI
         else
           launch(ew_contig_rowbcast<F, false>, blocks, 256, 0, f, out, in[0], in[1], nvec, uint32_t(C >> 2), mul, shift);
         check_launch("ew_contig_rowbcast");
+        return;
+      }
+    }
+  }
+
+  // (1c) dense [R, C] operands and at least one with a value per row
+  if constexpr (NIN >= 2 && !is_bound<F>::value && std::is_same<TI, float>::value && std::is_same<TO, float>::value) {
+    if (it.ndim == 2 && (it.shape[1] & 3) == 0 && (it.numel >> 2) < (int64_t(1) << 31) && it.strides[0][0] == it.shape[1] &&
+        it.strides[0][1] == 1 && aligned16(out)) {
+      int modes = 0;
+      bool fits = true;
+      for (int o = 0; o < NIN; ++o) {
+        if (it.strides[o + 1][0] == 1 && it.strides[o + 1][1] == 0) modes |= 1 << o;
+        else fits = fits && it.strides[o + 1][0] == it.shape[1] && it.strides[o + 1][1] == 1 && aligned16(in[o]);
+      }
+      if (fits && modes) {
+        uint32_t mul, shift;
+        ew_fast_divisor(it.shape[1] >> 2, &mul, &shift);
+        const int64_t nvec = it.numel >> 2;
+        launch(ew_contig_colbcast<F, NIN>, unsigned(ceil_div(nvec, 256 * 4)), 256, 0, f, out, in[0], in[1], in[2], modes, nvec, mul, shift);
+        check_launch("ew_contig_colbcast");
         return;
       }
     }

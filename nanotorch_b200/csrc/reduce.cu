@@ -152,48 +152,71 @@ __global__ void __launch_bounds__(256) reduce_rows(const float *__restrict__ in,
   }
 }
 
-// Short rows: a warp takes four rows at a time (their loads are issued together, so that a lane has four
-// 128-bit loads in flight instead of one), 32 rows per CTA.
-template <class Op>
+// Short rows: a warp takes RPW rows at a time, eight 128-bit loads in flight per lane either way -- two of each of four rows,
+// or eight of one.  Four rows need 4736 warps to fill the GPU, 18944 rows; with fewer a row per warp spreads them over more
+// SMs (4096 rows of 1000: 128 CTAs took 14 us, 512 take 5).
+template <class Op, int RPW>
 __global__ void __launch_bounds__(256) reduce_rows_warp(const float *__restrict__ in, float *__restrict__ out,
                                                         KeepIndex keep, int64_t n_rows, int64_t L, float divisor) {
+  pdl_trigger();
   pdl_wait();
-  const int64_t row0 = (int64_t(blockIdx.x) * 8 + (threadIdx.x >> 5)) * 4;
+  constexpr int DEPTH = 8 / RPW;
+  const int64_t row0 = (int64_t(blockIdx.x) * 8 + (threadIdx.x >> 5)) * RPW;
   if (row0 >= n_rows) return;
   const int lane = threadIdx.x & 31;
-  const float *p[4];
+  const float *p[RPW];
   bool vec = true;
 #pragma unroll
-  for (int r = 0; r < 4; ++r) {
+  for (int r = 0; r < RPW; ++r) {
     const int64_t row = (row0 + r < n_rows) ? row0 + r : n_rows - 1; // a row past the end re-reads the last one, unused
     p[r] = in + keep_offset(keep, row);
     vec = vec && ((reinterpret_cast<uintptr_t>(p[r]) & 15) == 0);
   }
-  float a[4] = {Op::neutral(), Op::neutral(), Op::neutral(), Op::neutral()};
+  float a[RPW];
+#pragma unroll
+  for (int r = 0; r < RPW; ++r) a[r] = Op::neutral();
   if (vec) {
-    const int64_t nvec = L >> 2;
-    for (int64_t i = lane; i < nvec; i += 32) {
-      float4 v[4];
+    const int nvec = int(L >> 2);
+    for (int i = lane; i < nvec; i += 32 * DEPTH) {
+      float4 v[DEPTH][RPW];
 #pragma unroll
-      for (int r = 0; r < 4; ++r) v[r] = __ldcs(reinterpret_cast<const float4 *>(p[r]) + i);
+      for (int u = 0; u < DEPTH; ++u)
 #pragma unroll
-      for (int r = 0; r < 4; ++r) a[r] = Op::combine(a[r], Op::combine(Op::combine(v[r].x, v[r].y), Op::combine(v[r].z, v[r].w)));
+        for (int r = 0; r < RPW; ++r)
+          v[u][r] = i + 32 * u < nvec ? __ldcs(reinterpret_cast<const float4 *>(p[r]) + i + 32 * u)
+                                      : make_float4(Op::neutral(), Op::neutral(), Op::neutral(), Op::neutral());
+#pragma unroll
+      for (int u = 0; u < DEPTH; ++u)
+#pragma unroll
+        for (int r = 0; r < RPW; ++r)
+          a[r] = Op::combine(a[r], Op::combine(Op::combine(v[u][r].x, v[u][r].y), Op::combine(v[u][r].z, v[u][r].w)));
     }
-    for (int64_t j = (nvec << 2) + lane; j < L; j += 32) {
+    for (int j = (nvec << 2) + lane; j < int(L); j += 32) {
 #pragma unroll
-      for (int r = 0; r < 4; ++r) a[r] = Op::combine(a[r], p[r][j]);
+      for (int r = 0; r < RPW; ++r) a[r] = Op::combine(a[r], p[r][j]);
     }
   } else {
-    for (int64_t j = lane; j < L; j += 32) {
+    for (int j = lane; j < int(L); j += 32 * DEPTH) {
 #pragma unroll
-      for (int r = 0; r < 4; ++r) a[r] = Op::combine(a[r], p[r][j]);
+      for (int u = 0; u < DEPTH; ++u)
+#pragma unroll
+        for (int r = 0; r < RPW; ++r)
+          if (j + 32 * u < int(L)) a[r] = Op::combine(a[r], p[r][j + 32 * u]);
     }
   }
 #pragma unroll
-  for (int r = 0; r < 4; ++r) {
+  for (int r = 0; r < RPW; ++r) {
     a[r] = warp_reduce<Op>(a[r]);
     if (lane == 0 && row0 + r < n_rows) out[row0 + r] = (divisor != 0.0f) ? a[r] / divisor : a[r];
   }
+}
+template <class Op>
+static void launch_rows_warp(const float *in, float *out, const KeepIndex &keep, int64_t n_rows, int64_t L, float divisor) {
+  if (n_rows >= int64_t(sm_count()) * 8 * 16)
+    launch(reduce_rows_warp<Op, 4>, unsigned(ceil_div(n_rows, 32)), 256, 0, in, out, keep, n_rows, L, divisor);
+  else
+    launch(reduce_rows_warp<Op, 1>, unsigned(ceil_div(n_rows, 8)), 256, 0, in, out, keep, n_rows, L, divisor);
+  check_launch("reduce_rows_warp");
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -615,8 +638,7 @@ template <class Op> static bool try_fast_f32(const nt_view *x, const Plan &pl, f
     if (L < 1024 && n_rows >= 64) {
       int64_t blocks = ceil_div(n_rows, 32);
       if (blocks > 0x7fffffffLL) return false;
-      launch(reduce_rows_warp<Op>, unsigned(blocks), 256, 0, in, out, pl.keep, n_rows, L, divisor);
-      check_launch("reduce_rows_warp");
+      launch_rows_warp<Op>(in, out, pl.keep, n_rows, L, divisor);
       return true;
     }
     int64_t S = ceil_div(target_ctas, n_rows);
@@ -1236,8 +1258,7 @@ int nt_sum_rows_noalloc(const float *in, int64_t n_rows, int64_t row_len, float 
   if (row_len < 1024 && n_rows >= 64) {
     int64_t blocks = ceil_div(n_rows, 32);
     if (blocks > 0x7fffffffLL) fail_invalid("nt_sum_rows_noalloc: too many rows for one launch.");
-    launch(reduce_rows_warp<RSum>, unsigned(blocks), 256, 0, in, out, keep, n_rows, row_len, 0.0f);
-    check_launch("reduce_rows_warp");
+    launch_rows_warp<RSum>(in, out, keep, n_rows, row_len, 0.0f);
     return NT_OK;
   }
   int64_t S = ceil_div(target_ctas, n_rows);
