@@ -638,6 +638,19 @@ static nt_view transposed(const TensorObj *t) { // the last two dims swapped
   return v;
 }
 
+// -g; a constant gradient, however expanded, stays one
+static PyObject *negated(TensorObj *g) {
+  const nt_view v = view_of(g);
+  if (v.storage->constant) {
+    Ref so(wrap_storage(constant(nt_scalar{2, 0, -double(v.storage->value)})));
+    PyObject *t = so ? reinterpret_cast<PyObject *>(new_view(so.p, g->nd, g->sh, g->st, g->offset)) : nullptr;
+    if (!t) throw PyErr{};
+    return t;
+  }
+  nt_storage *s = nullptr;
+  return fresh(checked(nt_neg(&v, &s), s), g->nd, g->sh);
+}
+
 // A product's operand as it took part: a scalar tensor keeps its own dtype in the graph, so only fast ones qualify.
 static bool fast_pair(FunctionObj *fn) {
   return is_fast(reinterpret_cast<PyObject *>(saved(fn, 0))) && is_fast(reinterpret_cast<PyObject *>(saved(fn, 1)));
@@ -653,10 +666,9 @@ static bool backward_op(FunctionObj *fn, TensorObj *g, PyObject **out, int *n_ou
       if (fn->op == OP_ADD) {
         out[1] = unbroadcast(g, input(fn, 1)).release();
       } else {
-        const nt_view v = view_of(g);
-        nt_storage *s = nullptr;
-        Ref neg(fresh(checked(nt_neg(&v, &s), s), g->nd, g->sh));
-        out[1] = unbroadcast(std::move(neg), input(fn, 1)).release();
+        // summed first: the sum of the negated values is the negated sum, bit for bit
+        Ref sum(unbroadcast(g, input(fn, 1)));
+        out[1] = negated(T_(sum.p));
       }
     }
     return true;
@@ -681,6 +693,21 @@ static bool backward_op(FunctionObj *fn, TensorObj *g, PyObject **out, int *n_ou
         out[1] = second;
         if (!first || !second) throw PyErr{};
         return true;
+      }
+    }
+    if (mul && vg.storage->constant && !both) {
+      // a constant gradient, as a sum or a mean sends it: the other factor times a number (see nt_scaled; not where a
+      // hook may change that factor during the sweep)
+      const int i = need(fn, 0) ? 0 : 1;
+      TensorObj *other = saved(fn, 1 - i), *own_input = saved(fn, i);
+      if (same_shape(g, other) && same_shape(g, own_input) && is_fast(reinterpret_cast<PyObject *>(other)) && !other->requires_grad) {
+        const nt_view vo = view_of(other);
+        nt_storage *s = nullptr;
+        checked(nt_scaled(&vo, vg.storage->value, &s), s);
+        if (s) {
+          out[i] = fresh(s, g->nd, g->sh);
+          return true;
+        }
       }
     }
     Operand o1, o2;
@@ -722,13 +749,10 @@ static bool backward_op(FunctionObj *fn, TensorObj *g, PyObject **out, int *n_ou
     if (fn->op == OP_LINEAR && need(fn, 2)) out[2] = unbroadcast(g, input(fn, 2)).release();
     return true;
   }
-  case OP_NEG: {
+  case OP_NEG:
     *n_out = 1;
-    const nt_view v = view_of(g);
-    nt_storage *s = nullptr;
-    out[0] = fresh(checked(nt_neg(&v, &s), s), g->nd, g->sh);
+    out[0] = negated(g);
     return true;
-  }
   case OP_EXP: case OP_LOG: case OP_SQRT: case OP_TANH: case OP_SIGMOID: case OP_RELU: {
     static const Fn2 fns[] = {nt_exp_backward, nt_log_backward, nt_sqrt_backward, nt_tanh_backward, nt_sigmoid_backward, nt_relu_backward};
     saved_ok(fn);

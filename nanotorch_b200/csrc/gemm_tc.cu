@@ -792,9 +792,14 @@ static std::atomic<int> g_tc_max_splits{max_splits_default()};
 
 static int *g_error_flag = nullptr;
 static int *error_flag_ptr();
+// Whether a kernel that may set the flag was launched since it was last read.  A synchronising call that finds it false
+// spares itself the read, a device-to-host copy of its own that took as long as a small result's.
+static std::atomic<bool> g_flag_dirty{false};
+void gemm_tc_mark_flag() { g_flag_dirty.store(true, std::memory_order_relaxed); }
 int *pipeline_error_flag() { return error_flag_ptr(); }
 static int *error_flag_ptr() {
   int *&flag = g_error_flag;
+  gemm_tc_mark_flag();
   if (!flag) {
     if (is_capturing())
       fail_runtime("gemm_3xtf32: first use inside a graph capture; run the step once eagerly before capturing it.");
@@ -809,7 +814,7 @@ static int *error_flag_ptr() {
 // synchronisation.  0 = no error.
 int gemm_tc_take_error() {
   int *flag = g_error_flag;
-  if (!flag) return 0; // the kernel never ran
+  if (!flag || !g_flag_dirty.exchange(false)) return 0;
   int host = 0;
   if (cudaMemcpy(&host, flag, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return -1;
   if (host != 0) {

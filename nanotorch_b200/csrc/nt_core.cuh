@@ -118,6 +118,7 @@ bool matmul_profile_active();
 void matmul_profile_extend(); // the launch just made belongs to the interval opened last
 void matmul_profile_end();
 bool cuda_ok();              // a device is present and usable
+void gemm_tc_mark_flag();     // a kernel that may set it has been launched behind the host's back (a graph replay)
 int gemm_tc_take_error();    // device-side error flag of the tensor-core GEMM (0 = none); call after a sync
 void check_device_errors();  // after a stream synchronisation: raises if a bounded device-side wait ran out
 long long wait_limit_clocks(); // limit of every bounded spin in device code, in SM clocks

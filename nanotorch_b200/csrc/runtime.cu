@@ -625,6 +625,38 @@ static nt_storage *full_impl(int64_t n, const nt_scalar *value, int dtype, int d
   return out.release();
 }
 
+// A small upload goes through a pinned slot of the library's own, so that the call need not wait for the copy before the
+// caller's buffer is free again (a sample of 3 KB: the wait cost more than the copy).  Eight slots of 256 KB, each reused
+// once its copy is done.  false: too large, or inside a capture.
+static bool upload_staged(void *dst, const void *src, size_t nbytes, cudaStream_t st) {
+  constexpr size_t SLOT = size_t(256) << 10;
+  constexpr int SLOTS = 8;
+  static struct {
+    std::mutex mu;
+    char *mem = nullptr;
+    cudaEvent_t done[SLOTS] = {};
+    int next = 0;
+  } ring;
+  if (nbytes > SLOT || is_capturing()) return false;
+  std::lock_guard<std::mutex> lk(ring.mu);
+  if (!ring.mem) {
+    void *p = nullptr;
+    if (cudaHostAlloc(&p, SLOT * SLOTS, cudaHostAllocDefault) != cudaSuccess) {
+      cudaGetLastError();
+      return false;
+    }
+    for (cudaEvent_t &e : ring.done) NT_CUDA_CHECK(cudaEventCreateWithFlags(&e, cudaEventDisableTiming));
+    ring.mem = static_cast<char *>(p);
+  }
+  const int k = ring.next;
+  ring.next = (k + 1) % SLOTS;
+  NT_CUDA_CHECK(cudaEventSynchronize(ring.done[k])); // returns at once for an event never recorded
+  std::memcpy(ring.mem + k * SLOT, src, nbytes);
+  NT_CUDA_CHECK(cudaMemcpyAsync(dst, ring.mem + k * SLOT, nbytes, cudaMemcpyHostToDevice, st));
+  NT_CUDA_CHECK(cudaEventRecord(ring.done[k], st));
+  return true;
+}
+
 static nt_storage *to_device_impl(nt_storage *s, int device) {
   if (s->device == device) {
     storage_retain(s);
@@ -873,6 +905,7 @@ int nt_graph_launch(int graph_id) {
   if (it == r.graph_exec.end()) fail_invalid("nt_graph_launch: unknown graph.");
   NT_CUDA_CHECK(cudaGraphLaunch(it->second, st));
   gemm_tc_new_epoch(); // the replay rewrites storages behind the host's counters
+  gemm_tc_mark_flag();
   count_launch();
   NT_API_END
 }
@@ -1020,8 +1053,10 @@ int nt_storage_upload(nt_storage *dst, const void *host_src, int64_t nbytes) {
     std::memcpy(dst->ptr(), host_src, size_t(nbytes));
   } else {
     cudaStream_t st = stream();
-    NT_CUDA_CHECK(cudaMemcpyAsync(dst->ptr(), host_src, size_t(nbytes), cudaMemcpyHostToDevice, st));
-    NT_CUDA_CHECK(cudaStreamSynchronize(st));
+    if (!upload_staged(dst->ptr(), host_src, size_t(nbytes), st)) {
+      NT_CUDA_CHECK(cudaMemcpyAsync(dst->ptr(), host_src, size_t(nbytes), cudaMemcpyHostToDevice, st));
+      NT_CUDA_CHECK(cudaStreamSynchronize(st));
+    }
   }
   storage_touch(dst);
   NT_API_END
