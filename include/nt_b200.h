@@ -350,6 +350,9 @@ int nt_div_backward_x2(const nt_view *g, const nt_view *x1, const nt_view *x2, n
  * the single-gradient kernels. */
 int nt_mul_backward(const nt_view *g, const nt_view *x1, const nt_view *x2, nt_storage **dx1, nt_storage **dx2);
 int nt_div_backward(const nt_view *g, const nt_view *x1, const nt_view *x2, nt_storage **dx1, nt_storage **dx2);
+/* The same with large transposed operands as well (2^20 elements and more, 16-byte aligned rows): the backward sweep's. */
+int nt_mul_gradients(const nt_view *g, const nt_view *x1, const nt_view *x2, nt_storage **dx1, nt_storage **dx2);
+int nt_div_gradients(const nt_view *g, const nt_view *x1, const nt_view *x2, nt_storage **dx1, nt_storage **dx2);
 /* Max/Min backward: g_expanded * mask where mask = (x == m_expanded) and zero on every tied slice
  * (integer-division quirk of the reference, autograd/ops_reduction.py:201-212, 275-286). */
 int nt_extremum_backward(const nt_view *g_expanded, const nt_view *x, const nt_view *m_expanded,

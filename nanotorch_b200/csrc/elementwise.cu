@@ -403,8 +403,8 @@ template <class T> struct NeqFlagF {
 };
 
 // Both gradients in one launch; *out1 stays NULL when the three views are not equally shaped dense fp32
-// runs (the caller then composes the single-gradient kernels).
-template <class F> static void binary_backward_both(F f, const nt_view *g, const nt_view *x1, const nt_view *x2,
+// runs (the caller then composes the single-gradient kernels).  `transposed`: nor operands that the tile pipeline takes.
+template <class F> static void binary_backward_both(F f, const nt_view *g, const nt_view *x1, const nt_view *x2, bool transposed,
                                                     nt_storage **out1, nt_storage **out2, const char *fname) {
   *out1 = *out2 = nullptr;
   const nt_view *chk[3] = {g, x1, x2};
@@ -412,19 +412,34 @@ template <class F> static void binary_backward_both(F f, const nt_view *g, const
   if constexpr (!is_bound<F>::value) {
     if (g->storage->scaled()) {
       const nt_view u = unscaled_view(*g);
-      return binary_backward_both(ScaledFirst<F>{f, g->storage->value}, &u, x1, x2, out1, out2, fname);
+      return binary_backward_both(ScaledFirst<F>{f, g->storage->value}, &u, x1, x2, transposed, out1, out2, fname);
     }
   }
   const int64_t n = view_numel(*g);
   const float *p[3];
+  bool dense = true;
   for (int i = 0; i < 3; ++i) {
-    int64_t acc = 1; // dense row-major?
-    for (int d = chk[i]->ndim - 1; d >= 0; --d) {
-      if (chk[i]->shape[d] != 1 && chk[i]->strides[d] != acc) return;
-      acc *= chk[i]->shape[d];
-    }
     p[i] = static_cast<const float *>(chk[i]->storage->ptr()) + chk[i]->offset;
-    if (!aligned16(p[i])) return;
+    dense = dense && row_major(chk[i]) && aligned16(p[i]);
+  }
+  if (!dense) {
+    if (!transposed || n < (int64_t(1) << 20)) return; // the pipeline's own lower limit: no results set up for nothing
+    StorageRef o1(storage_new(n, NT_FLOAT32, NT_CUDA)), o2(storage_new(n, NT_FLOAT32, NT_CUDA));
+    const nt_view v1 = fresh_view(o1.s, *g), v2 = fresh_view(o2.s, *g);
+    const nt_view *views[5] = {&v1, &v2, g, x1, x2};
+    const IterSpace<5> it = collapse<5>(views);
+    if (it.ndim < 2) return;
+    bool col[3], any = false;
+    for (int i = 0; i < 3; ++i) {
+      col[i] = it.strides[2 + i][it.ndim - 2] == 1 && it.strides[2 + i][it.ndim - 1] != 1;
+      any = any || col[i];
+    }
+    float *const outs[2] = {static_cast<float *>(o1->ptr()), static_cast<float *>(o2->ptr())};
+    if (any && ew_launch_tile_pipeline<F, 3, 2>(f, it, outs, p, col)) {
+      *out1 = o1.release();
+      *out2 = o2.release();
+    }
+    return;
   }
   if (n < 4) return;
   StorageRef o1(storage_new(n, NT_FLOAT32, NT_CUDA)), o2(storage_new(n, NT_FLOAT32, NT_CUDA));
@@ -798,12 +813,22 @@ int nt_div_backward_x2(const nt_view *g, const nt_view *x1, const nt_view *x2, n
 
 int nt_mul_backward(const nt_view *g, const nt_view *x1, const nt_view *x2, nt_storage **dx1, nt_storage **dx2) {
   NT_API_BEGIN
-  binary_backward_both(MulBwdBothF{}, g, x1, x2, dx1, dx2, "mul_backward");
+  binary_backward_both(MulBwdBothF{}, g, x1, x2, false, dx1, dx2, "mul_backward");
+  NT_API_END
+}
+int nt_mul_gradients(const nt_view *g, const nt_view *x1, const nt_view *x2, nt_storage **dx1, nt_storage **dx2) {
+  NT_API_BEGIN
+  binary_backward_both(MulBwdBothF{}, g, x1, x2, true, dx1, dx2, "mul_gradients");
   NT_API_END
 }
 int nt_div_backward(const nt_view *g, const nt_view *x1, const nt_view *x2, nt_storage **dx1, nt_storage **dx2) {
   NT_API_BEGIN
-  binary_backward_both(DivBwdBothF{}, g, x1, x2, dx1, dx2, "div_backward");
+  binary_backward_both(DivBwdBothF{}, g, x1, x2, false, dx1, dx2, "div_backward");
+  NT_API_END
+}
+int nt_div_gradients(const nt_view *g, const nt_view *x1, const nt_view *x2, nt_storage **dx1, nt_storage **dx2) {
+  NT_API_BEGIN
+  binary_backward_both(DivBwdBothF{}, g, x1, x2, true, dx1, dx2, "div_gradients");
   NT_API_END
 }
 

@@ -551,8 +551,9 @@ inline bool aligned16(const void *p) { return (reinterpret_cast<uintptr_t>(p) & 
 // along I (column-major), all other strides and the base 16-byte aligned, no broadcast operand, at most one
 // leading dim.  Returns false when the case does not qualify (the register-staged tile kernel takes it).
 extern std::atomic<int> g_tile_pipeline; // nt_set_transposed_tile_pipeline
-template <class F, int NIN>
-bool ew_launch_tile_pipeline(F f, const IterSpace<NIN + 1> &it, float *out, const float *const *in, const int *col_major) {
+// it: the outputs' views first, then the inputs'.  col_major[o]: input o has its unit stride along I.
+template <class F, int NIN, int NOUT>
+bool ew_launch_tile_pipeline(F f, const IterSpace<NIN + NOUT> &it, float *const *out, const float *const *in, const bool *col_major) {
   if (!g_tile_pipeline.load(std::memory_order_relaxed)) return false;
   if (it.ndim != 2 && it.ndim != 3) return false;
   const int dI = it.ndim - 2, dJ = it.ndim - 1;
@@ -560,10 +561,11 @@ bool ew_launch_tile_pipeline(F f, const IterSpace<NIN + 1> &it, float *out, cons
   if (nI < 64 || nJ < 64 || it.numel < (int64_t(1) << 20) || nI > 0x7fffffffLL || nJ > 0x7fffffffLL || lead > 0x7fffffffLL)
     return false;
   constexpr int64_t MAX_STRIDE = int64_t(1) << 37; // elements: 2^39 bytes, below the 2^40 of a tensor map
-  for (int o = 0; o <= NIN; ++o) {
-    const void *base = o == 0 ? static_cast<const void *>(out) : static_cast<const void *>(in[o - 1]);
-    if (!aligned16(base)) return false;
-    const bool col = o > 0 && col_major[o] != 0;
+  auto base_of = [&](int o) { return o < NOUT ? static_cast<const void *>(out[o]) : static_cast<const void *>(in[o - NOUT]); };
+  auto is_col = [&](int o) { return o >= NOUT && col_major[o - NOUT]; };
+  for (int o = 0; o < NIN + NOUT; ++o) {
+    if (!aligned16(base_of(o))) return false;
+    const bool col = is_col(o);
     const int64_t unit = it.strides[o][col ? dI : dJ], other = it.strides[o][col ? dJ : dI];
     if (unit != 1 || other <= 0 || (other & 3) != 0 || other >= MAX_STRIDE) return false;
     if (it.ndim == 3) {
@@ -572,12 +574,11 @@ bool ew_launch_tile_pipeline(F f, const IterSpace<NIN + 1> &it, float *out, cons
     }
   }
   auto map_of = [&](int o, bool prefetch_box = false) {
-    const void *base = o == 0 ? static_cast<const void *>(out) : static_cast<const void *>(in[o - 1]);
-    const bool col = o > 0 && col_major[o] != 0;
+    const bool col = is_col(o);
     const int64_t other = it.strides[o][col ? dJ : dI];
     const int64_t inner = col ? nI : nJ, rows = col ? nJ : nI;
     const int64_t ls = it.ndim == 3 ? it.strides[o][0] : other * rows;
-    return tile_tma::make_map(base, inner, rows, lead, other, ls, o == 0 ? 8u : 64u, prefetch_box);
+    return tile_tma::make_map(base_of(o), inner, rows, lead, other, ls, o < NOUT ? 8u : 64u, prefetch_box);
   };
   tile_tma::Args a{};
   a.tiles_i = int32_t(ceil_div(nI, tile_tma::T));
@@ -592,7 +593,7 @@ bool ew_launch_tile_pipeline(F f, const IterSpace<NIN + 1> &it, float *out, cons
   a.groups_j = (a.tiles_j + G - 1) / G;
   a.slots_per_lead = int64_t(G) * G * ((a.tiles_i + G - 1) / G) * a.groups_j;
   a.total = a.slots_per_lead * lead;
-  for (int o = 0; o < NIN; ++o) a.col[o] = col_major[o + 1] != 0;
+  for (int o = 0; o < NIN; ++o) a.col[o] = col_major[o];
   a.wait_limit = wait_limit_clocks();
   a.error_flag = pipeline_error_flag();
   // Measured on [4096, 4096]: with two operands the L2 prefetch two rounds ahead gains 3 % (0.83 -> 0.86 of
@@ -600,21 +601,26 @@ bool ew_launch_tile_pipeline(F f, const IterSpace<NIN + 1> &it, float *out, cons
   // that has less time per tile), so it is off there.  NT_TILE_PREFETCH overrides both.
   static const int prefetch_rounds = [] {
     const char *e = getenv("NT_TILE_PREFETCH");
-    const int v = (e && *e) ? atoi(e) : (NIN == 2 ? 2 : 0);
+    const int v = (e && *e) ? atoi(e) : (NIN >= 2 ? 2 : 0);
     return v < 0 ? 0 : (v > 8 ? 8 : v);
   }();
   a.prefetch_rounds = prefetch_rounds;
-  const CUtensorMap m_out = map_of(0), m0 = map_of(1), m1 = map_of(NIN == 2 ? 2 : 1);
-  const CUtensorMap pf0 = map_of(1, true), pf1 = map_of(NIN == 2 ? 2 : 1, true);
-  const size_t smem = tile_tma::smem_bytes(NIN);
+  tile_tma::Maps maps;
+  for (int o = 0; o < 2; ++o) maps.out[o] = map_of(o < NOUT ? o : 0);
+  for (int o = 0; o < 3; ++o) {
+    const int k = NOUT + (o < NIN ? o : 0);
+    maps.in[o] = map_of(k);
+    maps.pf[o] = map_of(k, true);
+  }
+  const size_t smem = tile_tma::smem_bytes(NIN, NOUT);
   static bool configured = false; // one per instantiation
   if (!configured) {
-    NT_CUDA_CHECK(cudaFuncSetAttribute(tile_tma::ew_tile_tma<F, NIN>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
+    NT_CUDA_CHECK(cudaFuncSetAttribute(tile_tma::ew_tile_tma<F, NIN, NOUT>, cudaFuncAttributeMaxDynamicSharedMemorySize, int(smem)));
     configured = true;
   }
   const int64_t tiles = int64_t(a.tiles_i) * a.tiles_j * lead;
   const unsigned grid = unsigned(std::min<int64_t>(tiles, sm_count()));
-  launch_ordered(tile_tma::ew_tile_tma<F, NIN>, grid, tile_tma::THREADS, smem, f, m_out, m0, m1, pf0, pf1, a);
+  launch_ordered(tile_tma::ew_tile_tma<F, NIN, NOUT>, grid, tile_tma::THREADS, smem, f, maps, a);
   check_launch("ew_tile_tma");
   return true;
 }
@@ -803,7 +809,10 @@ template <class F, int NIN> void ew_launch(F f, const nt_view *const (&views)[NI
             p.vec_mode[o] = vec_ok(o, dJ) ? 1 : 0;
         }
         if constexpr (NIN <= 2 && std::is_same<TI, float>::value && std::is_same<TO, float>::value) {
-          if (ew_launch_tile_pipeline<F, NIN>(f, it, out, in, p.col_major)) return;
+          float *const outs[1] = {out};
+          bool col[NIN];
+          for (int o = 0; o < NIN; ++o) col[o] = p.col_major[o + 1] != 0;
+          if (ew_launch_tile_pipeline<F, NIN, 1>(f, it, outs, in, col)) return;
         }
         dim3 grid(unsigned(ceil_div(it.shape[dJ], TILE)), unsigned(ceil_div(it.shape[dI], TILE)), unsigned(lead));
         const size_t smem = size_t(n_col) * TILE * TILE_PITCH * sizeof(TI); // at most 2 slots = 33 KB: below the 48 KB default limit

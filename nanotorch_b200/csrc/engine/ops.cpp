@@ -682,10 +682,10 @@ static bool backward_op(FunctionObj *fn, TensorObj *g, PyObject **out, int *n_ou
     const nt_view vg = view_of(g);
     const bool both = need(fn, 0) && need(fn, 1);
     if (both && !fast_pair(fn)) return false;
-    if (both && same_shape(g, x1) && same_shape(g, x2)) { // one pass when all three are dense
+    if (both && same_shape(g, x1) && same_shape(g, x2)) { // one pass when all three are dense, or large with a transpose
       const nt_view v1 = view_of(x1), v2 = view_of(x2);
       nt_storage *s1 = nullptr, *s2 = nullptr;
-      checked((mul ? nt_mul_backward : nt_div_backward)(&vg, &v1, &v2, &s1, &s2), s1);
+      checked((mul ? nt_mul_gradients : nt_div_gradients)(&vg, &v1, &v2, &s1, &s2), s1);
       if (s1) {
         PyObject *first = reinterpret_cast<PyObject *>(new_tensor(s1, g->nd, g->sh));
         PyObject *second = reinterpret_cast<PyObject *>(new_tensor(s2, g->nd, g->sh));
