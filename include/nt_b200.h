@@ -353,10 +353,17 @@ int nt_div_backward(const nt_view *g, const nt_view *x1, const nt_view *x2, nt_s
 /* The same with large transposed operands as well (2^20 elements and more, 16-byte aligned rows): the backward sweep's. */
 int nt_mul_gradients(const nt_view *g, const nt_view *x1, const nt_view *x2, nt_storage **dx1, nt_storage **dx2);
 int nt_div_gradients(const nt_view *g, const nt_view *x1, const nt_view *x2, nt_storage **dx1, nt_storage **dx2);
+/* The same where one operand holds a value per row ([..., 1] beside [..., C], all three dense): its gradient is [..., 1], the
+ * sum over the row.  Results stay NULL otherwise. */
+int nt_mul_gradients_row_value(const nt_view *g, const nt_view *x1, const nt_view *x2, nt_storage **dx1, nt_storage **dx2);
+int nt_div_gradients_row_value(const nt_view *g, const nt_view *x1, const nt_view *x2, nt_storage **dx1, nt_storage **dx2);
 /* Max/Min backward: g_expanded * mask where mask = (x == m_expanded) and zero on every tied slice
  * (integer-division quirk of the reference, autograd/ops_reduction.py:201-212, 275-286). */
 int nt_extremum_backward(const nt_view *g_expanded, const nt_view *x, const nt_view *m_expanded,
                          const int64_t *axes, int32_t n_axes, nt_storage **out);
+/* acc + that gradient (acc dense, of x's shape) for slices that are short dense rows; *out stays NULL for others. */
+int nt_extremum_backward_add(const nt_view *acc, const nt_view *g_expanded, const nt_view *x, const nt_view *m_expanded,
+                             const int64_t *axes, int32_t n_axes, nt_storage **out);
 /* SGD update p <- p - (g*lr), the two rounded steps of `p -= p.grad * lr` (nn/optimizers.py:45-51); bumps the version.
  * `grad_scale` multiplies g first when != 1 (data-parallel mean over ranks). */
 int nt_sgd_update(const nt_view *param, const nt_view *grad, float lr, float grad_scale);

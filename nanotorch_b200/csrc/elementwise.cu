@@ -450,6 +450,118 @@ template <class F> static void binary_backward_both(F f, const nt_view *g, const
   *out2 = o2.release();
 }
 
+// Both gradients of a product or a quotient of a dense operand and a value per row: the dense one is written, the other one's
+// is the row's sum of what would have been written.  Bound by memory: 12 bytes per element in one launch, where the two
+// elementwise kernels and the row sum moved 28 (4096 x 1000, out of the L2: 13 + 10 + 6 us; with the two steps for the row maximum a whole softmax with its
+// gradient went from 108 to 91 us).  W warps to a row: one, in the
+// order of the row sums, or all eight of the CTA for rows too few to fill the GPU that way.  V = 4: vectors, rows of whole
+// 16 bytes.  ROW1: the first operand is the value per row.
+template <class F, int V, int W, bool ROW1>
+__global__ void __launch_bounds__(256) ew_row_value_gradients(F f, float *__restrict__ out, float *__restrict__ row_out, const float *__restrict__ g,
+                                                              const float *__restrict__ x, const float *__restrict__ value, int64_t rows, int cols) {
+  pdl_trigger();
+  pdl_wait();
+  using vec = typename std::conditional<V == 4, float4, float>::type;
+  constexpr int DEPTH = 4, STEP = 32 * W;
+  __shared__ float part[8];
+  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int64_t row = W == 1 ? int64_t(blockIdx.x) * 8 + warp : int64_t(blockIdx.x);
+  if (row >= rows) return; // whole warps, and whole CTAs where they share a row
+  const int nvec = cols / V, first = W == 1 ? lane : int(threadIdx.x);
+  const float val = __ldg(value + row);
+  const vec *pg = reinterpret_cast<const vec *>(g + row * cols), *px = reinterpret_cast<const vec *>(x + row * cols);
+  vec *po = reinterpret_cast<vec *>(out + row * cols);
+  float acc = 0.0f;
+  auto one = [&](float gv, float xv, float *dense) {
+    float d1, d2;
+    f(gv, ROW1 ? val : xv, ROW1 ? xv : val, &d1, &d2);
+    *dense = ROW1 ? d2 : d1;
+    return ROW1 ? d1 : d2;
+  };
+  for (int i = first; i < nvec; i += STEP * DEPTH) {
+    vec gv[DEPTH], xv[DEPTH];
+#pragma unroll
+    for (int u = 0; u < DEPTH; ++u)
+      if (i + u * STEP < nvec) {
+        gv[u] = __ldcs(pg + i + u * STEP);
+        xv[u] = __ldcs(px + i + u * STEP);
+      }
+#pragma unroll
+    for (int u = 0; u < DEPTH; ++u)
+      if (i + u * STEP < nvec) {
+        vec y;
+        if constexpr (V == 4) {
+          const float a = one(gv[u].x, xv[u].x, &y.x), b = one(gv[u].y, xv[u].y, &y.y);
+          const float c = one(gv[u].z, xv[u].z, &y.z), d = one(gv[u].w, xv[u].w, &y.w);
+          acc += (a + b) + (c + d);
+        } else {
+          acc += one(gv[u], xv[u], &y);
+        }
+        if constexpr (V == 4) st_result(po + i + u * STEP, y, rows * nvec);
+        else po[i + u * STEP] = y;
+      }
+  }
+#pragma unroll
+  for (int s = 16; s > 0; s >>= 1) acc += __shfl_xor_sync(0xffffffffu, acc, s);
+  if constexpr (W == 1) {
+    if (lane == 0) row_out[row] = acc;
+  } else {
+    if (lane == 0) part[warp] = acc;
+    __syncthreads();
+    if (threadIdx.x == 0) {
+#pragma unroll
+      for (int w = 1; w < 8; ++w) acc += part[w];
+      row_out[row] = acc;
+    }
+  }
+}
+template <class F, bool ROW1>
+static void launch_row_value_gradients(F f, float *out, float *row_out, const float *g, const float *x, const float *value, int64_t rows, int cols) {
+  const bool v4 = (cols & 3) == 0 && aligned16(g) && aligned16(x) && aligned16(out);
+  // A warp per row until the rows are fewer than half the warps that the GPU holds and long enough to share.
+  const bool wide = rows < int64_t(sm_count()) * 32 && cols >= 1024;
+  const unsigned grid = unsigned(wide ? rows : ceil_div(rows, 8));
+  if (v4 && wide) launch(ew_row_value_gradients<F, 4, 8, ROW1>, grid, 256, 0, f, out, row_out, g, x, value, rows, cols);
+  else if (v4) launch(ew_row_value_gradients<F, 4, 1, ROW1>, grid, 256, 0, f, out, row_out, g, x, value, rows, cols);
+  else if (wide) launch(ew_row_value_gradients<F, 1, 8, ROW1>, grid, 256, 0, f, out, row_out, g, x, value, rows, cols);
+  else launch(ew_row_value_gradients<F, 1, 1, ROW1>, grid, 256, 0, f, out, row_out, g, x, value, rows, cols);
+  check_launch("ew_row_value_gradients");
+}
+// Results stay NULL where the views are no such pair, or where a few long rows would leave most SMs idle.
+template <class F> static void row_value_gradients(F f, const nt_view *g, const nt_view *x1, const nt_view *x2, nt_storage **out1,
+                                                   nt_storage **out2, const char *fname) {
+  *out1 = *out2 = nullptr;
+  const nt_view *chk[3] = {g, x1, x2};
+  for (const nt_view *v : chk) {
+    check_view(v, fname);
+    require_cuda(v, fname);
+    if (v->storage->dtype != NT_FLOAT32) fail_invalid(std::string(fname) + ": Float32 only.");
+    if (v->ndim != g->ndim || !row_major(v)) return;
+  }
+  if constexpr (!is_bound<F>::value) {
+    if (g->storage->scaled()) {
+      const nt_view u = unscaled_view(*g);
+      return row_value_gradients(ScaledFirst<F>{f, g->storage->value}, &u, x1, x2, out1, out2, fname);
+    }
+  }
+  const int nd = g->ndim;
+  if (nd < 1 || g->shape[nd - 1] < 2 || g->shape[nd - 1] > (int64_t(1) << 30)) return;
+  auto is_dense = [&](const nt_view *v) { return v->shape[nd - 1] == g->shape[nd - 1]; };
+  for (int d = 0; d + 1 < nd; ++d)
+    if (x1->shape[d] != g->shape[d] || x2->shape[d] != g->shape[d]) return;
+  const bool first = is_dense(x2) && x1->shape[nd - 1] == 1;
+  if (!first && !(is_dense(x1) && x2->shape[nd - 1] == 1)) return;
+  const int64_t n = view_numel(*g), cols = g->shape[nd - 1], rows = n / cols;
+  if (n == 0 || rows > 0x7fffffffLL || (rows < sm_count() && n > (int64_t(1) << 18))) return;
+  auto ptr = [](const nt_view *v) { return static_cast<const float *>(v->storage->ptr()) + v->offset; };
+  StorageRef dense(storage_new(n, NT_FLOAT32, NT_CUDA)), sums(storage_new(rows, NT_FLOAT32, NT_CUDA));
+  float *pd = static_cast<float *>(dense->ptr()), *ps = static_cast<float *>(sums->ptr());
+  if (first) launch_row_value_gradients<F, true>(f, pd, ps, ptr(g), ptr(x2), ptr(x1), rows, int(cols));
+  else launch_row_value_gradients<F, false>(f, pd, ps, ptr(g), ptr(x1), ptr(x2), rows, int(cols));
+  *out1 = first ? sums.release() : dense.release();
+  *out2 = first ? dense.release() : sums.release();
+}
+
 // ---- SGD.  A weight that has been a matmul operand: its TF32 planes follow the update.  When the parameter is the whole
 // of a dense 2-D storage the update writes them itself (20 bytes per element in one launch instead of 12 + 12 in two);
 // otherwise the cached views are split again behind the update.
@@ -824,6 +936,16 @@ int nt_mul_gradients(const nt_view *g, const nt_view *x1, const nt_view *x2, nt_
 int nt_div_backward(const nt_view *g, const nt_view *x1, const nt_view *x2, nt_storage **dx1, nt_storage **dx2) {
   NT_API_BEGIN
   binary_backward_both(DivBwdBothF{}, g, x1, x2, false, dx1, dx2, "div_backward");
+  NT_API_END
+}
+int nt_mul_gradients_row_value(const nt_view *g, const nt_view *x1, const nt_view *x2, nt_storage **dx1, nt_storage **dx2) {
+  NT_API_BEGIN
+  row_value_gradients(MulBwdBothF{}, g, x1, x2, dx1, dx2, "mul_gradients_row_value");
+  NT_API_END
+}
+int nt_div_gradients_row_value(const nt_view *g, const nt_view *x1, const nt_view *x2, nt_storage **dx1, nt_storage **dx2) {
+  NT_API_BEGIN
+  row_value_gradients(DivBwdBothF{}, g, x1, x2, dx1, dx2, "div_gradients_row_value");
   NT_API_END
 }
 int nt_div_gradients(const nt_view *g, const nt_view *x1, const nt_view *x2, nt_storage **dx1, nt_storage **dx2) {

@@ -292,8 +292,9 @@ PyObject *run_backward(TensorObj *root) {
     Ref fn(own(node->grad_fn)), g(own(node->grad));
     PyObject *out[3] = {};
     int n_out = 0;
+    bool added = false;
     Ref grads; // of the Python backward
-    const bool native = PyObject_TypeCheck(fn.p, &FunctionBase_Type) && backward_fast(F_(fn.p), T_(g.p), out, &n_out);
+    const bool native = PyObject_TypeCheck(fn.p, &FunctionBase_Type) && backward_fast(F_(fn.p), T_(g.p), out, &n_out, &added);
     Ref held[3] = {Ref(out[0]), Ref(out[1]), Ref(out[2])};
     if (!native) {
       if (PyErr_Occurred() || !settle(g.p)) return nullptr;
@@ -313,7 +314,8 @@ PyObject *run_backward(TensorObj *root) {
       PyObject *gx = native ? held[at].p : PySequence_Fast_GET_ITEM(grads.p, at);
       ++at;
       if (!requires_grad(T_(x))) continue;
-      if (gx && gx != Py_None && !accumulate(T_(x), gx)) return nullptr;
+      if (added) Py_XSETREF(T_(x)->grad, own(gx)); // one input, one gradient: the sum of both
+      else if (gx && gx != Py_None && !accumulate(T_(x), gx)) return nullptr;
       if (T_(x)->grad_fn || pending.empty()) continue;
       auto p = pending.find(x);
       if (p == pending.end()) continue;

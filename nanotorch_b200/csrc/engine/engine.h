@@ -167,7 +167,8 @@ PyObject *dims_tuple(int n, const int64_t *v);
 // ---- ops (ops.cpp): a new tensor, or null with an exception set, or null without one: "not a fast case"
 PyObject *forward(Op op, PyTypeObject *cls, PyObject *const *args, Py_ssize_t n);
 // the gradients of a node whose native forward ran; false: take the Python backward (no exception) or an exception
-bool backward_fast(FunctionObj *fn, TensorObj *g, PyObject **out, int *n_out);
+// *added: out[0] holds the gradient that its input had already, too.
+bool backward_fast(FunctionObj *fn, TensorObj *g, PyObject **out, int *n_out, bool *added);
 TensorObj *add_tensors(PyObject *a, PyObject *b); // a + b of two fast tensors of one shape, no graph; null otherwise
 PyObject *apply(PyTypeObject *cls, PyObject *const *args, Py_ssize_t n, PyObject *kwnames);
 PyObject *to_operand(PyObject *x, TensorObj *anchor); // totensor(x, anchor=anchor)

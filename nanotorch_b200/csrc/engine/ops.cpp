@@ -651,12 +651,31 @@ static PyObject *negated(TensorObj *g) {
   return fresh(checked(nt_neg(&v, &s), s), g->nd, g->sh);
 }
 
+// -(g summed down to like's shape): one axis of a dense gradient in one launch, the sum divided by -1
+static PyObject *negated_sum(TensorObj *g, const TensorObj *like) {
+  const nt_view v = view_of(g);
+  int64_t axis = -1;
+  int n = 0;
+  for (int d = 0; d < g->nd && g->nd == like->nd; ++d)
+    if (g->sh[d] != like->sh[d]) {
+      axis = d;
+      ++n;
+    }
+  if (n == 1 && !v.storage->constant && !v.storage->scaled()) {
+    nt_storage *s = nullptr;
+    checked(nt_mean_f32(&v, &axis, 1, -1.0f, &s), s);
+    if (s) return fresh(s, like->nd, like->sh);
+  }
+  Ref sum(unbroadcast(g, like));
+  return negated(T_(sum.p));
+}
+
 // A product's operand as it took part: a scalar tensor keeps its own dtype in the graph, so only fast ones qualify.
 static bool fast_pair(FunctionObj *fn) {
   return is_fast(reinterpret_cast<PyObject *>(saved(fn, 0))) && is_fast(reinterpret_cast<PyObject *>(saved(fn, 1)));
 }
 
-static bool backward_op(FunctionObj *fn, TensorObj *g, PyObject **out, int *n_out) {
+static bool backward_op(FunctionObj *fn, TensorObj *g, PyObject **out, int *n_out, bool *added) {
   switch (fn->op) {
   case OP_ADD:
   case OP_SUB: {
@@ -667,8 +686,7 @@ static bool backward_op(FunctionObj *fn, TensorObj *g, PyObject **out, int *n_ou
         out[1] = unbroadcast(g, input(fn, 1)).release();
       } else {
         // summed first: the sum of the negated values is the negated sum, bit for bit
-        Ref sum(unbroadcast(g, input(fn, 1)));
-        out[1] = negated(T_(sum.p));
+        out[1] = negated_sum(g, input(fn, 1));
       }
     }
     return true;
@@ -692,6 +710,17 @@ static bool backward_op(FunctionObj *fn, TensorObj *g, PyObject **out, int *n_ou
         out[0] = first;
         out[1] = second;
         if (!first || !second) throw PyErr{};
+        return true;
+      }
+    }
+    if (both && !vg.storage->constant && dense(g) && !(same_shape(g, x1) && same_shape(g, x2))) { // a value per row beside a dense operand
+      const nt_view v1 = view_of(x1), v2 = view_of(x2);
+      nt_storage *s1 = nullptr, *s2 = nullptr;
+      checked((mul ? nt_mul_gradients_row_value : nt_div_gradients_row_value)(&vg, &v1, &v2, &s1, &s2), s1);
+      if (s1) {
+        out[0] = reinterpret_cast<PyObject *>(new_tensor(s1, x1->nd, x1->sh));
+        out[1] = reinterpret_cast<PyObject *>(new_tensor(s2, x2->nd, x2->sh));
+        if (!out[0] || !out[1]) throw PyErr{};
         return true;
       }
     }
@@ -807,6 +836,16 @@ static bool backward_op(FunctionObj *fn, TensorObj *g, PyObject **out, int *n_ou
       Ref ge(expand_back(g, x, fn)), me(expand_back(saved(fn, 1), x, fn));
       const nt_view vg = view_of(T_(ge.p)), vx = view_of(saved(fn, 0)), vm = view_of(T_(me.p));
       nt_storage *s = nullptr;
+      TensorObj *in = input(fn, 0), *acc = in->grad ? T_(in->grad) : nullptr;
+      if (acc && in->nd == x->nd && is_fast(in->grad) && same_shape(acc, x) && !storage_of(acc)->constant) {
+        const nt_view va = view_of(acc);
+        checked(nt_extremum_backward_add(&va, &vg, &vx, &vm, fn->axes, fn->n_axes, &s), s);
+        if (s) {
+          out[0] = fresh(s, x->nd, x->sh);
+          *added = true;
+          return true;
+        }
+      }
       out[0] = fresh(checked(nt_extremum_backward(&vg, &vx, &vm, fn->axes, fn->n_axes, &s), s), x->nd, x->sh);
     }
     return true;
@@ -852,12 +891,12 @@ static bool backward_op(FunctionObj *fn, TensorObj *g, PyObject **out, int *n_ou
   }
 }
 
-bool backward_fast(FunctionObj *fn, TensorObj *g, PyObject **out, int *n_out) {
+bool backward_fast(FunctionObj *fn, TensorObj *g, PyObject **out, int *n_out, bool *added) {
   if (fn->op == OP_NONE || !is_fast(reinterpret_cast<PyObject *>(g))) return false;
   out[0] = out[1] = out[2] = nullptr;
   bool ok = false;
   try {
-    ok = backward_op(fn, g, out, n_out);
+    ok = backward_op(fn, g, out, n_out, added);
   } catch (const PyErr &) {
   }
   if (!ok)
