@@ -167,8 +167,12 @@ struct nt_storage {
   // squared error, inside a backward sweep (see nt_scaled).  Kernels that can take the factor read `src` itself.
   nt_storage *src = nullptr;
   int64_t src_offset = 0;
-  // The sum and the mean of all elements, when the kernel that wrote them left those too; handed out once.
-  nt_storage *side_sum = nullptr, *side_mean = nullptr;
+  // The sum and the mean of all elements, when the kernel that wrote them left those too.  Each is handed out once; what
+  // asks again gets a copy of side_kept (sum, mean), so that the same elements have the same sum every time.  They are
+  // good for the graph capture that recorded them (side_capture; 0: for eager work) and for nothing else: a replay rewrites
+  // the ones of its capture, and records no reduction over ones from outside.
+  nt_storage *side_sum = nullptr, *side_mean = nullptr, *side_kept = nullptr;
+  int side_capture = 0;
 
   bool scaled() const { return src && !block; }
   void *ptr() const {

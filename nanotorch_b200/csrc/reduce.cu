@@ -500,7 +500,7 @@ void reduce_prepare() { tickets(1); }
 constexpr int SQ_CHUNK = 4096; // values of a CTA and round
 __global__ void __launch_bounds__(256) square_sums(const float *__restrict__ in, float *__restrict__ out, int64_t n,
                                                    float *__restrict__ partials, unsigned *__restrict__ ticket,
-                                                   float *__restrict__ sum, float *__restrict__ mean) {
+                                                   float *__restrict__ sum, float *__restrict__ mean, float *__restrict__ kept) {
   pdl_trigger();
   pdl_wait();
   __shared__ float warp_part[8];
@@ -550,12 +550,12 @@ __global__ void __launch_bounds__(256) square_sums(const float *__restrict__ in,
     if (threadIdx.x == 0) *ticket = 0;
   }
   if (threadIdx.x == 0) {
-    *sum = v;
-    *mean = v / float(n);
+    *sum = kept[0] = v;
+    *mean = kept[1] = v / float(n);
   }
 }
 void square_with_sums(const float *in, nt_storage *out, int64_t n) {
-  StorageRef sum(storage_new(1, NT_FLOAT32, NT_CUDA)), mean(storage_new(1, NT_FLOAT32, NT_CUDA));
+  StorageRef sum(storage_new(1, NT_FLOAT32, NT_CUDA)), mean(storage_new(1, NT_FLOAT32, NT_CUDA)), kept(storage_new(2, NT_FLOAT32, NT_CUDA));
   const int64_t ctas = std::min(ceil_div(n, SQ_CHUNK), int64_t(sm_count()) * 8);
   size_t rounded = 0;
   float *partials = nullptr;
@@ -565,24 +565,31 @@ void square_with_sums(const float *in, nt_storage *out, int64_t n) {
     tk = tickets(1);
   }
   launch(square_sums, unsigned(ctas), 256, 0, in, static_cast<float *>(out->ptr()), n, partials, tk, static_cast<float *>(sum->ptr()),
-         static_cast<float *>(mean->ptr()));
+         static_cast<float *>(mean->ptr()), static_cast<float *>(kept->ptr()));
   check_launch("square_sums");
   if (partials) device_free(partials, rounded); // stream-ordered reuse
   out->side_sum = sum.release();
   out->side_mean = mean.release();
+  out->side_kept = kept.release();
+  out->side_capture = capture_id();
 }
 // The sum or mean of all elements that came with them, for a view of all of them with every dim dropped; null otherwise.
 static nt_storage *take_side(const nt_view *x, int64_t n_keep, int64_t n_drop, nt_storage *nt_storage::*side) {
   nt_storage *s = x->storage;
-  if (!(s->*side) || s->mutation != 0 || n_keep != 1 || n_drop != s->n || x->offset != 0) return nullptr;
+  if (!s->side_kept || s->mutation != 0 || n_keep != 1 || n_drop != s->n || x->offset != 0 || s->side_capture != capture_id()) return nullptr;
   int64_t acc = 1; // each element once, in whatever order
   for (int d = x->ndim - 1; d >= 0; --d) {
     if (x->shape[d] != 1 && x->strides[d] != acc) return nullptr;
     acc *= x->shape[d];
   }
-  nt_storage *r = s->*side;
-  s->*side = nullptr;
-  return r;
+  if (nt_storage *r = s->*side) {
+    s->*side = nullptr;
+    return r;
+  }
+  StorageRef again(storage_new(1, NT_FLOAT32, NT_CUDA));
+  const float *kept = static_cast<const float *>(s->side_kept->ptr()) + (side == &nt_storage::side_mean ? 1 : 0);
+  NT_CUDA_CHECK(cudaMemcpyAsync(again->ptr(), kept, sizeof(float), cudaMemcpyDeviceToDevice, stream()));
+  return again.release();
 }
 
 struct Plan {

@@ -420,7 +420,8 @@ nt_storage *storage_new_scaled(nt_storage *src, int64_t offset, int64_t n, float
 void drop_side_sums(nt_storage *s) {
   storage_release(s->side_sum);
   storage_release(s->side_mean);
-  s->side_sum = s->side_mean = nullptr;
+  storage_release(s->side_kept);
+  s->side_sum = s->side_mean = s->side_kept = nullptr;
 }
 void storage_release(nt_storage *s) {
   if (!s) return;

@@ -16,7 +16,7 @@ def test_mean_and_sum_of_squares(nt, shape):
     square = t ** 2
     assert np.array_equal(bits(square.numpy()), bits(x * x))
     want = np.square(x.astype(np.float64))
-    for _ in range(2):  # the second time the sums come from the square in memory
+    for _ in range(2):  # the second time they are copies of what the square left
         assert abs(float(nt.mean(square).numpy()) - want.mean()) <= 2e-6 * want.mean()
         assert abs(float(nt.sum(square).numpy()) - want.sum()) <= 2e-6 * want.sum()
     square = t ** 2
@@ -54,3 +54,49 @@ def test_a_leaf_under_the_square(nt):
     t = nt.Tensor.from_numpy(x, "cuda", requires_grad=True)
     (t ** 2).mean().backward()
     assert np.array_equal(bits(t.grad.numpy()), bits(np.float32(np.float32(1) / np.float32(x.size) * 2) * x))
+
+
+def test_the_same_elements_have_the_same_sums(nt):
+    square = nt.Tensor.from_numpy(np.random.default_rng(5).standard_normal((1200, 1027)).astype(np.float32), "cuda") ** 2
+    for f in (nt.mean, nt.sum):
+        first = f(square)
+        with nt.no_grad():
+            kept = first.numpy().copy()
+            first += 1.0  # the caller's own
+        assert {float(f(square).numpy()) for _ in range(2)} == {float(kept)}
+
+
+def put(t, values):
+    values = np.ascontiguousarray(values, np.float32)
+    t.storage.upload(values.ctypes.data, values.nbytes)
+
+
+@pytest.mark.parametrize("f", ["mean", "sum"])
+@pytest.mark.parametrize("square_inside", [True, False], ids=["square captured", "square before"])
+@pytest.mark.parametrize("sum_inside", [True, False], ids=["sum captured", "sum after"])
+def test_sums_of_a_square_and_a_graph_capture(nt, square_inside, sum_inside, f):
+    """Replays follow new values, and an eager sum taken after one replay keeps its value through the next."""
+    reduce = getattr(nt, f)
+    a, b = (np.random.default_rng(s).standard_normal((64, 33)).astype(np.float32) for s in (6, 7))
+    want = lambda v: np.float32(getattr(v.astype(np.float64), f)())  # noqa: E731
+    x = nt.Tensor.from_numpy(a, "cuda")
+    reduce(x ** 2), nt.sum(x)  # first-use set-up outside the capture
+    square = None if square_inside else x ** 2
+    total = None
+    graph = nt._C.Graph()
+    with graph.capture():
+        if square_inside:
+            square = x ** 2
+        if sum_inside:
+            total = reduce(square)
+        z = x + 1.0  # a launch in any case
+    graph.replay()
+    if not sum_inside:
+        total = reduce(square)
+    assert np.isclose(total.numpy(), want(a * a), rtol=2e-6)
+    put(x if square_inside else square, b if square_inside else b * b)
+    graph.replay()
+    assert np.isclose(total.numpy(), want(b * b if sum_inside else a * a), rtol=2e-6)
+    assert np.isclose(reduce(square).numpy(), want(b * b), rtol=2e-6)
+    graph.close()
+    del z
