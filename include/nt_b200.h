@@ -277,12 +277,10 @@ int nt_matmul_split_stats(uint64_t *split_launches, uint64_t *cache_hits);
  * NT_GEMM_PANEL): width in n-tiles of the panels the CTAs walk the output in, 0 = row by row. */
 int nt_set_matmul_schedule(int max_splits, int panel);
 /* Two independent products in one call, *out1 = a1 @ b1 and *out2 = a2 @ b2 -- what MatmulOp.backward computes
- * (autograd/ops_binary.py:253-267: g @ x2^T and x1^T @ g).  Same bits as two nt_matmul calls.  In mode 1, when the
- * second product's operand planes are already cached, its kernel can be launched as the programmatic dependent of
- * the first: its CTAs start on the SMs that the first product's last, partly filled wave leaves idle (256 tiles on
- * 148 SMs at a 2048-row batch) and wait for the first grid before they exit, so later work in the stream
- * still sees both complete.  The overlap is off by default (measured gain on the training step: 0.3-0.6 % at
- * 2048-4096 rows per GPU, none at 16384); nt_set_matmul_pair_overlap(1) or NT_GEMM_PAIR_OVERLAP=1 switches it on. */
+ * (autograd/ops_binary.py:253-267: g @ x2^T and x1^T @ g).  Same bits as two nt_matmul calls.  The second product
+ * starts when the first is complete: both may be split along k over the same counters and workspace, and letting the
+ * second one's CTAs in early was slower on the persistent kernel (4096^3 with both gradients 1594 -> 1705 us, 8192 x
+ * 1024 x 4096 934 -> 979).  nt_set_matmul_pair_overlap, which used to ask for that, is accepted and changes nothing. */
 int nt_matmul_pair(const nt_view *a1, const nt_view *b1, const nt_view *a2, const nt_view *b2, nt_storage **out1,
                    nt_storage **out2);
 int nt_set_matmul_pair_overlap(int on);

@@ -193,9 +193,6 @@ struct TcArgs {
   int32_t splits, kb_per_split;
   float *partials;
   unsigned int *tickets;
-  // promoted kernel: launched as the programmatic dependent of the product before it (nt_matmul_pair): it did not
-  // wait for that grid on entry, so every CTA waits for it before leaving -- this grid never completes first
-  int32_t wait_for_primary_at_end;
   int32_t tiles_m, tiles_n; // promoted kernel: output tiles of one batch
   int32_t work;             // tiles x splits x batches; a CTA takes items blockIdx.x, + gridDim.x, ...
 };
@@ -424,9 +421,7 @@ gemm_3xtf32_promoted_kernel(const __grid_constant__ CUtensorMap map_a, const __g
   volatile int *poison_slot = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  // A grid launched behind this one with the programmatic-serialization attribute may take the SMs this grid's
-  // last wave leaves idle; it has nothing to wait for here.
-  asm volatile("griddepcontrol.launch_dependents;" ::: "memory");
+  pdl_trigger(); // the kernel behind may be set up while this one runs (launch.cuh)
   // a work item: an output tile and, with split-K, this CTA's share of the contraction, k-blocks [kb0, kb0 + nkb)
   struct Item {
     int tile_m, tile_n, split, b, kb0, nkb, periods;
@@ -699,7 +694,6 @@ gemm_3xtf32_promoted_kernel(const __grid_constant__ CUtensorMap map_a, const __g
     while (clock64() - t0 < 2000000) {
     }
   }
-  if (g.wait_for_primary_at_end) asm volatile("griddepcontrol.wait;" ::: "memory");
   tcgen05_fence_before();
   __syncthreads();
   if (warp == 1) {
@@ -748,33 +742,6 @@ static int panel_default() {
   return 8;
 }
 static std::atomic<int> g_tc_panel{panel_default()};
-
-// nt_matmul_pair: the second of two independent products can be launched as the programmatic dependent of the
-// first when nothing was launched in between (its operand planes were cache hits) -- then its first CTAs fill the
-// SMs that the first product's last wave leaves idle.  g_promoted_seq is the launch count right after the last
-// promoted-kernel launch.  Off unless asked for (nt_set_matmul_pair_overlap, NT_GEMM_PAIR_OVERLAP=1): measured on
-// the training step it is worth 0.3 % at a 2048-row batch (256 + 512 tiles on 148 SMs), 0.6 % at 4096 rows and
-// nothing at 16384 -- under the power cap the SMs that stay busy in a thin last wave clock higher, which already
-// recovers most of what the idle ones lose.
-static thread_local bool t_pair_first = false, t_pair_second = false;
-static thread_local bool t_pair_end_pending = false; // the first product left its profile interval open
-static uint64_t g_promoted_seq = ~uint64_t(0);
-static int pair_overlap_default() {
-  const char *e = getenv("NT_GEMM_PAIR_OVERLAP");
-  return (e && *e) ? (atoi(e) != 0) : 0;
-}
-static std::atomic<int> g_pair_overlap{pair_overlap_default()};
-// role: 0 = not in a pair, 1 = first product, 2 = second.  Leaving a pair closes a profile interval the first
-// product left open for a second one that never joined it.
-void gemm_tc_pair_role(int role) {
-  t_pair_first = role == 1;
-  t_pair_second = role == 2;
-  if (role == 0 && t_pair_end_pending) {
-    t_pair_end_pending = false;
-    matmul_profile_end();
-  }
-}
-void gemm_tc_set_pair_overlap(bool on) { g_pair_overlap.store(on ? 1 : 0); }
 
 // Split-K tickets: one counter per output tile, zero between launches (the CTA that draws the last ticket of a
 // tile resets it).  GEMM launches are ordered on the compute stream, so one array serves them all.
@@ -1166,22 +1133,7 @@ static void launch_promoted(const CUtensorMap &ma, const CUtensorMap &mb, const 
                                        int(TC_SMEM_BYTES)));
     configured = true;
   }
-  if (!g.wait_for_primary_at_end) {
-    gemm_3xtf32_promoted_kernel<A_MN, B_MN><<<grid, 320, TC_SMEM_BYTES, stream()>>>(ma, mb, g);
-    return;
-  }
-  // programmatic dependent launch: this grid's CTAs may start while the previous kernel's last wave still runs
-  cudaLaunchConfig_t cfg{};
-  cfg.gridDim = grid;
-  cfg.blockDim = dim3(320, 1, 1);
-  cfg.dynamicSmemBytes = TC_SMEM_BYTES;
-  cfg.stream = stream();
-  cudaLaunchAttribute attr[1];
-  attr[0].id = cudaLaunchAttributeProgrammaticStreamSerialization;
-  attr[0].val.programmaticStreamSerializationAllowed = 1;
-  cfg.attrs = attr;
-  cfg.numAttrs = 1;
-  NT_CUDA_CHECK(cudaLaunchKernelEx(&cfg, gemm_3xtf32_promoted_kernel<A_MN, B_MN>, ma, mb, g));
+  gemm_3xtf32_promoted_kernel<A_MN, B_MN><<<grid, 320, TC_SMEM_BYTES, stream()>>>(ma, mb, g);
 }
 
 // How an operand matrix [P][Q] (strides s_p, s_q) is laid out: unit stride along Q, along P, or neither.
@@ -1284,28 +1236,14 @@ bool gemm_3xtf32_natural(nt_storage *sa, int64_t a_off, nt_storage *sb, int64_t 
     g.tiles_n = int32_t(tiles_n);
     g.work = int32_t(tiles_m * tiles_n * g.splits * batch);
     const dim3 grid{unsigned(std::min(g.work, sm_count())), 1, 1};
-    const bool overlap = g_pair_overlap.load(std::memory_order_relaxed) != 0;
-    g.wait_for_primary_at_end = (t_pair_second && overlap && launches_so_far() == g_promoted_seq) ? 1 : 0;
-    // the matmul profile times an overlapped pair as one interval of two launches: no event between them
-    if (t_pair_end_pending && !g.wait_for_primary_at_end) {
-      t_pair_end_pending = false;
-      matmul_profile_end();
-    }
-    if (g.wait_for_primary_at_end && t_pair_end_pending) matmul_profile_extend();
-    else matmul_profile_begin();
+    matmul_profile_begin();
     if (a_mn && b_mn) launch_promoted<true, true>(map_a, map_b, g, grid);
     else if (a_mn) launch_promoted<true, false>(map_a, map_b, g, grid);
     else if (b_mn) launch_promoted<false, true>(map_a, map_b, g, grid);
     else launch_promoted<false, false>(map_a, map_b, g, grid);
-    if (t_pair_first && overlap && matmul_profile_active()) {
-      t_pair_end_pending = true; // closed by the second product, or by gemm_tc_pair_role(0)
-    } else {
-      t_pair_end_pending = false;
-      matmul_profile_end();
-    }
+    matmul_profile_end();
     if (part_owned) device_free(g.partials, part_owned); // stream-ordered like the operand planes
     check_launch("gemm_3xtf32_promoted_kernel");
-    g_promoted_seq = launches_so_far();
   } catch (...) {
     if (a_owned) device_free(pa, a_owned);
     if (b_owned && pb) device_free(pb, b_owned);

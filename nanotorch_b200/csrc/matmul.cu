@@ -39,8 +39,6 @@ bool gemm_3xtf32_natural(nt_storage *sa, int64_t a_off, nt_storage *sb, int64_t 
                          int64_t b_sn, const float *bias, int64_t bias_stride, bool *bias_done);
 void gemm_tc_set_operand_cache(bool on);
 void gemm_tc_set_schedule(int max_splits, int panel);
-void gemm_tc_pair_role(int role);
-void gemm_tc_set_pair_overlap(bool on);
 void gemm_tc_split_stats(uint64_t *launches, uint64_t *hits);
 static std::atomic<int> g_natural_planes{1};
 static thread_local int t_reorder = 0; // nt_matmul_allow_reorder
@@ -384,12 +382,7 @@ int nt_matmul_pair(const nt_view *a1, const nt_view *b1, const nt_view *a2, cons
                    nt_storage **out2) {
   NT_API_BEGIN
   *out1 = *out2 = nullptr;
-  struct Leave {
-    ~Leave() { gemm_tc_pair_role(0); }
-  } leave;
-  gemm_tc_pair_role(1);
   nt_storage *first = matmul_impl(a1, b1, nullptr);
-  gemm_tc_pair_role(2);
   nt_storage *second = nullptr;
   try {
     second = matmul_impl(a2, b2, nullptr);
@@ -401,11 +394,7 @@ int nt_matmul_pair(const nt_view *a1, const nt_view *b1, const nt_view *a2, cons
   *out2 = second;
   NT_API_END
 }
-int nt_set_matmul_pair_overlap(int on) {
-  NT_API_BEGIN
-  gemm_tc_set_pair_overlap(on != 0);
-  NT_API_END
-}
+int nt_set_matmul_pair_overlap(int) { return NT_OK; } // see nt_b200.h
 
 int nt_linear(const nt_view *x, const nt_view *w, const nt_view *bias, nt_storage **out) {
   NT_API_BEGIN

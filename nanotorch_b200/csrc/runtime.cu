@@ -145,7 +145,6 @@ cudaStream_t update_stream() {
   ensure_streams_locked(r);
   return r.update;
 }
-uint64_t launches_so_far() { return rt().launches.load(); }
 int capture_id() {
   Runtime &r = rt();
   std::lock_guard<std::mutex> lk(r.mu);
@@ -217,13 +216,6 @@ void matmul_profile_begin() {
   NT_CUDA_CHECK(cudaEventRecord(a, r.compute));
   r.mm_events.emplace_back(a, b);
   r.mm_counts.push_back(1);
-}
-bool matmul_profile_active() { return rt().mm_profile; }
-// One more launch belongs to the interval that was opened last (the second product of an overlapped pair).
-void matmul_profile_extend() {
-  Runtime &r = rt();
-  if (!r.mm_profile || r.mm_counts.empty()) return;
-  r.mm_counts.back() += 1;
 }
 void matmul_profile_end() {
   Runtime &r = rt();

@@ -297,8 +297,8 @@ def test_fused_linear_is_the_composed_form_bit_for_bit(nt, mode):
 
 @pytest.mark.parametrize("graph_mode", [False, True])
 def test_overlapped_gradient_products_leave_the_step_unchanged(nt, graph_mode):
-    """Linear.backward launches its two products as an overlapping pair: six training steps, eagerly and as a
-    replayed graph, give the bits of the same steps with the overlap switched off."""
+    """Linear.backward hands its two products over as a pair: six training steps, eagerly and as a replayed graph, give
+    the same bits whatever the overlap setting (which is accepted and changes nothing)."""
     import nanotorch_b200.nn as nn
 
     X = nt.Tensor.from_numpy(np.random.default_rng(1).standard_normal((2048, 1024)).astype(np.float32), "cuda")

@@ -517,11 +517,11 @@ def test_split_k_products(nt, shape):
 
 
 @pytest.mark.parametrize("mode", [1, 0])
-@pytest.mark.parametrize("shape", [(2048, 1024, 1536), (300, 200, 260), (4096, 512, 4096)], ids=lambda s: "x".join(map(str, s)))
+@pytest.mark.parametrize("shape", [(2048, 1024, 1536), (300, 200, 260), (4096, 512, 4096), (4096, 256, 4096)], ids=lambda s: "x".join(map(str, s)))
 def test_matmul_pair_is_two_products(nt, shape, mode):
-    """Both gradients of a product in one call (the second tensor-core launch overlapping the first one's last
-    wave as its programmatic dependent): the bits of two separate products, also with the overlap switched off,
-    and a kernel queued behind the pair sees both results complete."""
+    """Both gradients of a product in one call: the bits of two separate products -- also where both are split along k
+    over the same counters and workspace, and whatever the overlap setting, which no longer does anything -- and a
+    kernel queued behind the pair sees both results complete."""
     _C = nt._C
     M, K, N = shape
     rng = np.random.default_rng(M + K)
