@@ -161,7 +161,8 @@ struct nt_storage {
   nt_storage *prev = nullptr, *next = nullptr; // constants without memory, see constants_materialize_all
 
   // value * (n elements of `src` from src_offset on), another storage's product with a known factor: the gradient of a
-  // squared error, inside a backward sweep (see nt_scaled).  Kernels that can take the factor read `src` itself.
+  // squared error, inside a backward sweep (see nt_scaled).  Kernels that can take the factor read `src` itself.  Once it is
+  // in memory of its own it no longer holds on to `src`.
   nt_storage *src = nullptr;
   int64_t src_offset = 0;
   // The sum and the mean of all elements, when the kernel that wrote them left those too.  Each is handed out once; what
@@ -171,7 +172,7 @@ struct nt_storage {
   nt_storage *side_sum = nullptr, *side_mean = nullptr, *side_kept = nullptr;
   int side_capture = 0;
 
-  bool scaled() const { return src && !block; }
+  bool scaled() const { return src != nullptr; }
   void *ptr() const {
     if (!block && (constant || src)) materialize();
     return block;

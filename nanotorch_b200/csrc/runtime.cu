@@ -419,13 +419,11 @@ void storage_release(nt_storage *s) {
   if (!s) return;
   if (s->refs.fetch_sub(1, std::memory_order_acq_rel) == 1) {
     drop_side_sums(s);
-    if (s->src) {
+    if (s->src) { // never written out
       storage_release(s->src);
-      if (!s->block) {
-        gemm_tc_forget(s);
-        delete s;
-        return;
-      }
+      gemm_tc_forget(s);
+      delete s;
+      return;
     }
     if (s->constant && !s->block) {
       constants_unlink(s);
@@ -688,6 +686,8 @@ void nt_storage::materialize() const {
     void *p = ntb::device_alloc(size_t(s->n) * sizeof(float), &s->rounded);
     ntb::scale_into(static_cast<float *>(p), static_cast<const float *>(s->src->ptr()) + s->src_offset, s->n, s->value);
     s->block = p;
+    ntb::storage_release(s->src); // a plain storage from here on; the source's memory is reused behind the kernel just launched
+    s->src = nullptr;
     return;
   }
   ntb::constants_unlink(s);

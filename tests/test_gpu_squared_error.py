@@ -100,3 +100,13 @@ def test_sums_of_a_square_and_a_graph_capture(nt, square_inside, sum_inside, f):
     assert np.isclose(reduce(square).numpy(), want(b * b), rtol=2e-6)
     graph.close()
     del z
+
+
+def test_a_written_gradient_does_not_keep_the_difference(nt):
+    n = 1 << 20
+    a, b = (nt.Tensor.from_numpy(np.full(n, v, np.float32), "cuda", requires_grad=True) for v in (1, 2))
+    target = nt.Tensor.from_numpy(np.zeros(n, np.float32), "cuda")
+    before = nt.cuda.memory_stats()["bytes_in_use"]
+    nt.mean(((a + b) - target) ** 2).backward()
+    assert nt.cuda.memory_stats()["bytes_in_use"] - before <= 4 * n  # one gradient, which both leaves have
+    assert (a.grad.numpy() == np.float32(6 / n)).all() and (b.grad.numpy() == np.float32(6 / n)).all()
