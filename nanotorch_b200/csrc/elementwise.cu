@@ -454,7 +454,7 @@ template <class F> static void binary_backward_both(F f, const nt_view *g, const
 // is the row's sum of what would have been written.  Bound by memory: 12 bytes per element in one launch, where the two
 // elementwise kernels and the row sum moved 28 (4096 x 1000, out of the L2: 13 + 10 + 6 us; with the two steps for the row maximum a whole softmax with its
 // gradient went from 108 to 91 us).  W warps to a row: one, in the
-// order of the row sums, or all eight of the CTA for rows too few to fill the GPU that way.  V = 4: vectors, rows of whole
+// order of the row sums, or all eight of the CTA (launch_row_value_gradients says when).  V = 4: vectors, rows of whole
 // 16 bytes.  ROW1: the first operand is the value per row.
 template <class F, int V, int W, bool ROW1>
 __global__ void __launch_bounds__(256) ew_row_value_gradients(F f, float *__restrict__ out, float *__restrict__ row_out, const float *__restrict__ g,
@@ -518,8 +518,13 @@ __global__ void __launch_bounds__(256) ew_row_value_gradients(F f, float *__rest
 template <class F, bool ROW1>
 static void launch_row_value_gradients(F f, float *out, float *row_out, const float *g, const float *x, const float *value, int64_t rows, int cols) {
   const bool v4 = (cols & 3) == 0 && aligned16(g) && aligned16(x) && aligned16(out);
-  // A warp per row until the rows are fewer than half the warps that the GPU holds and long enough to share.
-  const bool wide = rows < int64_t(sm_count()) * 32 && cols >= 1024;
+  // A CTA per row where a warp's chain of loads along the row takes longer than eight times as many CTAs do to come and go:
+  // long rows, or few of them.  Quotient, us with a warp / with a CTA per row, launches back to back: 450 x 512 2.7 / 2.0,
+  // 1500 x 512 4.1 / 4.2; 2000 x 1024 7.6 / 6.3, 3000 x 1024 8.3 / 9.0, 4096 x 1000 8.6 / 12.0; 3000 x 2048 15.4 / 13.0, 4096 x
+  // 2048 16.0 / 17.2; 4096 x 1027 (single values) 13.3 / 10.6, 6000 x 1027 13.3 / 15.5; from 4096 columns on at any number of
+  // rows: 150 x 4096 13.6 / 3.7, 9000 x 4096 73 / 70.
+  const int64_t nvec = v4 ? cols >> 2 : cols;
+  const bool wide = cols >= 4096 || (cols >= 256 && rows <= 8 * nvec && rows <= int64_t(sm_count()) * 32);
   const unsigned grid = unsigned(wide ? rows : ceil_div(rows, 8));
   if (v4 && wide) launch(ew_row_value_gradients<F, 4, 8, ROW1>, grid, 256, 0, f, out, row_out, g, x, value, rows, cols);
   else if (v4) launch(ew_row_value_gradients<F, 4, 1, ROW1>, grid, 256, 0, f, out, row_out, g, x, value, rows, cols);

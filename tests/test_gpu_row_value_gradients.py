@@ -7,7 +7,7 @@ import pytest
 pytestmark = pytest.mark.gpu
 
 SHAPES = [(1, 5), (7, 3), (8, 128), (9, 1000), (200, 1023), (149, 1028), (160, 4099), (4737, 1024), (3, 50, 1000), (200, 5000), (148, 16384),
-          (5, 70000)]
+          (5, 70000), (149, 255), (512, 256), (513, 256), (2048, 1024), (2049, 1024), (2056, 257), (2057, 257), (4736, 1027), (4737, 1027), (4737, 4096)]
 
 
 def close(got, want, scale):
