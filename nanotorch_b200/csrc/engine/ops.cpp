@@ -651,7 +651,8 @@ static PyObject *negated(TensorObj *g) {
   return fresh(checked(nt_neg(&v, &s), s), g->nd, g->sh);
 }
 
-// -(g summed down to like's shape): one axis of a dense gradient in one launch, the sum divided by -1
+// The sum of -g down to like's shape: one axis of a dense gradient in one launch.  Summed first, then subtracted from zero:
+// the bits of the sum of the negated values, which is +0 where they cancel.
 static PyObject *negated_sum(TensorObj *g, const TensorObj *like) {
   const nt_view v = view_of(g);
   int64_t axis = -1;
@@ -666,8 +667,15 @@ static PyObject *negated_sum(TensorObj *g, const TensorObj *like) {
     checked(nt_mean_f32(&v, &axis, 1, -1.0f, &s), s);
     if (s) return fresh(s, like->nd, like->sh);
   }
+  if (same_shape(g, like)) return negated(g);
   Ref sum(unbroadcast(g, like));
-  return negated(T_(sum.p));
+  TensorObj *t = T_(sum.p);
+  Held zero(constant(nt_scalar{2, 0, 0.0}));
+  nt_view z{};
+  z.storage = zero.s;
+  z.ndim = t->nd;
+  std::copy(t->sh, t->sh + t->nd, z.shape);
+  return elementwise(nt_subtract, z, view_of(t), t).release();
 }
 
 // A product's operand as it took part: a scalar tensor keeps its own dtype in the graph, so only fast ones qualify.
@@ -685,7 +693,6 @@ static bool backward_op(FunctionObj *fn, TensorObj *g, PyObject **out, int *n_ou
       if (fn->op == OP_ADD) {
         out[1] = unbroadcast(g, input(fn, 1)).release();
       } else {
-        // summed first: the sum of the negated values is the negated sum, bit for bit
         out[1] = negated_sum(g, input(fn, 1));
       }
     }

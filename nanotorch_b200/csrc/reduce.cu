@@ -44,6 +44,13 @@ struct RMin {
   static __device__ __forceinline__ float combine(float a, float b) { return fminf(a, b); }
 };
 
+// divisor != 0: the finished value is divided by it (one IEEE division of the rounded fp32 result: the bits of a sum kernel
+// followed by a divide kernel -- MeanOp's two steps in one launch).  -1 negates as the sum of the negated values would come
+// out: what cancels is +0, where a division would leave -0.
+__device__ __forceinline__ float finish(float v, float divisor) {
+  return divisor == 0.0f ? v : divisor == -1.0f ? 0.0f - v : v / divisor;
+}
+
 template <class Op> __device__ __forceinline__ float warp_reduce(float v) {
 #pragma unroll
   for (int s = 16; s > 0; s >>= 1) v = Op::combine(v, __shfl_xor_sync(0xffffffffu, v, s));
@@ -72,8 +79,6 @@ __global__ void __launch_bounds__(256) reduce_rows(const float *__restrict__ in,
                                                    float *__restrict__ partials, unsigned *__restrict__ tickets,
                                                    KeepIndex keep, int64_t L, int S, int64_t chunk, float divisor) {
   pdl_wait();
-  // divisor != 0: the finished value is divided by it (one IEEE division of the rounded fp32 result:
-  // the bits of a sum kernel followed by a divide kernel -- MeanOp's two steps in one launch)
   __shared__ float warp_part[8];
   __shared__ bool is_last;
   const int64_t row = blockIdx.x / S;
@@ -123,7 +128,7 @@ __global__ void __launch_bounds__(256) reduce_rows(const float *__restrict__ in,
     v = warp_reduce<Op>(v);
   }
   if (S == 1) {
-    if (threadIdx.x == 0) out[row] = (divisor != 0.0f) ? v / divisor : v;
+    if (threadIdx.x == 0) out[row] = finish(v, divisor);
     return;
   }
   // single-pass grid finish
@@ -146,7 +151,7 @@ __global__ void __launch_bounds__(256) reduce_rows(const float *__restrict__ in,
     acc = (lane < 8) ? warp_part[lane] : Op::neutral();
     acc = warp_reduce<Op>(acc);
     if (lane == 0) {
-      out[row] = (divisor != 0.0f) ? acc / divisor : acc;
+      out[row] = finish(acc, divisor);
       tickets[row] = 0; // leave the counter ready for the next launch
     }
   }
@@ -207,7 +212,7 @@ __global__ void __launch_bounds__(256) reduce_rows_warp(const float *__restrict_
 #pragma unroll
   for (int r = 0; r < RPW; ++r) {
     a[r] = warp_reduce<Op>(a[r]);
-    if (lane == 0 && row0 + r < n_rows) out[row0 + r] = (divisor != 0.0f) ? a[r] / divisor : a[r];
+    if (lane == 0 && row0 + r < n_rows) out[row0 + r] = finish(a[r], divisor);
   }
 }
 template <class Op>
@@ -287,7 +292,7 @@ __global__ void __launch_bounds__(256) reduce_cols(const float *__restrict__ in,
   }
   const int64_t out_base = z * C;
   if (S == 1) {
-    if (owner) out[out_base + c] = (divisor != 0.0f) ? v / divisor : v;
+    if (owner) out[out_base + c] = finish(v, divisor);
     return;
   }
   if (owner) partials[(z * S + split) * C + c] = v;
@@ -304,7 +309,7 @@ __global__ void __launch_bounds__(256) reduce_cols(const float *__restrict__ in,
   if (owner) {
     float a = Op::neutral();
     for (int s = 0; s < S; ++s) a = Op::combine(a, __ldcg(partials + (z * S + s) * C + c));
-    out[out_base + c] = (divisor != 0.0f) ? a / divisor : a;
+    out[out_base + c] = finish(a, divisor);
   }
   if (threadIdx.x == 0) tickets[tile_id] = 0;
 }
@@ -358,7 +363,7 @@ __global__ void __launch_bounds__(256) reduce_cols_wide(const float *__restrict_
   float *o = out + z * C + c0;
   if (S == 1) {
     if (live) {
-      if (divisor != 0.0f) acc = make_float4(acc.x / divisor, acc.y / divisor, acc.z / divisor, acc.w / divisor);
+      acc = make_float4(finish(acc.x, divisor), finish(acc.y, divisor), finish(acc.z, divisor), finish(acc.w, divisor));
       *reinterpret_cast<float4 *>(o) = acc;
     }
     return;
@@ -395,7 +400,7 @@ __global__ void __launch_bounds__(256) reduce_cols_wide(const float *__restrict_
       a.z = Op::combine(a.z, p0.z);
       a.w = Op::combine(a.w, p0.w);
     }
-    if (divisor != 0.0f) a = make_float4(a.x / divisor, a.y / divisor, a.z / divisor, a.w / divisor);
+    a = make_float4(finish(a.x, divisor), finish(a.y, divisor), finish(a.z, divisor), finish(a.w, divisor));
     *reinterpret_cast<float4 *>(o) = a;
   }
   if (threadIdx.x == 0) tickets[tile_id] = 0;

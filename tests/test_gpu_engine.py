@@ -41,6 +41,26 @@ def test_native_path_has_the_bits_of_the_op_classes(nt, case):
         assert a.shape == b.shape and np.array_equal(bits(a), bits(b))
 
 
+@pytest.mark.parametrize("shapes", [((64, 7), (1, 7)), ((128, 64), (128, 1)), ((4, 4096), (4, 1)), ((512, 2048), (1, 2048)),
+                                    ((2, 3, 4), (1, 3, 1)), ((6, 4), (4,)), ((2, 4), (2, 4))], ids=str)
+def test_gradients_that_cancel_are_the_same_zero(nt, shapes):
+    """The subtrahend's gradient is a sum of negated values: +0 where they cancel, on either path."""
+    from nanotorch_b200.autograd import SubOp
+
+    w = np.random.default_rng(5).integers(1, 9, shapes[0]).astype(np.float32)
+    pad = (1,) * (len(shapes[0]) - len(shapes[1])) + shapes[1]
+    for axis in [d for d, n in enumerate(pad) if n == 1 and shapes[0][d] % 2 == 0][:1]:  # w, -w, w, -w ... along a summed axis
+        w = np.take(w, np.arange(shapes[0][axis]) // 2 * 2, axis) * np.where(np.arange(shapes[0][axis]) % 2, -1, 1).reshape(
+            [-1 if d == axis else 1 for d in range(w.ndim)]).astype(np.float32)
+    got = []
+    for cls in (SubOp, type("SubOpPython", (SubOp,), {})):
+        x1, x2 = (nt.Tensor.from_numpy(np.ones(s, np.float32), "cuda", requires_grad=True) for s in shapes)
+        (cls.apply(x1, x2) * nt.Tensor.from_numpy(w, "cuda")).sum().backward()
+        got.append(x2.grad.numpy())
+    assert got[0].shape == got[1].shape == shapes[1] and np.array_equal(bits(got[0]), bits(got[1]))
+    assert shapes[0] == shapes[1] or not got[0].any()
+
+
 def test_results_are_freed_without_the_cycle_collector(nt):
     """A node that saves its own result must not keep it alive: memory comes back by reference count alone."""
     x = nt.Tensor.from_numpy(np.ones((64, 64), np.float32), "cuda", requires_grad=True)
