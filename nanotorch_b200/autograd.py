@@ -140,9 +140,13 @@ def _binary(x1: Tensor, x2: Tensor, op, op_inplace, out: Tensor | None) -> Tenso
     return result
 
 
+def _argument(fn: Function, i: int, name: str):
+    """An argument of the op's `apply`, whichever way it was given."""
+    return fn.inputs[i] if i < len(fn.inputs) else fn._inputs_kw[name]
+
+
 def _input_shapes(fn: Function) -> tuple[Shape, Shape]:
-    x1, x2 = fn.inputs[:2]
-    return x1.shape, x2.shape
+    return _argument(fn, 0, "x1").shape, _argument(fn, 1, "x2").shape
 
 
 class _BinaryOp(Function):
@@ -313,7 +317,7 @@ class LinearOp(Function):
         else:
             gx = g @ W.transpose(-2, -1) if _need(self, 0) else None
             gW = x.transpose(-2, -1) @ g if _need(self, 1) else None
-        gb = unbroadcast(g, self.inputs[2].shape) if _need(self, 2) else None
+        gb = unbroadcast(g, _argument(self, 2, "b").shape) if _need(self, 2) else None
         return gx, gW, gb
 
     @classmethod
@@ -619,7 +623,7 @@ class TransposeOp(Function):
         return Tensor._new_view(x.storage, tuple(shape), tuple(strides), x._offset)
 
     def backward(self, g):
-        return (g.transpose(*self.inputs[1:]),)
+        return (g.transpose(_argument(self, 1, "dim0"), _argument(self, 2, "dim1")),)
 
 
 ALL_OPS_ = [AddOp, ExpOp, ExpandOp, LogOp, MatmulOp, MeanOp, MulOp, NegOp, PowOp, ReluOp, ReshapeOp, SigmoidOp,

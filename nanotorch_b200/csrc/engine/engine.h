@@ -10,6 +10,8 @@
 #define PY_SSIZE_T_CLEAN
 #include <Python.h>
 
+#include <initializer_list>
+
 #include "../nt_core.cuh"
 
 namespace eng {
@@ -76,6 +78,12 @@ extern PyTypeObject StorageBase_Type, View_Type, TensorBase_Type, FunctionBase_T
 // ---- errors
 PyObject *raise_status(int status);     // the Python exception of a non-zero nt status; returns null
 struct PyErr {};                        // thrown after a Python exception has been set
+
+// Arguments of a METH_FASTCALL | METH_KEYWORDS function, each of `names` given once by position or by name, into out[];
+// false with a TypeError set.
+bool named_args(PyObject *const *args, Py_ssize_t n, PyObject *kwnames, std::initializer_list<const char *> names, PyObject **out);
+using FastKw = PyObject *(*)(PyObject *, PyObject *const *, Py_ssize_t, PyObject *);
+inline PyCFunction fast_kw(FastKw f) { return reinterpret_cast<PyCFunction>(reinterpret_cast<void *>(f)); }
 
 // ---- references
 struct Ref {

@@ -18,6 +18,33 @@ PyObject *raise_status(int status) {
   return nullptr;
 }
 
+bool named_args(PyObject *const *args, Py_ssize_t n, PyObject *kwnames, std::initializer_list<const char *> names, PyObject **out) {
+  const Py_ssize_t want = Py_ssize_t(names.size()), nkw = kwnames ? PyTuple_GET_SIZE(kwnames) : 0;
+  if (n > want) {
+    PyErr_Format(PyExc_TypeError, "expected %zd arguments, got %zd", want, n);
+    return false;
+  }
+  for (Py_ssize_t i = 0; i < want; ++i) out[i] = i < n ? args[i] : nullptr;
+  for (Py_ssize_t k = 0; k < nkw; ++k) {
+    Py_ssize_t at = 0;
+    for (const char *name : names) {
+      if (PyUnicode_CompareWithASCIIString(PyTuple_GET_ITEM(kwnames, k), name) == 0) break;
+      ++at;
+    }
+    if (at == want || out[at]) {
+      PyErr_Format(PyExc_TypeError, "unexpected or repeated keyword argument '%U'", PyTuple_GET_ITEM(kwnames, k));
+      return false;
+    }
+    out[at] = args[n + k];
+  }
+  for (Py_ssize_t i = 0; i < want; ++i)
+    if (!out[i]) {
+      PyErr_Format(PyExc_TypeError, "missing argument '%s'", names.begin()[i]);
+      return false;
+    }
+  return true;
+}
+
 int parse_dtype(PyObject *o) {
   for (int i = 0; i < 5; ++i)
     if (G.dtypes[i] == o) return i;
@@ -54,7 +81,9 @@ static int storage_init(PyObject *, PyObject *, PyObject *) {
   PyErr_SetString(PyExc_TypeError, "Storage: use Storage.allocate or Storage.from_iterable");
   return -1;
 }
-static PyObject *storage_wrap(PyObject *, PyObject *arg) {
+static PyObject *storage_wrap(PyObject *, PyObject *const *args, Py_ssize_t n, PyObject *kwnames) {
+  PyObject *arg;
+  if (!named_args(args, n, kwnames, {"handle"}, &arg)) return nullptr;
   void *p = PyLong_AsVoidPtr(arg);
   if (!p) {
     if (!PyErr_Occurred()) PyErr_SetString(PyExc_RuntimeError, "null storage");
@@ -62,16 +91,14 @@ static PyObject *storage_wrap(PyObject *, PyObject *arg) {
   }
   return wrap_storage(static_cast<nt_storage *>(p));
 }
-static PyObject *storage_allocate(PyObject *, PyObject *const *args, Py_ssize_t n) {
-  if (n != 3) {
-    PyErr_SetString(PyExc_TypeError, "allocate(n, dtype, device)");
-    return nullptr;
-  }
-  const long long count = PyLong_AsLongLong(args[0]);
+static PyObject *storage_allocate(PyObject *, PyObject *const *args, Py_ssize_t n, PyObject *kwnames) {
+  PyObject *a[3];
+  if (!named_args(args, n, kwnames, {"n", "dtype", "device"}, a)) return nullptr;
+  const long long count = PyLong_AsLongLong(a[0]);
   if (count == -1 && PyErr_Occurred()) return nullptr;
-  const int dt = parse_dtype(args[1]);
+  const int dt = parse_dtype(a[1]);
   if (dt < 0) return nullptr;
-  const int dev = parse_device(args[2]);
+  const int dev = parse_device(a[2]);
   if (dev < 0) return nullptr;
   nt_storage *s = nullptr;
   const int rc = nt_storage_allocate(count, dt, dev, &s);
@@ -82,7 +109,9 @@ static PyObject *storage_clone(PyObject *self, PyObject *) {
   const int rc = nt_storage_clone(handle(self), &s);
   return rc ? raise_status(rc) : wrap_storage(s);
 }
-static PyObject *storage_to(PyObject *self, PyObject *device) {
+static PyObject *storage_to(PyObject *self, PyObject *const *args, Py_ssize_t n, PyObject *kwnames) {
+  PyObject *device;
+  if (!named_args(args, n, kwnames, {"device"}, &device)) return nullptr;
   const int dev = parse_device(device);
   if (dev < 0) return nullptr;
   if (dev == handle(self)->device) return own(self);
@@ -92,7 +121,9 @@ static PyObject *storage_to(PyObject *self, PyObject *device) {
   Py_END_ALLOW_THREADS
   return rc ? raise_status(rc) : wrap_storage(s);
 }
-static PyObject *storage_cast(PyObject *self, PyObject *dtype) {
+static PyObject *storage_cast(PyObject *self, PyObject *const *args, Py_ssize_t n, PyObject *kwnames) {
+  PyObject *dtype;
+  if (!named_args(args, n, kwnames, {"dtype"}, &dtype)) return nullptr;
   const int dt = parse_dtype(dtype);
   if (dt < 0) return nullptr;
   if (dt == handle(self)->dtype) return own(self);
@@ -100,30 +131,28 @@ static PyObject *storage_cast(PyObject *self, PyObject *dtype) {
   const int rc = nt_storage_cast(handle(self), dt, &s);
   return rc ? raise_status(rc) : wrap_storage(s);
 }
-static bool pointer_and_bytes(PyObject *const *args, Py_ssize_t n, void **p, int64_t *nbytes) {
-  if (n != 2) {
-    PyErr_SetString(PyExc_TypeError, "expected (host_ptr, nbytes)");
-    return false;
-  }
-  *p = PyLong_AsVoidPtr(args[0]);
+static bool pointer_and_bytes(PyObject *const *args, Py_ssize_t n, PyObject *kwnames, void **p, int64_t *nbytes) {
+  PyObject *a[2];
+  if (!named_args(args, n, kwnames, {"host_ptr", "nbytes"}, a)) return false;
+  *p = PyLong_AsVoidPtr(a[0]);
   if (!*p && PyErr_Occurred()) return false;
-  *nbytes = PyLong_AsLongLong(args[1]);
+  *nbytes = PyLong_AsLongLong(a[1]);
   return !(*nbytes == -1 && PyErr_Occurred());
 }
-static PyObject *storage_upload(PyObject *self, PyObject *const *args, Py_ssize_t n) {
+static PyObject *storage_upload(PyObject *self, PyObject *const *args, Py_ssize_t n, PyObject *kwnames) {
   void *p;
   int64_t nbytes;
-  if (!pointer_and_bytes(args, n, &p, &nbytes)) return nullptr;
+  if (!pointer_and_bytes(args, n, kwnames, &p, &nbytes)) return nullptr;
   int rc;
   Py_BEGIN_ALLOW_THREADS rc = nt_storage_upload(handle(self), p, nbytes);
   Py_END_ALLOW_THREADS
   if (rc) return raise_status(rc);
   Py_RETURN_NONE;
 }
-static PyObject *storage_download(PyObject *self, PyObject *const *args, Py_ssize_t n) {
+static PyObject *storage_download(PyObject *self, PyObject *const *args, Py_ssize_t n, PyObject *kwnames) {
   void *p;
   int64_t nbytes;
-  if (!pointer_and_bytes(args, n, &p, &nbytes)) return nullptr;
+  if (!pointer_and_bytes(args, n, kwnames, &p, &nbytes)) return nullptr;
   int rc;
   Py_BEGIN_ALLOW_THREADS rc = nt_storage_download(handle(self), p, nbytes);
   Py_END_ALLOW_THREADS
@@ -141,13 +170,13 @@ static PyObject *storage_get_data_ptr(PyObject *self, void *) { return PyLong_Fr
 static PyObject *storage_get_h(PyObject *self, void *) { return PyLong_FromVoidPtr(handle(self)); }
 
 static PyMethodDef storage_methods[] = {
-    {"_wrap", storage_wrap, METH_O | METH_STATIC, "A storage over a native handle (takes its reference)."},
-    {"allocate", reinterpret_cast<PyCFunction>(storage_allocate), METH_FASTCALL | METH_STATIC, "allocate(n, dtype, device)"},
+    {"_wrap", fast_kw(storage_wrap), METH_FASTCALL | METH_KEYWORDS | METH_STATIC, "A storage over a native handle (takes its reference)."},
+    {"allocate", fast_kw(storage_allocate), METH_FASTCALL | METH_KEYWORDS | METH_STATIC, "allocate(n, dtype, device)"},
     {"clone", storage_clone, METH_NOARGS, nullptr},
-    {"to", storage_to, METH_O, nullptr},
-    {"cast", storage_cast, METH_O, nullptr},
-    {"upload", reinterpret_cast<PyCFunction>(storage_upload), METH_FASTCALL, nullptr},
-    {"download", reinterpret_cast<PyCFunction>(storage_download), METH_FASTCALL, nullptr},
+    {"to", fast_kw(storage_to), METH_FASTCALL | METH_KEYWORDS, "to(device)"},
+    {"cast", fast_kw(storage_cast), METH_FASTCALL | METH_KEYWORDS, "cast(dtype)"},
+    {"upload", fast_kw(storage_upload), METH_FASTCALL | METH_KEYWORDS, "upload(host_ptr, nbytes)"},
+    {"download", fast_kw(storage_download), METH_FASTCALL | METH_KEYWORDS, "download(host_ptr, nbytes)"},
     {}};
 static PyGetSetDef storage_getset[] = {{"size", storage_get_size},       {"itemsize", storage_get_itemsize},
                                        {"dtype", storage_get_dtype},     {"device", storage_get_device},
@@ -490,7 +519,9 @@ static int tensor_set_field(PyObject *self, PyObject *value, void *where) {
   Py_XDECREF(old);
   return 0;
 }
-static PyObject *tensor_attach_grad_fn(PyObject *self, PyObject *fn) {
+static PyObject *tensor_attach_grad_fn(PyObject *self, PyObject *const *args, Py_ssize_t n, PyObject *kwnames) {
+  PyObject *fn;
+  if (!named_args(args, n, kwnames, {"grad_fn"}, &fn)) return nullptr;
   tensor_set_field(self, fn, reinterpret_cast<void *>(offsetof(TensorObj, grad_fn)));
   Py_RETURN_NONE;
 }
@@ -628,19 +659,15 @@ static PyObject *make_view(PyTypeObject *cls, PyObject *storage, PyObject *shape
   t->strides = dims_tuple(int(st.size()), st.data());
   return t->shape && t->strides ? holder.release() : nullptr;
 }
-static PyObject *tensor_new_view(PyObject *cls, PyObject *const *args, Py_ssize_t n) {
-  if (n != 4) {
-    PyErr_SetString(PyExc_TypeError, "_new_view(storage, shape, strides, offset)");
-    return nullptr;
-  }
-  return make_view(reinterpret_cast<PyTypeObject *>(cls), args[0], args[1], args[2], args[3]);
+static PyObject *tensor_new_view(PyObject *cls, PyObject *const *args, Py_ssize_t n, PyObject *kwnames) {
+  PyObject *a[4];
+  if (!named_args(args, n, kwnames, {"storage", "shape", "strides", "offset"}, a)) return nullptr;
+  return make_view(reinterpret_cast<PyTypeObject *>(cls), a[0], a[1], a[2], a[3]);
 }
-static PyObject *tensor_new_contiguous(PyObject *cls, PyObject *const *args, Py_ssize_t n) {
-  if (n != 2) {
-    PyErr_SetString(PyExc_TypeError, "_new_contiguous(storage, shape)");
-    return nullptr;
-  }
-  return make_view(reinterpret_cast<PyTypeObject *>(cls), args[0], args[1], Py_None, Py_None);
+static PyObject *tensor_new_contiguous(PyObject *cls, PyObject *const *args, Py_ssize_t n, PyObject *kwnames) {
+  PyObject *a[2];
+  if (!named_args(args, n, kwnames, {"storage", "shape"}, a)) return nullptr;
+  return make_view(reinterpret_cast<PyTypeObject *>(cls), a[0], a[1], Py_None, Py_None);
 }
 
 // ---- operators: XxxOp.apply(self, totensor(other, anchor=self)), as the reference binds them
@@ -686,9 +713,9 @@ static PyObject *nb_imul(PyObject *a, PyObject *b) { return inplace(OP_MUL, a, b
 static PyObject *nb_idiv(PyObject *a, PyObject *b) { return inplace(OP_DIV, a, b); }
 
 template <Op OP> static PyObject *tensor_unary(PyObject *self, PyObject *) { return op_apply(OP, &self, 1); }
-static PyObject *tensor_pow(PyObject *self, PyObject *e) {
-  PyObject *args[2] = {self, e};
-  return op_apply(OP_POW, args, 2);
+static PyObject *tensor_pow(PyObject *self, PyObject *const *args, Py_ssize_t n, PyObject *kwnames) {
+  PyObject *full[2] = {self, nullptr};
+  return named_args(args, n, kwnames, {"exponent"}, full + 1) ? op_apply(OP_POW, full, 2) : nullptr;
 }
 // (axis=None, keepdim=False[, dtype=None]) after self
 template <Op OP, int N> static PyObject *tensor_reduce(PyObject *self, PyObject *const *args, Py_ssize_t n, PyObject *kwnames) {
@@ -728,21 +755,7 @@ template <Op OP> static PyObject *tensor_dims(PyObject *self, PyObject *const *a
 }
 static PyObject *tensor_transpose(PyObject *self, PyObject *const *args, Py_ssize_t n, PyObject *kwnames) {
   PyObject *full[3] = {self, nullptr, nullptr};
-  for (Py_ssize_t i = 0; i < n && i < 2; ++i) full[i + 1] = args[i];
-  for (Py_ssize_t k = 0; kwnames && k < PyTuple_GET_SIZE(kwnames); ++k) {
-    PyObject *name = PyTuple_GET_ITEM(kwnames, k);
-    const int at = PyUnicode_CompareWithASCIIString(name, "dim0") == 0 ? 1 : PyUnicode_CompareWithASCIIString(name, "dim1") == 0 ? 2 : 0;
-    if (!at || full[at]) {
-      PyErr_Format(PyExc_TypeError, "unexpected or repeated keyword argument '%U'", name);
-      return nullptr;
-    }
-    full[at] = args[n + k];
-  }
-  if (n > 2 || !full[1] || !full[2]) {
-    PyErr_SetString(PyExc_TypeError, "transpose(dim0, dim1)");
-    return nullptr;
-  }
-  return op_apply(OP_TRANSPOSE, full, 3);
+  return named_args(args, n, kwnames, {"dim0", "dim1"}, full + 1) ? op_apply(OP_TRANSPOSE, full, 3) : nullptr;
 }
 static PyObject *tensor_get_T(PyObject *self, void *) { return op_apply(OP_T, &self, 1); }
 
@@ -776,14 +789,14 @@ static PyObject *tensor_backward(PyObject *self, PyObject *) {
 }
 
 static PyMethodDef tensor_methods[] = {
-    {"_new_view", reinterpret_cast<PyCFunction>(tensor_new_view), METH_FASTCALL | METH_CLASS,
+    {"_new_view", fast_kw(tensor_new_view), METH_FASTCALL | METH_KEYWORDS | METH_CLASS,
      "_new_view(storage, shape, strides or None, offset or None): bounds-checked view of a storage"},
-    {"_new_contiguous", reinterpret_cast<PyCFunction>(tensor_new_contiguous), METH_FASTCALL | METH_CLASS,
+    {"_new_contiguous", fast_kw(tensor_new_contiguous), METH_FASTCALL | METH_KEYWORDS | METH_CLASS,
      "_new_contiguous(storage, shape)"},
-    {"_is_contiguous", reinterpret_cast<PyCFunction>(reinterpret_cast<void *>(tensor_is_contiguous)), METH_FASTCALL | METH_KEYWORDS,
+    {"_is_contiguous", fast_kw(tensor_is_contiguous), METH_FASTCALL | METH_KEYWORDS,
      "_is_contiguous(full_span=False)"},
     {"_alias", tensor_alias, METH_NOARGS, nullptr},
-    {"attach_grad_fn", tensor_attach_grad_fn, METH_O, nullptr},
+    {"attach_grad_fn", fast_kw(tensor_attach_grad_fn), METH_FASTCALL | METH_KEYWORDS, "attach_grad_fn(grad_fn)"},
     {"zero_grad", tensor_zero_grad, METH_NOARGS, nullptr},
     {"enable_grad", tensor_enable_grad, METH_NOARGS,
      "Enables gradient tracking after construction.  Unlike the constructor this does not look at the dtype, as in the "
@@ -795,14 +808,14 @@ static PyMethodDef tensor_methods[] = {
     {"tanh", tensor_unary<OP_TANH>, METH_NOARGS, nullptr},
     {"sigmoid", tensor_unary<OP_SIGMOID>, METH_NOARGS, nullptr},
     {"relu", tensor_unary<OP_RELU>, METH_NOARGS, nullptr},
-    {"pow", tensor_pow, METH_O, nullptr},
-    {"sum", reinterpret_cast<PyCFunction>(reinterpret_cast<void *>(tensor_reduce<OP_SUM, 3>)), METH_FASTCALL | METH_KEYWORDS, "sum(axis=None, keepdim=False, dtype=None)"},
-    {"mean", reinterpret_cast<PyCFunction>(reinterpret_cast<void *>(tensor_reduce<OP_MEAN, 3>)), METH_FASTCALL | METH_KEYWORDS, "mean(axis=None, keepdim=False, dtype=None)"},
-    {"max", reinterpret_cast<PyCFunction>(reinterpret_cast<void *>(tensor_reduce<OP_MAX, 2>)), METH_FASTCALL | METH_KEYWORDS, "max(axis=None, keepdim=False)"},
-    {"min", reinterpret_cast<PyCFunction>(reinterpret_cast<void *>(tensor_reduce<OP_MIN, 2>)), METH_FASTCALL | METH_KEYWORDS, "min(axis=None, keepdim=False)"},
+    {"pow", fast_kw(tensor_pow), METH_FASTCALL | METH_KEYWORDS, "pow(exponent)"},
+    {"sum", fast_kw(tensor_reduce<OP_SUM, 3>), METH_FASTCALL | METH_KEYWORDS, "sum(axis=None, keepdim=False, dtype=None)"},
+    {"mean", fast_kw(tensor_reduce<OP_MEAN, 3>), METH_FASTCALL | METH_KEYWORDS, "mean(axis=None, keepdim=False, dtype=None)"},
+    {"max", fast_kw(tensor_reduce<OP_MAX, 2>), METH_FASTCALL | METH_KEYWORDS, "max(axis=None, keepdim=False)"},
+    {"min", fast_kw(tensor_reduce<OP_MIN, 2>), METH_FASTCALL | METH_KEYWORDS, "min(axis=None, keepdim=False)"},
     {"reshape", reinterpret_cast<PyCFunction>(tensor_dims<OP_RESHAPE>), METH_FASTCALL, "reshape(*dims)"},
     {"expand", reinterpret_cast<PyCFunction>(tensor_dims<OP_EXPAND>), METH_FASTCALL, "expand(*dims)"},
-    {"transpose", reinterpret_cast<PyCFunction>(reinterpret_cast<void *>(tensor_transpose)), METH_FASTCALL | METH_KEYWORDS, "transpose(dim0, dim1)"},
+    {"transpose", fast_kw(tensor_transpose), METH_FASTCALL | METH_KEYWORDS, "transpose(dim0, dim1)"},
     {}};
 
 #define FIELD(name, member, set)                                                                   \

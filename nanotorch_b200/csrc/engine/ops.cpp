@@ -19,35 +19,36 @@ using FnIn = int (*)(const nt_view *, const nt_view *);
 using FnBoth = int (*)(const nt_view *, const nt_view *, const nt_view *, nt_storage **, nt_storage **);
 using FnAxes = int (*)(const nt_view *, const int64_t *, int32_t, nt_storage **);
 
-static bool count_is(Py_ssize_t n, Py_ssize_t want) {
-  if (n == want) return true;
-  PyErr_Format(PyExc_TypeError, "expected %zd arguments, got %zd", want, n);
-  return false;
-}
-template <Fn1 FN> static PyObject *c_unary(PyObject *, PyObject *const *a, Py_ssize_t n) {
+static constexpr char x_name[] = "x", src_name[] = "src";
+template <Fn1 FN, const char *NAME = x_name> static PyObject *c_unary(PyObject *, PyObject *const *args, Py_ssize_t n, PyObject *kwnames) {
   nt_view x;
-  if (!count_is(n, 1) || !view_arg(a[0], &x)) return nullptr;
+  PyObject *a;
+  if (!named_args(args, n, kwnames, {NAME}, &a) || !view_arg(a, &x)) return nullptr;
   nt_storage *out = nullptr;
   const int rc = FN(&x, &out);
   return rc ? raise_status(rc) : wrap_storage(out);
 }
-template <Fn2 FN> static PyObject *c_binary(PyObject *, PyObject *const *a, Py_ssize_t n) {
+template <Fn2 FN> static PyObject *c_binary(PyObject *, PyObject *const *args, Py_ssize_t n, PyObject *kwnames) {
   nt_view x, y;
-  if (!count_is(n, 2) || !view_arg(a[0], &x) || !view_arg(a[1], &y)) return nullptr;
+  PyObject *a[2];
+  if (!named_args(args, n, kwnames, {"x1", "x2"}, a) || !view_arg(a[0], &x) || !view_arg(a[1], &y)) return nullptr;
   nt_storage *out = nullptr;
   const int rc = FN(&x, &y, &out);
   return rc ? raise_status(rc) : wrap_storage(out);
 }
-template <Fn3 FN> static PyObject *c_ternary(PyObject *, PyObject *const *a, Py_ssize_t n) {
+static constexpr char w_name[] = "w", bias_name[] = "bias", g_name[] = "g", x1_name[] = "x1", x2_name[] = "x2";
+template <Fn3 FN, const char *N0, const char *N1, const char *N2> static PyObject *c_ternary(PyObject *, PyObject *const *args, Py_ssize_t n, PyObject *kwnames) {
   nt_view x, y, z;
-  if (!count_is(n, 3) || !view_arg(a[0], &x) || !view_arg(a[1], &y) || !view_arg(a[2], &z)) return nullptr;
+  PyObject *a[3];
+  if (!named_args(args, n, kwnames, {N0, N1, N2}, a) || !view_arg(a[0], &x) || !view_arg(a[1], &y) || !view_arg(a[2], &z)) return nullptr;
   nt_storage *out = nullptr;
   const int rc = FN(&x, &y, &z, &out);
   return rc ? raise_status(rc) : wrap_storage(out);
 }
-template <FnIn FN> static PyObject *c_inplace(PyObject *, PyObject *const *a, Py_ssize_t n) {
+template <FnIn FN> static PyObject *c_inplace(PyObject *, PyObject *const *args, Py_ssize_t n, PyObject *kwnames) {
   nt_view x, y;
-  if (!count_is(n, 2) || !view_arg(a[0], &x) || !view_arg(a[1], &y)) return nullptr;
+  PyObject *a[2];
+  if (!named_args(args, n, kwnames, {"x1", "x2"}, a) || !view_arg(a[0], &x) || !view_arg(a[1], &y)) return nullptr;
   const int rc = FN(&x, &y);
   if (rc) return raise_status(rc);
   Py_RETURN_NONE;
@@ -56,18 +57,20 @@ static PyObject *pair_of(nt_storage *s1, nt_storage *s2) {
   Ref a(wrap_storage(s1)), b(wrap_storage(s2));
   return a && b ? PyTuple_Pack(2, a.p, b.p) : nullptr;
 }
-template <FnBoth FN> static PyObject *c_both(PyObject *, PyObject *const *a, Py_ssize_t n) {
+template <FnBoth FN> static PyObject *c_both(PyObject *, PyObject *const *args, Py_ssize_t n, PyObject *kwnames) {
   nt_view g, x, y;
-  if (!count_is(n, 3) || !view_arg(a[0], &g) || !view_arg(a[1], &x) || !view_arg(a[2], &y)) return nullptr;
+  PyObject *a[3];
+  if (!named_args(args, n, kwnames, {"g", "x1", "x2"}, a) || !view_arg(a[0], &g) || !view_arg(a[1], &x) || !view_arg(a[2], &y)) return nullptr;
   nt_storage *s1 = nullptr, *s2 = nullptr;
   const int rc = FN(&g, &x, &y, &s1, &s2);
   if (rc) return raise_status(rc);
   if (!s1) Py_RETURN_NONE;
   return pair_of(s1, s2);
 }
-static PyObject *c_matmul_pair(PyObject *, PyObject *const *a, Py_ssize_t n) {
+static PyObject *c_matmul_pair(PyObject *, PyObject *const *args, Py_ssize_t n, PyObject *kwnames) {
   nt_view v[4];
-  if (!count_is(n, 4)) return nullptr;
+  PyObject *a[4];
+  if (!named_args(args, n, kwnames, {"a1", "b1", "a2", "b2"}, a)) return nullptr;
   for (int i = 0; i < 4; ++i)
     if (!view_arg(a[i], &v[i])) return nullptr;
   nt_storage *s1 = nullptr, *s2 = nullptr;
@@ -86,18 +89,20 @@ static bool axes_arg(PyObject *o, std::vector<int64_t> *out) {
   }
   return true;
 }
-template <FnAxes FN> static PyObject *c_reduce(PyObject *, PyObject *const *a, Py_ssize_t n) {
+template <FnAxes FN> static PyObject *c_reduce(PyObject *, PyObject *const *args, Py_ssize_t n, PyObject *kwnames) {
   nt_view x;
   std::vector<int64_t> ax;
-  if (!count_is(n, 2) || !view_arg(a[0], &x) || !axes_arg(a[1], &ax)) return nullptr;
+  PyObject *a[2];
+  if (!named_args(args, n, kwnames, {"x", "axis"}, a) || !view_arg(a[0], &x) || !axes_arg(a[1], &ax)) return nullptr;
   nt_storage *out = nullptr;
   const int rc = FN(&x, ax.data(), int32_t(ax.size()), &out);
   return rc ? raise_status(rc) : wrap_storage(out);
 }
-static PyObject *c_sum(PyObject *, PyObject *const *a, Py_ssize_t n) {
+static PyObject *c_sum(PyObject *, PyObject *const *args, Py_ssize_t n, PyObject *kwnames) {
   nt_view x;
   std::vector<int64_t> ax;
-  if (!count_is(n, 3) || !view_arg(a[0], &x) || !axes_arg(a[1], &ax)) return nullptr;
+  PyObject *a[3];
+  if (!named_args(args, n, kwnames, {"x", "axis", "dtype"}, a) || !view_arg(a[0], &x) || !axes_arg(a[1], &ax)) return nullptr;
   const int dt = parse_dtype(a[2]);
   if (dt < 0) return nullptr;
   nt_storage *out = nullptr;
@@ -105,26 +110,26 @@ static PyObject *c_sum(PyObject *, PyObject *const *a, Py_ssize_t n) {
   return rc ? raise_status(rc) : wrap_storage(out);
 }
 
-#define BINARY(name) {#name, reinterpret_cast<PyCFunction>(c_binary<nt_##name>), METH_FASTCALL, nullptr}
-#define UNARY(name) {#name, reinterpret_cast<PyCFunction>(c_unary<nt_##name>), METH_FASTCALL, nullptr}
-#define INPLACE(name) {#name, reinterpret_cast<PyCFunction>(c_inplace<nt_##name>), METH_FASTCALL, nullptr}
-#define REDUCE(name) {#name, reinterpret_cast<PyCFunction>(c_reduce<nt_##name>), METH_FASTCALL, nullptr}
-#define BOTH(name) {#name, reinterpret_cast<PyCFunction>(c_both<nt_##name>), METH_FASTCALL, nullptr}
+#define BINARY(name) {#name, fast_kw(c_binary<nt_##name>), METH_FASTCALL | METH_KEYWORDS, nullptr}
+#define UNARY(name) {#name, fast_kw(c_unary<nt_##name>), METH_FASTCALL | METH_KEYWORDS, nullptr}
+#define INPLACE(name) {#name, fast_kw(c_inplace<nt_##name>), METH_FASTCALL | METH_KEYWORDS, nullptr}
+#define REDUCE(name) {#name, fast_kw(c_reduce<nt_##name>), METH_FASTCALL | METH_KEYWORDS, nullptr}
+#define BOTH(name) {#name, fast_kw(c_both<nt_##name>), METH_FASTCALL | METH_KEYWORDS, nullptr}
 static PyMethodDef c_functions[] = {
     BINARY(add), BINARY(subtract), BINARY(multiply), BINARY(divide), BINARY(pw_equal), BINARY(pw_greater),
     BINARY(pw_greater_eq), BINARY(matmul), BINARY(relu_backward), BINARY(tanh_backward), BINARY(sigmoid_backward),
     BINARY(exp_backward), BINARY(log_backward), BINARY(sqrt_backward),
     UNARY(exp), UNARY(log), UNARY(sqrt), UNARY(tanh), UNARY(sigmoid), UNARY(neg), UNARY(relu),
-    UNARY(clone_contiguous_view_from),
+    {"clone_contiguous_view_from", fast_kw(c_unary<nt_clone_contiguous_view_from, src_name>), METH_FASTCALL | METH_KEYWORDS, nullptr},
     INPLACE(add_inplace), INPLACE(sub_inplace), INPLACE(mul_inplace), INPLACE(div_inplace), INPLACE(copy_inplace),
     REDUCE(max), REDUCE(min), REDUCE(argmax), REDUCE(argmin),
     BOTH(mul_backward), BOTH(div_backward),
-    {"linear", reinterpret_cast<PyCFunction>(c_ternary<nt_linear>), METH_FASTCALL,
+    {"linear", fast_kw(c_ternary<nt_linear, x_name, w_name, bias_name>), METH_FASTCALL | METH_KEYWORDS,
      "x @ w + bias with the bias add fused into the GEMM epilogue (addition to the reference's surface)."},
-    {"div_backward_x2", reinterpret_cast<PyCFunction>(c_ternary<nt_div_backward_x2>), METH_FASTCALL, nullptr},
-    {"matmul_pair", reinterpret_cast<PyCFunction>(c_matmul_pair), METH_FASTCALL,
+    {"div_backward_x2", fast_kw(c_ternary<nt_div_backward_x2, g_name, x1_name, x2_name>), METH_FASTCALL | METH_KEYWORDS, nullptr},
+    {"matmul_pair", fast_kw(c_matmul_pair), METH_FASTCALL | METH_KEYWORDS,
      "(a1 @ b1, a2 @ b2): two independent products in one call (addition to the reference's surface; the bits of two `matmul` calls)."},
-    {"sum", reinterpret_cast<PyCFunction>(c_sum), METH_FASTCALL, "sum(x, axes, dtype)"},
+    {"sum", fast_kw(c_sum), METH_FASTCALL | METH_KEYWORDS, "sum(x, axes, dtype)"},
     {}};
 
 bool init_ops(PyObject *m) { return PyModule_AddFunctions(m, c_functions) == 0; }

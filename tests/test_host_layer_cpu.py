@@ -1,6 +1,7 @@
 """Host logic of the Tensor/autograd mirror, no kernels: view bookkeeping, shape rules, error behaviour
 (the cases the reference's own tests pin in tests/test_ops/test_tensor_core*.py)."""
 
+import numpy as np
 import pytest
 
 from nanotorch_b200.autograd import _matmul_shapes, normalize_axes
@@ -159,3 +160,59 @@ def test_repr_has_the_references_format(nt):
                          "          [40, 41, 42, ..., 47, 48, 49]\n          [50, 51, 52, ..., 57, 58, 59])")
     assert repr(nt.zeros(2, 2, 2)) == "nt.Tensor(shape=(2, 2, 2), 8 x <Float32>, d: Cpu)"
     assert repr(six.T[1:3]) == "nt.Tensor([1, 11, 21, 31, 41, 51]\n          [2, 12, 22, 32, 42, 52])"   # through a view
+
+
+def test_native_functions_take_their_arguments_by_name(nt):
+    """Views of CPU storages reach the kernel's own refusal (a RuntimeError): the arguments were understood."""
+    C = nt._C
+    t = nt.Tensor([[1.0, 2.0], [3.0, 4.0]])
+    v = t._C_view
+    calls = {("x1", "x2"): ("add", "subtract", "multiply", "divide", "pw_equal", "matmul", "relu_backward", "add_inplace", "copy_inplace"),
+             ("x",): ("exp", "neg", "relu"), ("src",): ("clone_contiguous_view_from",), ("x", "w", "bias"): ("linear",),
+             ("g", "x1", "x2"): ("mul_backward", "div_backward", "div_backward_x2"), ("a1", "b1", "a2", "b2"): ("matmul_pair",)}
+    for names, functions in calls.items():
+        for f in functions:
+            for given in (dict.fromkeys(names, v), dict.fromkeys(names[1:], v)):
+                args = (v,) * (len(names) - len(given))
+                with pytest.raises((RuntimeError, ValueError)):
+                    getattr(C, f)(*args, **given)
+            with pytest.raises(TypeError):
+                getattr(C, f)(*(v,) * len(names), **{names[0]: v})
+            with pytest.raises(TypeError):
+                getattr(C, f)(*(v,) * (len(names) - 1), other=v)
+            with pytest.raises(TypeError):
+                getattr(C, f)(*(v,) * (len(names) - 1))
+    for f in ("max", "argmin"):
+        with pytest.raises((RuntimeError, ValueError)):
+            getattr(C, f)(x=v, axis=(0,))
+    with pytest.raises((RuntimeError, ValueError)):
+        C.sum(v, axis=(0,), dtype=nt.float32)
+    s = C.Storage.allocate(n=2, dtype=nt.float32, device=nt.Device.Cpu)
+    assert s.to(device=nt.Device.Cpu) is s and s.cast(dtype=nt.float32) is s and s.cast(dtype=nt.float64).dtype == nt.float64
+    data = np.array([1, 2], np.float32)
+    s.upload(host_ptr=data.ctypes.data, nbytes=8)
+    data[:] = 0
+    s.download(data.ctypes.data, nbytes=8)
+    assert data.tolist() == [1, 2]
+    u = nt.Tensor._new_contiguous(storage=s, shape=(2,))
+    u.attach_grad_fn(grad_fn=None)
+    assert nt.Tensor._new_view(s, shape=(1,), strides=None, offset=1).shape == (1,) and u.is_leaf
+    assert t.transpose(dim1=0, dim0=1).shape == (2, 2)
+    with pytest.raises(TypeError):
+        t.pow(power=2)
+    with pytest.raises(RuntimeError):
+        t.pow(exponent=2)  # no kernel takes a CPU tensor
+
+
+@pytest.mark.parametrize("op, args, kwargs", [("TransposeOp", ((2, 3),), {"dim0": 0, "dim1": 1}), ("TransposeOp", ((2, 3), 0), {"dim1": 1}),
+                                              ("AddOp", ((2, 3),), {"x2": (2, 3)})], ids=str)
+def test_an_op_given_an_argument_by_name_has_a_backward(nt, op, args, kwargs):
+    from nanotorch_b200 import autograd
+
+    shaped = lambda a: nt.Tensor._new_contiguous(nt._C.Storage.allocate(6, nt.float32, nt.Device.Cpu), a) if isinstance(a, tuple) else a  # noqa: E731
+    x = [shaped(a) for a in args]
+    native = type("Probe", (getattr(autograd, op),), {"forward": lambda self, *a, **k: x[0]._alias()})
+    x[0].enable_grad()
+    y = native.apply(*x, **{k: shaped(v) for k, v in kwargs.items()})
+    grads = y.grad_fn.backward(shaped(y.shape if op != "TransposeOp" else (3, 2)))
+    assert grads[0].shape == (2, 3)
