@@ -222,9 +222,12 @@ struct NoGrad {
   ~NoGrad() { G.grad_enabled = prev; }
 };
 
-// What leaves the sweep is in memory: see nt_scaled.
+// What leaves the sweep, and what Python code may come to see or change the source of, is in memory: see nt_scaled.
+static bool is_scaled(PyObject *g) {
+  return g && is_tensor(g) && T_(g)->storage && is_storage(T_(g)->storage) && storage_of(T_(g))->scaled();
+}
 static bool settle(PyObject *g) {
-  if (!is_tensor(g) || !T_(g)->storage || !is_storage(T_(g)->storage)) return true;
+  if (!g || !is_tensor(g) || !T_(g)->storage || !is_storage(T_(g)->storage)) return true;
   const int rc = nt_storage_settle(storage_of(T_(g)));
   if (rc) raise_status(rc);
   return rc == 0;
@@ -241,6 +244,8 @@ static bool accumulate(TensorObj *x, PyObject *gx) {
   Py_SETREF(x->grad, sum);
   return true;
 }
+
+static PyObject *sweep(std::vector<Ref> &order, std::vector<Ref>::reverse_iterator &it, std::unordered_map<PyObject *, int> &pending);
 
 PyObject *run_backward(TensorObj *root) {
   std::vector<Ref> order; // a node is followed by those it depends on... reversed below
@@ -283,7 +288,22 @@ PyObject *run_backward(TensorObj *root) {
     }
   }
   NoGrad no_grad; // gradients are values, not graph nodes
-  for (auto it = order.rbegin(); it != order.rend(); ++it) {
+  auto it = order.rbegin();
+  PyObject *done = sweep(order, it, pending);
+  if (!done) { // the gradients that the sweep leaves behind on its nodes
+    PyObject *type, *value, *trace;
+    PyErr_Fetch(&type, &value, &trace);
+    for (; it != order.rend(); ++it)
+      if (!settle(T_(it->p)->grad)) PyErr_Clear();
+    PyErr_Restore(type, value, trace);
+  }
+  return done;
+}
+
+// The nodes from `it` on, which is where it stops after an exception.
+static PyObject *sweep(std::vector<Ref> &order, std::vector<Ref>::reverse_iterator &it, std::unordered_map<PyObject *, int> &pending) {
+  bool any_scaled = false; // since Python code last ran
+  for (; it != order.rend(); ++it) {
     TensorObj *node = T_(it->p);
     if (!node->grad) {
       PyErr_SetString(PyExc_RuntimeError, "f_x.grad is None.");
@@ -296,8 +316,20 @@ PyObject *run_backward(TensorObj *root) {
     Ref grads; // of the Python backward
     const bool native = PyObject_TypeCheck(fn.p, &FunctionBase_Type) && backward_fast(F_(fn.p), T_(g.p), out, &n_out, &added);
     Ref held[3] = {Ref(out[0]), Ref(out[1]), Ref(out[2])};
+    // Before Python code runs, a custom op's backward or a hook, which may write to a tensor that a gradient still waiting in
+    // the sweep is a factor of.
+    auto settle_waiting = [&] {
+      if (!any_scaled) return true;
+      any_scaled = false;
+      for (Ref &h : held)
+        if (!settle(h.p)) return false;
+      for (auto later = it + 1; later != order.rend(); ++later)
+        if (!settle(T_(later->p)->grad)) return false;
+      return true;
+    };
+    for (Ref &h : held) any_scaled = any_scaled || is_scaled(h.p);
     if (!native) {
-      if (PyErr_Occurred() || !settle(g.p)) return nullptr;
+      if (PyErr_Occurred() || !settle(g.p) || !settle_waiting()) return nullptr;
       Ref r(PyObject_CallMethod(fn.p, "backward", "O", g.p));
       if (!r) return nullptr;
       grads = Ref(PySequence_Fast(r.p, "backward must return one gradient per tensor input"));
@@ -320,6 +352,7 @@ PyObject *run_backward(TensorObj *root) {
       auto p = pending.find(x);
       if (p == pending.end()) continue;
       if (p->second-- == 1 && T_(x)->grad) {
+        if (!settle_waiting()) return nullptr;
         Ref key(PyLong_FromVoidPtr(x));
         PyObject *hook = key ? PyDict_GetItemWithError(G.hooks, key.p) : nullptr;
         if (!hook) {

@@ -737,8 +737,8 @@ static bool backward_op(FunctionObj *fn, TensorObj *g, PyObject **out, int *n_ou
       }
     }
     if (mul && vg.storage->constant && !both) {
-      // a constant gradient, as a sum or a mean sends it: the other factor times a number (see nt_scaled; not where a
-      // hook may change that factor during the sweep)
+      // a constant gradient, as a sum or a mean sends it: the other factor times a number (see nt_scaled; not of a leaf,
+      // which a hook is likely to update during the sweep)
       const int i = need(fn, 0) ? 0 : 1;
       TensorObj *other = saved(fn, 1 - i), *own_input = saved(fn, i);
       if (same_shape(g, other) && same_shape(g, own_input) && is_fast(reinterpret_cast<PyObject *>(other)) && !other->requires_grad) {
@@ -810,8 +810,8 @@ static bool backward_op(FunctionObj *fn, TensorObj *g, PyObject **out, int *n_ou
     *n_out = 1;
     const nt_view vg = view_of(g), vx = view_of(x);
     nt_storage *s = nullptr;
-    // a squared error: the gradient is the saved difference times a number (unless that difference is a leaf, whose
-    // values a hook may change during the sweep)
+    // a squared error: the gradient is the saved difference times a number (unless that difference is a leaf, which a hook
+    // is likely to update during the sweep)
     if (fn->e == 2.0 && vg.storage->constant && x->grad_fn) {
       checked(nt_scaled(&vx, vg.storage->value * 2.0f, &s), s);
       if (s) {

@@ -110,3 +110,50 @@ def test_a_written_gradient_does_not_keep_the_difference(nt):
     nt.mean(((a + b) - target) ** 2).backward()
     assert nt.cuda.memory_stats()["bytes_in_use"] - before <= 4 * n  # one gradient, which both leaves have
     assert (a.grad.numpy() == np.float32(6 / n)).all() and (b.grad.numpy() == np.float32(6 / n)).all()
+
+
+@pytest.mark.parametrize("kind", ["backward", "hook", "error"])
+def test_a_waiting_gradient_survives_python_code(nt, kind):
+    """A custom op's backward, or a leaf's hook, overwrites the difference of which a gradient still waiting in the sweep is a
+    factor; and a sweep that ends in an exception leaves values behind, not factors."""
+    from nanotorch_b200 import autograd
+
+    class Scrub(autograd.Function):
+        """A sum whose backward zeroes its input and passes no gradient on."""
+
+        def forward(self, d):
+            self.d = d
+            return nt.Tensor._new_contiguous(nt._C.sum(d._C_view, (0,), d.dtype), ())
+
+        def backward(self, g):
+            scrub(self.d)
+            return (None,)
+
+    def scrub(d):
+        nt._C.mul_inplace(d._C_view, nt.Tensor.from_numpy(np.zeros(d.shape, np.float32), "cuda")._C_view)
+        if kind == "error":
+            raise ArithmeticError
+
+    x = np.arange(1, 9, dtype=np.float32)
+    kept = 0
+    for square_first in (True, False):  # one of the two has the square's gradient waiting when the difference is zeroed
+        t, leaf = (nt.Tensor.from_numpy(x, "cuda", requires_grad=True) for _ in range(2))
+        d = t - 0.5
+        other = (leaf * 1.0).sum() if kind == "hook" else Scrub.apply(d)
+        if kind == "hook":
+            autograd.leaf_grad_hooks[id(leaf)] = lambda p, d=d: scrub(d)
+        square = (d ** 2).sum()
+        try:
+            (square + other if square_first else other + square).backward()
+        except RuntimeError as refused:  # zeroed before the square's backward, which notices
+            assert "modified inplace" in str(refused)
+            continue
+        except ArithmeticError:
+            assert kind == "error"
+        finally:
+            autograd.leaf_grad_hooks.pop(id(leaf), None)
+        got = d.grad if kind == "error" else t.grad
+        if got is not None:
+            assert np.array_equal(got.numpy(), 2 * (x - 0.5))
+            kept += 1
+    assert kept == 1
