@@ -393,7 +393,9 @@ static bool axes_of(PyObject *axis, int nd, int64_t *axes, int *n) {
   *n = 0;
   if (axis != Py_None) {
     if (PyLong_CheckExact(axis)) {
-      axes[(*n)++] = PyLong_AsLongLong(axis);
+      int overflow = 0;
+      axes[(*n)++] = PyLong_AsLongLongAndOverflow(axis, &overflow);
+      if (overflow) return false;
     } else if (PyTuple_CheckExact(axis)) {
       if (!parse_dims(axis, axes, n)) return false;
     } else {

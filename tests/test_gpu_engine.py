@@ -86,3 +86,11 @@ def test_saved_tensor_modified_in_place_is_refused(nt):
         y += 1
     with pytest.raises(RuntimeError, match="modified inplace"):
         z.sum().backward()
+
+
+@pytest.mark.parametrize("axis", [2 ** 70, -2 ** 70, (0, 2 ** 70)], ids=str)
+@pytest.mark.parametrize("op", ["sum", "mean", "max"])
+def test_an_axis_beyond_64_bits_is_an_index_error(nt, op, axis):
+    x = nt.Tensor.from_numpy(np.ones((2, 3), np.float32), "cuda")
+    with pytest.raises(IndexError):
+        getattr(x, op)(axis=axis)
