@@ -694,7 +694,10 @@ static PyObject *nb_add(PyObject *a, PyObject *b) { return binary(OP_ADD, a, b, 
 static PyObject *nb_sub(PyObject *a, PyObject *b) { return binary(OP_SUB, a, b, false); }
 static PyObject *nb_mul(PyObject *a, PyObject *b) { return binary(OP_MUL, a, b, true); }
 static PyObject *nb_div(PyObject *a, PyObject *b) { return binary(OP_DIV, a, b, false); }
-static PyObject *nb_pow(PyObject *a, PyObject *b, PyObject *) { return binary(OP_POW, a, b, false); }
+static PyObject *nb_pow(PyObject *a, PyObject *b, PyObject *modulus) {
+  if (modulus != Py_None) Py_RETURN_NOTIMPLEMENTED;
+  return binary(OP_POW, a, b, false);
+}
 static PyObject *nb_matmul(PyObject *a, PyObject *b) {
   if (!is_tensor(a)) Py_RETURN_NOTIMPLEMENTED;
   return binary(OP_MATMUL, a, b, false);

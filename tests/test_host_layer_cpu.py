@@ -216,3 +216,10 @@ def test_an_op_given_an_argument_by_name_has_a_backward(nt, op, args, kwargs):
     y = native.apply(*x, **{k: shaped(v) for k, v in kwargs.items()})
     grads = y.grad_fn.backward(shaped(y.shape if op != "TransposeOp" else (3, 2)))
     assert grads[0].shape == (2, 3)
+
+
+def test_power_with_a_modulus_is_refused(nt):
+    t = nt.Tensor([1.0, 2.0])
+    for args in ((t, 2, 3), (2, t, 3), (t, 2, t)):
+        with pytest.raises(TypeError):
+            pow(*args)
