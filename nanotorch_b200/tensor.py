@@ -207,6 +207,12 @@ class Tensor(_engine.TensorBase):
         return f"nt.Tensor(shape={self.shape}, {self.numel} x <{self.dtype.name}>, d: {self.device.name})"
 
     # ------------------------------------------------------------------ moves and copies
+    def __copy__(self) -> "Tensor":
+        """The same storage, gradient and graph node under another tensor object."""
+        t = type(self)._new_view(self._storage, self._shape, self._strides, self._offset)
+        t._requires_grad, t._grad, t._grad_fn, t._pyvalue = self._requires_grad, self._grad, self._grad_fn, self._pyvalue
+        return t
+
     def to(self, target: Dtype | Device | str) -> "Tensor":
         """Cast to a dtype or move to a device; returns self when nothing changes."""
         src = self

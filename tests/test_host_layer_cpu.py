@@ -223,3 +223,15 @@ def test_power_with_a_modulus_is_refused(nt):
     for args in ((t, 2, 3), (2, t, 3), (t, 2, t)):
         with pytest.raises(TypeError):
             pow(*args)
+
+
+def test_shallow_copy_shares_the_storage(nt):
+    import copy
+
+    t = nt.Tensor([[1.0, 2.0], [3.0, 4.0]], requires_grad=True).T
+    t._grad = nt.Tensor([0.0])
+    c = copy.copy(t)
+    assert type(c) is type(t) and c is not t and c.storage is t.storage and c.tolist() == [[1.0, 3.0], [2.0, 4.0]]
+    assert c.strides == t.strides and c.grad is t.grad and c.grad_fn is t.grad_fn and c.requires_grad == t.requires_grad
+    deep = nt.Tensor._new_view(t.storage, (1,) * 10, None, None)
+    assert copy.copy(deep).shape == (1,) * 10
