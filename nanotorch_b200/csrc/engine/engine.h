@@ -127,6 +127,10 @@ TensorObj *new_tensor(nt_storage *s, int nd, const int64_t *shape);
 TensorObj *new_view(PyObject *storage, int nd, const int64_t *shape, const int64_t *strides, int64_t offset);
 inline TensorObj *alias_of(const TensorObj *t) { return new_view(t->storage, t->nd, t->sh, t->st, t->offset); }
 
+// The Python number that a 0-d tensor was made from, while its storage has not been written to; borrowed, or null.
+inline PyObject *pyvalue_of(const TensorObj *t) {
+  return t->pyvalue && t->storage && is_storage(t->storage) && storage_of(t)->mutation == 0 ? t->pyvalue : nullptr;
+}
 inline bool requires_grad(const TensorObj *t) { return t->requires_grad || t->grad_fn; }
 inline bool same_shape(const TensorObj *a, const TensorObj *b) {
   return a->nd == b->nd && std::memcmp(a->sh, b->sh, sizeof(int64_t) * size_t(a->nd < 0 ? 0 : a->nd)) == 0;

@@ -519,6 +519,10 @@ static int tensor_set_field(PyObject *self, PyObject *value, void *where) {
   Py_XDECREF(old);
   return 0;
 }
+static PyObject *tensor_get_pyvalue(PyObject *self, void *) {
+  PyObject *v = pyvalue_of(T_(self));
+  return own(v ? v : Py_None);
+}
 static PyObject *tensor_attach_grad_fn(PyObject *self, PyObject *const *args, Py_ssize_t n, PyObject *kwnames) {
   PyObject *fn;
   if (!named_args(args, n, kwnames, {"grad_fn"}, &fn)) return nullptr;
@@ -830,7 +834,7 @@ static PyGetSetDef tensor_getset[] = {
     FIELD("grad", grad, nullptr),
     FIELD("_grad_fn", grad_fn, tensor_set_field),
     FIELD("grad_fn", grad_fn, nullptr),
-    FIELD("_pyvalue", pyvalue, tensor_set_field),
+    {"_pyvalue", tensor_get_pyvalue, tensor_set_field, nullptr, reinterpret_cast<void *>(offsetof(TensorObj, pyvalue))},
     {"_shape", tensor_get_shape, tensor_set_shape},
     {"shape", tensor_get_shape},
     {"_strides", tensor_get_strides_, tensor_set_strides},

@@ -214,9 +214,8 @@ struct Operand {
     if (Py_TYPE(o) != G.tensor_type) return false;
     TensorObj *x = T_(o);
     nt_scalar v;
-    if (!x->pyvalue || x->nd != 0 || !is_storage(x->storage) || storage_of(x)->device != NT_CUDA ||
-        storage_of(x)->dtype > NT_FLOAT32 || !scalar_of(x->pyvalue, &v))
-      return false;
+    PyObject *value = pyvalue_of(x);
+    if (!value || x->nd != 0 || storage_of(x)->device != NT_CUDA || storage_of(x)->dtype > NT_FLOAT32 || !scalar_of(value, &v)) return false;
     t = x;
     scalar.s = constant(v);
     return true;
@@ -326,9 +325,8 @@ static PyObject *pow_forward(PyTypeObject *cls, PyObject *const *in) {
   nt_scalar e;
   if (is_tensor(in[1])) {
     TensorObj *t = T_(in[1]);
-    if (Py_TYPE(in[1]) != G.tensor_type || !t->pyvalue || t->nd != 0 || !is_storage(t->storage) ||
-        storage_of(t)->dtype > NT_FLOAT32 || !scalar_of(t->pyvalue, &e))
-      return nullptr;
+    PyObject *value = Py_TYPE(in[1]) == G.tensor_type ? pyvalue_of(t) : nullptr;
+    if (!value || t->nd != 0 || storage_of(t)->dtype > NT_FLOAT32 || !scalar_of(value, &e)) return nullptr;
     exponent = Ref(own(in[1]));
   } else {
     if (!scalar_of(in[1], &e)) return nullptr;

@@ -94,3 +94,27 @@ def test_an_axis_beyond_64_bits_is_an_index_error(nt, op, axis):
     x = nt.Tensor.from_numpy(np.ones((2, 3), np.float32), "cuda")
     with pytest.raises(IndexError):
         getattr(x, op)(axis=axis)
+
+
+@pytest.mark.parametrize("made_of", [3, 3.0, True], ids=str)
+def test_a_scalar_written_in_place_is_not_its_first_value(nt, made_of):
+    """A tensor made of a Python number takes part with that number only until it is written to, under whatever name."""
+    x = nt.Tensor.from_numpy(np.array([1.0, 2.0], np.float32), "cuda", requires_grad=True)
+    for write in ("add", "alias", "upload"):
+        t = nt.Tensor(made_of, device="cuda")
+        assert np.array_equal((x * t).numpy(), [made_of, 2 * made_of]) and np.array_equal((x ** t).numpy(), [1, 2 ** made_of])
+        if made_of is True:
+            continue
+        with nt.no_grad():
+            if write == "add":
+                nt.add(t, 2, out=t)
+            elif write == "alias":
+                t._alias().__iadd__(2)
+            else:
+                new = np.array(t.numpy() + 2, t.numpy().dtype)
+                t.storage.upload(new.ctypes.data, new.nbytes)
+        y = x * t
+        assert np.array_equal(y.numpy(), [5, 10]) and np.array_equal((x ** t).numpy(), [1, 32]) and np.array_equal((t - x).numpy(), [4, 3])
+        x.zero_grad()
+        y.sum().backward()
+        assert np.array_equal(x.grad.numpy(), [5, 5])
