@@ -972,7 +972,7 @@ int nt_sgd_update_many(const nt_view *params, const nt_view *grads, int32_t coun
     fused_checks(chk, 2, "sgd_update");
   }
   SgdBatch batch{};
-  nt_storage *of[SgdBatch::MAX];
+  nt_storage *of[SgdBatch::MAX], *grad_of[SgdBatch::MAX];
   auto flush = [&] {
     if (!batch.count) return;
     launch(sgd_batch, unsigned(batch.first[batch.count]), 256, 0, SgdF{lr, grad_scale, grad_scale != 1.0f}, batch);
@@ -988,15 +988,18 @@ int nt_sgd_update_many(const nt_view *params, const nt_view *grads, int32_t coun
   for (int32_t i = 0; i < count; ++i) {
     const nt_view *p = params + i, *g = grads + i;
     const int64_t n = view_numel(*p);
-    bool repeated = false; // a storage that is already in the batch: its update must see the one before
-    for (int k = 0; k < batch.count; ++k) repeated = repeated || of[k] == p->storage;
-    if (repeated) flush();
+    // The updates happen in the order of the list where they meet: one that writes what the batch writes, reads what it writes
+    // (a gradient that is another parameter) or writes what it reads comes behind it.
+    bool meets = false;
+    for (int k = 0; k < batch.count; ++k) meets = meets || of[k] == p->storage || of[k] == g->storage || grad_of[k] == p->storage;
+    if (meets) flush();
     if (n == 0 || n > SgdBatch::LARGE || !row_major(p) || !row_major(g)) {
       sgd_one(p, g, lr, grad_scale);
       continue;
     }
     const int k = batch.count++;
     of[k] = p->storage;
+    grad_of[k] = g->storage;
     batch.p[k] = static_cast<float *>(p->storage->ptr()) + p->offset;
     batch.g[k] = static_cast<const float *>(g->storage->ptr()) + g->offset;
     batch.n[k] = int32_t(n);

@@ -49,3 +49,21 @@ def test_many_updates_in_one_call(nt, scale):
     for p, q in zip(many, single):
         assert np.array_equal(bits(p.numpy()), bits(q.numpy())) and p.version == q.version
     assert np.array_equal(bits(base_m.numpy()), bits(base_s.numpy()))
+
+
+@pytest.mark.parametrize("sizes", [(7, 7, 7), (5000, 5000, 5000), (1 << 21, 1 << 21, 1 << 21)], ids=str)
+@pytest.mark.parametrize("order", [(0, 1, 2), (1, 0, 2), (2, 1, 0)], ids=str)
+def test_gradients_that_are_parameters(nt, sizes, order):
+    """Updates happen one after the other where a gradient is another parameter's storage: p1's gradient is p0, p2's is p1."""
+    import nanotorch_b200.nn as nn
+
+    n = sizes[0]
+    p = [nt.Tensor.from_numpy(np.full(n, 8.0 * (i + 1), np.float32), "cuda", requires_grad=True) for i in range(3)]
+    p[0]._grad = nt.Tensor.from_numpy(np.full(n, 2.0, np.float32), "cuda")
+    p[1]._grad, p[2]._grad = (nt.Tensor._new_view(p[i].storage, (n,), (1,), 0) for i in (0, 1))
+    want = [8.0, 16.0, 24.0]
+    for i in order:
+        want[i] -= 0.5 * (2.0 if i == 0 else want[i - 1])
+    nn.GradientDescent([p[i] for i in order], lr=0.5).step()
+    for got, w in zip(p, want):
+        assert (got.numpy() == w).all()
