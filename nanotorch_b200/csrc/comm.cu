@@ -233,11 +233,15 @@ int nt_comm_allreduce_sum(nt_storage *s) {
   Nccl &n = nccl();
   if (!n.comm) fail_runtime("nt_comm_allreduce_sum: communicator not initialised.");
   if (s->device != NT_CUDA || s->dtype != NT_FLOAT32) fail_invalid("nt_comm_allreduce_sum: Float32 Cuda storage only.");
+  const bool written_now = !s->block; // a value without memory is written on the compute stream: before the streams are joined
+  void *data = s->ptr();
   if (!n.in_group) {
     poll_async_error();
     comm_after_compute(); // the collective may start once everything enqueued on the compute stream so far has run
+  } else if (written_now) {
+    comm_after_compute(); // the group was opened before
   }
-  nccl_check(n.AllReduce(s->ptr(), s->ptr(), size_t(s->n), ncclFloat32, ncclSum, n.comm, comm_stream()), "ncclAllReduce");
+  nccl_check(n.AllReduce(data, data, size_t(s->n), ncclFloat32, ncclSum, n.comm, comm_stream()), "ncclAllReduce");
   storage_touch(s);
   count_launch();
   NT_API_END
@@ -248,6 +252,8 @@ int nt_comm_sgd_update(const nt_view *param, const nt_view *grad, float lr, floa
   // far on the communication stream (which itself is behind the kernels that produced the gradient)
   Nccl &n = nccl();
   try {
+    for (const nt_view *v : {param, grad})
+      if (v && v->storage) v->storage->ptr(); // see nt_comm_allreduce_sum
     comm_after_compute();
     NT_CUDA_CHECK(cudaEventRecord(n.exchanged, comm_stream()));
     NT_CUDA_CHECK(cudaStreamWaitEvent(update_stream(), n.exchanged, 0));

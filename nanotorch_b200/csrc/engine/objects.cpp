@@ -790,8 +790,13 @@ static PyObject *tensor_backward(PyObject *self, PyObject *) {
     seed = Ref(make_view(Py_TYPE(self), storage.p, sh.p, Py_None, Py_None));
     if (!seed) return nullptr;
   }
+  if (!t->grad_fn) { // a leaf's gradient is in memory, like those that leave a sweep
+    const int rc = nt_storage_settle(storage_of(T_(seed.p)));
+    if (rc) return raise_status(rc);
+    Py_XSETREF(t->grad, seed.release());
+    Py_RETURN_NONE;
+  }
   Py_XSETREF(t->grad, seed.release());
-  if (!t->grad_fn) Py_RETURN_NONE;
   return run_backward(t);
 }
 

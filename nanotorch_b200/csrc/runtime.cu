@@ -916,10 +916,11 @@ int nt_storage_upload_async(nt_storage *dst, const void *host_src, int64_t nbyte
   if (nbytes < 0 || size_t(nbytes) > size_t(dst->n) * dtype_itemsize(dst->dtype))
     fail_runtime("nt_storage_upload_async: byte count exceeds the storage.");
   cudaStream_t st = stream();
+  void *to = dst->ptr(); // a value without memory is written on the compute stream, before the copy
   Runtime &r = rt();
   NT_CUDA_CHECK(cudaEventRecord(r.copy_gate, st));
   NT_CUDA_CHECK(cudaStreamWaitEvent(r.copy, r.copy_gate, 0));
-  if (nbytes) NT_CUDA_CHECK(cudaMemcpyAsync(dst->ptr(), host_src, size_t(nbytes), cudaMemcpyHostToDevice, r.copy));
+  if (nbytes) NT_CUDA_CHECK(cudaMemcpyAsync(to, host_src, size_t(nbytes), cudaMemcpyHostToDevice, r.copy));
   storage_touch(dst);
   NT_API_END
 }

@@ -118,3 +118,26 @@ def test_a_scalar_written_in_place_is_not_its_first_value(nt, made_of):
         x.zero_grad()
         y.sum().backward()
         assert np.array_equal(x.grad.numpy(), [5, 5])
+
+
+def test_a_constant_is_written_before_another_stream_uses_it(nt):
+    """An upload on the copy stream into a value that had no memory yet comes after the value's own fill, however busy the
+    compute stream is; a leaf's own seed is in memory."""
+    import ctypes
+
+    big = nt.Tensor.from_numpy(np.ones((4096, 4096), np.float32), "cuda")
+    host = np.array([7.0], np.float32)
+    with nt.no_grad():
+        big @ big
+        nt.cuda.sync()
+        for _ in range(5):
+            s = nt._C.constant(3.0, nt.float32)
+            for _ in range(3):
+                big @ big
+            nt._C._check(nt._C._lib.nt_storage_upload_async(ctypes.c_void_p(s._h), ctypes.c_void_p(host.ctypes.data), ctypes.c_int64(4)))
+            nt._C._check(nt._C._lib.nt_upload_fence())
+            assert nt.Tensor._new_contiguous(s, ()).numpy() == 7.0
+    leaf = nt.Tensor.from_numpy(np.array([2.0], np.float32), "cuda", requires_grad=True)
+    used = nt.cuda.memory_stats()["bytes_in_use"]
+    leaf.backward()
+    assert nt.cuda.memory_stats()["bytes_in_use"] > used and leaf.grad.numpy() == 1.0
