@@ -125,7 +125,10 @@ void *nt_storage_data(nt_storage *s);                 /* host or device pointer 
 int nt_storage_clone(const nt_storage *s, nt_storage **out);            /* Storage::clone */
 int nt_storage_to(nt_storage *s, int device, nt_storage **out);         /* Storage::to; same device -> same storage, retained */
 int nt_storage_cast(nt_storage *s, int dtype, nt_storage **out);        /* Storage::cast; on device, no host round trip */
-int nt_storage_upload(nt_storage *dst, const void *host_src, int64_t nbytes);   /* H2D (or memcpy for CPU storages) */
+/* H2D (or memcpy for CPU storages).  host_src is free again when the call returns; small copies may still be on their way
+ * on the library stream then, unless the storage's address has been asked for: nt_storage_data waits for them, and
+ * later uploads to that storage wait themselves. */
+int nt_storage_upload(nt_storage *dst, const void *host_src, int64_t nbytes);
 int nt_storage_download(const nt_storage *src, void *host_dst, int64_t nbytes); /* D2H, synchronises */
 /* Overlapped input feed (no counterpart: the reference's Storage::to is a blocking cudaMemcpy).
  * The copy runs on a dedicated stream, ordered after everything enqueued on the compute stream so

@@ -160,6 +160,10 @@ struct nt_storage {
   nt_scalar scalar{};
   nt_storage *prev = nullptr, *next = nullptr; // constants without memory, see constants_materialize_all
 
+  // An upload that does not wait for its copy, and an address that has left the library: what reads through the address, on
+  // whatever stream, finds the uploaded values (nt_storage_data, nt_storage_upload).
+  bool uploading = false, exposed = false;
+
   // value * (n elements of `src` from src_offset on), another storage's product with a known factor: the gradient of a
   // squared error, inside a backward sweep (see nt_scaled).  Kernels that can take the factor read `src` itself.  Once it is
   // in memory of its own it no longer holds on to `src`.

@@ -617,8 +617,8 @@ static nt_storage *full_impl(int64_t n, const nt_scalar *value, int dtype, int d
 }
 
 // A small upload goes through a pinned slot of the library's own, so that the call need not wait for the copy before the
-// caller's buffer is free again (a sample of 3 KB: the wait cost more than the copy).  Eight slots of 256 KB, each reused
-// once its copy is done.  false: too large, or inside a capture.
+// caller's buffer is free again (a sample of 3 KB: the wait cost more than the copy).  Eight slots of 256 KB for the life of
+// the process, each reused once its copy is done.  false: too large, or inside a capture.
 static bool upload_staged(void *dst, const void *src, size_t nbytes, cudaStream_t st) {
   constexpr size_t SLOT = size_t(256) << 10;
   constexpr int SLOTS = 8;
@@ -975,6 +975,9 @@ uint64_t nt_storage_version(const nt_storage *s) { return s->version; }
 void *nt_storage_data(nt_storage *s) {
   try {
     void *p = s->ptr();
+    if (s->uploading && !is_capturing()) NT_CUDA_CHECK(cudaStreamSynchronize(stream()));
+    s->uploading = false;
+    s->exposed = true;
     s->constant = false; // the caller may write through the pointer
     drop_side_sums(s);
     return p;
@@ -1047,7 +1050,9 @@ int nt_storage_upload(nt_storage *dst, const void *host_src, int64_t nbytes) {
     std::memcpy(dst->ptr(), host_src, size_t(nbytes));
   } else {
     cudaStream_t st = stream();
-    if (!upload_staged(dst->ptr(), host_src, size_t(nbytes), st)) {
+    if (!dst->exposed && upload_staged(dst->ptr(), host_src, size_t(nbytes), st)) {
+      dst->uploading = true;
+    } else {
       NT_CUDA_CHECK(cudaMemcpyAsync(dst->ptr(), host_src, size_t(nbytes), cudaMemcpyHostToDevice, st));
       NT_CUDA_CHECK(cudaStreamSynchronize(st));
     }

@@ -141,3 +141,33 @@ def test_a_constant_is_written_before_another_stream_uses_it(nt):
     used = nt.cuda.memory_stats()["bytes_in_use"]
     leaf.backward()
     assert nt.cuda.memory_stats()["bytes_in_use"] > used and leaf.grad.numpy() == 1.0
+
+
+def test_an_uploads_address_is_handed_out_behind_its_copy(nt):
+    """A reader on another stream that goes through the storage's address finds the uploaded values while the library's own
+    stream is still busy: before the first look at the address, and for uploads after it."""
+    torch = pytest.importorskip("torch")
+
+    class Seen:
+        def __init__(self, t):
+            self.__cuda_array_interface__ = {"shape": t.shape, "typestr": "<f4", "version": 2, "data": (t.storage.data_ptr, False)}
+
+    big = nt.Tensor.from_numpy(np.ones((4096, 4096), np.float32), "cuda")
+    side = torch.cuda.Stream()
+    nt.Tensor.from_numpy(np.zeros(100, np.float32), "cuda")
+    with nt.no_grad():
+        big @ big
+        nt.cuda.sync()
+        for value in (5.0, 6.0):
+            for _ in range(20):
+                big @ big
+            t = nt.Tensor.from_numpy(np.full(100, value, np.float32), "cuda")
+            with torch.cuda.stream(side):
+                seen = torch.as_tensor(Seen(t), device="cuda")
+                assert (seen.clone().cpu() == value).all()
+            again = np.full(100, -value, np.float32)
+            for _ in range(20):
+                big @ big
+            t.storage.upload(again.ctypes.data, again.nbytes)
+            with torch.cuda.stream(side):
+                assert (seen.clone().cpu() == -value).all()
