@@ -782,6 +782,9 @@ static int *error_flag_ptr() {
 int gemm_tc_take_error() {
   int *flag = g_error_flag;
   if (!flag || !g_flag_dirty.exchange(false)) return 0;
+  // The wait that brought the caller here covered one stream, up to that moment.  A kernel that another thread has launched
+  // since, or that runs on a side stream, may still set the flag: it is read again behind the next wait.
+  if (!streams_idle()) gemm_tc_mark_flag();
   int host = 0;
   if (cudaMemcpy(&host, flag, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return -1;
   if (host != 0) {

@@ -101,6 +101,7 @@ cudaStream_t comm_stream();  // collectives
 cudaStream_t update_stream(); // the parameter updates that follow the collectives (lowest priority)
 cudaStream_t compute_stream(); // the compute stream itself, whatever redirection is active
 bool stream_redirected();      // stream() is not the compute stream
+bool streams_idle();           // nothing is enqueued on the compute, communication and update streams
 // While one of these lives, stream() returns `to`: kernels launched by the ordinary entry points go to
 // that stream instead (used to run a parameter update on the communication stream, right behind the
 // collective that produced its gradient).  Single-threaded use, like the rest of the library.

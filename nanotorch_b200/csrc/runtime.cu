@@ -122,6 +122,13 @@ cudaStream_t compute_stream() {
   return r.compute;
 }
 bool stream_redirected() { return rt().redirect != nullptr; }
+bool streams_idle() {
+  Runtime &r = rt();
+  std::lock_guard<std::mutex> lk(r.mu);
+  for (cudaStream_t s : {r.compute, r.comm, r.update})
+    if (s && cudaStreamQuery(s) != cudaSuccess) return false;
+  return true;
+}
 StreamRedirect::StreamRedirect(cudaStream_t to) {
   Runtime &r = rt();
   std::lock_guard<std::mutex> lk(r.mu);

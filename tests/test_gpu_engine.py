@@ -171,3 +171,39 @@ def test_an_uploads_address_is_handed_out_behind_its_copy(nt):
             t.storage.upload(again.ctypes.data, again.nbytes)
             with torch.cuda.stream(side):
                 assert (seen.clone().cpu() == -value).all()
+
+
+def test_a_wait_that_ran_out_beside_another_threads_sync_is_reported(nt):
+    """A kernel launched while another thread is inside a synchronising call is not covered by that call's look at the error
+    flag: whichever call comes behind the kernel reports that its wait ran out."""
+    import threading
+    import time
+
+    big = nt.Tensor.from_numpy(np.ones((4096, 4096), np.float32), "cuda")
+    reports = []
+
+    def sync():
+        try:
+            nt.cuda.sync()
+        except RuntimeError as e:
+            reports.append(str(e))
+
+    before = nt._C.get_wait_limit_clocks()
+    with nt.no_grad():
+        big @ big
+        nt.cuda.sync()
+        for _ in range(60):
+            big @ big
+        thread = threading.Thread(target=sync)
+        thread.start()
+        time.sleep(0.005)
+        nt._C.set_wait_limit_clocks(500_000_000)  # a quarter of a second
+        try:
+            nt._C.wait_probe()
+        finally:
+            nt._C.set_wait_limit_clocks(before)
+        thread.join()
+        sync()
+    assert len(reports) == 1 and "code 5" in reports[0]
+    sync()
+    assert len(reports) == 1
