@@ -179,7 +179,8 @@ struct nt_storage {
 
   bool scaled() const { return src != nullptr; }
   void *ptr() const {
-    if (!block && (constant || src)) materialize();
+    if (void *p = __atomic_load_n(&block, __ATOMIC_ACQUIRE)) return p;
+    if (constant || src) materialize();
     return block;
   }
   void materialize() const;

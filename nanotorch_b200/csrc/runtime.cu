@@ -590,9 +590,9 @@ static int grid_for(int64_t n, int block) {
   return int(g < 1 ? 1 : (g > cap ? cap : g));
 }
 
-template <class T> static void fill_device(nt_storage *s, T value) {
-  if (s->n == 0) return;
-  launch(fill_kernel<T>, grid_for(s->n, 256), 256, 0, static_cast<T *>(s->ptr()), s->n, value);
+template <class T> static void fill_device(T *p, int64_t n, T value) {
+  if (n == 0) return;
+  launch(fill_kernel<T>, grid_for(n, 256), 256, 0, p, n, value);
   check_launch("fill");
 }
 
@@ -606,15 +606,16 @@ template <class T> static T scalar_as(const nt_scalar *v) {
 }
 
 static void fill_constant(nt_storage *s) {
-  s->block = device_alloc(size_t(dtype_itemsize(s->dtype)), &s->rounded);
-  dispatch_all(s->dtype, [&]<class T>() { fill_device<T>(s, scalar_as<T>(&s->scalar)); });
+  void *p = device_alloc(size_t(dtype_itemsize(s->dtype)), &s->rounded);
+  dispatch_all(s->dtype, [&]<class T>() { fill_device(static_cast<T *>(p), 1, scalar_as<T>(&s->scalar)); });
+  __atomic_store_n(&s->block, p, __ATOMIC_RELEASE); // other threads may use it: their kernels come behind the fill
 }
 static nt_storage *full_impl(int64_t n, const nt_scalar *value, int dtype, int device) {
   StorageRef out(storage_new(n, dtype, device));
   dispatch_all(dtype, [&]<class T>() {
     T v = scalar_as<T>(value);
     if (device == NT_CUDA) {
-      fill_device<T>(out.s, v);
+      fill_device(static_cast<T *>(out->ptr()), n, v);
     } else {
       T *p = static_cast<T *>(out->ptr());
       for (int64_t i = 0; i < n; ++i) p[i] = v;
@@ -674,26 +675,37 @@ static nt_storage *to_device_impl(nt_storage *s, int device) {
 }
 
 void constants_materialize_all() {
-  for (;;) {
-    nt_storage *s;
-    {
-      std::lock_guard<std::mutex> lk(g_constants_mu);
-      s = g_constants;
+  std::vector<StorageRef> all; // those that no other thread is about to delete
+  {
+    std::lock_guard<std::mutex> lk(g_constants_mu);
+    for (nt_storage *c = g_constants; c; c = c->next) {
+      int64_t refs = c->refs.load();
+      while (refs > 0 && !c->refs.compare_exchange_weak(refs, refs + 1)) {
+      }
+      if (refs > 0) all.emplace_back(c);
     }
-    if (!s) return;
-    s->materialize();
   }
+  for (StorageRef &c : all) c->ptr();
 }
 
 } // namespace ntb
 
 void nt_storage::materialize() const {
-  nt_storage *s = const_cast<nt_storage *>(this);
+  // One thread at a time: a constant may be asked for by its user and by the start of a capture.  Recursive for a factor of
+  // something that has no memory itself; the source is let go of outside (its planes have a lock of their own).
+  static std::recursive_mutex mu;
+  nt_storage *s = const_cast<nt_storage *>(this), *source = nullptr;
+  struct Release {
+    nt_storage *&s;
+    ~Release() { ntb::storage_release(s); }
+  } release{source};
+  std::lock_guard<std::recursive_mutex> lk(mu);
+  if (s->block) return;
   if (s->src) {
     void *p = ntb::device_alloc(size_t(s->n) * sizeof(float), &s->rounded);
     ntb::scale_into(static_cast<float *>(p), static_cast<const float *>(s->src->ptr()) + s->src_offset, s->n, s->value);
     s->block = p;
-    ntb::storage_release(s->src); // a plain storage from here on; the source's memory is reused behind the kernel just launched
+    source = s->src; // a plain storage from here on; the source's memory is reused behind the kernel just launched
     s->src = nullptr;
     return;
   }

@@ -207,3 +207,34 @@ def test_a_wait_that_ran_out_beside_another_threads_sync_is_reported(nt):
     assert len(reports) == 1 and "code 5" in reports[0]
     sync()
     assert len(reports) == 1
+
+
+def test_captures_begin_while_another_thread_makes_constants(nt):
+    """The start of a capture gives the constants there are their memory, while another thread makes and drops some."""
+    import threading
+
+    x = nt.Tensor.from_numpy(np.ones(8, np.float32), "cuda")
+    stop = False
+
+    def churn():
+        held = []
+        while not stop:
+            held.append(nt._C.constant(2.0, nt.float32))
+            if len(held) > 5:
+                held.clear()
+
+    thread = threading.Thread(target=churn)
+    thread.start()
+    try:
+        mine = nt._C.constant(3.0, nt.float32)
+        for _ in range(100):
+            graph = nt._C.Graph()
+            with graph.capture():
+                y = x * 2.0
+            graph.replay()
+            assert (y.numpy() == 2.0).all()
+            graph.close()
+    finally:
+        stop = True
+        thread.join()
+    assert nt.Tensor._new_contiguous(mine, ()).numpy() == 3.0
