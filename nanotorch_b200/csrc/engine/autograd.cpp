@@ -49,7 +49,7 @@ static bool version_of(PyObject *tensor, uint64_t *out) {
   return !(*out == uint64_t(-1) && PyErr_Occurred());
 }
 static PyObject *function_save(PyObject *self, PyObject *const *args, Py_ssize_t n) {
-  if (!G.grad_enabled) Py_RETURN_NONE;
+  if (!grad_enabled()) Py_RETURN_NONE;
   FunctionObj *f = F_(self);
   PyObject *t = PyTuple_New(n);
   uint64_t *v = static_cast<uint64_t *>(PyMem_Malloc(sizeof(uint64_t) * size_t(n ? n : 1)));
@@ -149,7 +149,7 @@ PyObject *apply(PyTypeObject *cls, PyObject *const *args, Py_ssize_t n, PyObject
   if (!method) return nullptr;
   Ref out(PyObject_Vectorcall(method.p, args, size_t(n), kwnames));
   if (!out) return nullptr;
-  if (!G.grad_enabled) return out.release();
+  if (!grad_enabled()) return out.release();
   bool same = false;
   for (Py_ssize_t i = 0; i < n + nkw; ++i) same = same || args[i] == out.p;
   if (same) {
@@ -216,10 +216,11 @@ static Ref inputs_of(PyObject *fn) {
   return Ref(PyObject_GetAttrString(fn, "inputs"));
 }
 
+// This thread's own: what others record meanwhile is recorded.
+thread_local int t_sweeps = 0;
 struct NoGrad {
-  bool prev = G.grad_enabled;
-  NoGrad() { G.grad_enabled = false; }
-  ~NoGrad() { G.grad_enabled = prev; }
+  NoGrad() { ++t_sweeps; }
+  ~NoGrad() { --t_sweeps; }
 };
 
 // What leaves the sweep, and what Python code may come to see or change the source of, is in memory: see nt_scaled.
@@ -228,21 +229,27 @@ static bool is_scaled(PyObject *g) {
 }
 static bool settle(PyObject *g) {
   if (!g || !is_tensor(g) || !T_(g)->storage || !is_storage(T_(g)->storage)) return true;
-  const int rc = nt_storage_settle(storage_of(T_(g)));
+  const int rc = nogil([&] { return nt_storage_settle(storage_of(T_(g))); });
   if (rc) raise_status(rc);
   return rc == 0;
 }
 static bool accumulate(TensorObj *x, PyObject *gx) {
   if (!x->grad_fn && !settle(gx)) return false;
-  if (!x->grad) {
-    x->grad = own(gx);
-    return true;
+  for (;;) {
+    if (!x->grad) {
+      x->grad = own(gx);
+      return true;
+    }
+    Ref had(own(x->grad));
+    PyObject *sum = reinterpret_cast<PyObject *>(add_tensors(had.p, gx));
+    if (!sum && !PyErr_Occurred()) sum = PyNumber_Add(had.p, gx);
+    if (!sum) return false;
+    if (x->grad == had.p) {
+      Py_SETREF(x->grad, sum);
+      return true;
+    }
+    Py_DECREF(sum); // another thread's backward has added to it meanwhile
   }
-  PyObject *sum = reinterpret_cast<PyObject *>(add_tensors(x->grad, gx));
-  if (!sum && !PyErr_Occurred()) sum = PyNumber_Add(x->grad, gx);
-  if (!sum) return false;
-  Py_SETREF(x->grad, sum);
-  return true;
 }
 
 static PyObject *sweep(std::vector<Ref> &order, std::vector<Ref>::reverse_iterator &it, std::unordered_map<PyObject *, int> &pending);
@@ -378,7 +385,7 @@ static PyObject *m_run_backward(PyObject *, PyObject *root) {
   }
   return run_backward(T_(root));
 }
-static PyObject *m_is_grad_enabled(PyObject *, PyObject *) { return PyBool_FromLong(G.grad_enabled); }
+static PyObject *m_is_grad_enabled(PyObject *, PyObject *) { return PyBool_FromLong(grad_enabled()); }
 static PyObject *m_set_grad_enabled(PyObject *, PyObject *on) { // returns the previous setting
   const int v = PyObject_IsTrue(on);
   if (v < 0) return nullptr;
@@ -398,6 +405,7 @@ static PyObject *m_sgd_update(PyObject *, PyObject *const *args, Py_ssize_t n) {
   Ref seq(PySequence_Fast(args[0], "sgd_update: a sequence of tensors"));
   if (!seq) return nullptr;
   std::vector<nt_view> ps, gs;
+  std::vector<Ref> grads; // held while the lock is not
   for (Py_ssize_t i = 0; i < PySequence_Fast_GET_SIZE(seq.p); ++i) {
     PyObject *o = PySequence_Fast_GET_ITEM(seq.p, i);
     if (!is_tensor(o)) Py_RETURN_FALSE;
@@ -406,8 +414,9 @@ static PyObject *m_sgd_update(PyObject *, PyObject *const *args, Py_ssize_t n) {
     if (!is_fast(o) || !p->grad || !is_fast(p->grad) || !same_shape(p, T_(p->grad))) Py_RETURN_FALSE;
     ps.push_back(view_of(p));
     gs.push_back(view_of(T_(p->grad)));
+    grads.emplace_back(own(p->grad));
   }
-  const int rc = nt_sgd_update_many(ps.data(), gs.data(), int32_t(ps.size()), float(lr), float(scale));
+  const int rc = nogil([&] { return nt_sgd_update_many(ps.data(), gs.data(), int32_t(ps.size()), float(lr), float(scale)); });
   if (rc) return raise_status(rc);
   Py_RETURN_TRUE;
 }

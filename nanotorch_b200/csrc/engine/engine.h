@@ -11,6 +11,7 @@
 #include <Python.h>
 
 #include <initializer_list>
+#include <mutex>
 
 #include "../nt_core.cuh"
 
@@ -72,6 +73,8 @@ struct Globals {
   bool grad_enabled = true;
 };
 extern Globals G;
+extern thread_local int t_sweeps;         // this thread is inside a backward sweep: its gradients are values, not graph nodes
+inline bool grad_enabled() { return G.grad_enabled && !t_sweeps; }
 
 extern PyTypeObject StorageBase_Type, View_Type, TensorBase_Type, FunctionBase_Type;
 
@@ -84,6 +87,23 @@ struct PyErr {};                        // thrown after a Python exception has b
 bool named_args(PyObject *const *args, Py_ssize_t n, PyObject *kwnames, std::initializer_list<const char *> names, PyObject **out);
 using FastKw = PyObject *(*)(PyObject *, PyObject *const *, Py_ssize_t, PyObject *);
 inline PyCFunction fast_kw(FastKw f) { return reinterpret_cast<PyCFunction>(reinterpret_cast<void *>(f)); }
+
+// A call of the library without the interpreter lock: a launch waits while the stream's queue is full, and other Python
+// threads (one that prepares the next batch, a heartbeat) go on meanwhile.
+template <class F> int unlocked(F &&call) {
+  PyThreadState *state = PyEval_SaveThread();
+  const int rc = call();
+  PyEval_RestoreThread(state);
+  return rc;
+}
+// One that only enqueues work: one thread at a time, as the interpreter lock would have it.
+inline std::mutex g_launching;
+template <class F> int nogil(F &&call) {
+  return unlocked([&] {
+    std::lock_guard<std::mutex> lk(g_launching);
+    return call();
+  });
+}
 
 // ---- references
 struct Ref {

@@ -106,7 +106,7 @@ static PyObject *storage_allocate(PyObject *, PyObject *const *args, Py_ssize_t 
 }
 static PyObject *storage_clone(PyObject *self, PyObject *) {
   nt_storage *s = nullptr;
-  const int rc = nt_storage_clone(handle(self), &s);
+  const int rc = nogil([&] { return nt_storage_clone(handle(self), &s); });
   return rc ? raise_status(rc) : wrap_storage(s);
 }
 static PyObject *storage_to(PyObject *self, PyObject *const *args, Py_ssize_t n, PyObject *kwnames) {
@@ -116,9 +116,7 @@ static PyObject *storage_to(PyObject *self, PyObject *const *args, Py_ssize_t n,
   if (dev < 0) return nullptr;
   if (dev == handle(self)->device) return own(self);
   nt_storage *s = nullptr;
-  int rc;
-  Py_BEGIN_ALLOW_THREADS rc = nt_storage_to(handle(self), dev, &s);
-  Py_END_ALLOW_THREADS
+  const int rc = unlocked([&] { return nt_storage_to(handle(self), dev, &s); });
   return rc ? raise_status(rc) : wrap_storage(s);
 }
 static PyObject *storage_cast(PyObject *self, PyObject *const *args, Py_ssize_t n, PyObject *kwnames) {
@@ -128,7 +126,7 @@ static PyObject *storage_cast(PyObject *self, PyObject *const *args, Py_ssize_t 
   if (dt < 0) return nullptr;
   if (dt == handle(self)->dtype) return own(self);
   nt_storage *s = nullptr;
-  const int rc = nt_storage_cast(handle(self), dt, &s);
+  const int rc = nogil([&] { return nt_storage_cast(handle(self), dt, &s); });
   return rc ? raise_status(rc) : wrap_storage(s);
 }
 static bool pointer_and_bytes(PyObject *const *args, Py_ssize_t n, PyObject *kwnames, void **p, int64_t *nbytes) {
@@ -143,9 +141,7 @@ static PyObject *storage_upload(PyObject *self, PyObject *const *args, Py_ssize_
   void *p;
   int64_t nbytes;
   if (!pointer_and_bytes(args, n, kwnames, &p, &nbytes)) return nullptr;
-  int rc;
-  Py_BEGIN_ALLOW_THREADS rc = nt_storage_upload(handle(self), p, nbytes);
-  Py_END_ALLOW_THREADS
+  const int rc = unlocked([&] { return nt_storage_upload(handle(self), p, nbytes); });
   if (rc) return raise_status(rc);
   Py_RETURN_NONE;
 }
@@ -153,9 +149,7 @@ static PyObject *storage_download(PyObject *self, PyObject *const *args, Py_ssiz
   void *p;
   int64_t nbytes;
   if (!pointer_and_bytes(args, n, kwnames, &p, &nbytes)) return nullptr;
-  int rc;
-  Py_BEGIN_ALLOW_THREADS rc = nt_storage_download(handle(self), p, nbytes);
-  Py_END_ALLOW_THREADS
+  const int rc = unlocked([&] { return nt_storage_download(handle(self), p, nbytes); });
   if (rc) return raise_status(rc);
   Py_RETURN_NONE;
 }

@@ -25,7 +25,7 @@ template <Fn1 FN, const char *NAME = x_name> static PyObject *c_unary(PyObject *
   PyObject *a;
   if (!named_args(args, n, kwnames, {NAME}, &a) || !view_arg(a, &x)) return nullptr;
   nt_storage *out = nullptr;
-  const int rc = FN(&x, &out);
+  const int rc = nogil([&] { return FN(&x, &out); });
   return rc ? raise_status(rc) : wrap_storage(out);
 }
 template <Fn2 FN> static PyObject *c_binary(PyObject *, PyObject *const *args, Py_ssize_t n, PyObject *kwnames) {
@@ -33,7 +33,7 @@ template <Fn2 FN> static PyObject *c_binary(PyObject *, PyObject *const *args, P
   PyObject *a[2];
   if (!named_args(args, n, kwnames, {"x1", "x2"}, a) || !view_arg(a[0], &x) || !view_arg(a[1], &y)) return nullptr;
   nt_storage *out = nullptr;
-  const int rc = FN(&x, &y, &out);
+  const int rc = nogil([&] { return FN(&x, &y, &out); });
   return rc ? raise_status(rc) : wrap_storage(out);
 }
 static constexpr char w_name[] = "w", bias_name[] = "bias", g_name[] = "g", x1_name[] = "x1", x2_name[] = "x2";
@@ -42,14 +42,14 @@ template <Fn3 FN, const char *N0, const char *N1, const char *N2> static PyObjec
   PyObject *a[3];
   if (!named_args(args, n, kwnames, {N0, N1, N2}, a) || !view_arg(a[0], &x) || !view_arg(a[1], &y) || !view_arg(a[2], &z)) return nullptr;
   nt_storage *out = nullptr;
-  const int rc = FN(&x, &y, &z, &out);
+  const int rc = nogil([&] { return FN(&x, &y, &z, &out); });
   return rc ? raise_status(rc) : wrap_storage(out);
 }
 template <FnIn FN> static PyObject *c_inplace(PyObject *, PyObject *const *args, Py_ssize_t n, PyObject *kwnames) {
   nt_view x, y;
   PyObject *a[2];
   if (!named_args(args, n, kwnames, {"x1", "x2"}, a) || !view_arg(a[0], &x) || !view_arg(a[1], &y)) return nullptr;
-  const int rc = FN(&x, &y);
+  const int rc = nogil([&] { return FN(&x, &y); });
   if (rc) return raise_status(rc);
   Py_RETURN_NONE;
 }
@@ -62,7 +62,7 @@ template <FnBoth FN> static PyObject *c_both(PyObject *, PyObject *const *args, 
   PyObject *a[3];
   if (!named_args(args, n, kwnames, {"g", "x1", "x2"}, a) || !view_arg(a[0], &g) || !view_arg(a[1], &x) || !view_arg(a[2], &y)) return nullptr;
   nt_storage *s1 = nullptr, *s2 = nullptr;
-  const int rc = FN(&g, &x, &y, &s1, &s2);
+  const int rc = nogil([&] { return FN(&g, &x, &y, &s1, &s2); });
   if (rc) return raise_status(rc);
   if (!s1) Py_RETURN_NONE;
   return pair_of(s1, s2);
@@ -74,7 +74,7 @@ static PyObject *c_matmul_pair(PyObject *, PyObject *const *args, Py_ssize_t n, 
   for (int i = 0; i < 4; ++i)
     if (!view_arg(a[i], &v[i])) return nullptr;
   nt_storage *s1 = nullptr, *s2 = nullptr;
-  const int rc = nt_matmul_pair(&v[0], &v[1], &v[2], &v[3], &s1, &s2);
+  const int rc = nogil([&] { return nt_matmul_pair(&v[0], &v[1], &v[2], &v[3], &s1, &s2); });
   return rc ? raise_status(rc) : pair_of(s1, s2);
 }
 static bool axes_arg(PyObject *o, std::vector<int64_t> *out) {
@@ -95,7 +95,7 @@ template <FnAxes FN> static PyObject *c_reduce(PyObject *, PyObject *const *args
   PyObject *a[2];
   if (!named_args(args, n, kwnames, {"x", "axis"}, a) || !view_arg(a[0], &x) || !axes_arg(a[1], &ax)) return nullptr;
   nt_storage *out = nullptr;
-  const int rc = FN(&x, ax.data(), int32_t(ax.size()), &out);
+  const int rc = nogil([&] { return FN(&x, ax.data(), int32_t(ax.size()), &out); });
   return rc ? raise_status(rc) : wrap_storage(out);
 }
 static PyObject *c_sum(PyObject *, PyObject *const *args, Py_ssize_t n, PyObject *kwnames) {
@@ -106,7 +106,7 @@ static PyObject *c_sum(PyObject *, PyObject *const *args, Py_ssize_t n, PyObject
   const int dt = parse_dtype(a[2]);
   if (dt < 0) return nullptr;
   nt_storage *out = nullptr;
-  const int rc = nt_sum(&x, ax.data(), int32_t(ax.size()), dt, &out);
+  const int rc = nogil([&] { return nt_sum(&x, ax.data(), int32_t(ax.size()), dt, &out); });
   return rc ? raise_status(rc) : wrap_storage(out);
 }
 
@@ -247,7 +247,7 @@ struct Node {
   Ref holder;
 };
 static bool recording(PyObject *const *in, int n) {
-  if (!G.grad_enabled) return false;
+  if (!grad_enabled()) return false;
   for (int i = 0; i < n; ++i)
     if (is_tensor(in[i]) && requires_grad(T_(in[i]))) return true;
   return false;
@@ -295,7 +295,7 @@ static PyObject *binary_forward(Op op, PyTypeObject *cls, PyObject *const *in) {
   nt_view va, vb;
   if (!broadcast(a.t, b.t, &nd, shape) || !a.view(nd, shape, &va) || !b.view(nd, shape, &vb)) return nullptr;
   nt_storage *s = nullptr;
-  Ref out(fresh(checked(fns[op - OP_ADD](&va, &vb, &s), s), nd, shape));
+  Ref out(fresh(checked(nogil([&] { return fns[op - OP_ADD](&va, &vb, &s); }), s), nd, shape));
   if (recording(in, 2)) {
     FunctionObj *fn = attach(op, cls, out.p, in, 2);
     if (op == OP_MUL || op == OP_DIV) save(fn, out.p, {in[0], in[1]});
@@ -309,7 +309,7 @@ static PyObject *unary_forward(Op op, PyTypeObject *cls, PyObject *const *in) {
   TensorObj *x = T_(in[0]);
   const nt_view v = view_of(x);
   nt_storage *s = nullptr;
-  Ref out(fresh(checked(fns[op - OP_NEG](&v, &s), s), x->nd, x->sh));
+  Ref out(fresh(checked(nogil([&] { return fns[op - OP_NEG](&v, &s); }), s), x->nd, x->sh));
   if (recording(in, 1)) {
     FunctionObj *fn = attach(op, cls, out.p, in, 1);
     if (op == OP_LOG) save(fn, out.p, {in[0]});
@@ -336,7 +336,7 @@ static PyObject *pow_forward(PyTypeObject *cls, PyObject *const *in) {
   e = nt_scalar{2, 0, e.d};
   const nt_view v = view_of(x);
   nt_storage *s = nullptr;
-  Ref out(fresh(checked(nt_pow(&v, &e, &s), s), x->nd, x->sh));
+  Ref out(fresh(checked(nogil([&] { return nt_pow(&v, &e, &s); }), s), x->nd, x->sh));
   if (recording(in, 1) || (is_tensor(in[1]) && recording(in + 1, 1))) {
     FunctionObj *fn = attach(OP_POW, cls, out.p, in, 2);
     save(fn, out.p, {in[0], exponent.p});
@@ -367,7 +367,7 @@ static PyObject *matmul_forward(PyTypeObject *cls, PyObject *const *in) {
   const nt_view va = view_of(a), vb = view_of(b);
   const Reorder reorder(!recording(in, 2));
   nt_storage *s = nullptr;
-  Ref out(fresh(checked(nt_matmul(&va, &vb, &s), s), nd, shape));
+  Ref out(fresh(checked(nogil([&] { return nt_matmul(&va, &vb, &s); }), s), nd, shape));
   if (recording(in, 2)) save(attach(OP_MATMUL, cls, out.p, in, 2), out.p, {in[0], in[1]});
   return out.release();
 }
@@ -381,7 +381,7 @@ static PyObject *linear_forward(PyTypeObject *cls, PyObject *const *in) {
   const int64_t shape[2] = {x->sh[0], w->sh[1]};
   const Reorder reorder(!recording(in, 3));
   nt_storage *s = nullptr;
-  Ref out(fresh(checked(nt_linear(&vx, &vw, &vb, &s), s), 2, shape));
+  Ref out(fresh(checked(nogil([&] { return nt_linear(&vx, &vw, &vb, &s); }), s), 2, shape));
   if (recording(in, 3)) save(attach(OP_LINEAR, cls, out.p, in, 3), out.p, {in[0], in[1]});
   return out.release();
 }
@@ -437,15 +437,15 @@ static PyObject *reduce_forward(Op op, PyTypeObject *cls, PyObject *const *in, P
   nt_storage *s = nullptr;
   int64_t denom = 0;
   switch (op) {
-  case OP_SUM: checked(nt_sum(&v, axes, n_axes, NT_FLOAT32, &s), s); break;
+  case OP_SUM: checked(nogil([&] { return nt_sum(&v, axes, n_axes, NT_FLOAT32, &s); }), s); break;
   case OP_MEAN:
     denom = numel(x->nd, x->sh) / numel(nd, shape);
     if (denom > (int64_t(1) << 24)) return nullptr; // the count is no longer exact in fp32
-    checked(nt_mean_f32(&v, axes, n_axes, float(denom), &s), s);
+    checked(nogil([&] { return nt_mean_f32(&v, axes, n_axes, float(denom), &s); }), s);
     if (!s) return nullptr;
     break;
-  case OP_MAX: checked(nt_max(&v, axes, n_axes, &s), s); break;
-  default: checked(nt_min(&v, axes, n_axes, &s), s); break;
+  case OP_MAX: checked(nogil([&] { return nt_max(&v, axes, n_axes, &s); }), s); break;
+  default: checked(nogil([&] { return nt_min(&v, axes, n_axes, &s); }), s); break;
   }
   Ref out(fresh(s, nd, shape));
   if (recording(in, 1)) {
@@ -467,7 +467,7 @@ static PyObject *view_result(Op op, PyTypeObject *cls, PyObject *out, PyObject *
   return holder.release();
 }
 static PyObject *unchanged(Op op, PyTypeObject *cls, PyObject *const *in, Py_ssize_t n) { // the input itself, as a node of its own
-  return G.grad_enabled ? view_result(op, cls, reinterpret_cast<PyObject *>(alias_of(T_(in[0]))), in, n) : own(in[0]);
+  return grad_enabled() ? view_result(op, cls, reinterpret_cast<PyObject *>(alias_of(T_(in[0]))), in, n) : own(in[0]);
 }
 static bool dims_of(PyObject *const *in, Py_ssize_t n, int64_t *dims) {
   if (n > MAXD) return false;
@@ -583,7 +583,7 @@ static Ref unbroadcast(TensorObj *x, int nd, const int64_t *shape) {
     for (int d = 0; d < lead; ++d) axes[d] = d;
     const nt_view v = view_of(x);
     nt_storage *s = nullptr;
-    cur = Ref(fresh(checked(nt_sum(&v, axes, lead, NT_FLOAT32, &s), s), nd, x->sh + lead));
+    cur = Ref(fresh(checked(nogil([&] { return nt_sum(&v, axes, lead, NT_FLOAT32, &s); }), s), nd, x->sh + lead));
   }
   TensorObj *t = T_(cur.p);
   int n = 0;
@@ -598,7 +598,7 @@ static Ref unbroadcast(TensorObj *x, int nd, const int64_t *shape) {
   if (n) {
     const nt_view v = view_of(t);
     nt_storage *s = nullptr;
-    cur = Ref(fresh(checked(nt_sum(&v, axes, n, NT_FLOAT32, &s), s), nd, kept));
+    cur = Ref(fresh(checked(nogil([&] { return nt_sum(&v, axes, n, NT_FLOAT32, &s); }), s), nd, kept));
   }
   return cur;
 }
@@ -634,7 +634,7 @@ static nt_view expanded(const TensorObj *t, int nd, const int64_t *shape) {
 }
 static Ref elementwise(Fn2 f, const nt_view &a, const nt_view &b, const TensorObj *like) {
   nt_storage *s = nullptr;
-  return Ref(fresh(checked(f(&a, &b, &s), s), like->nd, like->sh));
+  return Ref(fresh(checked(nogil([&] { return f(&a, &b, &s); }), s), like->nd, like->sh));
 }
 static nt_view transposed(const TensorObj *t) { // the last two dims swapped
   nt_view v = view_of(t);
@@ -653,7 +653,7 @@ static PyObject *negated(TensorObj *g) {
     return t;
   }
   nt_storage *s = nullptr;
-  return fresh(checked(nt_neg(&v, &s), s), g->nd, g->sh);
+  return fresh(checked(nogil([&] { return nt_neg(&v, &s); }), s), g->nd, g->sh);
 }
 
 // The sum of -g down to like's shape: one axis of a dense gradient in one launch.  Summed first, then subtracted from zero:
@@ -669,7 +669,7 @@ static PyObject *negated_sum(TensorObj *g, const TensorObj *like) {
     }
   if (n == 1 && !v.storage->constant && !v.storage->scaled()) {
     nt_storage *s = nullptr;
-    checked(nt_mean_f32(&v, &axis, 1, -1.0f, &s), s);
+    checked(nogil([&] { return nt_mean_f32(&v, &axis, 1, -1.0f, &s); }), s);
     if (s) return fresh(s, like->nd, like->sh);
   }
   if (same_shape(g, like)) return negated(g);
@@ -715,7 +715,7 @@ static bool backward_op(FunctionObj *fn, TensorObj *g, PyObject **out, int *n_ou
     if (both && same_shape(g, x1) && same_shape(g, x2)) { // one pass when all three are dense, or large with a transpose
       const nt_view v1 = view_of(x1), v2 = view_of(x2);
       nt_storage *s1 = nullptr, *s2 = nullptr;
-      checked((mul ? nt_mul_gradients : nt_div_gradients)(&vg, &v1, &v2, &s1, &s2), s1);
+      checked(nogil([&] { return (mul ? nt_mul_gradients : nt_div_gradients)(&vg, &v1, &v2, &s1, &s2); }), s1);
       if (s1) {
         PyObject *first = reinterpret_cast<PyObject *>(new_tensor(s1, g->nd, g->sh));
         PyObject *second = reinterpret_cast<PyObject *>(new_tensor(s2, g->nd, g->sh));
@@ -728,7 +728,7 @@ static bool backward_op(FunctionObj *fn, TensorObj *g, PyObject **out, int *n_ou
     if (both && !vg.storage->constant && dense(g) && !(same_shape(g, x1) && same_shape(g, x2))) { // a value per row beside a dense operand
       const nt_view v1 = view_of(x1), v2 = view_of(x2);
       nt_storage *s1 = nullptr, *s2 = nullptr;
-      checked((mul ? nt_mul_gradients_row_value : nt_div_gradients_row_value)(&vg, &v1, &v2, &s1, &s2), s1);
+      checked(nogil([&] { return (mul ? nt_mul_gradients_row_value : nt_div_gradients_row_value)(&vg, &v1, &v2, &s1, &s2); }), s1);
       if (s1) {
         out[0] = reinterpret_cast<PyObject *>(new_tensor(s1, x1->nd, x1->sh));
         out[1] = reinterpret_cast<PyObject *>(new_tensor(s2, x2->nd, x2->sh));
@@ -763,7 +763,7 @@ static bool backward_op(FunctionObj *fn, TensorObj *g, PyObject **out, int *n_ou
       } else {
         if (!fast_pair(fn)) return false;
         nt_storage *s = nullptr;
-        out[1] = unbroadcast(Ref(fresh(checked(nt_div_backward_x2(&vg, &v1, &v2, &s), s), g->nd, g->sh)), x2).release();
+        out[1] = unbroadcast(Ref(fresh(checked(nogil([&] { return nt_div_backward_x2(&vg, &v1, &v2, &s); }), s), g->nd, g->sh)), x2).release();
       }
     }
     return true;
@@ -779,7 +779,7 @@ static bool backward_op(FunctionObj *fn, TensorObj *g, PyObject **out, int *n_ou
     if (need(fn, 0) && need(fn, 1) && g->nd == 2) {
       // both gradients in one call: the second product may start on the SMs the first one's last wave leaves idle
       nt_storage *s1 = nullptr, *s2 = nullptr;
-      checked(nt_matmul_pair(&vg, &vbt, &vat, &vg, &s1, &s2), s1);
+      checked(nogil([&] { return nt_matmul_pair(&vg, &vbt, &vat, &vg, &s1, &s2); }), s1);
       out[0] = reinterpret_cast<PyObject *>(new_tensor(s1, a->nd, a->sh));
       out[1] = reinterpret_cast<PyObject *>(new_tensor(s2, b->nd, b->sh));
       if (!out[0] || !out[1]) throw PyErr{};
@@ -819,7 +819,7 @@ static bool backward_op(FunctionObj *fn, TensorObj *g, PyObject **out, int *n_ou
         return true;
       }
     }
-    out[0] = fresh(checked(nt_pow_backward(&vg, &vx, float(fn->e), &s), s), g->nd, g->sh);
+    out[0] = fresh(checked(nogil([&] { return nt_pow_backward(&vg, &vx, float(fn->e), &s); }), s), g->nd, g->sh);
     return true;
   }
   case OP_SUM:
@@ -848,17 +848,23 @@ static bool backward_op(FunctionObj *fn, TensorObj *g, PyObject **out, int *n_ou
       Ref ge(expand_back(g, x, fn)), me(expand_back(saved(fn, 1), x, fn));
       const nt_view vg = view_of(T_(ge.p)), vx = view_of(saved(fn, 0)), vm = view_of(T_(me.p));
       nt_storage *s = nullptr;
-      TensorObj *in = input(fn, 0), *acc = in->grad ? T_(in->grad) : nullptr;
-      if (acc && in->nd == x->nd && is_fast(in->grad) && same_shape(acc, x) && !storage_of(acc)->constant) {
+      TensorObj *in = input(fn, 0);
+      Ref had(in->grad ? own(in->grad) : nullptr);
+      TensorObj *acc = T_(had.p);
+      if (acc && in->nd == x->nd && is_fast(had.p) && same_shape(acc, x) && !storage_of(acc)->constant) {
         const nt_view va = view_of(acc);
-        checked(nt_extremum_backward_add(&va, &vg, &vx, &vm, fn->axes, fn->n_axes, &s), s);
+        checked(nogil([&] { return nt_extremum_backward_add(&va, &vg, &vx, &vm, fn->axes, fn->n_axes, &s); }), s);
+        if (s && in->grad != had.p) { // another thread's backward has changed it meanwhile
+          nt_storage_release(s);
+          s = nullptr;
+        }
         if (s) {
           out[0] = fresh(s, x->nd, x->sh);
           *added = true;
           return true;
         }
       }
-      out[0] = fresh(checked(nt_extremum_backward(&vg, &vx, &vm, fn->axes, fn->n_axes, &s), s), x->nd, x->sh);
+      out[0] = fresh(checked(nogil([&] { return nt_extremum_backward(&vg, &vx, &vm, fn->axes, fn->n_axes, &s); }), s), x->nd, x->sh);
     }
     return true;
   }
@@ -920,7 +926,7 @@ TensorObj *add_tensors(PyObject *a, PyObject *b) {
   if (!is_fast(a) || !is_fast(b) || !same_shape(T_(a), T_(b))) return nullptr;
   const nt_view va = view_of(T_(a)), vb = view_of(T_(b));
   nt_storage *s = nullptr;
-  const int rc = nt_add(&va, &vb, &s);
+  const int rc = nogil([&] { return nt_add(&va, &vb, &s); });
   if (rc) {
     raise_status(rc);
     return nullptr;

@@ -238,3 +238,67 @@ def test_captures_begin_while_another_thread_makes_constants(nt):
         stop = True
         thread.join()
     assert nt.Tensor._new_contiguous(mine, ()).numpy() == 3.0
+
+
+def test_other_threads_run_while_a_launch_waits(nt):
+    """With the stream's launch queue full a launch waits for the GPU, without the interpreter lock: another thread gets all
+    of the processor that it asks for (half of it when the lock is held)."""
+    import threading
+    import time
+
+    a, b = (nt.Tensor.from_numpy(np.ones(s, np.float32), "cuda") for s in ((8192, 1024), (1024, 4096)))
+    used, stop = [], False
+
+    def busy():
+        start = time.thread_time()
+        while not stop:
+            pass
+        used.append(time.thread_time() - start)
+
+    nt._C.set_matmul_mode(nt._C.MATMUL_EXACT_FP32)  # 1.3 ms each
+    try:
+        with nt.no_grad():
+            a @ b
+            nt.cuda.sync()
+            for _ in range(1030):  # the queue takes 1024
+                a @ b
+            thread = threading.Thread(target=busy)
+            start = time.perf_counter()
+            thread.start()
+            while time.perf_counter() - start < 0.5:
+                a @ b
+            stop = True
+            thread.join()
+            wall = time.perf_counter() - start
+    finally:
+        nt._C.set_matmul_mode(nt._C.MATMUL_3XTF32)
+        nt.cuda.sync()
+    assert used[0] > 0.75 * wall
+
+
+def test_threads_with_graphs_of_their_own(nt):
+    """Forward and backward passes of several threads at once, each with its own input and all with one shared leaf: every
+    pass is recorded although another thread's sweep is running, and no contribution to the shared gradient is lost."""
+    import threading
+
+    threads, passes = 4, 50
+    shared = nt.Tensor.from_numpy(np.full(64, 2.0, np.float32), "cuda", requires_grad=True)
+    failures = []
+
+    def work(k):
+        try:
+            for _ in range(passes):
+                x = nt.Tensor.from_numpy(np.full((8, 64), float(k), np.float32), "cuda", requires_grad=True)
+                (x * shared).sum().backward()
+                if not (x.grad.numpy() == 2.0).all():
+                    failures.append(k)
+        except Exception as e:  # noqa: BLE001
+            failures.append(e)
+
+    pool = [threading.Thread(target=work, args=(k,)) for k in range(1, threads + 1)]
+    for t in pool:
+        t.start()
+    for t in pool:
+        t.join()
+    assert not failures
+    assert (shared.grad.numpy() == 8.0 * passes * sum(range(1, threads + 1))).all()
