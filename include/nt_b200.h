@@ -280,6 +280,13 @@ int nt_matmul_split_stats(uint64_t *split_launches, uint64_t *cache_hits);
  * by the CTA that finishes last, so the result does not depend on timing.  1 = never.  panel (default 8;
  * NT_GEMM_PANEL): width in n-tiles of the panels the CTAs walk the output in, 0 = row by row. */
 int nt_set_matmul_schedule(int max_splits, int panel);
+/* For tests and tuning: this thread's products of mode 1 above the threshold take the kernel that splits its operands itself
+ * (csrc/gemm_fused.cu), with output tiles of tile_n (32, 64, 128) columns and `cluster` (1, 2, 4, 8; with 128 columns 1)
+ * CTAs to a tile, whatever the expected times are.  Products that this kernel cannot take that way (128 columns and a
+ * contraction in several parts) go through planes.  0, 0 (default): by expected time. */
+int nt_matmul_force_fused(int tile_n, int cluster);
+/* Float32 products launched so far through planes, by that kernel, and on the CUDA cores. */
+int nt_matmul_kernel_counts(uint64_t *planes, uint64_t *fused, uint64_t *cuda_cores);
 /* Two independent products in one call, *out1 = a1 @ b1 and *out2 = a2 @ b2 -- what MatmulOp.backward computes
  * (autograd/ops_binary.py:253-267: g @ x2^T and x1^T @ g).  Same bits as two nt_matmul calls.  The second product
  * starts when the first is complete: both may be split along k over the same counters and workspace, and letting the

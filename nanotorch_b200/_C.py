@@ -503,6 +503,18 @@ def set_matmul_schedule(max_splits: int = 8, panel: int = 8) -> None:
     _check(_lib.nt_set_matmul_schedule(int(max_splits), int(panel)))
 
 
+def matmul_force_fused(tile_n: int = 0, cluster: int = 0) -> None:
+    """Which variant of the self-splitting tensor-core kernel this thread's products take; 0, 0 goes by expected time."""
+    _check(_lib.nt_matmul_force_fused(int(tile_n), int(cluster)))
+
+
+def matmul_kernel_counts() -> tuple[int, int, int]:
+    """Float32 products launched so far: through operand planes, by the self-splitting kernel, on the CUDA cores."""
+    counts = [C.c_uint64() for _ in range(3)]
+    _check(_lib.nt_matmul_kernel_counts(*map(C.byref, counts)))
+    return tuple(c.value for c in counts)
+
+
 def set_transposed_tile_pipeline(on: bool = True) -> None:
     """Large fp32 elementwise ops with a transposed operand: TMA-fed persistent kernel (default) or the
     register-staged tile kernel (see the header)."""

@@ -457,6 +457,9 @@ static FgPlan fg_plan(int64_t batch, int64_t M, int64_t N, int64_t K, bool parts
   }
   return best;
 }
+static thread_local FgPlan t_forced; // nt_matmul_force_fused
+bool gemm_fused_forced() { return t_forced.bn != 0; }
+void gemm_fused_force(int tile_n, int cluster) { t_forced = tile_n ? FgPlan{tile_n, cluster, 0.0} : FgPlan{}; }
 double gemm_fused_expected_us(int64_t batch, int64_t M, int64_t N, int64_t K) {
   return fg_plan(batch, M, N, K, gemm_tc_k_split(batch, M, N, K).splits > 1).us;
 }
@@ -480,7 +483,8 @@ bool gemm_fused(const float *A, const float *B, float *C, int64_t batch, int64_t
   // an operand without a unit-stride dim goes through the transposing split there, which never cuts k into parts
   const bool natural = (a_sk == 1 || a_sm == 1 || M == 1 || K == 1) && (b_sk == 1 || b_sn == 1 || N == 1 || K == 1);
   const KSplit ks = natural ? gemm_tc_k_split(batch, M, N, K) : KSplit{};
-  const FgPlan plan = fg_plan(batch, M, N, K, ks.splits > 1);
+  const FgPlan plan = gemm_fused_forced() ? t_forced : fg_plan(batch, M, N, K, ks.splits > 1);
+  if (plan.bn == 128 && ks.splits > 1) return false; // no room for the parts' buffer
   auto aligned = [](const float *p, int64_t s_r, int64_t s_k, int64_t s_b, int64_t K, int64_t batch) {
     return s_k == 1 && (reinterpret_cast<uintptr_t>(p) & 15) == 0 && s_r % 4 == 0 && K % 4 == 0 && (batch == 1 || s_b % 4 == 0);
   };

@@ -30,6 +30,8 @@ bool gemm_3xtf32(const float *A, const float *B, float *C, int64_t batch, int64_
 void gemm_tc_set_promoted(bool on);
 double gemm_tc_expected_us(int64_t batch, int64_t M, int64_t N, int64_t K);
 // gemm_fused.cu: mode 1 without planes
+bool gemm_fused_forced();
+void gemm_fused_force(int tile_n, int cluster);
 double gemm_fused_expected_us(int64_t batch, int64_t M, int64_t N, int64_t K);
 bool gemm_fused(const float *A, const float *B, float *C, int64_t batch, int64_t M, int64_t N, int64_t K, int64_t a_sb, int64_t a_sm,
                 int64_t a_sk, int64_t b_sb, int64_t b_sk, int64_t b_sn, const float *bias, int64_t bias_stride);
@@ -42,6 +44,7 @@ void gemm_tc_set_schedule(int max_splits, int panel);
 void gemm_tc_split_stats(uint64_t *launches, uint64_t *hits);
 static std::atomic<int> g_natural_planes{1};
 static thread_local int t_reorder = 0; // nt_matmul_allow_reorder
+static std::atomic<uint64_t> g_by_planes{0}, g_by_fused{0}, g_by_cuda_cores{0}; // nt_matmul_kernel_counts
 
 static std::atomic<int> g_matmul_mode{1};
 static std::atomic<int64_t> g_tc_min_macs{int64_t(1) << 21}; // batch*M*N*K at or below this: exact FP32 kernel
@@ -228,6 +231,21 @@ int nt_matmul_split_stats(uint64_t *split_launches, uint64_t *cache_hits) {
   gemm_tc_split_stats(split_launches, cache_hits);
   NT_API_END
 }
+int nt_matmul_force_fused(int tile_n, int cluster) {
+  NT_API_BEGIN
+  const bool off = tile_n == 0 && cluster == 0;
+  const bool tile = tile_n == 32 || tile_n == 64 || tile_n == 128, shared = cluster == 1 || cluster == 2 || cluster == 4 || cluster == 8;
+  if (!off && (!tile || !shared || (tile_n == 128 && cluster != 1))) fail_invalid("nt_matmul_force_fused: no such variant.");
+  gemm_fused_force(tile_n, cluster);
+  NT_API_END
+}
+int nt_matmul_kernel_counts(uint64_t *planes, uint64_t *fused, uint64_t *cuda_cores) {
+  NT_API_BEGIN
+  *planes = g_by_planes.load();
+  *fused = g_by_fused.load();
+  *cuda_cores = g_by_cuda_cores.load();
+  NT_API_END
+}
 int nt_wait_probe(void) {
   NT_API_BEGIN
   gemm_tc_wait_probe();
@@ -289,12 +307,12 @@ static nt_storage *matmul_impl(const nt_view *x1, const nt_view *x2, const nt_vi
     // Above that threshold mode 1 goes by expected time (a threshold of 0 sends everything through planes): planes, the
     // tensor-core kernel that does without them -- same bits -- and, where the caller does not need those very bits,
     // the CUDA cores, which finish first below some 5e8 multiply-adds (784 x 256 x 256: 7 us against 11.5 and 20).
-    const bool by_time = mode == 1 && big_enough && min_macs > 0;
+    const bool forced = gemm_fused_forced(), by_time = mode == 1 && big_enough && (min_macs > 0 || forced);
     const double tc_us = by_time ? gemm_tc_expected_us(nbatch, M, N, K) : 0, fused_us = by_time ? gemm_fused_expected_us(nbatch, M, N, K) : 0;
     const bool thin = M <= TH_M && b_sn == 1 && nbatch <= 65535;
     const bool may_split = (mode == 1 || mode == 3) && t_reorder >= (big_enough ? 1 : 2);
     const SimtPlan simt = plan_simt(nbatch, M, N, K, thin, may_split);
-    const bool on_cuda_cores = by_time && t_reorder && simt.us < std::min(tc_us, fused_us);
+    const bool on_cuda_cores = by_time && !forced && t_reorder && simt.us < std::min(tc_us, fused_us);
     if ((mode == 1 || mode == 3) && K > 0 && big_enough && !on_cuda_cores) {
       // the tensor-core path takes a single (collapsed) batch stride per operand
       int64_t a_sb = 0, b_sb = 0;
@@ -312,10 +330,12 @@ static nt_storage *matmul_impl(const nt_view *x1, const nt_view *x2, const nt_vi
         b_sb = bi.b_strides[bi.ndim - 1];
       }
       const float *bp = bias ? static_cast<const float *>(bias->storage->ptr()) + bias->offset : nullptr;
-      if (single && by_time && fused_us < tc_us) {
+      if (single && by_time && (forced || fused_us < tc_us)) {
         operands();
         bias_done = done = gemm_fused(g.A, g.B, g.C, nbatch, M, N, K, a_sb, a_sm, a_sk, b_sb, b_sk, b_sn, bp, bias ? bias->strides[0] : 0);
+        g_by_fused.fetch_add(done, std::memory_order_relaxed);
       }
+      const bool fused = done;
       if (single && !done && mode == 1 && g_natural_planes.load())
         done = gemm_3xtf32_natural(x1->storage, x1->offset, x2->storage, x2->offset, g.C, nbatch, M, N, K, a_sb, a_sm,
                                    a_sk, b_sb, b_sk, b_sn, bp, bias ? bias->strides[0] : 0, &bias_done);
@@ -324,9 +344,11 @@ static nt_storage *matmul_impl(const nt_view *x1, const nt_view *x2, const nt_vi
         done = gemm_3xtf32(g.A, g.B, g.C, nbatch, M, N, K, a_sb, a_sm, a_sk, b_sb, b_sk, b_sn, bp,
                            bias ? bias->strides[0] : 0, &bias_done);
       }
+      if (done && !fused) g_by_planes.fetch_add(1, std::memory_order_relaxed);
     }
     if (!done) {
       operands();
+      g_by_cuda_cores.fetch_add(1, std::memory_order_relaxed);
       g.bias = bias ? static_cast<const float *>(bias->storage->ptr()) + bias->offset : nullptr;
       g.bias_stride = bias ? bias->strides[0] : 0;
       bias_done = true;
