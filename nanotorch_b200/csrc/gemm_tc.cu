@@ -421,7 +421,6 @@ gemm_3xtf32_promoted_kernel(const __grid_constant__ CUtensorMap map_a, const __g
   volatile int *poison_slot = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
   const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
-  pdl_trigger(); // the kernel behind may be set up while this one runs (launch.cuh)
   // a work item: an output tile and, with split-K, this CTA's share of the contraction, k-blocks [kb0, kb0 + nkb)
   struct Item {
     int tile_m, tile_n, split, b, kb0, nkb, periods;

@@ -5,9 +5,12 @@
 // that free up, while the last CTAs of the kernel before it still run; such a kernel starts with pdl_wait(), which waits
 // until that kernel has completed and its writes are visible.  A kernel completes only after its own wait, so by
 // induction everything earlier in the stream has completed too.
-//   - pdl_trigger() lets the next kernel's CTAs in once every CTA of this one is running.  Only the elementwise kernels,
-//     whose CTAs come and go, call it: behind a kernel that holds its SMs to the end, the next one's CTAs piled up on the
-//     SMs that happened to have room (a 384 x 3584 x 1856 product with both gradients 549 -> 604 us).
+//   - pdl_trigger() lets the next kernel's CTAs in once every CTA of this one is running.  Kernels whose CTAs come and go
+//     call it: elementwise ops, fills and casts, operand splits, batched updates, squares with their sums, and row kernels
+//     with a warp per row.  Those that hold their SMs to the end do not -- products, tile pipelines, and the reductions and
+//     extremum gradients whose CTAs share a row or a column: behind them the next kernel's CTAs piled up on the SMs that
+//     happened to have room (a 384 x 3584 x 1856 product with both gradients 549 -> 604 us; with the trigger in the
+//     persistent product alone 4096^3 with both gradients 1538 -> 1547, 8192 x 1024 x 4096 930 -> 954).
 //   - launch_ordered() starts a kernel the ordinary way: those whose CTAs must be spread evenly over the SMs.
 //   - In a graph capture the same edges are recorded (a 17-launch step replays in 59.5 us instead of 61.4).
 //   - Not on other streams than the compute stream: kernels there follow events, not kernels.
