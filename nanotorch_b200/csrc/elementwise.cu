@@ -497,8 +497,7 @@ __global__ void __launch_bounds__(256) ew_row_value_gradients(F f, float *__rest
         } else {
           acc += one(gv[u], xv[u], &y);
         }
-        if constexpr (V == 4) st_result(po + i + u * STEP, y, rows * nvec);
-        else po[i + u * STEP] = y;
+        po[i + u * STEP] = y;
       }
   }
 #pragma unroll

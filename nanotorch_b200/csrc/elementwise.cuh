@@ -51,13 +51,9 @@ struct EwParams {
 
 __device__ __forceinline__ float4 ld_stream(const float4 *p) { return __ldcs(p); }
 __device__ __forceinline__ void st_stream(float4 *p, float4 v) { __stcs(p, v); }
-// A result of up to 96 MB stays in the L2 for the op that reads it next ((a * b - t) ** 2 at 4096 x 4096 with its
-// gradients: 131 -> 122 us); a larger one would only push itself out.  Operands are read with the streaming hint either
-// way: keeping them too displaced the results (139 us).
-__device__ __forceinline__ void st_result(float4 *p, float4 v, int64_t nvec) {
-  if (nvec <= (int64_t(6) << 20)) *p = v;
-  else __stcs(p, v);
-}
+// Results are stored without the streaming hint, at any size: what the next op reads of them is still in the L2.  The mean of
+// (a * b - t) ** 2 with both gradients, without and with the hint, us: operands of 16 MB 43 / 46, of 64 MB 123 / 144, of 112
+// MB 230 / 244, of 256 MB 522 / 531.  Operands are read with the hint: keeping them too displaced the results (64 MB: 139).
 
 // ---------------------------------------------------------------------------------------------
 // Contiguous fp32-sized kernel.  TI/TO are 4-byte types.  UNROLL vectors in flight per thread and operand.
@@ -97,7 +93,7 @@ __global__ void __launch_bounds__(256) ew_contig(F f, typename F::out_t *out, co
         if constexpr (NIN == 2) pr[e] = f(pa[e], pb[e]);
         if constexpr (NIN == 3) pr[e] = f(pa[e], pb[e], pc[e]);
       }
-      st_result(reinterpret_cast<float4 *>(out) + i, r, nvec);
+      reinterpret_cast<float4 *>(out)[i] = r;
     }
   }
   // ragged tail (n % 4 elements) by the first threads of block 0
@@ -175,7 +171,7 @@ __global__ void __launch_bounds__(256) ew_contig_rowbcast(F f, float *out, const
       float4 y;
       if constexpr (ROW_FIRST) y = make_float4(f(r.x, x.x), f(r.y, x.y), f(r.z, x.z), f(r.w, x.w));
       else y = make_float4(f(x.x, r.x), f(x.y, r.y), f(x.z, r.z), f(x.w, r.w));
-      st_result(reinterpret_cast<float4 *>(out) + i, y, nvec);
+      reinterpret_cast<float4 *>(out)[i] = y;
     }
   }
 }
@@ -219,7 +215,7 @@ __global__ void __launch_bounds__(256) ew_contig_colbcast(F f, float *out, const
         y = make_float4(f(v[u][0].x, v[u][1].x, v[u][2].x), f(v[u][0].y, v[u][1].y, v[u][2].y),
                         f(v[u][0].z, v[u][1].z, v[u][2].z), f(v[u][0].w, v[u][1].w, v[u][2].w));
       }
-      st_result(reinterpret_cast<float4 *>(out) + i, y, nvec);
+      reinterpret_cast<float4 *>(out)[i] = y;
     }
   }
 }

@@ -1104,7 +1104,7 @@ __global__ void __launch_bounds__(256) extremum_rows_onepass(const float *__rest
       r.z = gv * ((v[u].z == mv && unique) ? 1.0f : 0.0f);
       r.w = gv * ((v[u].w == mv && unique) ? 1.0f : 0.0f);
       if constexpr (ADD) r = add4(__ldcs(reinterpret_cast<const float4 *>(acc + row * L) + i), r);
-      st_result(po + i, r, int64_t(gridDim.x) * nvec);
+      po[i] = r;
     }
   }
 }
@@ -1146,7 +1146,7 @@ __global__ void __launch_bounds__(256) extremum_rows_warp(const float *__restric
       r.z = gv * ((v[u].z == mv && unique) ? 1.0f : 0.0f);
       r.w = gv * ((v[u].w == mv && unique) ? 1.0f : 0.0f);
       if constexpr (ADD) r = add4(a[u], r);
-      st_result(po + i, r, rows * nvec);
+      po[i] = r;
     }
   }
 }
