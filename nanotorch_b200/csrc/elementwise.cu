@@ -386,7 +386,7 @@ template <class F, int NIN> static nt_storage *produce_with_planes(F f, const nt
   if (!hi) return nullptr;
   const int64_t n = R * C;
   launch(ew_contig_planes<F, NIN>, unsigned(ceil_div(n >> 2, 256 * 4)), 256, 0, f, static_cast<float *>(out->ptr()), pa, pb, n,
-                                                                                      hi, hi + n);
+         hi, hi + n);
   check_launch("ew_contig_planes");
   return out.release();
 }
@@ -444,7 +444,7 @@ template <class F> static void binary_backward_both(F f, const nt_view *g, const
   if (n < 4) return;
   StorageRef o1(storage_new(n, NT_FLOAT32, NT_CUDA)), o2(storage_new(n, NT_FLOAT32, NT_CUDA));
   launch(ew_contig_two<F>, unsigned(ceil_div(n >> 2, 256 * 2)), 256, 0, f, static_cast<float *>(o1->ptr()),
-                                                                            static_cast<float *>(o2->ptr()), p[0], p[1], p[2], n);
+         static_cast<float *>(o2->ptr()), p[0], p[1], p[2], n);
   check_launch("ew_contig_two");
   *out1 = o1.release();
   *out2 = o2.release();

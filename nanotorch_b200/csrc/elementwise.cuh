@@ -677,7 +677,6 @@ template <class F, int NIN> void ew_launch(F f, const nt_view *const (&views)[NI
   }
   IterSpace<NIN + 1> it = collapse<NIN + 1>(views);
   if (it.numel == 0) return;
-  cudaStream_t st = stream();
 
   TO *out = static_cast<TO *>(views[0]->storage->ptr()) + it.offset[0];
   const TI *in[EW_MAX_IN] = {nullptr, nullptr, nullptr};

@@ -1,6 +1,8 @@
 // The ops of engine.h: the `_C` functions over TensorViews, and the forward and backward of the op classes for
-// ordinary Float32 Cuda tensors.  Each follows its class in nanotorch_b200/autograd.py call for call, so results are
-// bit for bit those of the Python path; whatever is out of the ordinary returns "not a fast case" and takes it.
+// ordinary Float32 Cuda tensors.  Each follows its class in nanotorch_b200/autograd.py call for call and has the bits of the
+// Python path, gradients of products excepted: they are summed in the order that is fastest here (Reorder), and in that of a
+// recorded product by the classes.  Whatever is out of the ordinary -- broadcast batches, subclasses, other dtypes --
+// returns "not a fast case" and takes the Python path.
 #include "engine.h"
 
 #include <algorithm>

@@ -253,8 +253,8 @@ int nt_wait_probe(void) {
 }
 
 // x1 @ x2, plus -- when `bias` is given (fp32, N values) -- the broadcast add of the bias as a second
-// rounded step: in the tensor-core kernel's epilogue where that kernel runs, by an in-place add launch
-// otherwise.  Either way the bits are those of matmul followed by add.
+// rounded step: where the kernel stores its result, or by an in-place add launch behind the kernel of mode 3,
+// which does not.  Either way the bits are those of matmul followed by add.
 static nt_storage *matmul_impl(const nt_view *x1, const nt_view *x2, const nt_view *bias) {
   check_view(x1, "matmul");
   check_view(x2, "matmul");
@@ -364,7 +364,7 @@ static nt_storage *matmul_impl(const nt_view *x1, const nt_view *x2, const nt_vi
         int64_t blocks = ceil_div(total, 256);
         if (blocks > 0x7fffffffLL) fail_runtime("matmul: output too large for one launch.");
         launch_ordered(matmul_naive<T>, unsigned(blocks), 256, 0, A, B, static_cast<T *>(o->ptr()), M, N, K, a_sm, a_sk,
-                                                                b_sk, b_sn, bi, total);
+                       b_sk, b_sn, bi, total);
         check_launch("matmul_naive");
       }
     });

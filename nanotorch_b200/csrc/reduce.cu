@@ -640,7 +640,6 @@ static Plan make_plan(const nt_view *x, const int64_t *axes, int32_t n_axes) {
 
 template <class Op> static bool try_fast_f32(const nt_view *x, const Plan &pl, float *out, float divisor = 0.0f) {
   const float *in = static_cast<const float *>(x->storage->ptr()) + x->offset;
-  cudaStream_t st = stream();
   const int sms = sm_count();
   const int64_t target_ctas = int64_t(sms) * 8;
 
@@ -741,7 +740,6 @@ template <class Op> static bool try_fast_f32(const nt_view *x, const Plan &pl, f
 
 template <class T, class O, class Op> static void launch_generic(const nt_view *x, const Plan &pl, void *out) {
   const T *in = static_cast<const T *>(x->storage->ptr()) + x->offset;
-  cudaStream_t st = stream();
   if (pl.n_drop > 256) {
     if (pl.n_keep > 0x7fffffffLL) fail_runtime("reduction: too many kept elements.");
     launch(reduce_generic<T, O, Op, 256>, unsigned(pl.n_keep), 256, 0, in, out, pl.keep, pl.drop, pl.n_keep, pl.n_drop);
@@ -944,38 +942,6 @@ __global__ void __launch_bounds__(256) extremum_apply(const float *__restrict__ 
     const float gv = g[slice_offset(sc.g_keep, slice)], mv = m[slice_offset(sc.m_keep, slice)];
     out[idx] = gv * ((xv == mv && count[slice] == 1) ? 1.0f : 0.0f);
   }
-}
-
-// Vector form of extremum_apply: a CTA owns 1024 consecutive elements of ONE outer index (a slice for
-// ROWS, a matrix row for COLS), so the outer index and -- for ROWS -- the slice's g, m and count are
-// block-uniform and no thread divides anything.
-template <bool ROWS>
-__global__ void __launch_bounds__(256) extremum_apply_vec(const float *__restrict__ x, const float *__restrict__ g,
-                                                          const float *__restrict__ m, const int *__restrict__ count,
-                                                          float *__restrict__ out, SliceScalars sc, int64_t L, int64_t sR,
-                                                          int chunks) {
-  pdl_wait();
-  const int64_t outer = blockIdx.x / chunks;
-  const int64_t inner = int64_t(blockIdx.x - outer * chunks) * 1024 + threadIdx.x * 4;
-  if (inner >= L) return;
-  const float *px = ROWS ? x + slice_offset(sc.x_keep, outer) + inner : x + outer * sR + inner;
-  const float4 v = __ldcs(reinterpret_cast<const float4 *>(px));
-  const float xv[4] = {v.x, v.y, v.z, v.w};
-  float res[4];
-  if (ROWS) {
-    const float gv = g[slice_offset(sc.g_keep, outer)], mv = m[slice_offset(sc.m_keep, outer)];
-    const bool unique = count[outer] == 1;
-#pragma unroll
-    for (int e = 0; e < 4; ++e) res[e] = gv * ((xv[e] == mv && unique) ? 1.0f : 0.0f);
-  } else {
-#pragma unroll
-    for (int e = 0; e < 4; ++e) {
-      const int64_t c = inner + e;
-      const float gv = g[slice_offset(sc.g_keep, c)], mv = m[slice_offset(sc.m_keep, c)];
-      res[e] = gv * ((xv[e] == mv && count[c] == 1) ? 1.0f : 0.0f);
-    }
-  }
-  __stcs(reinterpret_cast<float4 *>(out + outer * L + inner), make_float4(res[0], res[1], res[2], res[3]));
 }
 
 // Optimistic single pass for the long-slice and leading-dim cases: ties are rare, so write g * float(x == m)
@@ -1340,7 +1306,7 @@ int nt_sum_rows_noalloc(const float *in, int64_t n_rows, int64_t row_len, float 
   if (S > 1) // tickets must start at zero whatever the previous call left behind
     NT_CUDA_CHECK(cudaMemsetAsync(scratch->tickets, 0, size_t(n_rows) * sizeof(unsigned), st));
   launch(reduce_rows<RSum>, unsigned(n_rows * S), 256, 0, in, out, scratch->partials, scratch->tickets, keep, row_len,
-                                                        int(S), chunk, 0.0f);
+         int(S), chunk, 0.0f);
   check_launch("reduce_rows");
   NT_API_END
 }

@@ -1209,7 +1209,7 @@ int nt_uniform(int64_t n, int dtype, int device, nt_storage **out) {
       const int64_t blocks = ceil_div(n, per);
       if (n > 0) {
         launch(philox_uniform_kernel<T>, grid_for(blocks, 256), 256, 0, static_cast<T *>(o->ptr()), n,
-                                                                              rt().philox_seed, rt().philox_offset);
+               rt().philox_seed, rt().philox_offset);
         check_launch("philox_uniform");
       }
       rt().philox_offset += uint64_t(blocks);

@@ -1,8 +1,8 @@
 // Exact FP32 products on the CUDA cores: three kernels over strided operands, each output accumulated in ascending k
 // with one rounding per multiply-add (FUSED) or a rounded product and a rounded sum (the reference's CPU loop).
 //
-//   sgemm_small<T>  T x T output tiles (T = 64 or 32), cp.async into a 3-stage ring of 32-deep k-slices, 4 x 4 outputs
-//                   per thread.  What bounds a small product is not arithmetic but how many SMs take part and the
+//   sgemm_small<T>  T x T output tiles (T = 64, 32 or 16; 4 x 4, 4 x 2 or 2 x 2 outputs per thread), cp.async into a
+//                   4-stage ring of 32-deep k-slices.  What bounds a small product is not arithmetic but how many SMs take part and the
 //                   chain of loads each CTA waits for: 256 x 256 x 10 through one 128-wide tile per CTA used 2 SMs
 //                   and took 42 us.  With `splits` > 1 a cluster of CTAs shares a tile, each over its own k-range; the
 //                   partial tiles meet in distributed shared memory and are added in rank order, so the result
@@ -363,7 +363,7 @@ using f32x2 = unsigned long long;
 template <bool FUSED> __device__ __forceinline__ void mad2(f32x2 &c, f32x2 a, f32x2 b) {
   if constexpr (FUSED) {
     asm("fma.rn.f32x2 %0, %1, %2, %0;" : "+l"(c) : "l"(a), "l"(b));
-  } else { // as scalars: the packed multiply and add came out of the assembler as one fused operation
+  } else { // as scalars: results of a packed multiply and a packed add did not have the bits of two roundings
     float x, y, a0, a1, b0, b1;
     asm("mov.b64 {%0, %1}, %2;" : "=f"(x), "=f"(y) : "l"(c));
     asm("mov.b64 {%0, %1}, %2;" : "=f"(a0), "=f"(a1) : "l"(a));
