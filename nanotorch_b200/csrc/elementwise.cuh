@@ -694,8 +694,9 @@ template <class F, int NIN> void ew_launch(F f, const nt_view *const (&views)[NI
     if (all_contig && al && it.numel >= 4) {
       int64_t nvec = it.numel >> 2;
       // Four vectors per thread cover the memory latency of a full GPU.  Runs that do not give every SM a CTA that way take a
-      // vector per thread instead, whose values are computed side by side rather than one after the other (captured
-      // 784-256-10 training step of 256 rows: 56.6 -> 55.3 us; at 2^20 elements there is nothing to gain).
+      // vector per thread instead, whose values are computed side by side rather than one after the other (784-256-10
+      // training step of 256 rows issued eagerly 63.6 -> 62.8 us, captured 55.35 -> 55.3; an activation of up to 2^19 elements
+      // under a squared error is the same within noise).
       bool one = false;
       if constexpr (NIN <= 2 && std::is_same<TI, float>::value && std::is_same<TO, float>::value) {
         one = nvec <= int64_t(sm_count()) * 1024;
