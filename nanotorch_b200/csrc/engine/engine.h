@@ -96,9 +96,15 @@ template <class F> int unlocked(F &&call) {
   PyEval_RestoreThread(state);
   return rc;
 }
-// One that only enqueues work: one thread at a time, as the interpreter lock would have it.
+// One that only enqueues work: one thread at a time, as the interpreter lock would have it.  A program with a single Python
+// thread keeps the lock, which nobody waits for (an op under a squared error, some twenty calls: 30.0 us instead of 30.5).
 inline std::mutex g_launching;
+inline bool only_thread() {
+  PyThreadState *me = PyThreadState_Get();
+  return PyInterpreterState_ThreadHead(PyThreadState_GetInterpreter(me)) == me && !PyThreadState_Next(me);
+}
 template <class F> int nogil(F &&call) {
+  if (only_thread()) return call();
   return unlocked([&] {
     std::lock_guard<std::mutex> lk(g_launching);
     return call();
