@@ -176,7 +176,7 @@ template <int BN, bool CLUSTER> __global__ void __launch_bounds__(fg_threads<BN>
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(ring + bar_off + 96);
   volatile int *poison_slot = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int rank = CLUSTER ? int(blockIdx.x % unsigned(g.csize)) : 0;
   const int64_t n0 = int64_t(blockIdx.x / unsigned(g.csize)) * BN, m0 = int64_t(blockIdx.y) * FG_BM;
   const int rounds = (g.periods + g.csize - 1) / g.csize;
@@ -200,7 +200,7 @@ template <int BN, bool CLUSTER> __global__ void __launch_bounds__(fg_threads<BN>
   tcgen05_fence_before();
   __syncthreads();
   tcgen05_fence_after();
-  const uint32_t tmem_acc = *tmem_slot;
+  const uint32_t tmem_acc = __shfl_sync(0xffffffffu, *tmem_slot, 0); // uniform, and the compiler knows
   const bool poisoned = *poison_slot != 0;
 
   // blocks of 32 k in period p
@@ -264,14 +264,15 @@ template <int BN, bool CLUSTER> __global__ void __launch_bounds__(fg_threads<BN>
     }
   } else if (warp == EW + FG_PRODUCERS / 32) {
     // ------------------------------------------------------------------ MMA issuer
+    const uint32_t lead = elect_lane();
     int s = 0;
     uint32_t phase = 0;
     for (int round = 0; round < rounds; ++round) {
       const int p = round * g.csize + rank, buf = round & 1;
       const int nblk = p < g.periods ? blocks_of(p) : 0;
-      if (lane == 0 && nblk && ok) {
+      if (nblk && ok) {
         if (!mbar_wait(acc_empty0 + 8 * buf, ((round >> 1) & 1) ^ 1, g.wait_limit)) {
-          atomicExch(g.error_flag, 4);
+          if (lead) atomicExch(g.error_flag, 4);
           ok = false;
         }
         tcgen05_fence_after();
@@ -279,7 +280,7 @@ template <int BN, bool CLUSTER> __global__ void __launch_bounds__(fg_threads<BN>
         bool first = true;
         for (int blk = 0; blk < nblk && ok; ++blk) {
           if (!mbar_wait(full0 + 8 * s, phase, g.wait_limit)) {
-            atomicExch(g.error_flag, 2);
+            if (lead) atomicExch(g.error_flag, 2);
             ok = false;
             break;
           }
@@ -289,19 +290,19 @@ template <int BN, bool CLUSTER> __global__ void __launch_bounds__(fg_threads<BN>
           for (int ks = 0; ks < FG_BK / 8; ++ks) {
             const uint32_t pa = st + ks * 32u, pb = st + 2 * A_PLANE + ks * 32u;
             const uint64_t a_hi = fg_desc(pa), a_lo = fg_desc(pa + A_PLANE), b_hi = fg_desc(pb), b_lo = fg_desc(pb + B_PLANE);
-            umma_tf32_idesc(d, a_hi, b_lo, IDESC, first ? 0u : 1u); // small terms first, the large one last
-            umma_tf32_idesc(d, a_lo, b_hi, IDESC, 1);
-            umma_tf32_idesc(d, a_hi, b_hi, IDESC, 1);
+            umma_tf32_idesc(d, a_hi, b_lo, IDESC, first ? 0u : 1u, lead); // small terms first, the large one last
+            umma_tf32_idesc(d, a_lo, b_hi, IDESC, 1, lead);
+            umma_tf32_idesc(d, a_hi, b_hi, IDESC, 1, lead);
             first = false;
           }
-          umma_commit(empty0 + 8 * s);
+          umma_commit(empty0 + 8 * s, lead);
           if (++s == STAGES) {
             s = 0;
             phase ^= 1;
           }
         }
-        if (ok) umma_commit(acc_full0 + 8 * buf);
-        else mbar_arrive(acc_full0 + 8 * buf); // release the epilogue
+        if (ok) umma_commit(acc_full0 + 8 * buf, lead);
+        else if (lead) mbar_arrive(acc_full0 + 8 * buf); // release the epilogue
       }
       cluster_barrier();
       cluster_barrier();

@@ -172,8 +172,8 @@ __device__ __forceinline__ uint64_t umma_desc_mn_sw128(uint32_t smem_addr, uint3
 // [10,13); A and B K-major (0) in bits 15, 16; N >> 3 in [17,23); M >> 4 in [24,29).
 constexpr uint32_t TC_IDESC = (1u << 4) | (2u << 7) | (2u << 10) | (uint32_t(TC_BN >> 3) << 17) | (uint32_t(TC_BM >> 4) << 24);
 
-__device__ __forceinline__ void umma_tf32(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t accumulate) {
-  umma_tf32_idesc(tmem_d, adesc, bdesc, TC_IDESC, accumulate);
+__device__ __forceinline__ void umma_tf32(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t accumulate, uint32_t lead) {
+  umma_tf32_idesc(tmem_d, adesc, bdesc, TC_IDESC, accumulate, lead);
 }
 struct TcArgs {
   float *C;
@@ -231,7 +231,7 @@ gemm_3xtf32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem_raw + (bar_base - smem_u32(smem_raw)) + 72);
   volatile int *poison_slot = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   const int m0 = blockIdx.y * TC_BM, n0 = blockIdx.x * TC_BN, b = blockIdx.z;
 
   if (threadIdx.x == 0) {
@@ -252,7 +252,7 @@ gemm_3xtf32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
   tcgen05_fence_before();
   __syncthreads();
   tcgen05_fence_after();
-  const uint32_t tmem_acc = *tmem_slot;
+  const uint32_t tmem_acc = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   const bool poisoned = *poison_slot != 0;
 
   if (warp == 0) {
@@ -280,13 +280,14 @@ gemm_3xtf32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
     }
   } else if (warp == 1) {
     // ------------------------------------------------------------------ MMA issuer
-    if (lane == 0 && !poisoned) {
+    if (!poisoned) {
+      const uint32_t lead = elect_lane();
       uint32_t phase = 0;
       int s = 0;
       bool ok = true;
       for (int kb = 0; kb < g.num_kb; ++kb) {
         if (!mbar_wait(full0 + 8 * s, phase, g.wait_limit)) {
-          atomicExch(g.error_flag, 2);
+          if (lead) atomicExch(g.error_flag, 2);
           ok = false;
           break;
         }
@@ -302,18 +303,18 @@ gemm_3xtf32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
           // The tensor core's fp32 accumulation rounds toward zero, a bias that grows with the number
           // of accumulations into one accumulator.  The large term gets an accumulator of its own
           // (K/8 accumulations); the two cross terms, 2^-11 smaller, share the other one.
-          umma_tf32(tmem_acc, a_hi, b_hi, (kb | ks) != 0);
-          umma_tf32(tmem_acc + TC_BN, a_hi, b_lo, (kb | ks) != 0);
-          umma_tf32(tmem_acc + TC_BN, a_lo, b_hi, 1);
+          umma_tf32(tmem_acc, a_hi, b_hi, (kb | ks) != 0, lead);
+          umma_tf32(tmem_acc + TC_BN, a_hi, b_lo, (kb | ks) != 0, lead);
+          umma_tf32(tmem_acc + TC_BN, a_lo, b_hi, 1, lead);
         }
-        umma_commit(empty0 + 8 * s); // the stage may be refilled once these MMAs have read it
+        umma_commit(empty0 + 8 * s, lead); // the stage may be refilled once these MMAs have read it
         if (++s == TC_STAGES) {
           s = 0;
           phase ^= 1;
         }
       }
-      if (ok) umma_commit(acc_bar);
-      else asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(acc_bar) : "memory"); // release the epilogue
+      if (ok) umma_commit(acc_bar, lead);
+      else if (lead) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(acc_bar) : "memory"); // release the epilogue
     }
   } else {
     // ------------------------------------------------------------------ epilogue, warps 2..5
@@ -420,7 +421,7 @@ gemm_3xtf32_promoted_kernel(const __grid_constant__ CUtensorMap map_a, const __g
   uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem_raw + (bar_base - smem_u32(smem_raw)) + 96);
   volatile int *poison_slot = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
-  const int warp = threadIdx.x >> 5, lane = threadIdx.x & 31;
+  const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
   // a work item: an output tile and, with split-K, this CTA's share of the contraction, k-blocks [kb0, kb0 + nkb)
   struct Item {
     int tile_m, tile_n, split, b, kb0, nkb, periods;
@@ -454,7 +455,7 @@ gemm_3xtf32_promoted_kernel(const __grid_constant__ CUtensorMap map_a, const __g
   tcgen05_fence_before();
   __syncthreads();
   tcgen05_fence_after();
-  const uint32_t tmem_acc = *tmem_slot;
+  const uint32_t tmem_acc = __shfl_sync(0xffffffffu, *tmem_slot, 0);
   const bool poisoned = *poison_slot != 0;
 
   if (warp == 0) {
@@ -496,7 +497,8 @@ gemm_3xtf32_promoted_kernel(const __grid_constant__ CUtensorMap map_a, const __g
       }
     }
   } else if (warp == 1) {
-    if (lane == 0 && !poisoned) {
+    if (!poisoned) {
+      const uint32_t lead = elect_lane();
       uint32_t phase = 0;
       int s = 0;
       uint32_t done = 0; // periods of the items before
@@ -509,7 +511,7 @@ gemm_3xtf32_promoted_kernel(const __grid_constant__ CUtensorMap map_a, const __g
           const int buf = p & 1;
           // the epilogue must have drained this half (two periods ago) before it is overwritten
           if (!mbar_wait(acc_empty0 + 8 * buf, ((p >> 1) & 1) ^ 1, g.wait_limit)) {
-            atomicExch(g.error_flag, 4);
+            if (lead) atomicExch(g.error_flag, 4);
             ok = false;
             break;
           }
@@ -519,7 +521,7 @@ gemm_3xtf32_promoted_kernel(const __grid_constant__ CUtensorMap map_a, const __g
           bool first = true;
           for (; kb < kb_end; ++kb) {
             if (!mbar_wait(full0 + 8 * s, phase, g.wait_limit)) {
-              atomicExch(g.error_flag, 2);
+              if (lead) atomicExch(g.error_flag, 2);
               ok = false;
               break;
             }
@@ -539,22 +541,22 @@ gemm_3xtf32_promoted_kernel(const __grid_constant__ CUtensorMap map_a, const __g
               const uint64_t b_lo = B_MN ? umma_desc_mn_sw128(pb + TC_B_PLANE_BYTES, g.mn_lbo, g.mn_sbo)
                                          : umma_desc_sw64(pb + TC_B_PLANE_BYTES);
               // small terms first, the large one last
-              umma_tf32_idesc(d, a_hi, b_lo, IDESC, first ? 0u : 1u);
-              umma_tf32_idesc(d, a_lo, b_hi, IDESC, 1);
-              umma_tf32_idesc(d, a_hi, b_hi, IDESC, 1);
+              umma_tf32_idesc(d, a_hi, b_lo, IDESC, first ? 0u : 1u, lead);
+              umma_tf32_idesc(d, a_lo, b_hi, IDESC, 1, lead);
+              umma_tf32_idesc(d, a_hi, b_hi, IDESC, 1, lead);
               first = false;
             }
-            umma_commit(empty0 + 8 * s);
+            umma_commit(empty0 + 8 * s, lead);
             if (++s == TC_STAGES) {
               s = 0;
               phase ^= 1;
             }
           }
-          if (ok) umma_commit(acc_full0 + 8 * buf);
+          if (ok) umma_commit(acc_full0 + 8 * buf, lead);
         }
         done += it.periods;
       }
-      if (!ok) { // release the epilogue warps from whatever they wait on
+      if (!ok && lead) { // release the epilogue warps from whatever they wait on
         for (int i = 0; i < 2; ++i)
           asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(acc_full0 + 8 * i) : "memory");
       }
