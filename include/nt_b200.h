@@ -303,6 +303,12 @@ int nt_set_matmul_tc_min_macs(int64_t macs);
  * level 2 for gradients, 1 for products outside a recorded graph -- and not for a recorded forward product, whose
  * values decide the side of a ReLU's kink or which element is an extremum. */
 int nt_matmul_allow_reorder(int level);
+/* Whether this thread's products of mode 1 keep the rounding that they have on TF32 planes where they would otherwise go
+ * over fp16 planes, faster and closer to the exact product; returns the previous setting (default 0).  The host layer sets
+ * it for nn.Linear, forward and backward: a ReLU's mask is a decision on the last bit, and with masks that flip the gradients
+ * of eight layers differ by 3e-5 to 8e-4 from those of the same weights and data before.  Not in an nn.Sequential of Linear
+ * and Tanh layers (8e-6), and not for other products (2e-6 each, the bias of the TF32 path). */
+int nt_matmul_keep_rounding(int on);
 int64_t nt_get_matmul_tc_min_macs(void);
 
 /* ------------------------------------------------------------------ in-place (src/cpp/ops/inplace_ops.cu:75-79); bump the version */

@@ -503,6 +503,19 @@ def set_matmul_schedule(max_splits: int = 8, panel: int = 8) -> None:
     _check(_lib.nt_set_matmul_schedule(int(max_splits), int(panel)))
 
 
+class keep_rounding:
+    """While entered, this thread's products keep the rounding of TF32 planes (see nt_matmul_keep_rounding in the header)."""
+
+    def __init__(self, on: bool = True) -> None:
+        self._on = on
+
+    def __enter__(self) -> None:
+        self._was = _lib.nt_matmul_keep_rounding(int(self._on))
+
+    def __exit__(self, *_exc) -> None:
+        _lib.nt_matmul_keep_rounding(self._was)
+
+
 def matmul_force_fused(tile_n: int = 0, cluster: int = 0) -> None:
     """Which variant of the self-splitting tensor-core kernel this thread's products take; 0, 0 goes by expected time."""
     _check(_lib.nt_matmul_force_fused(int(tile_n), int(cluster)))

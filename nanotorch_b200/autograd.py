@@ -306,9 +306,16 @@ class LinearOp(Function):
 
     def forward(self, x, W, b):
         self.save_for_backward(x, W)
-        return Tensor._new_contiguous(_C.linear(x._C_view, W._C_view, b._C_view), (x.shape[0], W.shape[1]))
+        self._smooth = _engine.set_smooth(False)
+        _engine.set_smooth(self._smooth)
+        with _C.keep_rounding(not self._smooth):
+            return Tensor._new_contiguous(_C.linear(x._C_view, W._C_view, b._C_view), (x.shape[0], W.shape[1]))
 
     def backward(self, g):
+        with _C.keep_rounding(not self._smooth):
+            return self._gradients(g)
+
+    def _gradients(self, g):
         x, W = self.saved_tensors
         if _need(self, 0) and _need(self, 1) and g.dtype == Dtype.Float32 and g.ndim == 2:
             # both products in one call: the second starts on the SMs the first one's last wave leaves idle

@@ -2,6 +2,7 @@
 // the fused backward kernels and the SGD update.  All arithmetic is compiled with FMA contraction
 // off, so every functor rounds exactly where the reference's separate kernels round.
 #include "elementwise.cuh"
+#include "f16_split.cuh"
 #include "launch.cuh"
 #include "tanh_exact.h"
 #include "cr_math.h"
@@ -364,6 +365,22 @@ static bool dense_2d(const nt_view *v) {
   return v->ndim == 2 && v->strides[1] == 1 && v->strides[0] == v->shape[1] && v->storage->dtype == NT_FLOAT32 &&
          v->storage->device == NT_CUDA;
 }
+template <class F, int NIN>
+static void op_with_f16_planes(F f, void *planes, float *out, const float *a, const float *b, int64_t R, int64_t C) {
+  const F16Planes p = f16_planes_at(planes, 1, R, C);
+  F16SplitArgs g{};
+  g.a = a;
+  g.b = b;
+  g.out = out;
+  g.hi = p.planes;
+  g.lo = p.planes + R * C;
+  g.scale = p.scale;
+  g.header = p.header;
+  g.R = R;
+  g.C = g.Cp = g.s_r = C;
+  g.vec = 1;
+  launch_f16_planes<F, NIN, true>(f, g, 1);
+}
 template <class F, int NIN> static nt_storage *produce_with_planes(F f, const nt_view *a, const nt_view *b) {
   if constexpr (NIN == 2 && !is_bound<F>::value) {
     if (a->storage->scaled()) {
@@ -382,9 +399,16 @@ template <class F, int NIN> static nt_storage *produce_with_planes(F f, const nt
     if (!aligned16(pb)) return nullptr;
   }
   StorageRef out(storage_new(R * C, NT_FLOAT32, NT_CUDA));
-  float *hi = gemm_tc_adopt_planes(out.s, R, C);
-  if (!hi) return nullptr;
   const int64_t n = R * C;
+  // planes for the products that a square layer would make of it
+  const bool f16 = C % 64 == 0 && R <= 64 * 65535 && gemm_f16_wanted(1, R, C, C) && !matmul_keeps_rounding();
+  void *planes = gemm_tc_adopt_planes(out.s, R, C, f16);
+  if (!planes) return nullptr;
+  if (f16) {
+    op_with_f16_planes<F, NIN>(f, planes, static_cast<float *>(out->ptr()), pa, pb, R, C);
+    return out.release();
+  }
+  float *hi = static_cast<float *>(planes);
   launch(ew_contig_planes<F, NIN>, unsigned(ceil_div(n >> 2, 256 * 4)), 256, 0, f, static_cast<float *>(out->ptr()), pa, pb, n,
          hi, hi + n);
   check_launch("ew_contig_planes");
@@ -569,11 +593,11 @@ template <class F> static void row_value_gradients(F f, const nt_view *g, const 
 // ---- SGD.  A weight that has been a matmul operand: its TF32 planes follow the update.  When the parameter is the whole
 // of a dense 2-D storage the update writes them itself (20 bytes per element in one launch instead of 12 + 12 in two);
 // otherwise the cached views are split again behind the update.
-static float *sgd_planes(const nt_view *param) {
+static void *sgd_planes(const nt_view *param, bool *f16) {
   if (!g_producer_planes.load() || nt_get_matmul_mode() != 1 || !dense_2d(param) || param->offset != 0 ||
       param->shape[0] * param->shape[1] != param->storage->n)
     return nullptr;
-  return gemm_tc_refresh_target(param->storage, param->shape[0], param->shape[1]);
+  return gemm_tc_refresh_target(param->storage, param->shape[0], param->shape[1], f16);
 }
 static void sgd_one(const nt_view *param, const nt_view *grad, float lr, float grad_scale) {
   const nt_view *chk[2] = {param, grad};
@@ -583,10 +607,16 @@ static void sgd_one(const nt_view *param, const nt_view *grad, float lr, float g
     const int64_t n = param->shape[0] * param->shape[1];
     float *pp = static_cast<float *>(param->storage->ptr()) + param->offset;
     const float *pg = static_cast<const float *>(grad->storage->ptr()) + grad->offset;
-    float *hi = (n >= 4 && aligned16(pp) && aligned16(pg)) ? sgd_planes(param) : nullptr;
-    if (hi) {
-      launch(ew_contig_planes<SgdF, 2>, unsigned(ceil_div(n >> 2, 256 * 4)), 256, 0, f, pp, pp, pg, n, hi, hi + n);
-      check_launch("ew_contig_planes");
+    bool f16 = false;
+    void *planes = (n >= 4 && aligned16(pp) && aligned16(pg)) ? sgd_planes(param, &f16) : nullptr;
+    if (planes) {
+      if (f16) {
+        op_with_f16_planes<SgdF, 2>(f, planes, pp, pp, pg, param->shape[0], param->shape[1]);
+      } else {
+        float *hi = static_cast<float *>(planes);
+        launch(ew_contig_planes<SgdF, 2>, unsigned(ceil_div(n >> 2, 256 * 4)), 256, 0, f, pp, pp, pg, n, hi, hi + n);
+        check_launch("ew_contig_planes");
+      }
       param->storage->version += 1;
       storage_touch(param->storage);
       gemm_tc_mark_refreshed(param->storage);
@@ -1002,7 +1032,9 @@ int nt_sgd_update_many(const nt_view *params, const nt_view *grads, int32_t coun
     batch.p[k] = static_cast<float *>(p->storage->ptr()) + p->offset;
     batch.g[k] = static_cast<const float *>(g->storage->ptr()) + g->offset;
     batch.n[k] = int32_t(n);
-    batch.hi[k] = sgd_planes(p);
+    bool f16 = false;
+    void *planes = sgd_planes(p, &f16); // fp16 planes are split again behind the batch
+    batch.hi[k] = f16 ? nullptr : static_cast<float *>(planes);
     batch.first[k + 1] = batch.first[k] + int32_t(ceil_div(n, SgdBatch::CHUNK));
     if (batch.count == SgdBatch::MAX) flush();
   }

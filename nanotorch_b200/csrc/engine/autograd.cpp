@@ -204,6 +204,7 @@ static PyGetSetDef function_getset[] = {
     {}};
 static PyMemberDef function_members[] = {{"_e", T_DOUBLE, offsetof(FunctionObj, e), 0, nullptr},
                                          {"_denom", T_LONGLONG, offsetof(FunctionObj, denom), 0, nullptr},
+                                         {"_smooth", T_BOOL, offsetof(FunctionObj, smooth), 0, nullptr},
                                          {}};
 PyTypeObject FunctionBase_Type = {.ob_base = PyVarObject_HEAD_INIT(nullptr, 0)};
 
@@ -459,10 +460,16 @@ static PyObject *m_register_ops(PyObject *, PyObject *const *args, Py_ssize_t n)
   G.hooks = own(args[2]);
   Py_RETURN_NONE;
 }
+static PyObject *m_set_smooth(PyObject *, PyObject *on) {
+  const bool was = t_smooth;
+  t_smooth = on == Py_True;
+  return PyBool_FromLong(was);
+}
 static PyMethodDef m_functions[] = {
     {"run_backward", m_run_backward, METH_O, "Reverse-topological sweep from a tensor whose gradient holds the seed."},
     {"is_grad_enabled", m_is_grad_enabled, METH_NOARGS, nullptr},
     {"set_grad_enabled", m_set_grad_enabled, METH_O, nullptr},
+    {"set_smooth", m_set_smooth, METH_O, "Whether this thread runs a chain of layers without a kink; returns the previous setting."},
     {"sgd_update", reinterpret_cast<PyCFunction>(m_sgd_update), METH_FASTCALL, nullptr},
     {"register_storage", reinterpret_cast<PyCFunction>(m_register_storage), METH_FASTCALL, nullptr},
     {"register_tensor", m_register_tensor, METH_O, nullptr},

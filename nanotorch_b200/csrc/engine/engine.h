@@ -60,6 +60,7 @@ struct FunctionObj {
   int64_t axes[MAXD];
   double e;                            // pow
   int64_t denom;                       // mean
+  char smooth;                         // linear, unary: see set_smooth
 };
 
 struct Globals {
@@ -73,6 +74,7 @@ struct Globals {
   bool grad_enabled = true;
 };
 extern Globals G;
+extern thread_local bool t_smooth;        // see set_smooth
 extern thread_local int t_sweeps;         // this thread is inside a backward sweep: its gradients are values, not graph nodes
 inline bool grad_enabled() { return G.grad_enabled && !t_sweeps; }
 

@@ -305,15 +305,26 @@ static PyObject *binary_forward(Op op, PyTypeObject *cls, PyObject *const *in) {
   return out.release();
 }
 
+// The products of nn.Linear keep their rounding (nt_matmul_keep_rounding), and a tanh leaves the planes that they read --
+// except in a chain of layers without a kink in it (nn.Sequential says so with set_smooth), in its backward pass too.
+thread_local bool t_smooth = false;
+struct KeepRounding {
+  int was;
+  explicit KeepRounding(bool on) : was(nt_matmul_keep_rounding(on)) {}
+  ~KeepRounding() { nt_matmul_keep_rounding(was); }
+};
+
 static PyObject *unary_forward(Op op, PyTypeObject *cls, PyObject *const *in) {
   static const Fn1 fns[] = {nt_neg, nt_exp, nt_log, nt_sqrt, nt_tanh, nt_sigmoid, nt_relu};
   if (!is_fast(in[0])) return nullptr;
   TensorObj *x = T_(in[0]);
   const nt_view v = view_of(x);
+  const KeepRounding keep(!t_smooth);
   nt_storage *s = nullptr;
   Ref out(fresh(checked(nogil([&] { return fns[op - OP_NEG](&v, &s); }), s), x->nd, x->sh));
   if (recording(in, 1)) {
     FunctionObj *fn = attach(op, cls, out.p, in, 1);
+    fn->smooth = t_smooth;
     if (op == OP_LOG) save(fn, out.p, {in[0]});
     else if (op != OP_NEG) save(fn, out.p, {out.p});
   }
@@ -382,9 +393,14 @@ static PyObject *linear_forward(PyTypeObject *cls, PyObject *const *in) {
   const nt_view vx = view_of(x), vw = view_of(w), vb = view_of(b);
   const int64_t shape[2] = {x->sh[0], w->sh[1]};
   const Reorder reorder(!recording(in, 3));
+  const KeepRounding keep(!t_smooth);
   nt_storage *s = nullptr;
   Ref out(fresh(checked(nogil([&] { return nt_linear(&vx, &vw, &vb, &s); }), s), 2, shape));
-  if (recording(in, 3)) save(attach(OP_LINEAR, cls, out.p, in, 3), out.p, {in[0], in[1]});
+  if (recording(in, 3)) {
+    FunctionObj *fn = attach(OP_LINEAR, cls, out.p, in, 3);
+    fn->smooth = t_smooth;
+    save(fn, out.p, {in[0], in[1]});
+  }
   return out.release();
 }
 
@@ -776,6 +792,7 @@ static bool backward_op(FunctionObj *fn, TensorObj *g, PyObject **out, int *n_ou
     TensorObj *a = saved(fn, 0), *b = saved(fn, 1);
     if (g->nd != a->nd) return false;
     const Reorder reorder(2);
+    const KeepRounding keep(fn->op == OP_LINEAR && !fn->smooth);
     *n_out = fn->op == OP_LINEAR ? 3 : 2;
     const nt_view vg = view_of(g), vat = transposed(a), vbt = transposed(b);
     if (need(fn, 0) && need(fn, 1) && g->nd == 2) {
@@ -802,6 +819,7 @@ static bool backward_op(FunctionObj *fn, TensorObj *g, PyObject **out, int *n_ou
     TensorObj *x = saved(fn, 0);
     if (!same_shape(g, x)) return false;
     *n_out = 1;
+    const KeepRounding keep(!fn->smooth);
     out[0] = elementwise(fns[fn->op - OP_EXP], view_of(g), view_of(x), g).release();
     return true;
   }

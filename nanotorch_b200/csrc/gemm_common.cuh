@@ -21,7 +21,8 @@ __device__ __forceinline__ void tcgen05_fence_after() { asm volatile("tcgen05.fe
 // One lane of a converged warp.  The warps that issue products stay converged and predicate each instruction on this lane
 // instead of branching to it: in a branch of one lane every operand of a tcgen05.mma has to be brought into uniform registers
 // anew, 68 clocks per instruction against 36, and a pipeline wait cost 70 more -- of the 16 to 128 clocks that the tensor cores
-// take for one.  500 x 2000 x 300 with both gradients 88.1 -> 84.0 us, 900^3 124.8 -> 120.4, large products 0.5 %.
+// take for one.  500 x 2000 x 300 with both gradients 88.1 -> 84.0 us, 900^3 124.8 -> 120.4, large products over TF32 planes
+// 0.5 %, over fp16 planes, whose instructions are as short again, 4096^3 381 -> 301.
 __device__ __forceinline__ uint32_t elect_lane() {
   uint32_t r;
   asm volatile("{\n\t.reg .pred p;\n\t"

@@ -35,6 +35,8 @@
 #include <unordered_map>
 
 #include "gemm_common.cuh"
+#include "gemm_f16.cuh"
+#include "gemm_tile.cuh"
 #include "launch.cuh"
 #include "nt_core.cuh"
 #include "tf32_split.cuh"
@@ -42,8 +44,6 @@
 
 namespace ntb {
 
-constexpr int TC_BM = 128;   // UMMA M
-constexpr int TC_BN = 256;   // UMMA N
 constexpr int TC_BK = 16;    // k-block per stage: 16 fp32 = 64 bytes = one 64B-swizzle row
 constexpr int TC_STAGES = 4;
 constexpr int TC_UMMA_K = 8; // tf32: 32 bytes of k per instruction
@@ -51,7 +51,6 @@ constexpr int TC_TMEM_COLS = 512; // two fp32 accumulators of 256 columns: hi*hi
 constexpr uint32_t TC_A_PLANE_BYTES = TC_BM * TC_BK * 4;  // 8 KB
 constexpr uint32_t TC_B_PLANE_BYTES = TC_BN * TC_BK * 4;  // 16 KB
 constexpr uint32_t TC_STAGE_BYTES = 2 * TC_A_PLANE_BYTES + 2 * TC_B_PLANE_BYTES; // 48 KB
-constexpr uint32_t TC_CORNER_BYTES = 32 * 32 * 4; // per epilogue warp of the promoted kernel
 constexpr uint32_t TC_SMEM_BYTES = TC_STAGES * TC_STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/ + 8 * TC_CORNER_BYTES;
 
 // ---------------------------------------------------------------------------------------------
@@ -175,54 +174,8 @@ constexpr uint32_t TC_IDESC = (1u << 4) | (2u << 7) | (2u << 10) | (uint32_t(TC_
 __device__ __forceinline__ void umma_tf32(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t accumulate, uint32_t lead) {
   umma_tf32_idesc(tmem_d, adesc, bdesc, TC_IDESC, accumulate, lead);
 }
-struct TcArgs {
-  float *C;
-  int64_t M, N;
-  int32_t num_kb;   // k-blocks of TC_BK
-  int32_t batch;    // number of batches (plane index of `lo` = batch + b)
-  int32_t c_vec;    // rows of C may be written 128 bits at a time
-  const float *bias;    // promoted kernel only: C[m][n] = fl(fl(sum) + bias[n * bias_stride]) when non-null
-  int64_t bias_stride;
-  int *error_flag;
-  long long wait_limit; // SM clocks a pipeline wait may take before the kernel gives up
-  uint32_t mn_lbo, mn_sbo; // byte offsets of the MN-major descriptors (see umma_desc_mn_sw128)
-  int32_t panel;           // promoted kernel: tiles are walked in panels this many n-tiles wide (0 = row by row)
-  // promoted kernel, split-K: `splits` CTAs share an output tile, each over kb_per_split k-blocks; they leave
-  // their sums in `partials` ([tile][split][32 chunks][256 threads][4]) and the one that draws the last ticket
-  // adds them up in split order.  splits == 1: one CTA per tile, no workspace.
-  int32_t splits, kb_per_split;
-  float *partials;
-  unsigned int *tickets;
-  int32_t tiles_m, tiles_n; // promoted kernel: output tiles of one batch
-  int32_t work;             // tiles x splits x batches; a CTA takes items blockIdx.x, + gridDim.x, ...
-};
-
-// Output tile of a work item.  CTAs take items in the order of their index, one wave after the other; taking the n-tiles
-// of a whole row before the next m-tile would make every wave touch all of B, which at these
-// sizes (two planes of B: 134 MB for 4096 x 4096) no longer fits the L2 and is fetched from DRAM once per
-// wave.  With panels of `panel` n-tiles a wave covers more m-tiles and fewer n-tiles, and a panel's slice of
-// B stays in the L2 while the CTAs walk down the m-tiles.
-__device__ __forceinline__ void tile_of_work(const TcArgs &g, int w, int &tm, int &tn, int &split, int &b) {
-  const int splits = g.splits > 1 ? g.splits : 1, per_batch = g.tiles_m * g.tiles_n * splits;
-  b = w / per_batch;
-  int lin = w - b * per_batch;
-  const int t = lin / splits; // the CTAs of one tile are neighbours in the order: their partial sums meet in the L2
-  split = lin - t * splits;
-  lin = t;
-  tm = lin / g.tiles_n;
-  tn = lin - tm * g.tiles_n;
-  if (g.panel > 0) {
-    const int per_panel = g.panel * g.tiles_m;
-    const int p = lin / per_panel;
-    const int within = lin - p * per_panel;
-    const int pw = min(g.panel, g.tiles_n - p * g.panel);
-    tm = within / pw;
-    tn = p * g.panel + within % pw;
-  }
-}
-
 __global__ void __launch_bounds__(192, 1)
-gemm_3xtf32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, TcArgs g) {
+gemm_3xtf32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, TileArgs g) {
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t bar_base = smem_base + TC_STAGES * TC_STAGE_BYTES;
@@ -411,8 +364,12 @@ constexpr int TC_PERIOD_KB = TC_PERIOD / TC_BK; // k-blocks per accumulation cha
 // gradient (both MN-major) all read planes that were split once, without a transpose.
 template <bool A_MN, bool B_MN>
 __global__ void __launch_bounds__(320, 1)
-gemm_3xtf32_promoted_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, TcArgs g) {
+gemm_3xtf32_promoted_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, TileArgs g) {
   constexpr uint32_t IDESC = TC_IDESC | (A_MN ? (1u << 15) : 0u) | (B_MN ? (1u << 16) : 0u);
+  if (g.wide_a) { // behind a product over fp16 planes, which has done it unless one of them is wide
+    pdl_wait();
+    if (!(*g.wide_a | *g.wide_b)) return;
+  }
   extern __shared__ uint8_t smem_raw[];
   const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
   const uint32_t bar_base = smem_base + TC_STAGES * TC_STAGE_BYTES;
@@ -422,19 +379,6 @@ gemm_3xtf32_promoted_kernel(const __grid_constant__ CUtensorMap map_a, const __g
   volatile int *poison_slot = reinterpret_cast<volatile int *>(tmem_slot + 1);
 
   const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-  // a work item: an output tile and, with split-K, this CTA's share of the contraction, k-blocks [kb0, kb0 + nkb)
-  struct Item {
-    int tile_m, tile_n, split, b, kb0, nkb, periods;
-  };
-  auto item_of = [&](int w) {
-    Item it;
-    tile_of_work(g, w, it.tile_m, it.tile_n, it.split, it.b);
-    it.kb0 = g.splits > 1 ? it.split * g.kb_per_split : 0;
-    it.nkb = g.splits > 1 ? min(g.kb_per_split, g.num_kb - it.kb0) : g.num_kb;
-    it.periods = (it.nkb + TC_PERIOD_KB - 1) / TC_PERIOD_KB;
-    return it;
-  };
-
   if (threadIdx.x == 0) {
     for (int s = 0; s < TC_STAGES; ++s) {
       mbar_init(full0 + 8 * s, 1);
@@ -464,7 +408,7 @@ gemm_3xtf32_promoted_kernel(const __grid_constant__ CUtensorMap map_a, const __g
       int s = 0;
       bool ok = true;
       for (int w = blockIdx.x; w < g.work && ok; w += gridDim.x) {
-        const Item it = item_of(w);
+        const TileItem it = tile_item<TC_PERIOD_KB>(g, w);
         const int m0 = it.tile_m * TC_BM, n0 = it.tile_n * TC_BN, b = it.b;
         for (int kb = 0; kb < it.nkb; ++kb) {
           if (!mbar_wait(empty0 + 8 * s, phase ^ 1, g.wait_limit)) {
@@ -504,7 +448,7 @@ gemm_3xtf32_promoted_kernel(const __grid_constant__ CUtensorMap map_a, const __g
       uint32_t done = 0; // periods of the items before
       bool ok = true;
       for (int w = blockIdx.x; w < g.work && ok; w += gridDim.x) {
-        const Item it = item_of(w);
+        const TileItem it = tile_item<TC_PERIOD_KB>(g, w);
         int kb = 0;
         for (int q = 0; q < it.periods && ok; ++q) {
           const uint32_t p = done + q;
@@ -570,8 +514,7 @@ gemm_3xtf32_promoted_kernel(const __grid_constant__ CUtensorMap map_a, const __g
     bool ok = !poisoned;
     uint32_t done = 0; // periods of the items before
     for (int w = blockIdx.x; w < g.work && ok; w += gridDim.x) {
-      const Item it = item_of(w);
-      const int m0 = it.tile_m * TC_BM, n0 = it.tile_n * TC_BN, b = it.b;
+      const TileItem it = tile_item<TC_PERIOD_KB>(g, w);
       float sum[128];
 #pragma unroll
       for (int i = 0; i < 128; ++i) sum[i] = 0.0f;
@@ -601,92 +544,7 @@ gemm_3xtf32_promoted_kernel(const __grid_constant__ CUtensorMap map_a, const __g
         if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(acc_empty0 + 8 * buf) : "memory");
       }
       done += it.periods;
-      const int64_t m = int64_t(m0) + quad * 32 + lane;
-      bool last = ok; // this CTA finishes the tile
-      if (g.splits > 1 && !poisoned) {
-        // Split-K: leave this CTA's sums in the workspace; whoever draws the tile's last ticket adds the
-        // partial sums up in split order (the order never depends on which CTA finishes last).  All eight
-        // epilogue warps pass the two barriers whatever happened to them; a warp whose wait ran out says so.
-        volatile int *fail_slot = poison_slot + 1;
-        volatile unsigned int *ticket_slot = reinterpret_cast<volatile unsigned int *>(poison_slot + 2);
-        const int et = int(threadIdx.x) - 64; // 0..255 among the epilogue threads
-        const int64_t tile_lin = (int64_t(b) * g.tiles_m + it.tile_m) * g.tiles_n + it.tile_n;
-        float *mine = g.partials + ((tile_lin * g.splits + it.split) * 32 * 256 + et) * 4;
-        if (!ok) *fail_slot = 1;
-        if (ok && m < g.M) {
-#pragma unroll
-          for (int q = 0; q < 32; ++q)
-            __stcg(reinterpret_cast<float4 *>(mine + q * 1024), make_float4(sum[4 * q], sum[4 * q + 1], sum[4 * q + 2], sum[4 * q + 3]));
-        }
-        __threadfence();
-        asm volatile("bar.sync 1, 256;" ::: "memory");
-        if (et == 0) *ticket_slot = (*fail_slot != 0) ? 0xffffffffu : atomicAdd(g.tickets + tile_lin, 1u);
-        asm volatile("bar.sync 1, 256;" ::: "memory");
-        const unsigned int ticket = *ticket_slot;
-        last = ok && ticket == unsigned(g.splits - 1);
-        if (last) {
-          __threadfence();
-          if (m < g.M) {
-            const float *first = g.partials + (tile_lin * g.splits * 32 * 256 + et) * 4;
-#pragma unroll
-            for (int q = 0; q < 32; ++q) {
-              float4 acc = __ldcg(reinterpret_cast<const float4 *>(first + q * 1024));
-              for (int sp = 1; sp < g.splits; ++sp) {
-                const float4 v = __ldcg(reinterpret_cast<const float4 *>(first + int64_t(sp) * 32 * 256 * 4 + q * 1024));
-                acc.x += v.x;
-                acc.y += v.y;
-                acc.z += v.z;
-                acc.w += v.w;
-              }
-              sum[4 * q] = acc.x;
-              sum[4 * q + 1] = acc.y;
-              sum[4 * q + 2] = acc.z;
-              sum[4 * q + 3] = acc.w;
-            }
-          }
-          if (et == 0) g.tickets[tile_lin] = 0; // ready for the next launch
-        }
-      }
-      if (__all_sync(0xffffffffu, last)) {
-        // A lane holds a row; stored like that, every instruction would touch 32 lines with 16 bytes each.  The next item's
-        // products run meanwhile: tensor memory takes two periods before it needs this warp again.
-        float *C = g.C + (int64_t(b) * g.M + m0 + quad * 32) * g.N;
-        const int64_t rows = g.M - m0 - quad * 32;
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          const int64_t n = int64_t(n0) + half * 128 + c * 32;
-#pragma unroll
-          for (int j = 0; j < 8; ++j)
-            *reinterpret_cast<float4 *>(corner + lane * 128 + ((j ^ (lane & 7)) << 4)) =
-                make_float4(sum[c * 32 + 4 * j], sum[c * 32 + 4 * j + 1], sum[c * 32 + 4 * j + 2], sum[c * 32 + 4 * j + 3]);
-          __syncwarp();
-          // the second rounded step of x @ W + b: the fp32 product that a separate launch would have stored, plus the bias,
-          // rounded once more
-          if (g.c_vec) {
-            const int j = lane & 7;
-            const int64_t nn = n + 4 * j;
-            float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
-            if (g.bias && nn < g.N)
-              bias = make_float4(__ldg(g.bias + nn * g.bias_stride), __ldg(g.bias + (nn + 1) * g.bias_stride),
-                                 __ldg(g.bias + (nn + 2) * g.bias_stride), __ldg(g.bias + (nn + 3) * g.bias_stride));
-#pragma unroll
-            for (int i = 0; i < 8; ++i) {
-              const int r = 4 * i + (lane >> 3);
-              float4 v = *reinterpret_cast<const float4 *>(corner + r * 128 + ((j ^ (r & 7)) << 4));
-              if (g.bias) v = make_float4(v.x + bias.x, v.y + bias.y, v.z + bias.z, v.w + bias.w);
-              if (r < rows && nn < g.N) *reinterpret_cast<float4 *>(C + r * g.N + nn) = v;
-            }
-          } else {
-            const int64_t nn = n + lane;
-            const float bias = g.bias && nn < g.N ? __ldg(g.bias + nn * g.bias_stride) : 0.0f;
-            for (int r = 0; r < 32 && r < rows; ++r) {
-              const float v = *reinterpret_cast<const float *>(corner + r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4);
-              if (nn < g.N) C[r * g.N + nn] = g.bias ? v + bias : v;
-            }
-          }
-          __syncwarp();
-        }
-      }
+      if (!poisoned) finish_tile(g, it, ok, sum, corner, quad, half, lane, poison_slot);
     }
   }
 
@@ -877,14 +735,13 @@ struct NatSplitArgs {
   float factor;
 };
 
-__global__ void __launch_bounds__(256) split_planes(NatSplitArgs a) {
-  pdl_trigger();
-  pdl_wait();
-  const int64_t c = (int64_t(blockIdx.x) * 64 + (threadIdx.x & 63)) * 4;
+// 16 rows of 256 columns
+__device__ __forceinline__ void split_piece(const NatSplitArgs &a, int64_t piece_c, int64_t piece_r, int64_t batch) {
+  const int64_t c = (piece_c * 64 + (threadIdx.x & 63)) * 4;
   if (c >= a.Cp) return;
-  const int64_t r0 = int64_t(blockIdx.y) * 16 + (threadIdx.x >> 6);
-  const float *src = a.src + int64_t(blockIdx.z) * a.s_b;
-  const int64_t plane = int64_t(blockIdx.z) * a.R * a.Cp;
+  const int64_t r0 = piece_r * 16 + (threadIdx.x >> 6);
+  const float *src = a.src + batch * a.s_b;
+  const int64_t plane = batch * a.R * a.Cp;
   float4 x[4];
 #pragma unroll
   for (int i = 0; i < 4; ++i) { // rows r0, r0 + 4, r0 + 8, r0 + 12: all loads issued before the first use
@@ -916,10 +773,28 @@ __global__ void __launch_bounds__(256) split_planes(NatSplitArgs a) {
   }
 }
 
+__global__ void __launch_bounds__(256) split_planes(NatSplitArgs a) {
+  pdl_trigger();
+  pdl_wait();
+  split_piece(a, blockIdx.x, blockIdx.y, blockIdx.z);
+}
+// Both operands of a product whose fp16 planes are wide; otherwise a launch of CTAs that leave at once (few of them: one
+// for every piece of 4096 x 4096 took 5 us to come and go).
+__global__ void __launch_bounds__(256) split_planes_if_wide(NatSplitArgs a, NatSplitArgs b, int64_t batch, const int *wide_a, const int *wide_b) {
+  pdl_wait();
+  if (!(*wide_a | *wide_b)) return;
+  for (int i = 0; i < 2; ++i) {
+    const NatSplitArgs &s = i ? b : a;
+    const int64_t pc = (s.Cp + 255) / 256, pr = (s.R + 15) / 16;
+    for (int64_t p = blockIdx.x; p < pc * pr * batch; p += gridDim.x) split_piece(s, p % pc, p / pc % pr, p / (pc * pr));
+  }
+}
+
 struct PlaneEntry {
+  bool f16; // fp16 planes (f16_split.cuh) or TF32 planes
   int64_t offset, batch, s_b, R, C, s_r; // the view: element offset, batch count / stride, rows, columns, row stride
   int64_t Cp;
-  float *planes;
+  void *planes;
   size_t rounded;
   uint64_t mutation, epoch;
   int capture = 0;         // id of the capture that last split it, 0 = split eagerly
@@ -934,7 +809,17 @@ static uint64_t g_plane_epoch = 1;
 static std::atomic<int> g_operand_cache{1};
 static std::atomic<uint64_t> g_split_launches{0}, g_split_hits{0};
 
-static void run_split(const nt_storage *s, const PlaneEntry &e) {
+// Memory for the planes of an entry.
+static void plane_memory(PlaneEntry &e) {
+  if (!e.f16) {
+    e.planes = device_alloc(size_t(2 * e.batch * e.R * e.Cp) * 4, &e.rounded);
+    return;
+  }
+  e.planes = device_alloc(f16_planes_at(nullptr, e.batch, e.R, e.C).bytes, &e.rounded);
+  NT_CUDA_CHECK(cudaMemsetAsync(e.planes, 0, sizeof(F16Header), stream()));
+}
+
+static NatSplitArgs split_args(const nt_storage *s, const PlaneEntry &e) {
   NatSplitArgs a{};
   a.factor = 1.0f;
   if (s->scaled()) { // the product with the factor is rounded here, as it would be in memory
@@ -943,31 +828,52 @@ static void run_split(const nt_storage *s, const PlaneEntry &e) {
   } else {
     a.src = static_cast<const float *>(s->ptr()) + e.offset;
   }
-  a.hi = e.planes;
-  a.lo = e.planes + e.batch * e.R * e.Cp;
+  a.hi = static_cast<float *>(e.planes);
+  a.lo = a.hi + e.batch * e.R * e.Cp;
   a.R = e.R;
   a.C = e.C;
   a.Cp = e.Cp;
   a.s_r = e.s_r;
   a.s_b = e.s_b;
   a.vec = ((reinterpret_cast<uintptr_t>(a.src) & 15) == 0 && e.s_r % 4 == 0 && e.s_b % 4 == 0) ? 1 : 0;
+  return a;
+}
+
+static void run_split(const nt_storage *s, const PlaneEntry &e) {
+  const NatSplitArgs a = split_args(s, e);
+  g_split_launches.fetch_add(1, std::memory_order_relaxed);
+  if (e.f16) {
+    const F16Planes p = f16_planes_at(e.planes, e.batch, e.R, e.C);
+    F16SplitArgs h{};
+    h.a = a.src;
+    h.hi = p.planes;
+    h.lo = p.planes + e.batch * e.R * p.Cp;
+    h.scale = p.scale;
+    h.header = p.header;
+    h.R = e.R;
+    h.C = e.C;
+    h.Cp = p.Cp;
+    h.s_r = e.s_r;
+    h.s_b = e.s_b;
+    h.vec = a.vec;
+    launch_f16_planes<SplitScaledF, 1, false>(SplitScaledF{a.factor}, h, e.batch);
+    return;
+  }
   dim3 grid{unsigned(ceil_div(e.Cp, 256)), unsigned(ceil_div(e.R, 16)), unsigned(e.batch)};
   launch(split_planes, grid, 256, 0, a);
   check_launch("split_planes");
-  g_split_launches.fetch_add(1, std::memory_order_relaxed);
 }
 
 // Planes of the view (rows R, columns C with unit stride, row stride s_r, `batch` matrices s_b apart) of
 // storage s.  `owned` is set when the caller must free them after its launch (cache off).
-static float *natural_planes(nt_storage *s, int64_t offset, int64_t batch, int64_t s_b, int64_t R, int64_t C, int64_t s_r,
-                             int64_t *Cp_out, size_t *owned_rounded) {
-  const int64_t Cp = ceil_div(C, 32) * 32;
+static void *natural_planes(nt_storage *s, bool f16, int64_t offset, int64_t batch, int64_t s_b, int64_t R, int64_t C, int64_t s_r,
+                            int64_t *Cp_out, size_t *owned_rounded) {
+  const int64_t Cp = f16 ? ceil_div(C, 64) * 64 : ceil_div(C, 32) * 32;
   *Cp_out = Cp;
   *owned_rounded = 0;
-  const size_t bytes = size_t(2 * batch * R * Cp) * 4;
   if (!g_operand_cache.load()) {
-    PlaneEntry e{offset, batch, s_b, R, C, s_r, Cp, nullptr, 0, 0, 0};
-    e.planes = static_cast<float *>(device_alloc(bytes, &e.rounded));
+    PlaneEntry e{f16, offset, batch, s_b, R, C, s_r, Cp, nullptr, 0, 0, 0};
+    plane_memory(e);
     *owned_rounded = e.rounded;
     run_split(s, e);
     return e.planes;
@@ -977,7 +883,7 @@ static float *natural_planes(nt_storage *s, int64_t offset, int64_t batch, int64
   const uint64_t tick = ++g_plane_tick;
   auto &list = g_plane_cache[s];
   for (PlaneEntry &e : list) {
-    if (e.offset == offset && e.batch == batch && e.s_b == s_b && e.R == R && e.C == C && e.s_r == s_r) {
+    if (e.f16 == f16 && e.offset == offset && e.batch == batch && e.s_b == s_b && e.R == R && e.C == C && e.s_r == s_r) {
       const bool current = e.mutation == s->mutation && e.epoch == g_plane_epoch;
       e.last_use = tick;
       if (current && (cid == 0 || e.capture == cid || e.maintained)) {
@@ -1006,23 +912,23 @@ static float *natural_planes(nt_storage *s, int64_t offset, int64_t batch, int64
       list.erase(list.begin() + victim);
     }
   }
-  PlaneEntry e{offset, batch, s_b, R, C, s_r, Cp, nullptr, 0, s->mutation, g_plane_epoch, cid, false, tick};
-  e.planes = static_cast<float *>(device_alloc(bytes, &e.rounded));
+  PlaneEntry e{f16, offset, batch, s_b, R, C, s_r, Cp, nullptr, 0, s->mutation, g_plane_epoch, cid, false, tick};
+  plane_memory(e);
   run_split(s, e);
   list.push_back(e);
   return e.planes;
 }
 
 // Planes that a producer kernel fills itself while it still holds its output in registers: registers a
-// valid entry for the dense [R][C] view of `s` (C a multiple of 32, so the planes index like the output)
-// and returns its hi plane (lo follows R * C values later); nullptr when the cache is off.
-float *gemm_tc_adopt_planes(nt_storage *s, int64_t R, int64_t C) {
-  if (!g_operand_cache.load() || C % 32 != 0) return nullptr;
+// valid entry for the dense [R][C] view of `s` (C a multiple of 32, or of 64 for fp16 planes, so the planes index like the
+// output) and returns its planes; nullptr when the cache is off.
+void *gemm_tc_adopt_planes(nt_storage *s, int64_t R, int64_t C, bool f16) {
+  if (!g_operand_cache.load() || C % (f16 ? 64 : 32) != 0) return nullptr;
   const int cid = capture_id();
   std::lock_guard<std::mutex> lk(g_plane_mu);
   auto &list = g_plane_cache[s];
-  PlaneEntry e{0, 1, 0, R, C, C, C, nullptr, 0, s->mutation, g_plane_epoch, cid, false};
-  e.planes = static_cast<float *>(device_alloc(size_t(2 * R * C) * 4, &e.rounded));
+  PlaneEntry e{f16, 0, 1, 0, R, C, C, C, nullptr, 0, s->mutation, g_plane_epoch, cid, false};
+  plane_memory(e);
   list.push_back(e);
   return e.planes;
 }
@@ -1055,16 +961,17 @@ void gemm_tc_refresh(nt_storage *s) {
   }
 }
 
-// For a writer that rewrites a whole dense [R][C] fp32 storage and can write the TF32 planes in the same pass
+// For a writer that rewrites a whole dense [R][C] fp32 storage and can write the planes in the same pass
 // (the SGD update): the plane buffer to write, if the storage has exactly one cached view and that view is the
 // whole storage with unpadded rows; the caller then calls gemm_tc_mark_refreshed instead of gemm_tc_refresh.
-float *gemm_tc_refresh_target(nt_storage *s, int64_t R, int64_t C) {
+void *gemm_tc_refresh_target(nt_storage *s, int64_t R, int64_t C, bool *f16) {
   if (!g_operand_cache.load() || C % 32 != 0) return nullptr;
   std::lock_guard<std::mutex> lk(g_plane_mu);
   auto it = g_plane_cache.find(s);
   if (it == g_plane_cache.end() || it->second.size() != 1) return nullptr;
   const PlaneEntry &e = it->second.front();
   if (e.offset != 0 || e.batch != 1 || e.R != R || e.C != C || e.s_r != C || e.Cp != C) return nullptr;
+  *f16 = e.f16;
   return e.planes;
 }
 void gemm_tc_mark_refreshed(nt_storage *s) {
@@ -1130,14 +1037,14 @@ constexpr uint32_t TC_MN_LBO = TC_BK * 128; // next 32 values of m|n
 constexpr uint32_t TC_MN_SBO = 4 * 128;     // next swizzle atom (4 rows of k)
 
 template <bool A_MN, bool B_MN>
-static void launch_promoted(const CUtensorMap &ma, const CUtensorMap &mb, const TcArgs &g, dim3 grid) {
+static void launch_promoted(const CUtensorMap &ma, const CUtensorMap &mb, const TileArgs &g, dim3 grid) {
   static bool configured = false;
   if (!configured) {
     NT_CUDA_CHECK(cudaFuncSetAttribute(gemm_3xtf32_promoted_kernel<A_MN, B_MN>, cudaFuncAttributeMaxDynamicSharedMemorySize,
                                        int(TC_SMEM_BYTES)));
     configured = true;
   }
-  gemm_3xtf32_promoted_kernel<A_MN, B_MN><<<grid, 320, TC_SMEM_BYTES, stream()>>>(ma, mb, g);
+  launch_with(g.wide_a != nullptr, 1, gemm_3xtf32_promoted_kernel<A_MN, B_MN>, grid, 320, TC_SMEM_BYTES, ma, mb, g);
 }
 
 // How an operand matrix [P][Q] (strides s_p, s_q) is laid out: unit stride along Q, along P, or neither.
@@ -1163,21 +1070,35 @@ KSplit gemm_tc_k_split(int64_t batch, int64_t M, int64_t N, int64_t K) {
   return best;
 }
 
+// Whether a product goes over fp16 planes: three products at twice the rate of TF32, from operands of half the bytes, but
+// two more launches, of kernels that only look whether they are needed (2 us each).  From 2^30 multiply-adds on that pays
+// nearly everywhere: us of a product, and of one with both gradients and two splits, over TF32 planes (or without planes)
+// and over fp16 planes: 2048 x 1024 x 1024 37.7 / 34.0, 154 / 147; 4096 x 512 x 640 23.9 / 21.5, 153 / 139; 300 x 4096 x 1024
+// 61.7 / 54.6, 132 / 121; 4096 x 130 x 2500 28.8 / 29.6, 197 / 181; 2048^3 67.8 / 44.8, 230 / 172; 8192 x 1024 x 4096 252 /
+// 168, 868 / 582.  Below, kernels without planes or on the CUDA cores finish in the time of the launches.  A short extent
+// leaves blocks of 64 x 64 and tiles half empty.
+bool gemm_f16_wanted(int64_t batch, int64_t M, int64_t N, int64_t K) {
+  return std::min({M, N, K}) >= 128 && double(batch) * double(M) * double(N) * double(K) > double(int64_t(1) << 30);
+}
+
 // Expected time of a product through planes: half a microsecond per 16-deep k-block of a tile, one tile per SM at a time;
 // 11 us around it (pipeline fill, epilogue, one operand split); 4.5 us per part for the finish of a k-split.  Measured, with
 // one split: 256 x 64 x 256 14 us, 784 x 256 x 256 20, 1024 x 512 x 512 26, 1024^3 40, 100 x 2000 x 60 (4 parts) 44.
-double gemm_tc_expected_us(int64_t batch, int64_t M, int64_t N, int64_t K) {
+// Over fp16 planes half of that per k-block, 6 us for the end of every tile of a CTA and 4 for the launches behind it: 2048^3
+// 45 us, 32 x 512^3 41, 8192 x 1024 x 4096 168.
+double gemm_tc_expected_us(int64_t batch, int64_t M, int64_t N, int64_t K, bool f16) {
   const int64_t tiles = ceil_div(M, TC_BM) * ceil_div(N, TC_BN) * batch, num_kb = ceil_div(K, TC_BK);
   const KSplit ks = gemm_tc_k_split(batch, M, N, K);
   const double waves = double(ceil_div(tiles * ks.splits, sm_count()));
-  return 11.0 + waves * double(ks.splits > 1 ? ks.kb_per_split : num_kb) * 0.5 + (ks.splits > 1 ? 4.5 * ks.splits : 0.0);
+  const double kb = double(ks.splits > 1 ? ks.kb_per_split : num_kb);
+  return (f16 ? 13.0 + waves * (kb * 0.26 + 6.0) : 11.0 + waves * kb * 0.5) + (ks.splits > 1 ? 4.5 * ks.splits : 0.0);
 }
 
-// The promoted-accumulation kernel over natural-layout planes.  Returns false when an operand has no
+// A product over natural-layout planes.  Returns false when an operand has no
 // unit-stride matrix dim (the caller then takes the transposing split below).
 bool gemm_3xtf32_natural(nt_storage *sa, int64_t a_off, nt_storage *sb, int64_t b_off, float *C, int64_t batch, int64_t M,
                          int64_t N, int64_t K, int64_t a_sb, int64_t a_sm, int64_t a_sk, int64_t b_sb, int64_t b_sk,
-                         int64_t b_sn, const float *bias, int64_t bias_stride, bool *bias_done) {
+                         int64_t b_sn, const float *bias, int64_t bias_stride, bool *bias_done, bool f16) {
   if (bias_done) *bias_done = false;
   if (!g_promoted.load()) return false;
   if (batch < 1 || batch > 32767 || M < 1 || N < 1 || K < 1) return false;
@@ -1194,14 +1115,22 @@ bool gemm_3xtf32_natural(nt_storage *sa, int64_t a_off, nt_storage *sb, int64_t 
   if (ceil_div(aR, 16) > 65535 || ceil_div(bR, 16) > 65535) return false; // grid.y of split_planes
   gemm_tc_prepare();
   int64_t aCp = 0, bCp = 0;
-  size_t a_owned = 0, b_owned = 0;
-  float *pa = natural_planes(sa, a_off, batch, batch > 1 ? a_sb : 0, aR, aC, a_sr, &aCp, &a_owned);
-  float *pb = nullptr;
+  size_t a_owned = 0, b_owned = 0, part_owned = 0;
+  f16 = f16 && ceil_div(aR, 64) <= 65535 && ceil_div(bR, 64) <= 65535;
+  void *pa = natural_planes(sa, f16, a_off, batch, batch > 1 ? a_sb : 0, aR, aC, a_sr, &aCp, &a_owned);
+  void *pb = nullptr;
+  float *partials = nullptr;
+  PlaneEntry ea{false, a_off, batch, batch > 1 ? a_sb : 0, aR, aC, a_sr}, eb{false, b_off, batch, batch > 1 ? b_sb : 0, bR, bC, b_sr};
+  auto free_all = [&] { // stream-ordered: what reads them is already queued
+    if (a_owned) device_free(pa, a_owned);
+    if (b_owned && pb) device_free(pb, b_owned);
+    if (partials) device_free(partials, part_owned);
+    for (PlaneEntry *e : {&ea, &eb})
+      if (e->planes) device_free(e->planes, e->rounded);
+  };
   try {
-    pb = natural_planes(sb, b_off, batch, batch > 1 ? b_sb : 0, bR, bC, b_sr, &bCp, &b_owned);
-    CUtensorMap map_a = a_mn ? make_map_mn(pa, aR, aCp, 2 * batch, TC_BM) : make_map_k(pa, aR, K, aCp, 2 * batch, TC_BM);
-    CUtensorMap map_b = b_mn ? make_map_mn(pb, bR, bCp, 2 * batch, TC_BN) : make_map_k(pb, bR, K, bCp, 2 * batch, TC_BN);
-    TcArgs g{};
+    pb = natural_planes(sb, f16, b_off, batch, batch > 1 ? b_sb : 0, bR, bC, b_sr, &bCp, &b_owned);
+    TileArgs g{};
     g.C = C;
     g.M = M;
     g.N = N;
@@ -1222,14 +1151,13 @@ bool gemm_3xtf32_natural(nt_storage *sa, int64_t a_off, nt_storage *sb, int64_t 
     // Not for wave quantisation of larger products: measured on the 2048-row training step (256 tiles on 148
     // SMs, 2 waves against 1.75 with four k-quarters) the split costs more than it saves, 10.4 ms per step
     // against 8.3 -- four short pipelines with four epilogues and 134 MB of partial sums per launch.
-    size_t part_owned = 0;
     {
       const int64_t tiles = tiles_m * tiles_n * batch;
       const KSplit ks = gemm_tc_k_split(batch, M, N, K);
       g.splits = ks.splits;
       g.kb_per_split = ks.kb_per_split;
       if (g.splits > 1) {
-        g.partials = static_cast<float *>(device_alloc(size_t(tiles) * g.splits * TC_BM * TC_BN * 4, &part_owned));
+        g.partials = partials = static_cast<float *>(device_alloc(size_t(tiles) * g.splits * TC_BM * TC_BN * 4, &part_owned));
         g.tickets = g_tickets;
       }
     }
@@ -1241,20 +1169,37 @@ bool gemm_3xtf32_natural(nt_storage *sa, int64_t a_off, nt_storage *sb, int64_t 
     g.work = int32_t(tiles_m * tiles_n * g.splits * batch);
     const dim3 grid{unsigned(std::min(g.work, sm_count())), 1, 1};
     matmul_profile_begin();
+    float *ta = static_cast<float *>(pa), *tb = static_cast<float *>(pb);
+    if (f16) {
+      const F16Operand oa{f16_planes_at(pa, batch, aR, aC), aR, aC, a_mn}, ob{f16_planes_at(pb, batch, bR, bC), bR, bC, b_mn};
+      gemm_f16_launch(oa, ob, g, K);
+      // what it left alone because an operand is wide: both operands split again, into TF32 planes, and multiplied
+      for (PlaneEntry *e : {&ea, &eb}) {
+        e->Cp = ceil_div(e->C, 32) * 32;
+        plane_memory(*e);
+      }
+      aCp = ea.Cp;
+      bCp = eb.Cp;
+      ta = static_cast<float *>(ea.planes);
+      tb = static_cast<float *>(eb.planes);
+      g.wide_a = &oa.p.header->wide;
+      g.wide_b = &ob.p.header->wide;
+      launch(split_planes_if_wide, unsigned(4 * sm_count()), 256, 0, split_args(sa, ea), split_args(sb, eb), batch, g.wide_a, g.wide_b);
+      check_launch("split_planes_if_wide");
+    }
+    const CUtensorMap map_a = a_mn ? make_map_mn(ta, aR, aCp, 2 * batch, TC_BM) : make_map_k(ta, aR, K, aCp, 2 * batch, TC_BM);
+    const CUtensorMap map_b = b_mn ? make_map_mn(tb, bR, bCp, 2 * batch, TC_BN) : make_map_k(tb, bR, K, bCp, 2 * batch, TC_BN);
     if (a_mn && b_mn) launch_promoted<true, true>(map_a, map_b, g, grid);
     else if (a_mn) launch_promoted<true, false>(map_a, map_b, g, grid);
     else if (b_mn) launch_promoted<false, true>(map_a, map_b, g, grid);
     else launch_promoted<false, false>(map_a, map_b, g, grid);
     matmul_profile_end();
-    if (part_owned) device_free(g.partials, part_owned); // stream-ordered like the operand planes
     check_launch("gemm_3xtf32_promoted_kernel");
   } catch (...) {
-    if (a_owned) device_free(pa, a_owned);
-    if (b_owned && pb) device_free(pb, b_owned);
+    free_all();
     throw;
   }
-  if (a_owned) device_free(pa, a_owned);
-  if (b_owned) device_free(pb, b_owned);
+  free_all();
   return true;
 }
 
@@ -1280,7 +1225,7 @@ bool gemm_3xtf32(const float *A, const float *B, float *C, int64_t batch, int64_
     launch_split(B, pb, batch, N, K, Kp, b_sb, b_sn, b_sk);
     CUtensorMap map_a = make_map(pa, M, Kp, 2 * batch, TC_BM);
     CUtensorMap map_b = make_map(pb, N, Kp, 2 * batch, TC_BN);
-    TcArgs g{};
+    TileArgs g{};
     g.C = C;
     g.M = M;
     g.N = N;

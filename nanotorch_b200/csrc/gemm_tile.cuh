@@ -1,0 +1,171 @@
+// What the two persistent tensor-core products over operand planes (gemm_tc.cu, gemm_f16.cu) share: the walk over 128 x 256
+// output tiles, the k-parts of a tile and their sum, and the way a finished tile takes from registers to memory.
+#pragma once
+
+#include <cstdint>
+
+namespace ntb {
+
+constexpr int TC_BM = 128; // UMMA M
+constexpr int TC_BN = 256; // UMMA N
+constexpr uint32_t TC_CORNER_BYTES = 32 * 32 * 4; // per epilogue warp, see finish_tile
+
+struct TileArgs {
+  float *C;
+  int64_t M, N;
+  int32_t num_kb;   // k-blocks
+  int32_t batch;    // number of batches (plane index of `lo` = batch + b)
+  int32_t c_vec;    // rows of C may be written 128 bits at a time
+  const float *bias;    // promoted kernels only: C[m][n] = fl(fl(sum) + bias[n * bias_stride]) when non-null
+  int64_t bias_stride;
+  int *error_flag;
+  long long wait_limit; // SM clocks a pipeline wait may take before the kernel gives up
+  uint32_t mn_lbo, mn_sbo; // byte offsets of the MN-major descriptors (see umma_desc_mn_sw128)
+  int32_t panel;           // tiles are walked in panels this many n-tiles wide (0 = row by row)
+  // split-K: `splits` CTAs share an output tile, each over kb_per_split k-blocks; they leave
+  // their sums in `partials` ([tile][split][32 chunks][256 threads][4]) and the one that draws the last ticket
+  // adds them up in split order.  splits == 1: one CTA per tile, no workspace.
+  int32_t splits, kb_per_split;
+  float *partials;
+  unsigned int *tickets;
+  int32_t tiles_m, tiles_n; // output tiles of one batch
+  int32_t work;             // tiles x splits x batches; a CTA takes items blockIdx.x, + gridDim.x, ...
+  // Whether either operand has a block that two fp16 numbers per value do not hold (gemm_f16.cu), one flag per operand: the
+  // kernel over fp16 planes leaves such a product alone, and the TF32 launches behind it, which have these set, do it.
+  const int *wide_a, *wide_b;
+};
+
+// Output tile of a work item.  CTAs take items in the order of their index, one wave after the other; taking the n-tiles
+// of a whole row before the next m-tile would make every wave touch all of B, which at these
+// sizes (two planes of B: 134 MB for 4096 x 4096) no longer fits the L2 and is fetched from DRAM once per
+// wave.  With panels of `panel` n-tiles a wave covers more m-tiles and fewer n-tiles, and a panel's slice of
+// B stays in the L2 while the CTAs walk down the m-tiles.
+__device__ __forceinline__ void tile_of_work(const TileArgs &g, int w, int &tm, int &tn, int &split, int &b) {
+  const int splits = g.splits > 1 ? g.splits : 1, per_batch = g.tiles_m * g.tiles_n * splits;
+  b = w / per_batch;
+  int lin = w - b * per_batch;
+  const int t = lin / splits; // the CTAs of one tile are neighbours in the order: their partial sums meet in the L2
+  split = lin - t * splits;
+  lin = t;
+  tm = lin / g.tiles_n;
+  tn = lin - tm * g.tiles_n;
+  if (g.panel > 0) {
+    const int per_panel = g.panel * g.tiles_m;
+    const int p = lin / per_panel;
+    const int within = lin - p * per_panel;
+    const int pw = min(g.panel, g.tiles_n - p * g.panel);
+    tm = within / pw;
+    tn = p * g.panel + within % pw;
+  }
+}
+
+// A work item: an output tile and, with split-K, this CTA's share of the contraction, k-blocks [kb0, kb0 + nkb), in
+// `periods` accumulation chains of PERIOD_KB blocks.
+struct TileItem {
+  int tile_m, tile_n, split, b, kb0, nkb, periods;
+};
+template <int PERIOD_KB> __device__ __forceinline__ TileItem tile_item(const TileArgs &g, int w) {
+  TileItem it;
+  tile_of_work(g, w, it.tile_m, it.tile_n, it.split, it.b);
+  it.kb0 = g.splits > 1 ? it.split * g.kb_per_split : 0;
+  it.nkb = g.splits > 1 ? min(g.kb_per_split, g.num_kb - it.kb0) : g.num_kb;
+  it.periods = (it.nkb + PERIOD_KB - 1) / PERIOD_KB;
+  return it;
+}
+
+// The end of a tile in an epilogue warp (eight of them, threads 64..319 of the CTA): `sum` holds 128 columns (`half`) of the
+// row `lane` of the warp's 32 (`quad`).  `corner`: the warp's TC_CORNER_BYTES of shared memory, a 32 x 32 corner of the
+// tile on its way from a lane per row to whole 128-byte lines, 16-byte groups swizzled.  slots[1]: an epilogue warp gave up;
+// slots[2]: the ticket drawn.
+__device__ __forceinline__ void finish_tile(const TileArgs &g, const TileItem &it, bool ok, float (&sum)[128], char *corner, int quad,
+                                            int half, int lane, volatile int *slots) {
+  const int m0 = it.tile_m * TC_BM, n0 = it.tile_n * TC_BN, b = it.b;
+  const int64_t m = int64_t(m0) + quad * 32 + lane;
+  bool last = ok; // this CTA finishes the tile
+  if (g.splits > 1) {
+    // Split-K: leave this CTA's sums in the workspace; whoever draws the tile's last ticket adds the
+    // partial sums up in split order (the order never depends on which CTA finishes last).  All eight
+    // epilogue warps pass the two barriers whatever happened to them; a warp whose wait ran out says so.
+    volatile int *fail_slot = slots + 1;
+    volatile unsigned int *ticket_slot = reinterpret_cast<volatile unsigned int *>(slots + 2);
+    const int et = int(threadIdx.x) - 64; // 0..255 among the epilogue threads
+    const int64_t tile_lin = (int64_t(b) * g.tiles_m + it.tile_m) * g.tiles_n + it.tile_n;
+    float *mine = g.partials + ((tile_lin * g.splits + it.split) * 32 * 256 + et) * 4;
+    if (!ok) *fail_slot = 1;
+    if (ok && m < g.M) {
+#pragma unroll
+      for (int q = 0; q < 32; ++q)
+        __stcg(reinterpret_cast<float4 *>(mine + q * 1024), make_float4(sum[4 * q], sum[4 * q + 1], sum[4 * q + 2], sum[4 * q + 3]));
+    }
+    __threadfence();
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+    if (et == 0) *ticket_slot = (*fail_slot != 0) ? 0xffffffffu : atomicAdd(g.tickets + tile_lin, 1u);
+    asm volatile("bar.sync 1, 256;" ::: "memory");
+    const unsigned int ticket = *ticket_slot;
+    last = ok && ticket == unsigned(g.splits - 1);
+    if (last) {
+      __threadfence();
+      if (m < g.M) {
+        const float *first = g.partials + (tile_lin * g.splits * 32 * 256 + et) * 4;
+#pragma unroll
+        for (int q = 0; q < 32; ++q) {
+          float4 acc = __ldcg(reinterpret_cast<const float4 *>(first + q * 1024));
+          for (int sp = 1; sp < g.splits; ++sp) {
+            const float4 v = __ldcg(reinterpret_cast<const float4 *>(first + int64_t(sp) * 32 * 256 * 4 + q * 1024));
+            acc.x += v.x;
+            acc.y += v.y;
+            acc.z += v.z;
+            acc.w += v.w;
+          }
+          sum[4 * q] = acc.x;
+          sum[4 * q + 1] = acc.y;
+          sum[4 * q + 2] = acc.z;
+          sum[4 * q + 3] = acc.w;
+        }
+      }
+      if (et == 0) g.tickets[tile_lin] = 0; // ready for the next launch
+    }
+  }
+  if (__all_sync(0xffffffffu, last)) {
+    // A lane holds a row; stored like that, every instruction would touch 32 lines with 16 bytes each.  The next item's
+    // products run meanwhile: tensor memory takes two periods before it needs this warp again.
+    float *C = g.C + (int64_t(b) * g.M + m0 + quad * 32) * g.N;
+    const int64_t rows = g.M - m0 - quad * 32;
+#pragma unroll
+    for (int c = 0; c < 4; ++c) {
+      const int64_t n = int64_t(n0) + half * 128 + c * 32;
+#pragma unroll
+      for (int j = 0; j < 8; ++j)
+        *reinterpret_cast<float4 *>(corner + lane * 128 + ((j ^ (lane & 7)) << 4)) =
+            make_float4(sum[c * 32 + 4 * j], sum[c * 32 + 4 * j + 1], sum[c * 32 + 4 * j + 2], sum[c * 32 + 4 * j + 3]);
+      __syncwarp();
+      // the second rounded step of x @ W + b: the fp32 product that a separate launch would have stored, plus the bias,
+      // rounded once more
+      if (g.c_vec) {
+        const int j = lane & 7;
+        const int64_t nn = n + 4 * j;
+        float4 bias = make_float4(0.f, 0.f, 0.f, 0.f);
+        if (g.bias && nn < g.N)
+          bias = make_float4(__ldg(g.bias + nn * g.bias_stride), __ldg(g.bias + (nn + 1) * g.bias_stride),
+                             __ldg(g.bias + (nn + 2) * g.bias_stride), __ldg(g.bias + (nn + 3) * g.bias_stride));
+#pragma unroll
+        for (int i = 0; i < 8; ++i) {
+          const int r = 4 * i + (lane >> 3);
+          float4 v = *reinterpret_cast<const float4 *>(corner + r * 128 + ((j ^ (r & 7)) << 4));
+          if (g.bias) v = make_float4(v.x + bias.x, v.y + bias.y, v.z + bias.z, v.w + bias.w);
+          if (r < rows && nn < g.N) *reinterpret_cast<float4 *>(C + r * g.N + nn) = v;
+        }
+      } else {
+        const int64_t nn = n + lane;
+        const float bias = g.bias && nn < g.N ? __ldg(g.bias + nn * g.bias_stride) : 0.0f;
+        for (int r = 0; r < 32 && r < rows; ++r) {
+          const float v = *reinterpret_cast<const float *>(corner + r * 128 + (((lane >> 2) ^ (r & 7)) << 4) + (lane & 3) * 4);
+          if (nn < g.N) C[r * g.N + nn] = g.bias ? v + bias : v;
+        }
+      }
+      __syncwarp();
+    }
+  }
+}
+
+} // namespace ntb

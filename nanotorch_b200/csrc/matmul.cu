@@ -28,7 +28,7 @@ bool gemm_3xtf32(const float *A, const float *B, float *C, int64_t batch, int64_
                  int64_t a_sb, int64_t a_sm, int64_t a_sk, int64_t b_sb, int64_t b_sk, int64_t b_sn,
                  const float *bias, int64_t bias_stride, bool *bias_done);
 void gemm_tc_set_promoted(bool on);
-double gemm_tc_expected_us(int64_t batch, int64_t M, int64_t N, int64_t K);
+double gemm_tc_expected_us(int64_t batch, int64_t M, int64_t N, int64_t K, bool f16);
 // gemm_fused.cu: mode 1 without planes
 bool gemm_fused_forced();
 void gemm_fused_force(int tile_n, int cluster);
@@ -38,12 +38,14 @@ bool gemm_fused(const float *A, const float *B, float *C, int64_t batch, int64_t
 // mode 1 over natural-layout, cached operand planes; false when an operand has no unit-stride matrix dim
 bool gemm_3xtf32_natural(nt_storage *sa, int64_t a_off, nt_storage *sb, int64_t b_off, float *C, int64_t batch, int64_t M,
                          int64_t N, int64_t K, int64_t a_sb, int64_t a_sm, int64_t a_sk, int64_t b_sb, int64_t b_sk,
-                         int64_t b_sn, const float *bias, int64_t bias_stride, bool *bias_done);
+                         int64_t b_sn, const float *bias, int64_t bias_stride, bool *bias_done, bool f16);
 void gemm_tc_set_operand_cache(bool on);
 void gemm_tc_set_schedule(int max_splits, int panel);
 void gemm_tc_split_stats(uint64_t *launches, uint64_t *hits);
 static std::atomic<int> g_natural_planes{1};
 static thread_local int t_reorder = 0; // nt_matmul_allow_reorder
+static thread_local bool t_keep = false; // nt_matmul_keep_rounding
+bool matmul_keeps_rounding() { return t_keep; }
 static std::atomic<uint64_t> g_by_planes{0}, g_by_fused{0}, g_by_cuda_cores{0}; // nt_matmul_kernel_counts
 
 static std::atomic<int> g_matmul_mode{1};
@@ -204,6 +206,11 @@ int nt_matmul_allow_reorder(int level) {
   t_reorder = level < 0 ? 0 : level;
   return was;
 }
+int nt_matmul_keep_rounding(int on) {
+  const bool was = t_keep;
+  t_keep = on != 0;
+  return was;
+}
 int nt_get_matmul_mode(void) { return g_matmul_mode.load(); }
 int nt_set_matmul_schedule(int max_splits, int panel) {
   NT_API_BEGIN
@@ -305,10 +312,12 @@ static nt_storage *matmul_impl(const nt_view *x1, const nt_view *x2, const nt_vi
     const int64_t min_macs = g_tc_min_macs.load();
     const bool big_enough = double(nbatch) * double(M) * double(N) * double(K) > double(min_macs);
     // Above that threshold mode 1 goes by expected time (a threshold of 0 sends everything through planes): planes, the
-    // tensor-core kernel that does without them -- same bits -- and, where the caller does not need those very bits,
+    // tensor-core kernel that does without them -- same bits as TF32 planes; a product that is wanted on fp16 planes always
+    // goes there, so that its bits do not depend on a setting -- and, where the caller does not need those very bits,
     // the CUDA cores, which finish first below some 5e8 multiply-adds (784 x 256 x 256: 7 us against 11.5 and 20).
     const bool forced = gemm_fused_forced(), by_time = mode == 1 && big_enough && (min_macs > 0 || forced);
-    const double tc_us = by_time ? gemm_tc_expected_us(nbatch, M, N, K) : 0, fused_us = by_time ? gemm_fused_expected_us(nbatch, M, N, K) : 0;
+    const bool f16 = !t_keep && gemm_f16_wanted(nbatch, M, N, K);
+    const double tc_us = by_time ? gemm_tc_expected_us(nbatch, M, N, K, f16) : 0, fused_us = by_time ? gemm_fused_expected_us(nbatch, M, N, K) : 0;
     const bool thin = M <= TH_M && b_sn == 1 && nbatch <= 65535;
     const bool may_split = (mode == 1 || mode == 3) && t_reorder >= (big_enough ? 1 : 2);
     const SimtPlan simt = plan_simt(nbatch, M, N, K, thin, may_split);
@@ -330,7 +339,7 @@ static nt_storage *matmul_impl(const nt_view *x1, const nt_view *x2, const nt_vi
         b_sb = bi.b_strides[bi.ndim - 1];
       }
       const float *bp = bias ? static_cast<const float *>(bias->storage->ptr()) + bias->offset : nullptr;
-      if (single && by_time && (forced || fused_us < tc_us)) {
+      if (single && by_time && (forced || (fused_us < tc_us && !f16))) {
         operands();
         bias_done = done = gemm_fused(g.A, g.B, g.C, nbatch, M, N, K, a_sb, a_sm, a_sk, b_sb, b_sk, b_sn, bp, bias ? bias->strides[0] : 0);
         g_by_fused.fetch_add(done, std::memory_order_relaxed);
@@ -338,7 +347,7 @@ static nt_storage *matmul_impl(const nt_view *x1, const nt_view *x2, const nt_vi
       const bool fused = done;
       if (single && !done && mode == 1 && g_natural_planes.load())
         done = gemm_3xtf32_natural(x1->storage, x1->offset, x2->storage, x2->offset, g.C, nbatch, M, N, K, a_sb, a_sm,
-                                   a_sk, b_sb, b_sk, b_sn, bp, bias ? bias->strides[0] : 0, &bias_done);
+                                   a_sk, b_sb, b_sk, b_sn, bp, bias ? bias->strides[0] : 0, &bias_done, f16);
       if (single && !done) {
         operands();
         done = gemm_3xtf32(g.A, g.B, g.C, nbatch, M, N, K, a_sb, a_sm, a_sk, b_sb, b_sk, b_sn, bp,

@@ -96,10 +96,16 @@ class Sequential(Module):
         return self
 
     def forward(self, *args: Any, **kwargs: Any) -> Any:
-        x = self._modules[0](*args, **kwargs)
-        for m in self._modules[1:]:
-            x = m(x)
-        return x
+        # Linear layers with nothing but Tanh between them: no ReLU's mask hangs on the last bit of a product, so the large
+        # ones may take the fp16 planes in both passes (nt_matmul_keep_rounding says what the others keep, and why)
+        was = _engine.set_smooth(all(type(m) is Linear or type(m) is Tanh for m in self._modules))
+        try:
+            x = self._modules[0](*args, **kwargs)
+            for m in self._modules[1:]:
+                x = m(x)
+            return x
+        finally:
+            _engine.set_smooth(was)
 
 
 class Optimizer:

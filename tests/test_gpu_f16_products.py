@@ -1,0 +1,188 @@
+"""Products over fp16 planes (more than 2^30 multiply-adds): the edges of their tiles, blocks and chains in every operand
+layout, k-parts and batches, the planes that producers write, and matrices that two fp16 numbers per value do not hold."""
+
+import numpy as np
+import pytest
+
+from tests.util import assert_bit_exact, assert_scaled
+
+pytestmark = pytest.mark.gpu
+
+SHAPES = [(1, 1100, 1028, 1000), (1, 1024, 1056, 1024), (1, 1025, 1023, 1089), (1, 4100, 130, 2500), (1, 130, 9000, 1000),
+          (1, 512, 4096, 1024), (1, 128, 8200, 1030), (5, 700, 640, 500), (33, 257, 520, 290)]
+
+
+def dev(nt, x, turned=False):
+    return nt.Tensor.from_numpy(np.ascontiguousarray(np.swapaxes(x, -1, -2)), "cuda").transpose(-2, -1) if turned else nt.Tensor.from_numpy(x, "cuda")
+
+
+@pytest.mark.parametrize("shape", SHAPES, ids=str)
+@pytest.mark.parametrize("values", ["uniform", "normal"])
+def test_every_layout(nt, shape, values):
+    batch, M, K, N = shape
+    rng = np.random.default_rng(M + K + N)
+    lead = (batch,) if batch > 1 else ()
+    draw = (lambda *s: rng.uniform(-1, 1, s).astype(np.float32)) if values == "uniform" else (lambda *s: rng.standard_normal(s).astype(np.float32))
+    a, b = draw(*lead, M, K), draw(*lead, K, N)
+    with nt.no_grad():
+        got = [(dev(nt, a, ta) @ dev(nt, b, tb)).numpy() for ta in (False, True) for tb in (False, True)]
+    for g in got[1:]:
+        assert_bit_exact(g, got[0], "same bits whatever the operand order")
+    rows = slice(M - 67, M)
+    a64, b64 = a[..., rows, :].astype(np.float64), b.astype(np.float64)
+    # 2^-23 of each operand and 2^-24 for the dropped lo * lo; at most 2^-22 of a chain of 64; 2^-24 of each sum of chains
+    bound = 5 * 2.0 ** -23 + (K / 64 + 1) * 2.0 ** -24
+    assert_scaled(got[0][..., rows, :], a64 @ b64, np.abs(a64) @ np.abs(b64), bound, f"{shape}")
+    if batch == 1:
+        bias = draw(N)
+        fused = nt._C.linear(dev(nt, a)._C_view, dev(nt, b)._C_view, dev(nt, bias)._C_view)
+        assert_bit_exact(nt.Tensor._new_contiguous(fused, (M, N)).numpy(), got[0] + bias, "bias in the epilogue")
+
+
+def _wide(name, rng, n):
+    a = rng.standard_normal((n, n)).astype(np.float32)
+    if name == "faint row":
+        a[77] *= 1e-12
+    elif name == "faint column":
+        a[:, n - 1] *= 1e-12
+    elif name == "faint block":
+        a[100:170, 260:330] *= 1e-15  # across blocks: one of their parts is faint beside the rest of its block
+    elif name == "tiny value":
+        a[n - 1, n - 1] = 1e-30
+    elif name == "denormal matrix":
+        a *= 1e-39
+    elif name == "small matrix":
+        a *= 1e-21
+    elif name == "large matrix":
+        a *= 1e25
+    elif name == "infinity":
+        a[3, 4] = np.inf
+    elif name == "nan":
+        a[3, 4] = np.nan
+    elif name == "lowest":
+        a[5, ::2] = np.finfo(np.float32).min
+    return a
+
+
+WIDE = ["faint row", "faint column", "faint block", "tiny value", "denormal matrix", "small matrix", "large matrix", "infinity", "nan", "lowest"]
+
+
+@pytest.mark.parametrize("name", WIDE)
+@pytest.mark.parametrize("side", ["a", "b"])
+def test_what_fp16_does_not_hold_goes_through_tf32(nt, name, side):
+    """The bits of the kernel over TF32 planes, which the first 128 rows alone, a smaller product, still take."""
+    n = 1280
+    rng = np.random.default_rng(3)
+    wide, plain = _wide(name, rng, n), rng.standard_normal((n, n)).astype(np.float32)
+    a, b = (wide, plain) if side == "a" else (plain, wide)
+    nt._C.set_matmul_schedule(1, 8)
+    try:
+        with nt.no_grad():
+            got = (dev(nt, a) @ dev(nt, b)).numpy()
+            want = np.concatenate([(dev(nt, a[i:i + 128]) @ dev(nt, b)).numpy() for i in range(0, n, 128)])
+    finally:
+        nt._C.set_matmul_schedule(8, 8)
+    assert_bit_exact(got, want, name)
+
+
+def test_values_at_the_end_of_the_range(nt):
+    """Magnitudes from 2^-28 of the largest on are held to 2^-22, factors of 2^+-60 included; a block may hold a few fainter
+    ones.  A diagonal matrix shows every value by itself."""
+    n = 1280
+    rng = np.random.default_rng(4)
+    eye = np.eye(n, dtype=np.float32)
+    for scale in (2.0 ** -70, 2.0 ** -40, 1.0, 2.0 ** 40, 2.0 ** 73):
+        d = rng.uniform(1, 2, n) * 2.0 ** rng.integers(-27, 1, n) * scale
+        d[::64] = 1.5 * scale  # the largest of every block
+        with nt.no_grad():
+            got = np.diagonal((dev(nt, np.diag(d.astype(np.float32))) @ dev(nt, eye)).numpy()).astype(np.float64)
+        assert_scaled(got, d.astype(np.float32), np.abs(d), 2.0 ** -22, f"scale {scale}")
+        d[5] = 2.0 ** -33 * scale  # one faint value: to 2^-17 of itself, 2^-52 of the block's largest
+        with nt.no_grad():
+            got = np.diagonal((dev(nt, np.diag(d.astype(np.float32))) @ dev(nt, eye)).numpy()).astype(np.float64)
+        assert_scaled(got, d.astype(np.float32), np.abs(d), 2.0 ** -16, f"faint value at {scale}")
+
+
+def test_a_replayed_product_follows_its_operands(nt):
+    """Whether an operand is wide is found out on the device, in every replay again."""
+    n = 1280
+    rng = np.random.default_rng(5)
+    x, w = dev(nt, rng.standard_normal((n, n)).astype(np.float32)), dev(nt, rng.standard_normal((n, n)).astype(np.float32))
+    with nt.no_grad():
+        (x @ w).numpy()
+        graph = nt._C.Graph()
+        with graph.capture():
+            y = x @ w
+        for name in ("plain", "faint row", "plain", "tiny value", "plain"):
+            data = _wide(name, rng, n)
+            x.storage.upload(data.ctypes.data, data.nbytes)
+            graph.replay()
+            assert_bit_exact(y.numpy(), (dev(nt, data) @ w).numpy(), name)
+        graph.close()
+
+
+def test_producers_write_fp16_planes(nt):
+    """tanh, tanh_backward and the SGD update on matrices whose products go over fp16 planes: the bits of the plain kernels,
+    no split for the products that follow, and the products of split operands."""
+    import nanotorch_b200.nn as nn
+
+    _C = nt._C
+    rng = np.random.default_rng(6)
+    shape = (1100, 1088)
+    z, g, w = (rng.standard_normal(s).astype(np.float32) for s in (shape, shape, (1088, 1152)))
+    z[500] *= 1e-13  # tanh of it: a wide matrix
+    tanh = nn.Sequential(nn.Tanh())  # a chain without a kink
+    for faint in (False, True):
+        zt = dev(nt, z if faint else np.abs(z) + 1)
+        out = []
+        for planes in (False, True):
+            _C.set_producer_planes(planes)
+            try:
+                W, G = dev(nt, w), dev(nt, g)
+                with nt.no_grad():
+                    (dev(nt, g) @ W).numpy()  # the weight's planes exist from here on
+                    h = tanh(zt)
+                    d = nt.Tensor._new_contiguous(_C.tanh_backward(G._C_view, h._C_view), shape)
+                    step = dev(nt, rng.standard_normal(w.shape).astype(np.float32) if not planes else kept)
+                    kept = step.numpy()
+                    _C.sgd_update(W._C_view, step._C_view, 0.25, 1.0)
+                    s0, _ = _C.matmul_split_stats()
+                    y1, y2 = h @ W, h.T @ d
+                    s1, _ = _C.matmul_split_stats()
+                    out.append([t.numpy() for t in (h, d, W, y1, y2)])
+            finally:
+                _C.set_producer_planes(True)
+            assert s1 - s0 == (0 if planes else 2)
+        for plain, with_planes in zip(*out):
+            assert_bit_exact(with_planes, plain, "with planes of its own")
+
+
+def test_linear_keeps_its_rounding_where_a_kink_may_follow(nt):
+    """nn.Linear by itself or in a chain with a ReLU has the bits of the products over TF32 planes, forward and backward; in a
+    chain of Linear and Tanh those over fp16 planes, closer to the exact ones."""
+    import nanotorch_b200.nn as nn
+
+    _C = nt._C
+    rng = np.random.default_rng(7)
+    x_np, w_np, b_np, g_np = (rng.standard_normal(s).astype(np.float32) for s in ((1100, 1088), (1088, 1152), (1152,), (1100, 1152)))
+    results = {}
+    for name in ("alone", "relu", "tanh"):
+        layer = nn.Linear(1088, 1152).to("cuda")
+        layer._W, layer._b = (nt.Tensor.from_numpy(v, "cuda", requires_grad=True) for v in (w_np, b_np))
+        x, g = nt.Tensor.from_numpy(x_np, "cuda", requires_grad=True), dev(nt, g_np)
+        chain = {"alone": layer, "relu": nn.Sequential(layer, nn.ReLU()), "tanh": nn.Sequential(layer, nn.Tanh())}[name]
+        y = chain(x)
+        z = y if name == "alone" else y.grad_fn.inputs[0]
+        assert z.grad_fn._smooth == (name == "tanh")
+        (z * g).sum().backward()
+        results[name] = [z.numpy(), x.grad.numpy(), layer._W.grad.numpy()]
+    X, W, G = dev(nt, x_np), dev(nt, w_np), dev(nt, g_np)
+    products = lambda: [(X @ W).numpy() + b_np, (G @ W.T).numpy(), (X.T @ G).numpy()]
+    with nt.no_grad():
+        with _C.keep_rounding():
+            kept = products()
+        free = products()
+    for got, want in zip(results["alone"] + results["relu"] + results["tanh"], kept + kept + free):
+        assert_bit_exact(got, want)
+    exact = x_np.astype(np.float64) @ w_np.astype(np.float64) + b_np
+    assert np.linalg.norm(free[0] - exact) < 0.3 * np.linalg.norm(kept[0] - exact)
