@@ -2,7 +2,7 @@
 #pragma once
 
 #include "f16_split.cuh"
-#include "gemm_tile.cuh"
+#include "gemm_tf32.cuh"
 
 namespace ntb {
 
@@ -29,7 +29,15 @@ inline F16Scales f16_scales(const F16Operand &o) {
   s.count_mn = int(o.mn ? o.p.CB : o.p.RB);
   return s;
 }
-// C = A B (+ bias) over planes; `t` as for the kernel over TF32 planes, num_kb aside.  Does nothing where a header says wide.
-void gemm_f16_launch(const F16Operand &a, const F16Operand &b, TileArgs t, int64_t K);
+// What the kernel does instead where a header says wide, which only the device knows: every CTA splits its share of both
+// operands into TF32 planes, all wait for one another, and the product goes over those.
+struct F16Fallback {
+  CUtensorMap map_a, map_b; // of the TF32 planes
+  TileArgs t;
+  NatSplitArgs a, b;
+  unsigned int *arrived; // CTAs at the wait; zero between launches
+};
+// C = A B (+ bias) over planes; `t` as for the kernel over TF32 planes, num_kb aside.
+void gemm_f16_launch(const F16Operand &a, const F16Operand &b, TileArgs t, int64_t K, const F16Fallback &f);
 
 } // namespace ntb

@@ -36,7 +36,7 @@
 
 #include "gemm_common.cuh"
 #include "gemm_f16.cuh"
-#include "gemm_tile.cuh"
+#include "gemm_tf32.cuh"
 #include "launch.cuh"
 #include "nt_core.cuh"
 #include "tf32_split.cuh"
@@ -44,14 +44,7 @@
 
 namespace ntb {
 
-constexpr int TC_BK = 16;    // k-block per stage: 16 fp32 = 64 bytes = one 64B-swizzle row
-constexpr int TC_STAGES = 4;
-constexpr int TC_UMMA_K = 8; // tf32: 32 bytes of k per instruction
 constexpr int TC_TMEM_COLS = 512; // two fp32 accumulators of 256 columns: hi*hi, and hi*lo + lo*hi
-constexpr uint32_t TC_A_PLANE_BYTES = TC_BM * TC_BK * 4;  // 8 KB
-constexpr uint32_t TC_B_PLANE_BYTES = TC_BN * TC_BK * 4;  // 16 KB
-constexpr uint32_t TC_STAGE_BYTES = 2 * TC_A_PLANE_BYTES + 2 * TC_B_PLANE_BYTES; // 48 KB
-constexpr uint32_t TC_SMEM_BYTES = TC_STAGES * TC_STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/ + 8 * TC_CORNER_BYTES;
 
 // ---------------------------------------------------------------------------------------------
 // split_pack
@@ -139,38 +132,6 @@ __global__ void __launch_bounds__(256) split_pack(SplitArgs a) {
 }
 
 // ---------------------------------------------------------------------------------------------
-// K-major operand tile in the 64-byte swizzle layout that TMA wrote: rows of 64 bytes, groups of 8
-// rows (512 bytes) back to back.  Fields: start address >> 4 in bits [0,14); leading byte offset >> 4
-// in [16,30) (unused for this layout, set to 1); stride byte offset >> 4 in [32,46) = 512 bytes between
-// 8-row groups; descriptor version 1 in [46,48); layout type SWIZZLE_64B = 4 in [61,64).
-__device__ __forceinline__ uint64_t umma_desc_sw64(uint32_t smem_addr) {
-  uint64_t d = 0;
-  d |= uint64_t((smem_addr & 0x3FFFF) >> 4);
-  d |= uint64_t(1) << 16;
-  d |= uint64_t(512 >> 4) << 32;
-  d |= uint64_t(1) << 46;
-  d |= uint64_t(4) << 61;
-  return d;
-}
-// MN-major operand tile of 32-bit values.  The one shared-memory layout the tensor core accepts for it is
-// the 128-byte swizzle with 32-byte atoms: a row of 128 bytes holds 32 consecutive values of the m (or n)
-// index for one k, the 32-byte chunks of a row are permuted by the row number modulo 4, so 4 rows (512
-// bytes) form one swizzle atom -- what the tensor map mode SWIZZLE_128B_ATOM_32B writes.  An instruction
-// of kind::tf32 consumes 8 values of k = two atoms, `sbo` bytes apart; the atoms of the next 32 m (or n)
-// values lie `lbo` bytes further.  Same field positions as above; layout type 1.
-__device__ __forceinline__ uint64_t umma_desc_mn_sw128(uint32_t smem_addr, uint32_t lbo, uint32_t sbo) {
-  uint64_t d = 0;
-  d |= uint64_t((smem_addr & 0x3FFFF) >> 4);
-  d |= uint64_t((lbo >> 4) & 0x3FFF) << 16;
-  d |= uint64_t((sbo >> 4) & 0x3FFF) << 32;
-  d |= uint64_t(1) << 46;
-  d |= uint64_t(1) << 61;
-  return d;
-}
-// Instruction descriptor, kind::tf32: D format F32 (1) in bits [4,6); A and B format TF32 (2) in [7,10) and
-// [10,13); A and B K-major (0) in bits 15, 16; N >> 3 in [17,23); M >> 4 in [24,29).
-constexpr uint32_t TC_IDESC = (1u << 4) | (2u << 7) | (2u << 10) | (uint32_t(TC_BN >> 3) << 17) | (uint32_t(TC_BM >> 4) << 24);
-
 __device__ __forceinline__ void umma_tf32(uint32_t tmem_d, uint64_t adesc, uint64_t bdesc, uint32_t accumulate, uint32_t lead) {
   umma_tf32_idesc(tmem_d, adesc, bdesc, TC_IDESC, accumulate, lead);
 }
@@ -340,225 +301,11 @@ gemm_3xtf32_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_const
 }
 
 // ---------------------------------------------------------------------------------------------
-// Variant with promoted accumulation (matmul mode 1, the default; the kernel above is mode 3).
-//
-// One persistent CTA per SM walks over the output tiles: the producer runs ahead into the next tile's k-blocks, and the
-// epilogue warps store a tile while the MMA warp works on the next.  With a CTA per tile every tile paid for its own
-// start, pipeline fill and drain (32 x 512^3: two waves of 30 us for 13 us of products; 142 -> 161 TFLOP/s; 8192 x 1024 x
-// 4096 237 -> 266, 4096^3 250 -> 256).
-//
-// The tensor core adds into its fp32 accumulator with round-toward-zero, so a long accumulation chain
-// carries a bias that grows with its length.  Here a chain is only TC_PERIOD_KB k-blocks (256 values of
-// k, 96 MMAs) long: the two 256-column halves of tensor memory alternate as the accumulator of
-// successive periods; while the MMA warp fills one, eight epilogue warps drain the other with
-// tcgen05.ld and add it -- round-to-nearest -- into running sums they keep in registers (128 per
-// thread).  The result has the error of an ordinary fp32 summation (2e-6 of max|C| at K = 4096 and 16384;
-// chains of 128 measured 1e-6 at 3 % more time, one chain per output 1e-5 .. 4e-5).
-constexpr int TC_PERIOD_KB = TC_PERIOD / TC_BK; // k-blocks per accumulation chain
-
-// A_MN / B_MN: the operand's planes keep the source tensor's own row-major order and the contraction
-// index k runs down the rows (A seen as its transpose, B as stored): the tile arrives through a 4-D
-// tensor map {32 m|n, k, (m|n)/32, plane} into 128-byte-swizzle / 32-byte-atom rows and the instruction
-// reads it MN-major.  Otherwise k runs along the rows (K-major): 3-D map, 64-byte swizzle.  Every combination is
-// one instantiation, so forward (A K-major, B MN-major), input gradient (both K-major) and weight
-// gradient (both MN-major) all read planes that were split once, without a transpose.
+// The tiles of gemm_tf32.cuh, the kernel of matmul mode 1 (the kernel above is mode 3).
 template <bool A_MN, bool B_MN>
 __global__ void __launch_bounds__(320, 1)
-gemm_3xtf32_promoted_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, TileArgs g) {
-  constexpr uint32_t IDESC = TC_IDESC | (A_MN ? (1u << 15) : 0u) | (B_MN ? (1u << 16) : 0u);
-  if (g.wide_a) { // behind a product over fp16 planes, which has done it unless one of them is wide
-    pdl_wait();
-    if (!(*g.wide_a | *g.wide_b)) return;
-  }
-  extern __shared__ uint8_t smem_raw[];
-  const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
-  const uint32_t bar_base = smem_base + TC_STAGES * TC_STAGE_BYTES;
-  // full[s] at +8 s, empty[s] at +32 + 8 s, acc_full[b] at +64 + 8 b, acc_empty[b] at +80 + 8 b, tmem slot at +96
-  const uint32_t full0 = bar_base, empty0 = bar_base + 32, acc_full0 = bar_base + 64, acc_empty0 = bar_base + 80;
-  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem_raw + (bar_base - smem_u32(smem_raw)) + 96);
-  volatile int *poison_slot = reinterpret_cast<volatile int *>(tmem_slot + 1);
-
-  const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
-  if (threadIdx.x == 0) {
-    for (int s = 0; s < TC_STAGES; ++s) {
-      mbar_init(full0 + 8 * s, 1);
-      mbar_init(empty0 + 8 * s, 1);
-    }
-    for (int i = 0; i < 2; ++i) {
-      mbar_init(acc_full0 + 8 * i, 1);
-      mbar_init(acc_empty0 + 8 * i, 8); // one arrival per epilogue warp
-    }
-    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
-    *poison_slot = *reinterpret_cast<volatile int *>(g.error_flag); // see gemm_3xtf32_kernel
-    poison_slot[1] = 0; // split-K: an epilogue warp gave up
-  }
-  if (warp == 1) {
-    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512) : "memory");
-    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
-  }
-  tcgen05_fence_before();
-  __syncthreads();
-  tcgen05_fence_after();
-  const uint32_t tmem_acc = __shfl_sync(0xffffffffu, *tmem_slot, 0);
-  const bool poisoned = *poison_slot != 0;
-
-  if (warp == 0) {
-    if (lane == 0 && !poisoned) {
-      uint32_t phase = 0;
-      int s = 0;
-      bool ok = true;
-      for (int w = blockIdx.x; w < g.work && ok; w += gridDim.x) {
-        const TileItem it = tile_item<TC_PERIOD_KB>(g, w);
-        const int m0 = it.tile_m * TC_BM, n0 = it.tile_n * TC_BN, b = it.b;
-        for (int kb = 0; kb < it.nkb; ++kb) {
-          if (!mbar_wait(empty0 + 8 * s, phase ^ 1, g.wait_limit)) {
-            atomicExch(g.error_flag, 1);
-            ok = false;
-            break;
-          }
-          const uint32_t st = smem_base + s * TC_STAGE_BYTES;
-          mbar_expect_tx(full0 + 8 * s, TC_STAGE_BYTES);
-          const int k = (it.kb0 + kb) * TC_BK;
-          if constexpr (A_MN) {
-            tma_load_4d(st, &map_a, full0 + 8 * s, 0, k, m0 >> 5, b);
-            tma_load_4d(st + TC_A_PLANE_BYTES, &map_a, full0 + 8 * s, 0, k, m0 >> 5, g.batch + b);
-          } else {
-            tma_load_3d(st, &map_a, full0 + 8 * s, k, m0, b);
-            tma_load_3d(st + TC_A_PLANE_BYTES, &map_a, full0 + 8 * s, k, m0, g.batch + b);
-          }
-          if constexpr (B_MN) {
-            tma_load_4d(st + 2 * TC_A_PLANE_BYTES, &map_b, full0 + 8 * s, 0, k, n0 >> 5, b);
-            tma_load_4d(st + 2 * TC_A_PLANE_BYTES + TC_B_PLANE_BYTES, &map_b, full0 + 8 * s, 0, k, n0 >> 5, g.batch + b);
-          } else {
-            tma_load_3d(st + 2 * TC_A_PLANE_BYTES, &map_b, full0 + 8 * s, k, n0, b);
-            tma_load_3d(st + 2 * TC_A_PLANE_BYTES + TC_B_PLANE_BYTES, &map_b, full0 + 8 * s, k, n0, g.batch + b);
-          }
-          if (++s == TC_STAGES) {
-            s = 0;
-            phase ^= 1;
-          }
-        }
-      }
-    }
-  } else if (warp == 1) {
-    if (!poisoned) {
-      const uint32_t lead = elect_lane();
-      uint32_t phase = 0;
-      int s = 0;
-      uint32_t done = 0; // periods of the items before
-      bool ok = true;
-      for (int w = blockIdx.x; w < g.work && ok; w += gridDim.x) {
-        const TileItem it = tile_item<TC_PERIOD_KB>(g, w);
-        int kb = 0;
-        for (int q = 0; q < it.periods && ok; ++q) {
-          const uint32_t p = done + q;
-          const int buf = p & 1;
-          // the epilogue must have drained this half (two periods ago) before it is overwritten
-          if (!mbar_wait(acc_empty0 + 8 * buf, ((p >> 1) & 1) ^ 1, g.wait_limit)) {
-            if (lead) atomicExch(g.error_flag, 4);
-            ok = false;
-            break;
-          }
-          tcgen05_fence_after();
-          const uint32_t d = tmem_acc + uint32_t(buf * TC_BN);
-          const int kb_end = min(kb + TC_PERIOD_KB, it.nkb);
-          bool first = true;
-          for (; kb < kb_end; ++kb) {
-            if (!mbar_wait(full0 + 8 * s, phase, g.wait_limit)) {
-              if (lead) atomicExch(g.error_flag, 2);
-              ok = false;
-              break;
-            }
-            tcgen05_fence_after();
-            const uint32_t st = smem_base + s * TC_STAGE_BYTES;
-#pragma unroll
-            for (int ks = 0; ks < TC_BK / TC_UMMA_K; ++ks) {
-              // one instruction consumes 8 values of k: 32 bytes along a K-major row, 8 rows of 128 bytes
-              // of an MN-major tile
-              const uint32_t a_off = A_MN ? ks * 1024u : ks * TC_UMMA_K * 4u;
-              const uint32_t b_off = B_MN ? ks * 1024u : ks * TC_UMMA_K * 4u;
-              const uint32_t pa = st + a_off, pb = st + 2 * TC_A_PLANE_BYTES + b_off;
-              const uint64_t a_hi = A_MN ? umma_desc_mn_sw128(pa, g.mn_lbo, g.mn_sbo) : umma_desc_sw64(pa);
-              const uint64_t a_lo = A_MN ? umma_desc_mn_sw128(pa + TC_A_PLANE_BYTES, g.mn_lbo, g.mn_sbo)
-                                         : umma_desc_sw64(pa + TC_A_PLANE_BYTES);
-              const uint64_t b_hi = B_MN ? umma_desc_mn_sw128(pb, g.mn_lbo, g.mn_sbo) : umma_desc_sw64(pb);
-              const uint64_t b_lo = B_MN ? umma_desc_mn_sw128(pb + TC_B_PLANE_BYTES, g.mn_lbo, g.mn_sbo)
-                                         : umma_desc_sw64(pb + TC_B_PLANE_BYTES);
-              // small terms first, the large one last
-              umma_tf32_idesc(d, a_hi, b_lo, IDESC, first ? 0u : 1u, lead);
-              umma_tf32_idesc(d, a_lo, b_hi, IDESC, 1, lead);
-              umma_tf32_idesc(d, a_hi, b_hi, IDESC, 1, lead);
-              first = false;
-            }
-            umma_commit(empty0 + 8 * s, lead);
-            if (++s == TC_STAGES) {
-              s = 0;
-              phase ^= 1;
-            }
-          }
-          if (ok) umma_commit(acc_full0 + 8 * buf, lead);
-        }
-        done += it.periods;
-      }
-      if (!ok && lead) { // release the epilogue warps from whatever they wait on
-        for (int i = 0; i < 2; ++i)
-          asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(acc_full0 + 8 * i) : "memory");
-      }
-    }
-  } else {
-    // ------------------------------------------------------------------ epilogue, warps 2..9
-    const int quad = warp & 3;          // 32-lane group of tensor memory this warp may read
-    const int half = (warp - 2) >> 2;   // which 128 of the 256 columns
-    // a 32 x 32 corner of the tile on its way from a lane per row to whole 128-byte lines, 16-byte groups swizzled
-    char *corner = reinterpret_cast<char *>(smem_raw + (bar_base - smem_u32(smem_raw))) + 256 + (warp - 2) * TC_CORNER_BYTES;
-    bool ok = !poisoned;
-    uint32_t done = 0; // periods of the items before
-    for (int w = blockIdx.x; w < g.work && ok; w += gridDim.x) {
-      const TileItem it = tile_item<TC_PERIOD_KB>(g, w);
-      float sum[128];
-#pragma unroll
-      for (int i = 0; i < 128; ++i) sum[i] = 0.0f;
-      for (int q = 0; q < it.periods; ++q) {
-        const uint32_t p = done + q;
-        const int buf = p & 1;
-        if (ok && !mbar_wait(acc_full0 + 8 * buf, (p >> 1) & 1, g.wait_limit)) {
-          atomicExch(g.error_flag, 3);
-          ok = false;
-        }
-        if (!ok || *reinterpret_cast<volatile int *>(g.error_flag) != 0) {
-          ok = false;
-          break;
-        }
-        tcgen05_fence_after();
-        const uint32_t taddr = tmem_acc + (uint32_t(quad * 32) << 16) + uint32_t(buf * TC_BN + half * 128);
-#pragma unroll
-        for (int c = 0; c < 4; ++c) {
-          uint32_t v[32];
-          tmem_ld32(taddr + uint32_t(c * 32), v);
-          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
-#pragma unroll
-          for (int e = 0; e < 32; ++e) sum[c * 32 + e] = sum[c * 32 + e] + __uint_as_float(v[e]);
-        }
-        tcgen05_fence_before();
-        __syncwarp();
-        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(acc_empty0 + 8 * buf) : "memory");
-      }
-      done += it.periods;
-      if (!poisoned) finish_tile(g, it, ok, sum, corner, quad, half, lane, poison_slot);
-    }
-  }
-
-  if (!poisoned && *reinterpret_cast<volatile int *>(g.error_flag) != 0) {
-    const long long t0 = clock64();
-    while (clock64() - t0 < 2000000) {
-    }
-  }
-  tcgen05_fence_before();
-  __syncthreads();
-  if (warp == 1) {
-    tcgen05_fence_after();
-    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_acc), "r"(512) : "memory");
-  }
+gemm_3xtf32_promoted_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_constant__ CUtensorMap map_b, const __grid_constant__ TileArgs g) {
+  tf32_tiles<A_MN, B_MN>(map_a, map_b, g);
 }
 
 // ---------------------------------------------------------------------------------------------
@@ -606,6 +353,7 @@ static std::atomic<int> g_tc_panel{panel_default()};
 // tile resets it).  GEMM launches are ordered on the compute stream, so one array serves them all.
 constexpr int64_t TC_MAX_TICKETS = 65536;
 static unsigned int *g_tickets = nullptr;
+static unsigned int *g_grid_barrier = nullptr; // see F16Fallback; behind the tickets
 static int max_splits_default() {
   const char *e = getenv("NT_GEMM_SPLITK");
   if (e && *e) {
@@ -648,7 +396,7 @@ int gemm_tc_take_error() {
   if (cudaMemcpy(&host, flag, sizeof(int), cudaMemcpyDeviceToHost) != cudaSuccess) return -1;
   if (host != 0) {
     cudaMemset(flag, 0, sizeof(int));
-    if (g_tickets) cudaMemset(g_tickets, 0, size_t(TC_MAX_TICKETS) * 4); // tiles that never completed left theirs behind
+    if (g_tickets) cudaMemset(g_tickets, 0, size_t(TC_MAX_TICKETS + 1) * 4); // tiles that never completed left theirs behind
   }
   return host;
 }
@@ -687,8 +435,9 @@ void gemm_tc_prepare() {
     if (is_capturing())
       fail_runtime("gemm_3xtf32: first use inside a graph capture; run the step once eagerly before capturing it.");
     size_t rounded;
-    g_tickets = static_cast<unsigned int *>(device_alloc(size_t(TC_MAX_TICKETS) * 4, &rounded));
-    NT_CUDA_CHECK(cudaMemsetAsync(g_tickets, 0, size_t(TC_MAX_TICKETS) * 4, stream()));
+    g_tickets = static_cast<unsigned int *>(device_alloc(size_t(TC_MAX_TICKETS + 1) * 4, &rounded));
+    g_grid_barrier = g_tickets + TC_MAX_TICKETS;
+    NT_CUDA_CHECK(cudaMemsetAsync(g_tickets, 0, size_t(TC_MAX_TICKETS + 1) * 4, stream()));
   }
 }
 
@@ -727,69 +476,11 @@ void gemm_tc_wait_probe() {
 // inside the capture, so that a replay sees whatever the buffer holds by then.
 // A storage keeps at most PLANE_ENTRIES_PER_STORAGE entries (views at different offsets of one big tensor
 // would otherwise pile up); the least recently used entry that no capture relies on makes room.
-struct NatSplitArgs {
-  const float *src;
-  float *hi, *lo;
-  int64_t R, C, Cp, s_r, s_b;
-  int vec; // rows of the source may be read 128 bits at a time
-  float factor;
-};
-
-// 16 rows of 256 columns
-__device__ __forceinline__ void split_piece(const NatSplitArgs &a, int64_t piece_c, int64_t piece_r, int64_t batch) {
-  const int64_t c = (piece_c * 64 + (threadIdx.x & 63)) * 4;
-  if (c >= a.Cp) return;
-  const int64_t r0 = piece_r * 16 + (threadIdx.x >> 6);
-  const float *src = a.src + batch * a.s_b;
-  const int64_t plane = batch * a.R * a.Cp;
-  float4 x[4];
-#pragma unroll
-  for (int i = 0; i < 4; ++i) { // rows r0, r0 + 4, r0 + 8, r0 + 12: all loads issued before the first use
-    const int64_t r = r0 + 4 * i;
-    x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
-    if (r < a.R) {
-      const float *p = src + r * a.s_r + c;
-      if (a.vec && c + 3 < a.C) {
-        x[i] = __ldg(reinterpret_cast<const float4 *>(p));
-      } else {
-        if (c + 0 < a.C) x[i].x = p[0];
-        if (c + 1 < a.C) x[i].y = p[1];
-        if (c + 2 < a.C) x[i].z = p[2];
-        if (c + 3 < a.C) x[i].w = p[3];
-      }
-      x[i] = make_float4(a.factor * x[i].x, a.factor * x[i].y, a.factor * x[i].z, a.factor * x[i].w);
-    }
-  }
-#pragma unroll
-  for (int i = 0; i < 4; ++i) {
-    const int64_t r = r0 + 4 * i;
-    if (r < a.R) {
-      const int64_t idx = plane + r * a.Cp + c;
-      const float h0 = split_hi(x[i].x), h1 = split_hi(x[i].y), h2 = split_hi(x[i].z), h3 = split_hi(x[i].w);
-      *reinterpret_cast<float4 *>(a.hi + idx) = make_float4(h0, h1, h2, h3);
-      *reinterpret_cast<float4 *>(a.lo + idx) =
-          make_float4(split_lo(x[i].x, h0), split_lo(x[i].y, h1), split_lo(x[i].z, h2), split_lo(x[i].w, h3));
-    }
-  }
-}
-
 __global__ void __launch_bounds__(256) split_planes(NatSplitArgs a) {
   pdl_trigger();
   pdl_wait();
   split_piece(a, blockIdx.x, blockIdx.y, blockIdx.z);
 }
-// Both operands of a product whose fp16 planes are wide; otherwise a launch of CTAs that leave at once (few of them: one
-// for every piece of 4096 x 4096 took 5 us to come and go).
-__global__ void __launch_bounds__(256) split_planes_if_wide(NatSplitArgs a, NatSplitArgs b, int64_t batch, const int *wide_a, const int *wide_b) {
-  pdl_wait();
-  if (!(*wide_a | *wide_b)) return;
-  for (int i = 0; i < 2; ++i) {
-    const NatSplitArgs &s = i ? b : a;
-    const int64_t pc = (s.Cp + 255) / 256, pr = (s.R + 15) / 16;
-    for (int64_t p = blockIdx.x; p < pc * pr * batch; p += gridDim.x) split_piece(s, p % pc, p / pc % pr, p / (pc * pr));
-  }
-}
-
 struct PlaneEntry {
   bool f16; // fp16 planes (f16_split.cuh) or TF32 planes
   int64_t offset, batch, s_b, R, C, s_r; // the view: element offset, batch count / stride, rows, columns, row stride
@@ -1044,7 +735,7 @@ static void launch_promoted(const CUtensorMap &ma, const CUtensorMap &mb, const 
                                        int(TC_SMEM_BYTES)));
     configured = true;
   }
-  launch_with(g.wide_a != nullptr, 1, gemm_3xtf32_promoted_kernel<A_MN, B_MN>, grid, 320, TC_SMEM_BYTES, ma, mb, g);
+  gemm_3xtf32_promoted_kernel<A_MN, B_MN><<<grid, 320, TC_SMEM_BYTES, stream()>>>(ma, mb, g);
 }
 
 // How an operand matrix [P][Q] (strides s_p, s_q) is laid out: unit stride along Q, along P, or neither.
@@ -1070,13 +761,14 @@ KSplit gemm_tc_k_split(int64_t batch, int64_t M, int64_t N, int64_t K) {
   return best;
 }
 
-// Whether a product goes over fp16 planes: three products at twice the rate of TF32, from operands of half the bytes, but
-// two more launches, of kernels that only look whether they are needed (2 us each).  From 2^30 multiply-adds on that pays
-// nearly everywhere: us of a product, and of one with both gradients and two splits, over TF32 planes (or without planes)
-// and over fp16 planes: 2048 x 1024 x 1024 37.7 / 34.0, 154 / 147; 4096 x 512 x 640 23.9 / 21.5, 153 / 139; 300 x 4096 x 1024
-// 61.7 / 54.6, 132 / 121; 4096 x 130 x 2500 28.8 / 29.6, 197 / 181; 2048^3 67.8 / 44.8, 230 / 172; 8192 x 1024 x 4096 252 /
-// 168, 868 / 582.  Below, kernels without planes or on the CUDA cores finish in the time of the launches.  A short extent
-// leaves blocks of 64 x 64 and tiles half empty.
+// Whether a product goes over fp16 planes: three products at twice the rate of TF32, from operands of half the bytes.  From 2^30 multiply-adds on that pays
+// everywhere: us of a product, and of one with both gradients and two splits, over TF32 planes (or without planes) and over
+// fp16 planes: 2048 x 1024 x 1024 37.7 / 29.8, 154 / 112; 4096 x 512 x 640 23.9 / 17.5, 153 / 105; 300 x 4096 x 1024 61.7 /
+// 40.8, 132 / 93; 4096 x 130 x 2500 28.8 / 27.3, 197 / 154; 2048^3 67.8 / 40.5, 230 / 147; 8192 x 1024 x 4096 252 / 163, 868 /
+// 567.  Below, kernels without planes or on the CUDA cores are as fast, and the kernel without planes has the bits of the one
+// over TF32 planes.  A short extent leaves blocks of 64 x 64 and tiles half empty.
+// Where an operand turns out to be wide the same launch splits both again and goes over TF32 planes, 2048^3 133 us instead of
+// 71, 4096^3 729 instead of 537; one matrix of 67 million normally distributed values in a hundred is.
 bool gemm_f16_wanted(int64_t batch, int64_t M, int64_t N, int64_t K) {
   return std::min({M, N, K}) >= 128 && double(batch) * double(M) * double(N) * double(K) > double(int64_t(1) << 30);
 }
@@ -1084,14 +776,14 @@ bool gemm_f16_wanted(int64_t batch, int64_t M, int64_t N, int64_t K) {
 // Expected time of a product through planes: half a microsecond per 16-deep k-block of a tile, one tile per SM at a time;
 // 11 us around it (pipeline fill, epilogue, one operand split); 4.5 us per part for the finish of a k-split.  Measured, with
 // one split: 256 x 64 x 256 14 us, 784 x 256 x 256 20, 1024 x 512 x 512 26, 1024^3 40, 100 x 2000 x 60 (4 parts) 44.
-// Over fp16 planes half of that per k-block, 6 us for the end of every tile of a CTA and 4 for the launches behind it: 2048^3
-// 45 us, 32 x 512^3 41, 8192 x 1024 x 4096 168.
+// Over fp16 planes half of that per k-block and 6 us for the end of every tile of a CTA; with no split, 2048^3 takes 41 us, 32 x
+// 512^3 32, 8192 x 1024 x 4096 163, 1056 x 1024 x 1024 29.
 double gemm_tc_expected_us(int64_t batch, int64_t M, int64_t N, int64_t K, bool f16) {
   const int64_t tiles = ceil_div(M, TC_BM) * ceil_div(N, TC_BN) * batch, num_kb = ceil_div(K, TC_BK);
   const KSplit ks = gemm_tc_k_split(batch, M, N, K);
   const double waves = double(ceil_div(tiles * ks.splits, sm_count()));
   const double kb = double(ks.splits > 1 ? ks.kb_per_split : num_kb);
-  return (f16 ? 13.0 + waves * (kb * 0.26 + 6.0) : 11.0 + waves * kb * 0.5) + (ks.splits > 1 ? 4.5 * ks.splits : 0.0);
+  return (f16 ? 9.0 + waves * (kb * 0.26 + 6.0) : 11.0 + waves * kb * 0.5) + (ks.splits > 1 ? 4.5 * ks.splits : 0.0);
 }
 
 // A product over natural-layout planes.  Returns false when an operand has no
@@ -1169,32 +861,32 @@ bool gemm_3xtf32_natural(nt_storage *sa, int64_t a_off, nt_storage *sb, int64_t 
     g.work = int32_t(tiles_m * tiles_n * g.splits * batch);
     const dim3 grid{unsigned(std::min(g.work, sm_count())), 1, 1};
     matmul_profile_begin();
-    float *ta = static_cast<float *>(pa), *tb = static_cast<float *>(pb);
     if (f16) {
       const F16Operand oa{f16_planes_at(pa, batch, aR, aC), aR, aC, a_mn}, ob{f16_planes_at(pb, batch, bR, bC), bR, bC, b_mn};
-      gemm_f16_launch(oa, ob, g, K);
-      // what it left alone because an operand is wide: both operands split again, into TF32 planes, and multiplied
+      // what the kernel takes instead where an operand is wide: both split again, into TF32 planes
       for (PlaneEntry *e : {&ea, &eb}) {
         e->Cp = ceil_div(e->C, 32) * 32;
         plane_memory(*e);
       }
-      aCp = ea.Cp;
-      bCp = eb.Cp;
-      ta = static_cast<float *>(ea.planes);
-      tb = static_cast<float *>(eb.planes);
-      g.wide_a = &oa.p.header->wide;
-      g.wide_b = &ob.p.header->wide;
-      launch(split_planes_if_wide, unsigned(4 * sm_count()), 256, 0, split_args(sa, ea), split_args(sb, eb), batch, g.wide_a, g.wide_b);
-      check_launch("split_planes_if_wide");
+      F16Fallback f{};
+      f.t = g;
+      f.a = split_args(sa, ea);
+      f.b = split_args(sb, eb);
+      f.arrived = g_grid_barrier;
+      f.map_a = a_mn ? make_map_mn(f.a.hi, aR, ea.Cp, 2 * batch, TC_BM) : make_map_k(f.a.hi, aR, K, ea.Cp, 2 * batch, TC_BM);
+      f.map_b = b_mn ? make_map_mn(f.b.hi, bR, eb.Cp, 2 * batch, TC_BN) : make_map_k(f.b.hi, bR, K, eb.Cp, 2 * batch, TC_BN);
+      gemm_f16_launch(oa, ob, g, K, f);
+    } else {
+      float *ta = static_cast<float *>(pa), *tb = static_cast<float *>(pb);
+      const CUtensorMap map_a = a_mn ? make_map_mn(ta, aR, aCp, 2 * batch, TC_BM) : make_map_k(ta, aR, K, aCp, 2 * batch, TC_BM);
+      const CUtensorMap map_b = b_mn ? make_map_mn(tb, bR, bCp, 2 * batch, TC_BN) : make_map_k(tb, bR, K, bCp, 2 * batch, TC_BN);
+      if (a_mn && b_mn) launch_promoted<true, true>(map_a, map_b, g, grid);
+      else if (a_mn) launch_promoted<true, false>(map_a, map_b, g, grid);
+      else if (b_mn) launch_promoted<false, true>(map_a, map_b, g, grid);
+      else launch_promoted<false, false>(map_a, map_b, g, grid);
+      check_launch("gemm_3xtf32_promoted_kernel");
     }
-    const CUtensorMap map_a = a_mn ? make_map_mn(ta, aR, aCp, 2 * batch, TC_BM) : make_map_k(ta, aR, K, aCp, 2 * batch, TC_BM);
-    const CUtensorMap map_b = b_mn ? make_map_mn(tb, bR, bCp, 2 * batch, TC_BN) : make_map_k(tb, bR, K, bCp, 2 * batch, TC_BN);
-    if (a_mn && b_mn) launch_promoted<true, true>(map_a, map_b, g, grid);
-    else if (a_mn) launch_promoted<true, false>(map_a, map_b, g, grid);
-    else if (b_mn) launch_promoted<false, true>(map_a, map_b, g, grid);
-    else launch_promoted<false, false>(map_a, map_b, g, grid);
     matmul_profile_end();
-    check_launch("gemm_3xtf32_promoted_kernel");
   } catch (...) {
     free_all();
     throw;

@@ -1,0 +1,319 @@
+// The products over TF32 planes with promoted accumulation: what a CTA of gemm_tc.cu's kernel does, and one of gemm_f16.cu's
+// where an operand has no fp16 planes.
+#pragma once
+
+#include <cuda.h>
+
+#include <cstdint>
+
+#include "gemm_common.cuh"
+#include "gemm_tile.cuh"
+#include "tf32_split.cuh"
+#include "tma.cuh"
+
+namespace ntb {
+
+constexpr int TC_BK = 16;    // k-block per stage: 16 fp32 = 64 bytes = one 64B-swizzle row
+constexpr int TC_STAGES = 4;
+constexpr int TC_UMMA_K = 8; // tf32: 32 bytes of k per instruction
+constexpr uint32_t TC_A_PLANE_BYTES = TC_BM * TC_BK * 4;  // 8 KB
+constexpr uint32_t TC_B_PLANE_BYTES = TC_BN * TC_BK * 4;  // 16 KB
+constexpr uint32_t TC_STAGE_BYTES = 2 * TC_A_PLANE_BYTES + 2 * TC_B_PLANE_BYTES; // 48 KB
+constexpr uint32_t TC_SMEM_BYTES = TC_STAGES * TC_STAGE_BYTES + 1024 /*align*/ + 256 /*barriers*/ + 8 * TC_CORNER_BYTES;
+
+// K-major operand tile in the 64-byte swizzle layout that TMA wrote: rows of 64 bytes, groups of 8
+// rows (512 bytes) back to back.  Fields: start address >> 4 in bits [0,14); leading byte offset >> 4
+// in [16,30) (unused for this layout, set to 1); stride byte offset >> 4 in [32,46) = 512 bytes between
+// 8-row groups; descriptor version 1 in [46,48); layout type SWIZZLE_64B = 4 in [61,64).
+__device__ __forceinline__ uint64_t umma_desc_sw64(uint32_t smem_addr) {
+  uint64_t d = 0;
+  d |= uint64_t((smem_addr & 0x3FFFF) >> 4);
+  d |= uint64_t(1) << 16;
+  d |= uint64_t(512 >> 4) << 32;
+  d |= uint64_t(1) << 46;
+  d |= uint64_t(4) << 61;
+  return d;
+}
+// MN-major operand tile of 32-bit values.  The one shared-memory layout the tensor core accepts for it is
+// the 128-byte swizzle with 32-byte atoms: a row of 128 bytes holds 32 consecutive values of the m (or n)
+// index for one k, the 32-byte chunks of a row are permuted by the row number modulo 4, so 4 rows (512
+// bytes) form one swizzle atom -- what the tensor map mode SWIZZLE_128B_ATOM_32B writes.  An instruction
+// of kind::tf32 consumes 8 values of k = two atoms, `sbo` bytes apart; the atoms of the next 32 m (or n)
+// values lie `lbo` bytes further.  Same field positions as above; layout type 1.
+__device__ __forceinline__ uint64_t umma_desc_mn_sw128(uint32_t smem_addr, uint32_t lbo, uint32_t sbo) {
+  uint64_t d = 0;
+  d |= uint64_t((smem_addr & 0x3FFFF) >> 4);
+  d |= uint64_t((lbo >> 4) & 0x3FFF) << 16;
+  d |= uint64_t((sbo >> 4) & 0x3FFF) << 32;
+  d |= uint64_t(1) << 46;
+  d |= uint64_t(1) << 61;
+  return d;
+}
+// Instruction descriptor, kind::tf32: D format F32 (1) in bits [4,6); A and B format TF32 (2) in [7,10) and
+// [10,13); A and B K-major (0) in bits 15, 16; N >> 3 in [17,23); M >> 4 in [24,29).
+constexpr uint32_t TC_IDESC = (1u << 4) | (2u << 7) | (2u << 10) | (uint32_t(TC_BN >> 3) << 17) | (uint32_t(TC_BM >> 4) << 24);
+
+struct NatSplitArgs {
+  const float *src;
+  float *hi, *lo;
+  int64_t R, C, Cp, s_r, s_b;
+  int vec; // rows of the source may be read 128 bits at a time
+  float factor;
+};
+
+// 16 rows of 256 columns
+__device__ __forceinline__ void split_piece(const NatSplitArgs &a, int64_t piece_c, int64_t piece_r, int64_t batch) {
+  const int64_t c = (piece_c * 64 + (threadIdx.x & 63)) * 4;
+  if (c >= a.Cp) return;
+  const int64_t r0 = piece_r * 16 + (threadIdx.x >> 6);
+  const float *src = a.src + batch * a.s_b;
+  const int64_t plane = batch * a.R * a.Cp;
+  float4 x[4];
+#pragma unroll
+  for (int i = 0; i < 4; ++i) { // rows r0, r0 + 4, r0 + 8, r0 + 12: all loads issued before the first use
+    const int64_t r = r0 + 4 * i;
+    x[i] = make_float4(0.f, 0.f, 0.f, 0.f);
+    if (r < a.R) {
+      const float *p = src + r * a.s_r + c;
+      if (a.vec && c + 3 < a.C) {
+        x[i] = __ldg(reinterpret_cast<const float4 *>(p));
+      } else {
+        if (c + 0 < a.C) x[i].x = p[0];
+        if (c + 1 < a.C) x[i].y = p[1];
+        if (c + 2 < a.C) x[i].z = p[2];
+        if (c + 3 < a.C) x[i].w = p[3];
+      }
+      x[i] = make_float4(a.factor * x[i].x, a.factor * x[i].y, a.factor * x[i].z, a.factor * x[i].w);
+    }
+  }
+#pragma unroll
+  for (int i = 0; i < 4; ++i) {
+    const int64_t r = r0 + 4 * i;
+    if (r < a.R) {
+      const int64_t idx = plane + r * a.Cp + c;
+      const float h0 = split_hi(x[i].x), h1 = split_hi(x[i].y), h2 = split_hi(x[i].z), h3 = split_hi(x[i].w);
+      *reinterpret_cast<float4 *>(a.hi + idx) = make_float4(h0, h1, h2, h3);
+      *reinterpret_cast<float4 *>(a.lo + idx) =
+          make_float4(split_lo(x[i].x, h0), split_lo(x[i].y, h1), split_lo(x[i].z, h2), split_lo(x[i].w, h3));
+    }
+  }
+}
+
+// Matmul mode 1, the default.
+//
+// One persistent CTA per SM walks over the output tiles: the producer runs ahead into the next tile's k-blocks, and the
+// epilogue warps store a tile while the MMA warp works on the next.  With a CTA per tile every tile paid for its own
+// start, pipeline fill and drain (32 x 512^3: two waves of 30 us for 13 us of products; 142 -> 161 TFLOP/s; 8192 x 1024 x
+// 4096 237 -> 266, 4096^3 250 -> 256).
+//
+// The tensor core adds into its fp32 accumulator with round-toward-zero, so a long accumulation chain
+// carries a bias that grows with its length.  Here a chain is only TC_PERIOD_KB k-blocks (256 values of
+// k, 96 MMAs) long: the two 256-column halves of tensor memory alternate as the accumulator of
+// successive periods; while the MMA warp fills one, eight epilogue warps drain the other with
+// tcgen05.ld and add it -- round-to-nearest -- into running sums they keep in registers (128 per
+// thread).  The result has the error of an ordinary fp32 summation (2e-6 of max|C| at K = 4096 and 16384;
+// chains of 128 measured 1e-6 at 3 % more time, one chain per output 1e-5 .. 4e-5).
+constexpr int TC_PERIOD_KB = TC_PERIOD / TC_BK; // k-blocks per accumulation chain
+
+// A_MN / B_MN: the operand's planes keep the source tensor's own row-major order and the contraction
+// index k runs down the rows (A seen as its transpose, B as stored): the tile arrives through a 4-D
+// tensor map {32 m|n, k, (m|n)/32, plane} into 128-byte-swizzle / 32-byte-atom rows and the instruction
+// reads it MN-major.  Otherwise k runs along the rows (K-major): 3-D map, 64-byte swizzle.  Every combination is
+// one instantiation, so forward (A K-major, B MN-major), input gradient (both K-major) and weight
+// gradient (both MN-major) all read planes that were split once, without a transpose.
+// For CTAs of at least 320 threads, with TC_SMEM_BYTES of shared memory.
+template <bool A_MN, bool B_MN>
+__device__ __forceinline__ void tf32_tiles(const CUtensorMap &map_a, const CUtensorMap &map_b, const TileArgs &g) {
+  constexpr uint32_t IDESC = TC_IDESC | (A_MN ? (1u << 15) : 0u) | (B_MN ? (1u << 16) : 0u);
+  extern __shared__ uint8_t smem_raw[];
+  const uint32_t smem_base = (smem_u32(smem_raw) + 1023u) & ~1023u;
+  const uint32_t bar_base = smem_base + TC_STAGES * TC_STAGE_BYTES;
+  // full[s] at +8 s, empty[s] at +32 + 8 s, acc_full[b] at +64 + 8 b, acc_empty[b] at +80 + 8 b, tmem slot at +96
+  const uint32_t full0 = bar_base, empty0 = bar_base + 32, acc_full0 = bar_base + 64, acc_empty0 = bar_base + 80;
+  uint32_t *tmem_slot = reinterpret_cast<uint32_t *>(smem_raw + (bar_base - smem_u32(smem_raw)) + 96);
+  volatile int *poison_slot = reinterpret_cast<volatile int *>(tmem_slot + 1);
+
+  const int warp = __shfl_sync(0xffffffffu, int(threadIdx.x >> 5), 0), lane = threadIdx.x & 31;
+  if (threadIdx.x == 0) {
+    for (int s = 0; s < TC_STAGES; ++s) {
+      mbar_init(full0 + 8 * s, 1);
+      mbar_init(empty0 + 8 * s, 1);
+    }
+    for (int i = 0; i < 2; ++i) {
+      mbar_init(acc_full0 + 8 * i, 1);
+      mbar_init(acc_empty0 + 8 * i, 8); // one arrival per epilogue warp
+    }
+    asm volatile("fence.mbarrier_init.release.cluster;" ::: "memory");
+    *poison_slot = *reinterpret_cast<volatile int *>(g.error_flag); // see gemm_3xtf32_kernel
+    poison_slot[1] = 0; // split-K: an epilogue warp gave up
+  }
+  if (warp == 1) {
+    asm volatile("tcgen05.alloc.cta_group::1.sync.aligned.shared::cta.b32 [%0], %1;" ::"r"(smem_u32(tmem_slot)), "r"(512) : "memory");
+    asm volatile("tcgen05.relinquish_alloc_permit.cta_group::1.sync.aligned;" ::: "memory");
+  }
+  tcgen05_fence_before();
+  __syncthreads();
+  tcgen05_fence_after();
+  const uint32_t tmem_acc = __shfl_sync(0xffffffffu, *tmem_slot, 0);
+  const bool poisoned = *poison_slot != 0;
+
+  if (warp == 0) {
+    if (lane == 0 && !poisoned) {
+      uint32_t phase = 0;
+      int s = 0;
+      bool ok = true;
+      for (int w = blockIdx.x; w < g.work && ok; w += gridDim.x) {
+        const TileItem it = tile_item<TC_PERIOD_KB>(g, w);
+        const int m0 = it.tile_m * TC_BM, n0 = it.tile_n * TC_BN, b = it.b;
+        for (int kb = 0; kb < it.nkb; ++kb) {
+          if (!mbar_wait(empty0 + 8 * s, phase ^ 1, g.wait_limit)) {
+            atomicExch(g.error_flag, 1);
+            ok = false;
+            break;
+          }
+          const uint32_t st = smem_base + s * TC_STAGE_BYTES;
+          mbar_expect_tx(full0 + 8 * s, TC_STAGE_BYTES);
+          const int k = (it.kb0 + kb) * TC_BK;
+          if constexpr (A_MN) {
+            tma_load_4d(st, &map_a, full0 + 8 * s, 0, k, m0 >> 5, b);
+            tma_load_4d(st + TC_A_PLANE_BYTES, &map_a, full0 + 8 * s, 0, k, m0 >> 5, g.batch + b);
+          } else {
+            tma_load_3d(st, &map_a, full0 + 8 * s, k, m0, b);
+            tma_load_3d(st + TC_A_PLANE_BYTES, &map_a, full0 + 8 * s, k, m0, g.batch + b);
+          }
+          if constexpr (B_MN) {
+            tma_load_4d(st + 2 * TC_A_PLANE_BYTES, &map_b, full0 + 8 * s, 0, k, n0 >> 5, b);
+            tma_load_4d(st + 2 * TC_A_PLANE_BYTES + TC_B_PLANE_BYTES, &map_b, full0 + 8 * s, 0, k, n0 >> 5, g.batch + b);
+          } else {
+            tma_load_3d(st + 2 * TC_A_PLANE_BYTES, &map_b, full0 + 8 * s, k, n0, b);
+            tma_load_3d(st + 2 * TC_A_PLANE_BYTES + TC_B_PLANE_BYTES, &map_b, full0 + 8 * s, k, n0, g.batch + b);
+          }
+          if (++s == TC_STAGES) {
+            s = 0;
+            phase ^= 1;
+          }
+        }
+      }
+    }
+  } else if (warp == 1) {
+    if (!poisoned) {
+      const uint32_t lead = elect_lane();
+      uint32_t phase = 0;
+      int s = 0;
+      uint32_t done = 0; // periods of the items before
+      bool ok = true;
+      for (int w = blockIdx.x; w < g.work && ok; w += gridDim.x) {
+        const TileItem it = tile_item<TC_PERIOD_KB>(g, w);
+        int kb = 0;
+        for (int q = 0; q < it.periods && ok; ++q) {
+          const uint32_t p = done + q;
+          const int buf = p & 1;
+          // the epilogue must have drained this half (two periods ago) before it is overwritten
+          if (!mbar_wait(acc_empty0 + 8 * buf, ((p >> 1) & 1) ^ 1, g.wait_limit)) {
+            if (lead) atomicExch(g.error_flag, 4);
+            ok = false;
+            break;
+          }
+          tcgen05_fence_after();
+          const uint32_t d = tmem_acc + uint32_t(buf * TC_BN);
+          const int kb_end = min(kb + TC_PERIOD_KB, it.nkb);
+          bool first = true;
+          for (; kb < kb_end; ++kb) {
+            if (!mbar_wait(full0 + 8 * s, phase, g.wait_limit)) {
+              if (lead) atomicExch(g.error_flag, 2);
+              ok = false;
+              break;
+            }
+            tcgen05_fence_after();
+            const uint32_t st = smem_base + s * TC_STAGE_BYTES;
+#pragma unroll
+            for (int ks = 0; ks < TC_BK / TC_UMMA_K; ++ks) {
+              // one instruction consumes 8 values of k: 32 bytes along a K-major row, 8 rows of 128 bytes
+              // of an MN-major tile
+              const uint32_t a_off = A_MN ? ks * 1024u : ks * TC_UMMA_K * 4u;
+              const uint32_t b_off = B_MN ? ks * 1024u : ks * TC_UMMA_K * 4u;
+              const uint32_t pa = st + a_off, pb = st + 2 * TC_A_PLANE_BYTES + b_off;
+              const uint64_t a_hi = A_MN ? umma_desc_mn_sw128(pa, g.mn_lbo, g.mn_sbo) : umma_desc_sw64(pa);
+              const uint64_t a_lo = A_MN ? umma_desc_mn_sw128(pa + TC_A_PLANE_BYTES, g.mn_lbo, g.mn_sbo)
+                                         : umma_desc_sw64(pa + TC_A_PLANE_BYTES);
+              const uint64_t b_hi = B_MN ? umma_desc_mn_sw128(pb, g.mn_lbo, g.mn_sbo) : umma_desc_sw64(pb);
+              const uint64_t b_lo = B_MN ? umma_desc_mn_sw128(pb + TC_B_PLANE_BYTES, g.mn_lbo, g.mn_sbo)
+                                         : umma_desc_sw64(pb + TC_B_PLANE_BYTES);
+              // small terms first, the large one last
+              umma_tf32_idesc(d, a_hi, b_lo, IDESC, first ? 0u : 1u, lead);
+              umma_tf32_idesc(d, a_lo, b_hi, IDESC, 1, lead);
+              umma_tf32_idesc(d, a_hi, b_hi, IDESC, 1, lead);
+              first = false;
+            }
+            umma_commit(empty0 + 8 * s, lead);
+            if (++s == TC_STAGES) {
+              s = 0;
+              phase ^= 1;
+            }
+          }
+          if (ok) umma_commit(acc_full0 + 8 * buf, lead);
+        }
+        done += it.periods;
+      }
+      if (!ok && lead) { // release the epilogue warps from whatever they wait on
+        for (int i = 0; i < 2; ++i)
+          asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(acc_full0 + 8 * i) : "memory");
+      }
+    }
+  } else if (warp < 10) {
+    // ------------------------------------------------------------------ epilogue, warps 2..9
+    const int quad = warp & 3;          // 32-lane group of tensor memory this warp may read
+    const int half = (warp - 2) >> 2;   // which 128 of the 256 columns
+    // a 32 x 32 corner of the tile on its way from a lane per row to whole 128-byte lines, 16-byte groups swizzled
+    char *corner = reinterpret_cast<char *>(smem_raw + (bar_base - smem_u32(smem_raw))) + 256 + (warp - 2) * TC_CORNER_BYTES;
+    bool ok = !poisoned;
+    uint32_t done = 0; // periods of the items before
+    for (int w = blockIdx.x; w < g.work && ok; w += gridDim.x) {
+      const TileItem it = tile_item<TC_PERIOD_KB>(g, w);
+      float sum[128];
+#pragma unroll
+      for (int i = 0; i < 128; ++i) sum[i] = 0.0f;
+      for (int q = 0; q < it.periods; ++q) {
+        const uint32_t p = done + q;
+        const int buf = p & 1;
+        if (ok && !mbar_wait(acc_full0 + 8 * buf, (p >> 1) & 1, g.wait_limit)) {
+          atomicExch(g.error_flag, 3);
+          ok = false;
+        }
+        if (!ok || *reinterpret_cast<volatile int *>(g.error_flag) != 0) {
+          ok = false;
+          break;
+        }
+        tcgen05_fence_after();
+        const uint32_t taddr = tmem_acc + (uint32_t(quad * 32) << 16) + uint32_t(buf * TC_BN + half * 128);
+#pragma unroll
+        for (int c = 0; c < 4; ++c) {
+          uint32_t v[32];
+          tmem_ld32(taddr + uint32_t(c * 32), v);
+          asm volatile("tcgen05.wait::ld.sync.aligned;" ::: "memory");
+#pragma unroll
+          for (int e = 0; e < 32; ++e) sum[c * 32 + e] = sum[c * 32 + e] + __uint_as_float(v[e]);
+        }
+        tcgen05_fence_before();
+        __syncwarp();
+        if (lane == 0) asm volatile("mbarrier.arrive.shared::cta.b64 _, [%0];" ::"r"(acc_empty0 + 8 * buf) : "memory");
+      }
+      done += it.periods;
+      if (!poisoned) finish_tile(g, it, ok, sum, corner, quad, half, lane, int(threadIdx.x) - 64, poison_slot);
+    }
+  }
+
+  if (!poisoned && *reinterpret_cast<volatile int *>(g.error_flag) != 0) {
+    const long long t0 = clock64();
+    while (clock64() - t0 < 2000000) {
+    }
+  }
+  tcgen05_fence_before();
+  __syncthreads();
+  if (warp == 1) {
+    tcgen05_fence_after();
+    asm volatile("tcgen05.dealloc.cta_group::1.sync.aligned.b32 %0, %1;" ::"r"(tmem_acc), "r"(512) : "memory");
+  }
+}
+
+} // namespace ntb

@@ -30,9 +30,6 @@ struct TileArgs {
   unsigned int *tickets;
   int32_t tiles_m, tiles_n; // output tiles of one batch
   int32_t work;             // tiles x splits x batches; a CTA takes items blockIdx.x, + gridDim.x, ...
-  // Whether either operand has a block that two fp16 numbers per value do not hold (gemm_f16.cu), one flag per operand: the
-  // kernel over fp16 planes leaves such a product alone, and the TF32 launches behind it, which have these set, do it.
-  const int *wide_a, *wide_b;
 };
 
 // Output tile of a work item.  CTAs take items in the order of their index, one wave after the other; taking the n-tiles
@@ -73,12 +70,15 @@ template <int PERIOD_KB> __device__ __forceinline__ TileItem tile_item(const Til
   return it;
 }
 
-// The end of a tile in an epilogue warp (eight of them, threads 64..319 of the CTA): `sum` holds 128 columns (`half`) of the
-// row `lane` of the warp's 32 (`quad`).  `corner`: the warp's TC_CORNER_BYTES of shared memory, a 32 x 32 corner of the
-// tile on its way from a lane per row to whole 128-byte lines, 16-byte groups swizzled.  slots[1]: an epilogue warp gave up;
-// slots[2]: the ticket drawn.
+// The end of a tile in an epilogue warp (eight of them; `et` is the thread's number among their 256): `sum` holds 128 columns
+// (`half`) of the row `lane` of the warp's 32 (`quad`).  `corner`: the warp's TC_CORNER_BYTES of shared memory, a 32 x 32
+// corner of the tile on its way from a lane per row to whole 128-byte lines, 16-byte groups swizzled.  slots[1]: an epilogue
+// warp gave up; slots[2]: the ticket drawn.
+// 5000 clocks, and 8000 when all SMs store at once, of which a next tile's first two chains hide 3700.  What was tried: pieces
+// through the copy engine (32 rows of 64 bytes, two on their way: 10800), whole rows of 512 bytes per instruction (13000), 256-
+// bit stores from the registers (as long).
 __device__ __forceinline__ void finish_tile(const TileArgs &g, const TileItem &it, bool ok, float (&sum)[128], char *corner, int quad,
-                                            int half, int lane, volatile int *slots) {
+                                            int half, int lane, int et, volatile int *slots) {
   const int m0 = it.tile_m * TC_BM, n0 = it.tile_n * TC_BN, b = it.b;
   const int64_t m = int64_t(m0) + quad * 32 + lane;
   bool last = ok; // this CTA finishes the tile
@@ -88,7 +88,6 @@ __device__ __forceinline__ void finish_tile(const TileArgs &g, const TileItem &i
     // epilogue warps pass the two barriers whatever happened to them; a warp whose wait ran out says so.
     volatile int *fail_slot = slots + 1;
     volatile unsigned int *ticket_slot = reinterpret_cast<volatile unsigned int *>(slots + 2);
-    const int et = int(threadIdx.x) - 64; // 0..255 among the epilogue threads
     const int64_t tile_lin = (int64_t(b) * g.tiles_m + it.tile_m) * g.tiles_n + it.tile_n;
     float *mine = g.partials + ((tile_lin * g.splits + it.split) * 32 * 256 + et) * 4;
     if (!ok) *fail_slot = 1;
