@@ -95,7 +95,7 @@ __device__ __forceinline__ bool grid_wait(unsigned int *arrived, int *error_flag
     const long long t0 = clock64();
     while ((all = *reinterpret_cast<volatile unsigned int *>(arrived) >= gridDim.x) == false && clock64() - t0 <= limit) {
     }
-    if (!all) atomicExch(error_flag, 6);
+    if (!all) atomicExch(error_flag, 7);
     else if (atomicAdd(arrived, 1u) == 2 * gridDim.x - 1) *arrived = 0; // the last to leave
     __threadfence();
   }
@@ -261,7 +261,7 @@ gemm_3xf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
     const int quad = warp & 3;        // 32-lane group of tensor memory this warp may read
     const int half = warp >> 2;       // which 128 of the 256 columns
     char *corner = reinterpret_cast<char *>(smem_raw + (bar_base - smem_u32(smem_raw))) + 256 + warp * TC_CORNER_BYTES;
-    bool ok = !poisoned;
+    bool ok = !poisoned, reached = false;
     uint32_t done = 0; // chains of the items before
     for (int w = blockIdx.x; w < g.work && ok; w += gridDim.x) {
       const TileItem it = tile_item<FH_CHAIN>(g, w);
@@ -307,7 +307,9 @@ gemm_3xf16_kernel(const __grid_constant__ CUtensorMap map_a, const __grid_consta
       // chain the tensor cores waited for the epilogue (63 % busy).
       ok = ok && *reinterpret_cast<volatile int *>(g.error_flag) == 0;
       if (!poisoned) finish_tile(g, it, ok, sum, corner, quad, half, lane, int(threadIdx.x), poison_slot);
+      reached = reached || it.shared >= 0;
     }
+    if (!poisoned && !ok) give_up_tile(g, reached, poison_slot);
   }
 
   if (!poisoned && *reinterpret_cast<volatile int *>(g.error_flag) != 0) {

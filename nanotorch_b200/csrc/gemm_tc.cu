@@ -773,6 +773,26 @@ bool gemm_f16_wanted(int64_t batch, int64_t M, int64_t N, int64_t K) {
   return std::min({M, N, K}) >= 128 && double(batch) * double(M) * double(N) * double(K) > double(int64_t(1) << 30);
 }
 
+// Over fp16 planes: the tiles that do not fill a wave of SMs -- all of them, where there are few, or those left over by whole
+// waves -- in parts along k, as many as take up to all SMs at once.  4096^3 has 512 tiles, 68 of them beyond three waves of
+// 148; in two parts they take half a tile's time on all SMs (with both gradients 1017-1113 us, 947-1087 so; 2048 x 4100 x 2500
+// 134 / 114).  A part of 512 of k at least, and 12 us saved at 0.26 us per 16 of k: the sums of the parts take some 10 (3000 x
+// 600 x 700 in parts of 512 and 88 30 us, 20 in one).  Not over TF32 planes, whose products have the bits of the kernel without
+// planes (and gemm_tc_k_split's parts).
+static KSplit gemm_f16_k_split(int64_t tiles, int64_t K, int64_t *whole) {
+  KSplit best;
+  const int64_t sms = sm_count(), left = tiles % sms, num_kb = ceil_div(K, TC_BK);
+  const int max_splits = g_tc_max_splits.load(std::memory_order_relaxed);
+  for (int sp = 2; sp <= max_splits && left > 0 && left * sp <= sms; ++sp) {
+    const int per = int(ceil_div(ceil_div(num_kb, int64_t(sp)), int64_t(TC_PERIOD_KB))) * TC_PERIOD_KB;
+    if (per < 2 * TC_PERIOD_KB || int64_t(sp - 1) * per >= num_kb || double(num_kb - per) * 0.26 < 12.0) continue;
+    best.splits = sp;
+    best.kb_per_split = per;
+  }
+  *whole = best.splits > 1 ? tiles - left : tiles;
+  return best;
+}
+
 // Expected time of a product through planes: half a microsecond per 16-deep k-block of a tile, one tile per SM at a time;
 // 11 us around it (pipeline fill, epilogue, one operand split); 4.5 us per part for the finish of a k-split.  Measured, with
 // one split: 256 x 64 x 256 14 us, 784 x 256 x 256 20, 1024 x 512 x 512 26, 1024^3 40, 100 x 2000 x 60 (4 parts) 44.
@@ -780,10 +800,14 @@ bool gemm_f16_wanted(int64_t batch, int64_t M, int64_t N, int64_t K) {
 // 512^3 32, 8192 x 1024 x 4096 163, 1056 x 1024 x 1024 29.
 double gemm_tc_expected_us(int64_t batch, int64_t M, int64_t N, int64_t K, bool f16) {
   const int64_t tiles = ceil_div(M, TC_BM) * ceil_div(N, TC_BN) * batch, num_kb = ceil_div(K, TC_BK);
+  if (f16) {
+    int64_t whole;
+    const KSplit ks = gemm_f16_k_split(tiles, K, &whole);
+    return 9.0 + double(ceil_div(whole, sm_count())) * (double(num_kb) * 0.26 + 6.0) + (ks.splits > 1 ? double(ks.kb_per_split) * 0.26 + 12.0 : 0.0);
+  }
   const KSplit ks = gemm_tc_k_split(batch, M, N, K);
   const double waves = double(ceil_div(tiles * ks.splits, sm_count()));
-  const double kb = double(ks.splits > 1 ? ks.kb_per_split : num_kb);
-  return (f16 ? 9.0 + waves * (kb * 0.26 + 6.0) : 11.0 + waves * kb * 0.5) + (ks.splits > 1 ? 4.5 * ks.splits : 0.0);
+  return 11.0 + waves * double(ks.splits > 1 ? ks.kb_per_split : num_kb) * 0.5 + (ks.splits > 1 ? 4.5 * ks.splits : 0.0);
 }
 
 // A product over natural-layout planes.  Returns false when an operand has no
@@ -840,25 +864,25 @@ bool gemm_3xtf32_natural(nt_storage *sa, int64_t a_off, nt_storage *sb, int64_t 
     }
     // Split-K for products that leave most SMs without a tile (a skinny output with a long contraction: 4
     // tiles at 256 x 8192 x 512): up to max_splits CTAs share a tile while tiles x splits still fit one wave.
-    // Not for wave quantisation of larger products: measured on the 2048-row training step (256 tiles on 148
-    // SMs, 2 waves against 1.75 with four k-quarters) the split costs more than it saves, 10.4 ms per step
-    // against 8.3 -- four short pipelines with four epilogues and 134 MB of partial sums per launch.
-    {
-      const int64_t tiles = tiles_m * tiles_n * batch;
-      const KSplit ks = gemm_tc_k_split(batch, M, N, K);
-      g.splits = ks.splits;
-      g.kb_per_split = ks.kb_per_split;
-      if (g.splits > 1) {
-        g.partials = partials = static_cast<float *>(device_alloc(size_t(tiles) * g.splits * TC_BM * TC_BN * 4, &part_owned));
-        g.tickets = g_tickets;
-      }
-    }
+    const int64_t tiles = tiles_m * tiles_n * batch;
+    int64_t whole = 0;
+    const KSplit ks = gemm_tc_k_split(batch, M, N, K), hs = f16 ? gemm_f16_k_split(tiles, K, &whole) : KSplit{};
+    auto shared = [&](TileArgs &t, const KSplit &split, int64_t whole_tiles) {
+      t.splits = split.splits;
+      t.kb_per_split = split.kb_per_split;
+      t.whole = int32_t(whole_tiles);
+      t.work = int32_t(whole_tiles + (tiles - whole_tiles) * split.splits);
+      t.partials = partials;
+      t.tickets = g_tickets;
+    };
+    const int64_t parts = std::max(ks.splits > 1 ? tiles * ks.splits : 0, (tiles - whole) * hs.splits * f16);
+    if (parts) partials = static_cast<float *>(device_alloc(size_t(parts) * TC_BM * TC_BN * 4, &part_owned));
     g.bias = bias;
     g.bias_stride = bias ? bias_stride : 0;
     if (bias && bias_done) *bias_done = true;
     g.tiles_m = int32_t(tiles_m);
     g.tiles_n = int32_t(tiles_n);
-    g.work = int32_t(tiles_m * tiles_n * g.splits * batch);
+    shared(g, ks, ks.splits > 1 ? 0 : tiles);
     const dim3 grid{unsigned(std::min(g.work, sm_count())), 1, 1};
     matmul_profile_begin();
     if (f16) {
@@ -870,6 +894,7 @@ bool gemm_3xtf32_natural(nt_storage *sa, int64_t a_off, nt_storage *sb, int64_t 
       }
       F16Fallback f{};
       f.t = g;
+      shared(g, hs, whole);
       f.a = split_args(sa, ea);
       f.b = split_args(sb, eb);
       f.arrived = g_grid_barrier;
@@ -938,7 +963,7 @@ bool gemm_3xtf32(const float *A, const float *B, float *C, int64_t batch, int64_
     if (g_promoted.load()) {
       g.tiles_m = int32_t(grid.y);
       g.tiles_n = int32_t(grid.x);
-      g.work = int32_t(grid.x * grid.y * grid.z);
+      g.whole = g.work = int32_t(grid.x * grid.y * grid.z);
       gemm_3xtf32_promoted_kernel<false, false><<<unsigned(std::min(g.work, sm_count())), 320, TC_SMEM_BYTES, stream()>>>(map_a, map_b, g);
     } else
       gemm_3xtf32_kernel<<<grid, 192, TC_SMEM_BYTES, stream()>>>(map_a, map_b, g);

@@ -266,7 +266,7 @@ __device__ __forceinline__ void tf32_tiles(const CUtensorMap &map_a, const CUten
     const int half = (warp - 2) >> 2;   // which 128 of the 256 columns
     // a 32 x 32 corner of the tile on its way from a lane per row to whole 128-byte lines, 16-byte groups swizzled
     char *corner = reinterpret_cast<char *>(smem_raw + (bar_base - smem_u32(smem_raw))) + 256 + (warp - 2) * TC_CORNER_BYTES;
-    bool ok = !poisoned;
+    bool ok = !poisoned, reached = false;
     uint32_t done = 0; // periods of the items before
     for (int w = blockIdx.x; w < g.work && ok; w += gridDim.x) {
       const TileItem it = tile_item<TC_PERIOD_KB>(g, w);
@@ -300,7 +300,9 @@ __device__ __forceinline__ void tf32_tiles(const CUtensorMap &map_a, const CUten
       }
       done += it.periods;
       if (!poisoned) finish_tile(g, it, ok, sum, corner, quad, half, lane, int(threadIdx.x) - 64, poison_slot);
+      reached = reached || it.shared >= 0;
     }
+    if (!poisoned && !ok) give_up_tile(g, reached, poison_slot);
   }
 
   if (!poisoned && *reinterpret_cast<volatile int *>(g.error_flag) != 0) {

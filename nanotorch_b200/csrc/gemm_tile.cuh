@@ -22,14 +22,14 @@ struct TileArgs {
   long long wait_limit; // SM clocks a pipeline wait may take before the kernel gives up
   uint32_t mn_lbo, mn_sbo; // byte offsets of the MN-major descriptors (see umma_desc_mn_sw128)
   int32_t panel;           // tiles are walked in panels this many n-tiles wide (0 = row by row)
-  // split-K: `splits` CTAs share an output tile, each over kb_per_split k-blocks; they leave
+  // Items from `whole` on are parts of tiles: `splits` CTAs share an output tile, each over kb_per_split k-blocks; they leave
   // their sums in `partials` ([tile][split][32 chunks][256 threads][4]) and the one that draws the last ticket
-  // adds them up in split order.  splits == 1: one CTA per tile, no workspace.
-  int32_t splits, kb_per_split;
+  // adds them up in split order.  A CTA has one such item at most, its last.
+  int32_t whole, splits, kb_per_split;
   float *partials;
   unsigned int *tickets;
   int32_t tiles_m, tiles_n; // output tiles of one batch
-  int32_t work;             // tiles x splits x batches; a CTA takes items blockIdx.x, + gridDim.x, ...
+  int32_t work;             // whole tiles and parts; a CTA takes items blockIdx.x, + gridDim.x, ...
 };
 
 // Output tile of a work item.  CTAs take items in the order of their index, one wave after the other; taking the n-tiles
@@ -37,13 +37,18 @@ struct TileArgs {
 // sizes (two planes of B: 134 MB for 4096 x 4096) no longer fits the L2 and is fetched from DRAM once per
 // wave.  With panels of `panel` n-tiles a wave covers more m-tiles and fewer n-tiles, and a panel's slice of
 // B stays in the L2 while the CTAs walk down the m-tiles.
-__device__ __forceinline__ void tile_of_work(const TileArgs &g, int w, int &tm, int &tn, int &split, int &b) {
-  const int splits = g.splits > 1 ? g.splits : 1, per_batch = g.tiles_m * g.tiles_n * splits;
-  b = w / per_batch;
-  int lin = w - b * per_batch;
-  const int t = lin / splits; // the CTAs of one tile are neighbours in the order: their partial sums meet in the L2
-  split = lin - t * splits;
-  lin = t;
+__device__ __forceinline__ void tile_of_work(const TileArgs &g, int w, int &tm, int &tn, int &split, int &shared, int &b) {
+  int t = w;
+  shared = -1;
+  split = 0;
+  if (w >= g.whole) { // the CTAs of one tile are neighbours in the order: their partial sums meet in the L2
+    shared = (w - g.whole) / g.splits;
+    split = (w - g.whole) - shared * g.splits;
+    t = g.whole + shared;
+  }
+  const int per_batch = g.tiles_m * g.tiles_n;
+  b = t / per_batch;
+  const int lin = t - b * per_batch;
   tm = lin / g.tiles_n;
   tn = lin - tm * g.tiles_n;
   if (g.panel > 0) {
@@ -56,16 +61,16 @@ __device__ __forceinline__ void tile_of_work(const TileArgs &g, int w, int &tm, 
   }
 }
 
-// A work item: an output tile and, with split-K, this CTA's share of the contraction, k-blocks [kb0, kb0 + nkb), in
-// `periods` accumulation chains of PERIOD_KB blocks.
+// A work item: an output tile and, where it is the shared-th that CTAs share (otherwise -1), this CTA's share of the
+// contraction, k-blocks [kb0, kb0 + nkb), in `periods` accumulation chains of PERIOD_KB blocks.
 struct TileItem {
-  int tile_m, tile_n, split, b, kb0, nkb, periods;
+  int tile_m, tile_n, split, shared, b, kb0, nkb, periods;
 };
 template <int PERIOD_KB> __device__ __forceinline__ TileItem tile_item(const TileArgs &g, int w) {
   TileItem it;
-  tile_of_work(g, w, it.tile_m, it.tile_n, it.split, it.b);
-  it.kb0 = g.splits > 1 ? it.split * g.kb_per_split : 0;
-  it.nkb = g.splits > 1 ? min(g.kb_per_split, g.num_kb - it.kb0) : g.num_kb;
+  tile_of_work(g, w, it.tile_m, it.tile_n, it.split, it.shared, it.b);
+  it.kb0 = it.shared >= 0 ? it.split * g.kb_per_split : 0;
+  it.nkb = it.shared >= 0 ? min(g.kb_per_split, g.num_kb - it.kb0) : g.num_kb;
   it.periods = (it.nkb + PERIOD_KB - 1) / PERIOD_KB;
   return it;
 }
@@ -82,13 +87,13 @@ __device__ __forceinline__ void finish_tile(const TileArgs &g, const TileItem &i
   const int m0 = it.tile_m * TC_BM, n0 = it.tile_n * TC_BN, b = it.b;
   const int64_t m = int64_t(m0) + quad * 32 + lane;
   bool last = ok; // this CTA finishes the tile
-  if (g.splits > 1) {
+  if (it.shared >= 0) {
     // Split-K: leave this CTA's sums in the workspace; whoever draws the tile's last ticket adds the
     // partial sums up in split order (the order never depends on which CTA finishes last).  All eight
-    // epilogue warps pass the two barriers whatever happened to them; a warp whose wait ran out says so.
+    // epilogue warps pass the two barriers whatever happened to them; a warp whose wait ran out says so (see give_up_tile).
     volatile int *fail_slot = slots + 1;
     volatile unsigned int *ticket_slot = reinterpret_cast<volatile unsigned int *>(slots + 2);
-    const int64_t tile_lin = (int64_t(b) * g.tiles_m + it.tile_m) * g.tiles_n + it.tile_n;
+    const int64_t tile_lin = it.shared;
     float *mine = g.partials + ((tile_lin * g.splits + it.split) * 32 * 256 + et) * 4;
     if (!ok) *fail_slot = 1;
     if (ok && m < g.M) {
@@ -165,6 +170,16 @@ __device__ __forceinline__ void finish_tile(const TileArgs &g, const TileItem &i
       __syncwarp();
     }
   }
+}
+
+// For an epilogue warp that leaves its items because a wait ran out, with `reached` saying whether it has been through a
+// shared tile: the CTA's other warps may be on their way to one, whose two barriers it passes too.
+__device__ __forceinline__ void give_up_tile(const TileArgs &g, bool reached, volatile int *slots) {
+  const int last = int(blockIdx.x) + (g.work - 1 - int(blockIdx.x)) / int(gridDim.x) * int(gridDim.x);
+  if (reached || last < g.whole) return;
+  slots[1] = 1;
+  asm volatile("bar.sync 1, 256;" ::: "memory");
+  asm volatile("bar.sync 1, 256;" ::: "memory");
 }
 
 } // namespace ntb

@@ -186,3 +186,31 @@ def test_linear_keeps_its_rounding_where_a_kink_may_follow(nt):
         assert_bit_exact(got, want)
     exact = x_np.astype(np.float64) @ w_np.astype(np.float64) + b_np
     assert np.linalg.norm(free[0] - exact) < 0.3 * np.linalg.norm(kept[0] - exact)
+
+
+@pytest.mark.parametrize("shape", [(1, 2600, 1600, 2000), (1, 2048, 4100, 2500), (3, 1100, 2100, 1500)], ids=str)
+def test_tiles_left_over_by_the_last_wave_are_shared(nt, shape):
+    """Few tiles more than a multiple of the SMs (168, 160 and 162 for 148): those are cut along k.  Close to the uncut product --
+    the parts' sums are rounded once more --, the same bits on every run and in every layout, bias in the epilogue."""
+    _C = nt._C
+    batch, M, K, N = shape
+    rng = np.random.default_rng(M)
+    lead = (batch,) if batch > 1 else ()
+    a, b, bias = (rng.standard_normal(s).astype(np.float32) for s in ((*lead, M, K), (*lead, K, N), (N,)))
+    with nt.no_grad():
+        got = [(dev(nt, a, ta) @ dev(nt, b, tb)).numpy() for ta, tb in ((False, False), (False, True), (True, False), (True, True), (False, False))]
+        for g in got[1:]:
+            assert_bit_exact(g, got[0], "same bits whatever the operand order")
+        if batch == 1:
+            fused = _C.linear(dev(nt, a)._C_view, dev(nt, b)._C_view, dev(nt, bias)._C_view)
+            assert_bit_exact(nt.Tensor._new_contiguous(fused, (M, N)).numpy(), got[0] + bias, "bias in the epilogue")
+        _C.set_matmul_schedule(1, 8)
+        try:
+            uncut = (dev(nt, a) @ dev(nt, b)).numpy()
+        finally:
+            _C.set_matmul_schedule(8, 8)
+    bound = np.abs(a).astype(np.float64) @ np.abs(b).astype(np.float64)
+    assert (got[0] != uncut).any()
+    assert (np.abs(got[0].astype(np.float64) - uncut) <= 8 * 2.0 ** -24 * bound).all()  # up to eight parts
+    rows = slice(M - 300, M)
+    assert_scaled(got[0][..., rows, :], a[..., rows, :].astype(np.float64) @ b.astype(np.float64), bound[..., rows, :], 5 * 2.0 ** -23 + (K / 64 + 9) * 2.0 ** -24)
