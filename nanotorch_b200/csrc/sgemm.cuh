@@ -264,22 +264,26 @@ template <int T, bool A_K, bool B_K, bool FUSED> __global__ void __launch_bounds
 // ---------------------------------------------------------------------------------------------
 // A few rows (M <= 8) times a row-major matrix: a prediction for one sample or a handful.  A CTA owns 32 columns and
 // keeps up to TH_STAGES slices of 64 k on their way; warp w multiplies rows w and w + 4, a column per lane: a chain of
-// one multiply-add per k and row, which is what bounds it.  (The 32 x 32 tiles spend 31 of 32 rows on nothing.)
-constexpr int TH_M = 8, TH_N = 32, TH_BK = 64, TH_STAGES = 10, TH_NT = 128;
+// one multiply-add per k and row, which is what bounds it.  (The 32 x 32 tiles spend 31 of 32 rows on nothing.)  Four warps
+// of their own start the copies: by the multiplying warps, the copies of a slice, some 30 instructions with their addresses,
+// came between its multiply-adds (1 x 4096 x 512 28.9 us, now 22.6; 1 x 784 x 256 7.0 / 6.5; 8 x 2000 x 100 21.2 / 17.3).
+constexpr int TH_M = 8, TH_N = 32, TH_BK = 64, TH_STAGES = 10, TH_NT = 256, TH_COPY = 128;
 constexpr int TH_STAGE = TH_BK * (TH_N + TH_M); // floats: [k][32] of B, then [row][64] of A
 constexpr int TH_SMEM = TH_STAGES * TH_STAGE * 4;
 
 // FOUR: M <= 4
 template <bool FUSED, bool FOUR> __global__ void __launch_bounds__(TH_NT) sgemm_thin(GemmArgs g) {
+  pdl_wait();
   extern __shared__ __align__(16) float th_smem[];
-  const int tid = threadIdx.x, lane = tid & 31, warp = tid >> 5;
+  const bool copies = threadIdx.x >= TH_NT - TH_COPY;
+  const int tid = threadIdx.x % TH_COPY, lane = tid & 31, warp = tid >> 5;
   const int64_t n0 = int64_t(blockIdx.x) * TH_N;
   const float *A = g.A, *B = g.B;
   gemm_batch_base(g, blockIdx.z, A, B);
   const int steps = int((g.K + TH_BK - 1) / TH_BK);
   // copies of B: rows kb, kb + kb_step, ... of a slice, 16 bytes (or single values) each; of A: k = tid % 64 of every
   // second row
-  const int W = g.b_vec ? 4 : 1, kb = tid / (TH_N / W), nb = (tid % (TH_N / W)) * W, kb_step = TH_NT / (TH_N / W);
+  const int W = g.b_vec ? 4 : 1, kb = tid / (TH_N / W), nb = (tid % (TH_N / W)) * W, kb_step = TH_COPY / (TH_N / W);
   const bool nb_in = n0 + nb < g.N;
   const float *pb = B + kb * g.b_sk + n0 + nb, *pa = A + (tid / TH_BK) * g.a_sm + (tid % TH_BK) * g.a_sk;
   const int64_t b_step = kb_step * g.b_sk, b_next = TH_BK * g.b_sk, a_next = TH_BK * g.a_sk;
@@ -291,19 +295,19 @@ template <bool FUSED, bool FOUR> __global__ void __launch_bounds__(TH_NT) sgemm_
       float *d = st + kb * TH_N + nb;
       if (W == 4) {
 #pragma unroll
-        for (int i = 0; i < TH_BK * TH_N / 4 / TH_NT; ++i, q += b_step, d += kb_step * TH_N) {
+        for (int i = 0; i < TH_BK * TH_N / 4 / TH_COPY; ++i, q += b_step, d += kb_step * TH_N) {
           const bool live = nb_in && kb + i * kb_step < left;
           cp_async16(d, live ? q : B, live);
         }
       } else {
 #pragma unroll 4
-        for (int i = 0; i < TH_BK * TH_N / TH_NT; ++i, q += b_step, d += kb_step * TH_N) {
+        for (int i = 0; i < TH_BK * TH_N / TH_COPY; ++i, q += b_step, d += kb_step * TH_N) {
           const bool live = nb_in && kb + i * kb_step < left;
           cp_async4(d, live ? q : B, live);
         }
       }
       const float *qa = pa;
-      for (int m = tid / TH_BK; m < g.M; m += TH_NT / TH_BK, qa += (TH_NT / TH_BK) * g.a_sm) {
+      for (int m = tid / TH_BK; m < g.M; m += TH_COPY / TH_BK, qa += (TH_COPY / TH_BK) * g.a_sm) {
         const bool live = tid % TH_BK < left;
         cp_async4(st + TH_BK * TH_N + m * TH_BK + tid % TH_BK, live ? qa : A, live);
       }
@@ -313,11 +317,15 @@ template <bool FUSED, bool FOUR> __global__ void __launch_bounds__(TH_NT) sgemm_
     cp_async_commit();
   };
   float acc[2] = {0.0f, 0.0f};
-  for (int s = 0; s < TH_STAGES - 1; ++s) fetch(s);
+  if (copies)
+    for (int s = 0; s < TH_STAGES - 1; ++s) fetch(s);
   for (int s = 0; s < steps; ++s) {
     cp_async_wait<TH_STAGES - 2>();
     __syncthreads(); // slice s has landed for everyone, slice s - 1 has been read by everyone
-    fetch(s + TH_STAGES - 1);
+    if (copies) {
+      fetch(s + TH_STAGES - 1);
+      continue;
+    }
     const float *bs = th_smem + (s % TH_STAGES) * TH_STAGE + lane, *as = th_smem + (s % TH_STAGES) * TH_STAGE + TH_BK * TH_N + warp * TH_BK;
     if (warp < g.M) {
       // 16 values of k at a time, the next 16 on their way while these multiply
@@ -344,6 +352,7 @@ template <bool FUSED, bool FOUR> __global__ void __launch_bounds__(TH_NT) sgemm_
       }
     }
   }
+  if (copies) return;
   const int64_t n = n0 + lane;
   float *C = g.C + int64_t(blockIdx.z) * g.M * g.N;
 #pragma unroll
