@@ -5,14 +5,14 @@
 Headline (the line's `metric`/`value`): training throughput, in samples/s, of the data-parallel MLP
 configuration -- 8 x Linear(4096, 4096) with Tanh between them, MSE loss against N(0,1) targets,
 global batch 16384 of N(0,1) rows sharded over N ranks, SGD lr 1e-3, Kaiming-uniform init from seed
-0, fp32 with 3xTF32 tensor-core products -- on synthetic data.  A step is forward + backward +
+0, fp32 products of three fp16 tensor-core products each -- on synthetic data.  A step is forward + backward +
 gradient all-reduce + update on one global batch.  `value` is measured with the batch resident in
 HBM; `e2e` feeds every step's batch from pinned host memory (double-buffered host->device copies
 inside the timed region) and reads the loss back to the host every step.
 
 At N = 1 the same line also carries, under "ops", the per-op sweep of the other configurations
 (elementwise and reductions in GB/s against the measured HBM copy rate, matmul in TFLOP/s), the
-`roofline` of the dominant kernel of the step (the 3xTF32 GEMM) and `cpu_baseline`, the reference's
+`roofline` of the dominant kernel of the step (the GEMM over fp16 planes) and `cpu_baseline`, the reference's
 own CPU path timed on this box on a bounded sample.
 
 `--impl reference` times the reference's CPU implementation of the same step (its native module
@@ -982,16 +982,16 @@ def product_arm(args, rank: int, local_rank: int, world: int) -> None:
         m, k, n = local, WIDTH, WIDTH
         flops_per_launch = 2.0 * m * n * k            # algorithmic: one fp32 multiply-add per (m, n, k)
         avg_ms = gemm_ms / max(gemm_launches, 1)
-        tf32_peak = peaks["tf32_tflops_sustained"]    # the kernel is timed inside a long, power-capped step
+        # the kernel is timed inside a long, power-capped step; fp16 products run at the rate of bf16
+        fp16_peak = peaks["bf16_tflops_sustained"]
         achieved = flops_per_launch / avg_ms / 1e9 if gemm_launches else None
-        full = local == GLOBAL_BATCH and _C.get_matmul_mode() == 1
         line = {
             "metric": "mlp_train_samples_per_s", "value": value, "unit": "samples/s", "n_gpus": world,
             "steps": args.steps, "warmup": args.warmup, "ms_per_step": ms_resident / args.steps,
             "higher_is_better": True, "scaling": "strong", "vs_baseline": None, "dtype": "f32",
             "data": "synthetic",
             "config": {"workload": WORKLOAD, "global_batch": GLOBAL_BATCH, "per_rank_batch": local, "width": WIDTH,
-                       "layers": LAYERS, "matmul_mode": "3xTF32 (tcgen05)" if _C.get_matmul_mode() == 1 else "fp32",
+                       "layers": LAYERS, "matmul_mode": "3 fp16 products per fp32 product (tcgen05)" if _C.get_matmul_mode() == 1 else "fp32",
                        "parallelism": f"dp{world}", "l2": "inputs larger than L2 (weights 537 MB, activations 268 MB each)",
                        # cross-world parity: the global-batch loss of the first 5 steps from the seed-0 state and
                        # the fp64 sum (and sum of magnitudes) of the first layer's weights after them; they agree
@@ -1010,28 +1010,22 @@ def product_arm(args, rank: int, local_rank: int, world: int) -> None:
             "gpu_launches": launches,
             "clocks": sampler.summary(*clock_window),
             "roofline": {
-                "kernel": "gemm_3xtf32 (tcgen05.mma kind::tf32; fp32 product = 3 TF32 products)",
+                "kernel": "gemm_3xf16 (tcgen05.mma kind::f16; fp32 product = 3 fp16 products)",
                 "bound": "tensor", "unit": "TFLOP/s",
-                # algorithmic work 2*M*N*K per launch over the average launch time, against the TF32 rate
-                # cuBLAS sustains on this GPU; a 3xTF32 product issues three tensor-core products per
-                # multiply-add, so 1/3 is the ceiling of this fraction
-                "achieved": achieved, "peak": tf32_peak, "frac": (achieved / tf32_peak) if achieved else None,
+                # algorithmic work 2*M*N*K per launch over the average launch time, against the 16-bit rate that
+                # cuBLAS sustains on this GPU; three tensor-core products per multiply-add, so 1/3 is the ceiling
+                "achieved": achieved, "peak": fp16_peak, "frac": (achieved / fp16_peak) if achieved else None,
                 "frac_ceiling_3_products": 1.0 / 3.0,
-                "tensor_pipe": {"achieved": 3 * achieved if achieved else None, "peak": tf32_peak,
-                                "frac": (3 * achieved / tf32_peak) if achieved else None,
-                                "what": "TF32 tensor FLOP/s actually issued (3 per algorithmic one) over the same peak"},
-                "peak_source": f"{peaks['gemm_peaks_source']}: cuBLAS TF32 8192^3 sustained {peaks['tf32_tflops_sustained']:.0f}, "
-                               f"burst {peaks['tf32_tflops']:.0f}; cross-check bf16/2 from MEASURED_PEAKS.json "
-                               f"({peaks['source']}) = {peaks['bf16_tflops_sustained'] / 2:.0f} sustained / "
-                               f"{peaks['bf16_tflops'] / 2:.0f} burst; cuBLAS SGEMM (no tensor cores) {peaks['fp32_tflops']:.0f}",
+                "tensor_pipe": {"achieved": 3 * achieved if achieved else None, "peak": fp16_peak,
+                                "frac": (3 * achieved / fp16_peak) if achieved else None,
+                                "what": "fp16 tensor FLOP/s actually issued (3 per algorithmic one) over the same peak"},
+                "peak_source": f"MEASURED_PEAKS.json ({peaks['source']}): cuBLAS bf16 {peaks['bf16_tflops_sustained']:.0f} sustained, "
+                               f"{peaks['bf16_tflops']:.0f} burst; {peaks['gemm_peaks_source']}: cuBLAS TF32 8192^3 sustained "
+                               f"{peaks['tf32_tflops_sustained']:.0f}, burst {peaks['tf32_tflops']:.0f}; cuBLAS SGEMM (no tensor "
+                               f"cores) {peaks['fp32_tflops']:.0f}",
                 "launches": gemm_launches, "avg_launch_ms": avg_ms,
                 "flops_per_launch": flops_per_launch,
-                # DRAM bytes of one launch, from the ncu capture of the step's two GEMM shapes at the full
-                # per-GPU batch, weighted 15 : 8 as in one step; none for other shapes (re-reads do not scale)
-                "traffic": GEMM_TRAFFIC_BYTES_PER_LAUNCH if full else None,
-                "traffic_unit": "bytes/launch (dram__bytes_read.sum + dram__bytes_write.sum)",
-                "traffic_source": GEMM_TRAFFIC_SOURCE if full else None,
-                "algorithmic_bytes_per_launch": GEMM_ALGORITHMIC_BYTES_PER_LAUNCH if full else None,
+                "traffic": None,  # DRAM bytes of a launch have been captured of the kernel over TF32 planes only
             },
         }
         if world == 1 and not args.no_ops:
@@ -1055,12 +1049,6 @@ def product_arm(args, rank: int, local_rank: int, world: int) -> None:
     if dist is not None:
         dist.destroy_process_group()
 
-
-# (15 * 2882.6 MB + 8 * 3027.4 MB) / 23: forward / input-gradient shape and weight-gradient shape of the step
-GEMM_TRAFFIC_BYTES_PER_LAUNCH = 2.422e9
-GEMM_TRAFFIC_SOURCE = "profiles/gemm_3xtf32_step_shapes_dram_traffic.md (ncu, third capture: one launch per shape)"
-# fp32 operands read once, hi/lo planes written and read once, output written once, same 15 : 8 weighting
-GEMM_ALGORITHMIC_BYTES_PER_LAUNCH = (15 * 939.5e6 + 8 * 1140.9e6) / 23
 
 PROFILE_CASES = ("gemm4096", "add4096", "add4096_transposed", "pow2_4096_transposed", "add4096_broadcast", "tanh4096", "tanh4096_exact", "exp4096",
                  "sigmoid4096", "sum8192_dim0", "sum8192_dim1", "sum8192_full", "max_backward8192", "gather8192_rows", "gemm_step_shapes",

@@ -236,7 +236,8 @@ int nt_linear(const nt_view *x, const nt_view *w, const nt_view *bias, nt_storag
  *   0  exact FP32 on the CUDA cores (FMA, sequential in k: the rounding of the reference's CUDA kernels);
  *   1  (default) 3xTF32 on the tcgen05 tensor cores with promoted accumulation: chains of 256 values of k
  *      accumulate in tensor memory, their sums are added round-to-nearest in registers -- the error of an
- *      ordinary fp32 summation (2e-6 of max|C| at K = 4096 and at K = 16384);
+ *      ordinary fp32 summation (2e-6 of max|C| at K = 4096 and at K = 16384); products of more than 2^30
+ *      multiply-adds go over fp16 planes instead (2e-7), see nt_matmul_keep_rounding;
  *   2  FP32 on the CUDA cores with separate multiply and add, sequential in k: bit-for-bit the reference's
  *      CPU loop (src/cpp/ops/matmul.cu:31-45);
  *   3  3xTF32 with a single accumulation chain per output: ~1 % faster than mode 1; the tensor core's
@@ -263,9 +264,9 @@ int nt_get_matmul_mode(void);
  * nt_storage_data() pointers are not seen.  nt_matmul_split_stats: operand-split launches and cache hits since load. */
 int nt_set_matmul_operand_planes(int natural, int cached);
 /* on != 0 (default): nt_tanh and nt_tanh_backward, when their result is a dense 2-D Float32 matrix of at
- * least 2^20 elements whose rows are whole 128-byte lines, also write the result's TF32 planes and register
- * them in the cache above -- an activation or its gradient is then never read back by an operand split.
- * Costs 8 extra bytes written per element if no product ever uses the result. */
+ * least 2^20 elements whose rows are whole 128-byte lines, also write the result's planes (TF32, or fp16 where a square
+ * layer's products would go over those) and register them in the cache above -- an activation or its gradient is then never read back by an operand split.
+ * Costs 8 (or 4) extra bytes written per element if no product ever uses the result. */
 int nt_set_producer_planes(int on);
 /* on != 0 (default): an elementwise op on Float32 operands of at least 2^20 elements, one of which is
  * transposed over the last two dims (unit stride on the second-to-last), runs as a persistent kernel fed

@@ -357,8 +357,8 @@ template <class F> static nt_storage *fused2(F f, const nt_view *a, const nt_vie
 }
 
 // A producer of GEMM operands (an activation, its gradient): a dense 2-D fp32 result, large enough for the
-// tensor-core path, with rows that are whole 128-byte lines -- it writes its own TF32 planes (ew_contig_planes)
-// and registers them in the operand-plane cache, so the products that follow find them ready.
+// tensor-core path, with rows that are whole 128-byte lines -- it writes its own planes (ew_contig_planes,
+// f16_planes_kernel) and registers them in the operand-plane cache, so the products that follow find them ready.
 std::atomic<int> g_tile_pipeline{1};
 static std::atomic<int> g_producer_planes{1};
 static bool dense_2d(const nt_view *v) {
@@ -590,7 +590,7 @@ template <class F> static void row_value_gradients(F f, const nt_view *g, const 
   *out2 = first ? dense.release() : sums.release();
 }
 
-// ---- SGD.  A weight that has been a matmul operand: its TF32 planes follow the update.  When the parameter is the whole
+// ---- SGD.  A weight that has been a matmul operand: its planes follow the update.  When the parameter is the whole
 // of a dense 2-D storage the update writes them itself (20 bytes per element in one launch instead of 12 + 12 in two);
 // otherwise the cached views are split again behind the update.
 static void *sgd_planes(const nt_view *param, bool *f16) {

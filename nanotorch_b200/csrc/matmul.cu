@@ -1,7 +1,8 @@
 // nt_matmul: batched C[..., M, N] = A[..., M, K] x B[..., K, N] over arbitrary strided views.
 //
 // fp32 has three modes (nt_set_matmul_mode):
-//   1 (default) 3xTF32 on the tcgen05 tensor cores with promoted accumulation, see gemm_tc.cu;
+//   1 (default) 3xTF32 on the tcgen05 tensor cores with promoted accumulation, see gemm_tc.cu; large products as three
+//               fp16 products, see gemm_f16.cu;
 //   3           3xTF32 with one accumulation chain per output (1 % faster, 5-20x the rounding bias);
 //   0           exact FP32 on the CUDA cores (sgemm.cuh), one FMA per multiply-add, accumulated in
 //               ascending k -- the rounding of the reference's CUDA kernels (src/cpp/ops/matmul.cu:60-205);
